@@ -25,17 +25,19 @@
 // (the staged contraction computes it from exactly that), and every entry has
 // the key triple of its class.  The values are then scattered once into a
 // table indexed by the sorted key triple, and dense entries are generated by
-// key arithmetic and one table read.  The projection's first contraction (the
-// O(N^4 M) one) computes its slab that way inside the FP64 tensor-core GEMM
-// as it stages the operand tiles (KeyedSlabOp, at most 32 orbitals), or fills
-// the slab first (k_fill_slab_keyed) and contracts it.
+// key arithmetic and one table read.  The projection (at most 32 orbitals) and
+// the apply contract each pair class once (pair_classes.cuh) where the points
+// make a box that fits its kernel.  Otherwise the projection's first
+// contraction (the O(N^4 M) one) computes its slab inside the FP64 tensor-core
+// GEMM as it stages the operand tiles (KeyedSlabOp, at most 32 orbitals), or
+// fills the slab first (k_fill_slab_keyed) and contracts it.
 #include <algorithm>
 #include <map>
 #include <mutex>
 
 #include "dmma.cuh"
+#include "pair_classes.cuh"
 #include "symmetry.cuh"
-#include "tables.cuh"
 
 namespace gli {
 
@@ -105,19 +107,10 @@ __global__ void k_fill_eri_rows(SymGrid G, DenseGrid D, const int64_t* __restric
 
 // ---------------------------------------------------------------------------
 // complete class lists: values by sorted per-axis key triple
-__host__ __device__ inline i64 tetra_index(i64 k1, i64 k2, i64 k3) {  // k1 <= k2 <= k3
-    return k3 * (k3 + 1) * (k3 + 2) / 6 + k2 * (k2 + 1) / 2 + k1;
-}
-// the same in 32-bit arithmetic, for key tables of at most 2^29 slots (the
-// only ones built): then k3 (k3 + 1) (k3 + 2) <= 6 * 2^29 < 2^32
-__device__ __forceinline__ uint32_t tetra_index32(uint32_t k1, uint32_t k2, uint32_t k3) {
-    return k3 * (k3 + 1) * (k3 + 2) / 6u + k2 * (k2 + 1) / 2u + k1;
-}
-
 __device__ inline i64 eri_key_slot(const int p[4][3], i64 L) {
     i64 k[3];
     for (int a = 0; a < 3; ++a)
-        k[a] = eri_axis_key(p[0][a] - p[1][a], p[2][a] - p[3][a], (p[0][a] + p[1][a]) - (p[2][a] + p[3][a]), L);
+        k[a] = pair_axis_key(p[0][a] - p[1][a], p[2][a] - p[3][a], (p[0][a] + p[1][a]) - (p[2][a] + p[3][a]), (int)L);
     if (k[0] > k[1]) { i64 t = k[0]; k[0] = k[1]; k[1] = t; }
     if (k[1] > k[2]) { i64 t = k[1]; k[1] = k[2]; k[2] = t; }
     if (k[0] > k[1]) { i64 t = k[0]; k[0] = k[1]; k[1] = t; }
@@ -196,9 +189,9 @@ __global__ void __launch_bounds__(256) k_fill_slab_keyed(const short4* __restric
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
         const uint32_t row = e / N, l = e - row * N, j = row / N, k = row - j * N;
         const short4 pj = pt[j], pk = pt[k], pl = pt[l];
-        int a = eri_axis_key32(pi.x - pj.x, pk.x - pl.x, (pi.x + pj.x) - (pk.x + pl.x), L);
-        int b = eri_axis_key32(pi.y - pj.y, pk.y - pl.y, (pi.y + pj.y) - (pk.y + pl.y), L);
-        int c = eri_axis_key32(pi.z - pj.z, pk.z - pl.z, (pi.z + pj.z) - (pk.z + pl.z), L);
+        int a = pair_axis_key(pi.x - pj.x, pk.x - pl.x, (pi.x + pj.x) - (pk.x + pl.x), L);
+        int b = pair_axis_key(pi.y - pj.y, pk.y - pl.y, (pi.y + pj.y) - (pk.y + pl.y), L);
+        int c = pair_axis_key(pi.z - pj.z, pk.z - pl.z, (pi.z + pj.z) - (pk.z + pl.z), L);
         if (a > b) { const int t = a; a = b; b = t; }
         if (b > c) { const int t = b; b = c; c = t; }
         if (a > b) { const int t = a; a = b; b = t; }
@@ -281,9 +274,9 @@ struct KeyedSlabOp {
             const double* src = table;
             if (v) {
                 const short4 pl = pt[l];
-                int a = eri_axis_key32(st.d[0], st.k[0] - pl.x, st.s[0] - (st.k[0] + pl.x), L);
-                int c = eri_axis_key32(st.d[1], st.k[1] - pl.y, st.s[1] - (st.k[1] + pl.y), L);
-                int e = eri_axis_key32(st.d[2], st.k[2] - pl.z, st.s[2] - (st.k[2] + pl.z), L);
+                int a = pair_axis_key(st.d[0], st.k[0] - pl.x, st.s[0] - (st.k[0] + pl.x), L);
+                int c = pair_axis_key(st.d[1], st.k[1] - pl.y, st.s[1] - (st.k[1] + pl.y), L);
+                int e = pair_axis_key(st.d[2], st.k[2] - pl.z, st.s[2] - (st.k[2] + pl.z), L);
                 if (a > c) { const int t = a; a = c; c = t; }
                 if (c > e) { const int t = c; c = e; e = t; }
                 if (a > c) { const int t = a; a = c; c = t; }
@@ -544,7 +537,7 @@ static void build_key_table(const SymGrid& G, const GridDesc& g, const int64_t* 
     kt.ok = false;
     if (m <= 0) return;
     const i64 L = G.L;
-    const i64 nk = L * (L + 1) / 2 * (2 * L - 1);
+    const i64 nk = pair_axis_keys((int)L);
     const i64 slots = nk * (nk + 1) * (nk + 2) / 6;
     if (slots > ((i64)1 << 29)) return;  // above 4 GB: keep the lookups
     const CanonicalList canon = canonical_eri_list(g, G.e, s);
@@ -594,20 +587,65 @@ void grid_perms_device(const GridDesc& g, int64_t* d_perm, cudaStream_t s) {
     GLI_CHECK_LAUNCH();
 }
 
-// ret[(i k), s] = sum_{j l} V[i j k l] states[(j l), s], rows expanded in chunks
+// ret[(i k)][col0 + c] = sum_j C[(i j)][k][c], c < cols
+__global__ void __launch_bounds__(256) k_apply_sum(const double* __restrict__ C, int N, int cols, int ns, int col0,
+                                                   double* __restrict__ ret) {
+    const i64 row = (i64)N * cols, total = N * row;
+    const i64 e = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= total) return;
+    const i64 i = e / row, kc = e - i * row;
+    const double* c = C + i * N * row + kc;
+    double v = 0.0;
+    int j = 0;
+    for (; j + 8 <= N; j += 8) {
+        double t[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) t[u] = c[(j + u) * row];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v += t[u];
+    }
+    for (; j < N; ++j) v += c[j * row];
+    const i64 k = kc / cols;
+    ret[(i * N + k) * ns + col0 + (kc - k * cols)] = v;
+}
+
+// ret[(i k), s] = sum_{j l} V[i j k l] states[(j l), s].  Complete lists:
+// C[(i j)] = V[i j] X_j once per pair class (k_pair_contract), then the sum over
+// j in order; the contributions C take 8 N^3 bytes a state, at most 2 GB a
+// turn.  (5^3 points, 4 states: 1000 launches of a slab fill and products over
+// single j took 11.4 ms of kernels.)  Other lists: rows expanded in chunks.
 void apply_eri_device(const GridDesc& g, const int64_t* d_idx, const double* d_val, i64 m, const double* d_states,
                       i64 ns, double* d_ret, cudaStream_t s) {
     const SymGrid G = sym_of(g);
     const DenseGrid D = dense_of(g);
     const i64 N = D.N, N2 = N * N;
+    KeyTable kt;
+    build_key_table(G, g, d_idx, d_val, m, kt, s);
+    if (kt.ok && G.L <= PAIR_MAX_AXIS) {
+        std::vector<int> coords[3];
+        for (int a = 0; a < 3; ++a)
+            for (int k = 0; k < G.L; ++k) coords[a].push_back(k - G.e);
+        const PairBox box = make_pair_box(G.L, coords);
+        if (pair_box_fits(box, 4)) {
+            const i64 per = std::min<i64>(ns, std::max<i64>(1, ((i64)2 << 30) / (N2 * N * 8)));
+            DevBuf<double> C(N2 * N * per, s);
+            for (i64 c0 = 0; c0 < ns; c0 += per) {
+                const int cols = (int)std::min(per, ns - c0);
+                // a class has up to eight ordered pairs, one column tile of 8 per state
+                pair_contract<false>(box, std::min(4, cols), kt.t.p, d_states, cols, (int)ns, (int)c0, C.p, s);
+                const i64 total = N2 * cols;
+                k_apply_sum<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(C.p, (int)N, cols, (int)ns, (int)c0, d_ret);
+                GLI_CHECK_LAUNCH();
+            }
+            return;
+        }
+    }
     // chunk of rows i of V[i][j][k][l]: for one i, the (j, k, l) block is N^3
     const i64 per_i = N2 * N;
     i64 ci = (i64)(256 << 20) / (per_i * 8);
     if (ci < 1) ci = 1;
     if (ci > N) ci = N;
     DevBuf<double> V(ci * per_i, s);
-    KeyTable kt;
-    build_key_table(G, g, d_idx, d_val, m, kt, s);
     for (i64 i0 = 0; i0 < N; i0 += ci) {
         const i64 ni = std::min(ci, N - i0);
         // V rows (i, j) for i in [i0, i0 + ni): layout [i][j][k][l]
@@ -658,6 +696,105 @@ __global__ void __launch_bounds__(256) k_symmetrize_pairs(const double* __restri
         blk[e] = v;
         if (j < i) mir[e] = v;
     }
+}
+
+// rows of B (M columns) to the rows at[] of out
+__global__ void k_scatter_rows(const double* __restrict__ B, const int* __restrict__ at, i64 total, int M,
+                               double* __restrict__ out) {
+    const i64 e = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= total) return;
+    const i64 r = e / M;
+    out[(i64)at[r] * M + (e - r * M)] = B[e];
+}
+
+// class of every ordered pair of box points
+__global__ void k_pair_class_map(PairBox box, int* __restrict__ cls) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < box.N * box.N) cls[e] = pair_class(box, e / box.N, e % box.N);
+}
+
+// A3[i][m][q] = sum_j Y[class(i, j)][m] B[j][q]: rows m are the packed (r >= s)
+// entries of the class blocks, q the orbitals (at most 32, one column tile),
+// batch i.  The A operand's rows are the unit-stride direction; each k reads
+// the block of its pair's class, so no N x N array of blocks is made (382 MB
+// at 216 points and 32 orbitals, and 352 us for writing and contracting it).
+struct ClassBlocksOp {
+    static constexpr bool A_KMAJOR = true, B_KMAJOR = false;
+    static constexpr int BN = 32;
+    const double* Y;
+    const int* cls;  // N x N
+    const double* B;  // N x M
+    double* out;
+    int N, M, P;
+    struct Block {
+        int mvalid, nvalid, nk;
+        int m0;
+        const int* cls;
+        double* c;
+    };
+    struct AState {};
+    struct BState {};
+    __device__ bool begin(Block& b) const {
+        b.m0 = blockIdx.x * DM_BM;
+        b.mvalid = min(DM_BM, P - b.m0);
+        b.nvalid = M;
+        b.nk = (N + DM_BK - 1) / DM_BK;
+        b.cls = cls + (i64)blockIdx.y * N;
+        b.c = out + ((i64)blockIdx.y * P + b.m0) * M;
+        return b.mvalid > 0;
+    }
+    __device__ void a_init(const Block&, AState&) const {}
+    __device__ void b_init(const Block&, BState&) const {}
+    __device__ void a_issue(const Block& b, AState&, int kc, double* tile) const {
+        const int r = dm_kmajor_row(threadIdx.x);
+#pragma unroll
+        for (int q = 0; q < DM_ELEMS; ++q) {
+            const int k = dm_kmajor_k(threadIdx.x, q), j = kc * DM_BK + k;
+            const bool v = r < b.mvalid && j < N;
+            dm_cp8(tile + dm_kmajor_at(r, k), v ? Y + (i64)__ldg(&b.cls[j]) * P + b.m0 + r : Y, v);
+        }
+    }
+    __device__ void b_issue(const Block& b, BState&, int kc, double* tile) const {
+#pragma unroll
+        for (int q = 0; q < BN * DM_BK / DM_THREADS; ++q) {
+            const int n = dm_rowmajor_row(threadIdx.x, q), k = dm_rowmajor_k(threadIdx.x), j = kc * DM_BK + k;
+            const bool v = n < b.nvalid && j < N;
+            dm_cp8(tile + dm_rowmajor_at(n, k), v ? B + (i64)j * M + n : B, v);
+        }
+    }
+    __device__ void store(const Block& b, int m, int n, double v0, double v1) const {
+        if (m >= b.mvalid) return;
+        double* c = b.c + (i64)m * M + n;
+        if (n < b.nvalid) c[0] = v0;
+        if (n + 1 < b.nvalid) c[1] = v1;
+    }
+};
+
+// E[p][q][r][s] from T[(r s)][q][p], (r s) packed r >= s
+__global__ void k_expand_projection(const double* __restrict__ T, int M, double* __restrict__ E) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= M * M * M * M) return;
+    const int s = e % M, r = e / M % M, q = e / (M * M) % M, p = e / (M * M * M);
+    const int hi = max(r, s), lo = min(r, s);
+    E[e] = T[((i64)(hi * (hi + 1) / 2 + lo) * M + q) * M + p];
+}
+
+// The projection of a complete list onto M <= 32 orbitals on a box of points:
+// Y[c] = B^T V[c] B per pair class, then the two indices of the other pair
+static void project_pair_classes(const PairBox& box, int nt, const double* table, const double* basis, int M,
+                                 double* d_out, cudaStream_t s) {
+    const i64 N = box.N, P = (i64)M * (M + 1) / 2;
+    DevBuf<double> Y(box.classes * P, s), A3(N * P * M, s), T(P * M * M, s);
+    DevBuf<int> cls(N * N, s);
+    pair_contract<true>(box, nt, table, basis, M, M, 0, Y.p, s);
+    k_pair_class_map<<<(unsigned)((N * N + 255) / 256), 256, 0, s>>>(box, cls.p);
+    GLI_CHECK_LAUNCH();
+    dmma_launch(ClassBlocksOp{Y.p, cls.p, basis, A3.p, (int)N, M, (int)P},
+                dim3((unsigned)((P + DM_BM - 1) / DM_BM), (unsigned)N), s);
+    // T[(rs q)][p] = sum_i A3[i][(rs q)] B[i][p]
+    dgemm((int)(P * M), M, (int)N, MatView{A3.p, 0, 1, P * M}, MatView{basis, 0, M, 1}, T.p, 0, M, 1, 1, false, s);
+    k_expand_projection<<<(unsigned)(((i64)M * M * M * M + 255) / 256), 256, 0, s>>>(T.p, M, d_out);
+    GLI_CHECK_LAUNCH();
 }
 
 void project_device(int kind, const GridDesc& g, const int64_t* d_idx, const double* d_val, i64 m,
@@ -732,6 +869,56 @@ void project_device(int kind, const GridDesc& g, const int64_t* d_idx, const dou
             GLI_CUDA(cudaMemcpyAsync(bcomp.p, hbc.data(), Nx * M * sizeof(double), cudaMemcpyHostToDevice, s));
             GLI_CUDA(cudaStreamSynchronize(s));  // the host vectors go out of scope
             bx = bcomp.p;
+        }
+    }
+    if (slab32 && M <= 32) {
+        // The active points in their box (the product of their coordinates per
+        // axis; a sub-grid is its own box): the first two contractions once per
+        // pair class.  A box of over twice the active points (orbitals on
+        // scattered points) would contract mostly zero rows, and one beyond the
+        // kernel's rows or shared memory does not fit it.
+        std::vector<int> coords[3];
+        for (i64 a = 0; a < Nx; ++a) {
+            const int c[3] = {hpt[a].x, hpt[a].y, hpt[a].z};
+            for (int x = 0; x < 3; ++x) coords[x].push_back(c[x]);
+        }
+        for (auto& c : coords) {
+            std::sort(c.begin(), c.end());
+            c.erase(std::unique(c.begin(), c.end()), c.end());
+        }
+        const int nt = (int)((M + 7) / 8);
+        bool fits = true;
+        i64 points = 1;
+        for (auto& c : coords) {
+            fits = fits && c.size() <= PAIR_MAX_AXIS;
+            points *= (i64)c.size();
+        }
+        if (fits && points <= 2 * Nx) {
+            const PairBox box = make_pair_box((int)G.L, coords);
+            if (pair_box_fits(box, nt)) {
+                const double* bb = bx;
+                DevBuf<double> bbox;
+                if (points != Nx) {  // zero rows for the box's other points
+                    bbox.alloc(points * M, s);
+                    bbox.zero();
+                    std::vector<int> at((size_t)Nx);
+                    for (i64 a = 0; a < Nx; ++a) {
+                        const int c[3] = {hpt[a].x, hpt[a].y, hpt[a].z};
+                        i64 lin = 0;
+                        for (int x = 0; x < 3; ++x)
+                            lin = lin * box.n[x] + (std::lower_bound(coords[x].begin(), coords[x].end(), c[x]) - coords[x].begin());
+                        at[(size_t)a] = (int)lin;
+                    }
+                    DevBuf<int> d_at(Nx, s);
+                    GLI_CUDA(cudaMemcpyAsync(d_at.p, at.data(), Nx * sizeof(int), cudaMemcpyHostToDevice, s));
+                    k_scatter_rows<<<(unsigned)((Nx * M + 255) / 256), 256, 0, s>>>(bx, d_at.p, Nx * M, (int)M, bbox.p);
+                    GLI_CHECK_LAUNCH();
+                    GLI_CUDA(cudaStreamSynchronize(s));  // the host vector goes out of scope
+                    bb = bbox.p;
+                }
+                project_pair_classes(box, nt, kt.t.p, bb, (int)M, d_out, s);
+                return;
+            }
         }
     }
     // V[i j k l] = V[j i k l]: the two first contractions run over the pairs

@@ -1,0 +1,469 @@
+// Contractions of a complete ERI tensor by pair classes.
+//
+// V[i j k l] depends on the point pair (i, j) only through its class: per axis
+// the unordered pair of coordinates.  On a box of n0 x n1 x n2 points
+// (a product of coordinate lists) the N^2 ordered pairs fall into F0 F1 F2
+// classes, Fa = na (na + 1) / 2 (6^3 points: 9,261 classes of 46,656 ordered
+// pairs; 7^3: 21,952 of 117,649), and V[c][k l] = V[c'][k l] as matrices in
+// (k, l) for every pair of class c.  So every contraction over (k, l) is made
+// once per class:
+//   projection   Y[c] = B^T V[c] B                     (an M x M block per class)
+//   apply        C[(i j)] = V[c] X_j for the pairs (i, j) of class c
+// and V[c] itself holds one value per class c' of (k, l).
+//
+// The values come from the key table of the complete list (dense.cu): slot
+// tetra_index of the sorted triple of axis keys.  An axis key joins the fields
+// (|d|, s) and (|d'|, s') of the two pairs' coordinates, d = difference and
+// s = sum: the unordered {|d|, |d'|} and |s - s'|.  s - s' has the parity of
+// d + d', so |s - s'| / 2 (rounded down) tells the keys apart, and a grid of L
+// points per axis has L (L + 1) / 2 L of them.  (With |s - s'| itself half of
+// the keys never occur: at 7^3 the table takes 64 MB, and the values that a
+// warp reads lie every other slot; now 10 MB, neighbours in one sector.)
+#pragma once
+
+#include "dmma.cuh"
+#include "gli_internal.cuh"
+
+namespace gli {
+
+// axis keys of the key table
+__host__ __device__ __forceinline__ int pair_axis_keys(int L) { return L * (L + 1) / 2 * L; }
+__host__ __device__ __forceinline__ int pair_axis_key(int d01, int d23, int cc, int L) {
+    int a = d01 < 0 ? -d01 : d01;
+    int b = d23 < 0 ? -d23 : d23;
+    if (a > b) { const int t = a; a = b; b = t; }
+    const int c = cc < 0 ? -cc : cc;
+    return (b * (b + 1) / 2 + a) * L + (c >> 1);
+}
+
+__host__ __device__ inline i64 tetra_index(i64 k1, i64 k2, i64 k3) {  // k1 <= k2 <= k3
+    return k3 * (k3 + 1) * (k3 + 2) / 6 + k2 * (k2 + 1) / 2 + k1;
+}
+// the same in 32-bit arithmetic, for key tables of at most 2^29 slots (the
+// only ones built): then k3 (k3 + 1) (k3 + 2) <= 6 * 2^29 < 2^32
+__device__ __forceinline__ uint32_t tetra_index32(uint32_t k1, uint32_t k2, uint32_t k3) {
+    return k3 * (k3 + 1) * (k3 + 2) / 6u + k2 * (k2 + 1) / 2u + k1;
+}
+
+constexpr int PAIR_MAX_AXIS = 16, PAIR_MAX_WARPS = 16;
+constexpr int PAIR_MAX_TILES = 2;                                      // 16-row tiles per warp
+constexpr int PAIR_MAX_POINTS = 16 * PAIR_MAX_WARPS * PAIR_MAX_TILES;  // 512
+
+// A box of points, x-major: coordinate lists (ascending) per axis
+struct PairBox {
+    int L;        // points per axis of the class list's grid (key range)
+    int n[3], F[3];
+    int N, nyz;   // points; points of one x plane
+    int F2, PS;   // F1 F2; plane stride: F2 values and a zero
+    int S;        // k steps of 4 per x plane
+    int classes;  // F0 F1 F2
+    short c[3][PAIR_MAX_AXIS];
+};
+
+inline PairBox make_pair_box(int L, const std::vector<int> coords[3]) {
+    PairBox b = {};
+    b.L = L;
+    for (int a = 0; a < 3; ++a) {
+        b.n[a] = (int)coords[a].size();
+        b.F[a] = b.n[a] * (b.n[a] + 1) / 2;
+        for (int k = 0; k < b.n[a]; ++k) b.c[a][k] = (short)coords[a][k];
+    }
+    b.nyz = b.n[1] * b.n[2];
+    b.N = b.n[0] * b.nyz;
+    b.F2 = b.F[1] * b.F[2];
+    b.PS = b.F2 + 1;
+    b.S = (b.nyz + 3) / 4;
+    b.classes = b.F[0] * b.F2;
+    return b;
+}
+
+// field f = hi (hi + 1) / 2 + lo of an axis -> coordinate positions lo <= hi
+__device__ __forceinline__ void pair_field(int f, int& lo, int& hi) {
+    int h = 0;
+    while ((h + 1) * (h + 2) / 2 <= f) ++h;
+    hi = h;
+    lo = f - h * (h + 1) / 2;
+}
+
+// class of the ordered pair of box points (i, j)
+__device__ __forceinline__ int pair_class(const PairBox& b, int i, int j) {
+    int f[3];
+#pragma unroll
+    for (int a = 2; a >= 0; --a) {
+        const int n = b.n[a], x = a ? i % n : i, y = a ? j % n : j;
+        i /= n;
+        j /= n;
+        const int lo = min(x, y), hi = max(x, y);
+        f[a] = hi * (hi + 1) / 2 + lo;
+    }
+    return (f[0] * b.F[1] + f[1]) * b.F[2] + f[2];
+}
+
+// Shared memory of k_pair_contract (the launch and the kernel agree on it)
+struct PairSmem {
+    int ldb;      // doubles per row of B: 4 or 12 mod 16, so that fragment reads have no bank conflicts
+    int planes;   // doubles: two buffers of n0 planes (the epilogue's tiles reuse them)
+    int brows;    // rows of B
+    int map_ld;   // uint16 per row of the (y z) x (y z) maps
+    size_t bytes;
+    __host__ __device__ PairSmem(const PairBox& b, int warps, int nt) {
+        ldb = 8 * nt + 4;
+        const int rows = b.N < 16 * warps ? (b.N + 15) / 16 * 16 : 16 * warps;
+        planes = 2 * b.n[0] * b.PS;
+        if (planes < rows * ldb) planes = rows * ldb;
+        if (planes < 8 * nt * (8 * nt + 1)) planes = 8 * nt * (8 * nt + 1);
+        brows = b.N + 4;
+        map_ld = 4 * b.S;
+        bytes = 8 * ((size_t)planes + (size_t)brows * ldb + 2 * 8 * (size_t)nt) + 4 * ((size_t)b.F2 + b.F[0] + b.F[1] + b.F[2]) +
+                2 * ((size_t)2 * b.nyz + 1) * map_ld;
+    }
+};
+
+// One class c per turn of a persistent block: A = V[c] B over the box's points,
+// V[c] the N x N matrix of the class and B of at most 8 NT columns.
+//
+//   SYM   B is the basis (N x cols); V[c] is taken as U + U^T, U its upper
+//         triangle with half the diagonal, so only U B is formed, and
+//         Y = B^T (U B) gives B^T V B = Y + Y^T; out[c] holds its lower
+//         triangle (r >= s, packed).
+//   else  (apply) B holds the columns [state rows of j] of the ordered pairs
+//         (i, j) of class c, states col0 .. col0 + cols of each:
+//         out[(i N + j) N + k][state] = sum_l V[c][k l] x[j N + l][state].
+//
+// The k loop runs over the x planes of l.  V[c] restricted to l's plane needs
+// one plane of values per x coordinate of k (F1 F2 each): they are copied from
+// the key table with 8-byte cp.async into one of two buffers while the previous
+// plane is contracted.  A fragments are read from there through a map
+// (yz of k, yz of l) -> value, 16 bits each, the same for every plane; rows
+// and columns outside the triangle (or the box) point at the plane's zero.
+// Bound: the FP64 tensor pipe, 47% busy (343 points, 20 orbitals); the rest is
+// the planes' copies, the barriers between planes and the blocks' start and
+// end.  Measured on a B200, first two contractions: 216 points and 32 orbitals
+// 1.09 ms (a contraction per point pair, its slab staged from the key table:
+// 5.25 ms), 343 points and 20 orbitals 5.2 ms (23.7 ms); the whole projection
+// calls 9.9 to 5.4 ms and 28.0 to 9.2 ms, the apply at 5^3 points and 4 states
+// 12.8 to 0.57 ms (0.24 ms of kernels).
+//
+// A warp owns up to two 16-row tiles (rows 16 (w + W t)) and keeps their
+// accumulators over all planes, so each B fragment serves all its tiles.  The
+// FP64 MMAs of four warps per scheduler hide each other's issue gaps and the
+// map and value loads (two warps with three tiles each kept the FP64 tensor
+// pipe 39% busy): two blocks of 8 warps on an SM, or one of 16 where the
+// planes and B of one box take more than half of the shared memory.
+template <int W, int NT, int TPW, bool SYM>
+__global__ void __launch_bounds__(32 * W, W == 8 ? 2 : 1)
+    k_pair_contract(const PairBox box, const double* __restrict__ table, const double* __restrict__ bsrc, int cols,
+                    int ld, int col0, double* __restrict__ out) {
+    extern __shared__ __align__(16) double sm[];
+    constexpr int PAIR_WARPS = W, PAIR_THREADS = 32 * W;
+    const PairSmem lay(box, W, NT);
+    const int LDB = 8 * NT + 4;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = lane & 3, c8 = lane >> 2;
+    const int N = box.N, nyz = box.nyz, PS = box.PS, F2 = box.F2, map_ld = lay.map_ld;
+    double* planes = sm;
+    double* B = sm + lay.planes;
+    i64* csrc = reinterpret_cast<i64*>(B + lay.brows * LDB);  // (apply) source and destination of each column
+    i64* cdst = csrc + 8 * NT;
+    uint32_t* yz = reinterpret_cast<uint32_t*>(cdst + 8 * NT);  // (min, max, diagonal) of the y and z keys
+    int* kx = reinterpret_cast<int*>(yz + F2);
+    int* ky = kx + box.F[0];
+    int* kz = ky + box.F[1];
+    uint16_t* map = reinterpret_cast<uint16_t*>(kz + box.F[2]);  // nyz rows: every l
+    uint16_t* tmap = map + nyz * map_ld;                          // nyz rows: l >= k only
+    uint16_t* zrow = tmap + nyz * map_ld;                         // a row of zeros
+    // the maps, and B where every class has the same
+    for (int e = tid; e < nyz * map_ld; e += PAIR_THREADS) {
+        const int k = e / map_ld, l = e - k * map_ld;
+        int v = F2;
+        if (l < nyz) {
+            const int n2 = box.n[2], yk = k / n2, zk = k - yk * n2, yl = l / n2, zl = l - yl * n2;
+            const int yh = max(yk, yl), zh = max(zk, zl);
+            v = (yh * (yh + 1) / 2 + min(yk, yl)) * box.F[2] + zh * (zh + 1) / 2 + min(zk, zl);
+        }
+        map[e] = (uint16_t)v;
+        tmap[e] = (uint16_t)(l >= k ? v : F2);
+    }
+    for (int e = tid; e < map_ld; e += PAIR_THREADS) zrow[e] = (uint16_t)F2;
+    for (int e = tid; e < lay.brows * 8 * NT; e += PAIR_THREADS) {
+        const int r = e / (8 * NT), c = e - r * (8 * NT);
+        B[r * LDB + c] = SYM && r < N && c < cols ? bsrc[(i64)r * ld + c] : 0.0;
+    }
+    // this thread's rows: x plane and the offsets of its rows of the two maps
+    const int tiles = (N + 15) / 16, mine = tiles > warp ? (tiles - warp + PAIR_WARPS - 1) / PAIR_WARPS : 0;
+    int row_k[TPW][2], row_m[TPW][2];
+#pragma unroll
+    for (int t = 0; t < TPW; ++t)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int r = 16 * (warp + PAIR_WARPS * t) + 8 * i + c8;
+            row_k[t][i] = r / nyz;
+            row_m[t][i] = (r - row_k[t][i] * nyz) * map_ld + q;
+        }
+
+    for (int cls = blockIdx.x; cls < box.classes; cls += gridDim.x) {
+        int f[3], lo[3], hi[3], d[3], s[3];
+        f[2] = cls % box.F[2];
+        f[1] = cls / box.F[2] % box.F[1];
+        f[0] = cls / F2;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            pair_field(f[a], lo[a], hi[a]);
+            d[a] = box.c[a][hi[a]] - box.c[a][lo[a]];
+            s[a] = box.c[a][hi[a]] + box.c[a][lo[a]];
+        }
+        __syncthreads();  // the previous class is done with the tables, the planes and (apply) B
+        for (int a = 0, o = 0; a < 3; o += box.F[a], ++a)
+            for (int g = tid; g < box.F[a]; g += PAIR_THREADS) {
+                int l2, h2;
+                pair_field(g, l2, h2);
+                const int d2 = box.c[a][h2] - box.c[a][l2], s2 = box.c[a][h2] + box.c[a][l2];
+                kx[o + g] = pair_axis_key(d[a], d2, s[a] - s2, box.L);
+            }
+        for (int e = tid; e < 2 * box.n[0]; e += PAIR_THREADS) planes[e * PS + F2] = 0.0;
+        __syncthreads();
+        for (int e = tid; e < F2; e += PAIR_THREADS) {
+            const int fy = e / box.F[2], fz = e - fy * box.F[2];
+            int l2, h2, l3, h3;
+            pair_field(fy, l2, h2);
+            pair_field(fz, l3, h3);
+            const uint32_t a = min(ky[fy], kz[fz]), b = max(ky[fy], kz[fz]);
+            yz[e] = a | b << 15 | (l2 == h2 && l3 == h3 ? 1u << 31 : 0u);
+        }
+        int axes = 0;  // (apply) axes on which the class's two coordinates differ
+        if (!SYM) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) axes += lo[a] != hi[a];
+        }
+        // the ordered pair p of the class: bit per differing axis
+        auto pair_points = [&](int p, int& i, int& j) {
+            i = j = 0;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                bool flip = false;
+                if (lo[a] != hi[a]) {
+                    flip = p & 1;
+                    p >>= 1;
+                }
+                i = i * box.n[a] + (flip ? hi[a] : lo[a]);
+                j = j * box.n[a] + (flip ? lo[a] : hi[a]);
+            }
+        };
+        const int bcols = SYM ? cols : cols << axes;
+        for (int ct = 0; ct < bcols; ct += 8 * NT) {  // (SYM: one turn)
+        if (!SYM) {
+            if (tid < 8 * NT) {
+                const int cc = ct + tid;
+                i64 from = -1, to = -1;
+                if (cc < bcols) {
+                    int i, j;
+                    pair_points(cc / cols, i, j);
+                    from = (i64)j * N * ld + col0 + cc % cols;
+                    to = ((i64)i * N + j) * N * cols + cc % cols;
+                }
+                csrc[tid] = from;
+                cdst[tid] = to;
+            }
+            __syncthreads();
+            for (int e = tid; e < 8 * NT * N; e += PAIR_THREADS) {
+                const int r = e / (8 * NT), c = e - r * (8 * NT);
+                const i64 from = csrc[c];
+                dm_cp8(B + r * LDB + c, from >= 0 ? bsrc + from + (i64)r * ld : bsrc, from >= 0);
+            }
+        }
+        __syncthreads();
+        // copies the values of l's plane lx into a buffer
+        auto stage = [&](int lx, double* buf) {
+            const int cnt = SYM ? lx + 1 : box.n[0];
+            for (int kxi = 0; kxi < cnt; ++kxi) {
+                const int h = max(kxi, lx);
+                const uint32_t x = kx[h * (h + 1) / 2 + min(kxi, lx)];
+                double* dst = buf + kxi * PS;
+                for (int e = tid; e < F2; e += PAIR_THREADS) {
+                    const uint32_t v = yz[e], a = v & 0x7fffu, b = v >> 15 & 0x7fffu;
+                    dm_cp8(dst + e, table + tetra_index32(min(a, x), max(a, min(b, x)), max(b, x)), true);
+                }
+            }
+            dm_commit();
+        };
+        double acc[TPW][2][NT][2];
+#pragma unroll
+        for (int t = 0; t < TPW; ++t)
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < NT; ++j) acc[t][i][j][0] = acc[t][i][j][1] = 0.0;
+        stage(0, planes);
+        for (int lx = 0; lx < box.n[0]; ++lx) {
+            double* buf = planes + (lx & 1) * box.n[0] * PS;
+            dm_wait<0>();
+            if (SYM)  // the diagonal k = l, halved by the thread that copied it
+                for (int e = tid; e < F2; e += PAIR_THREADS)
+                    if (yz[e] >> 31) buf[lx * PS + e] *= 0.5;
+            __syncthreads();  // the plane has landed everywhere; the other buffer is consumed
+            if (lx + 1 < box.n[0]) stage(lx + 1, planes + ((lx + 1) & 1) * box.n[0] * PS);
+            // rows that meet this plane (offsets into the maps and the values)
+            const int rows = SYM ? (lx + 1) * nyz : N, xmax = SYM ? lx + 1 : box.n[0];
+            int mo[TPW][2], po[TPW][2];
+            int nact = 0;
+#pragma unroll
+            for (int t = 0; t < TPW; ++t) {
+                if (16 * (warp + PAIR_WARPS * t) < rows) nact = t + 1;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int k = row_k[t][i];
+                    const bool in = k < xmax;
+                    mo[t][i] = in ? row_m[t][i] + (SYM && k == lx ? nyz * map_ld : 0) : 2 * nyz * map_ld + q;
+                    po[t][i] = (lx & 1) * box.n[0] * PS + (in ? k * PS : 0);
+                }
+            }
+            const int bo = lay.planes + (lx * nyz + q) * LDB + c8;
+            auto steps = [&](auto active) {
+                constexpr int A = decltype(active)::value;
+                auto step = [&](int st, bool last) {
+                    // (past the plane's last point B is taken as zero, not only
+                    // A: a state or orbital may hold infinities in the next plane)
+                    const bool in = !last || 4 * st + q < nyz;
+                    double bf[NT];
+#pragma unroll
+                    for (int j = 0; j < NT; ++j) bf[j] = in ? sm[bo + st * 4 * LDB + 8 * j] : 0.0;
+#pragma unroll
+                    for (int t = 0; t < A; ++t) {
+                        const double a0 = sm[po[t][0] + map[mo[t][0] + 4 * st]], a1 = sm[po[t][1] + map[mo[t][1] + 4 * st]];
+#pragma unroll
+                        for (int j = 0; j < NT; ++j) dm_mma(acc[t][0][j], a0, bf[j]);
+#pragma unroll
+                        for (int j = 0; j < NT; ++j) dm_mma(acc[t][1][j], a1, bf[j]);
+                    }
+                };
+#pragma unroll 2
+                for (int st = 0; st < box.S - 1; ++st) step(st, false);
+                step(box.S - 1, true);
+            };
+            if constexpr (TPW >= 2)
+                if (nact == 2) steps(std::integral_constant<int, 2>{});
+            if (nact == 1) steps(std::integral_constant<int, 1>{});
+        }
+        if constexpr (SYM) {
+            // Y[r][s] = sum_k B[k][r] A[k][s]: the rows of A through shared memory,
+            // 128 at a time; NT^2 tiles of Y over the warps
+            constexpr int YT = (NT * NT + PAIR_WARPS - 1) / PAIR_WARPS;
+            // (two chains of MMAs per tile of Y: one chain over 343 rows waits
+            // on its own latency)
+            double y[YT][2][2];
+#pragma unroll
+            for (int t = 0; t < YT; ++t) y[t][0][0] = y[t][0][1] = y[t][1][0] = y[t][1][1] = 0.0;
+            double* X = planes;
+#pragma unroll
+            for (int t = 0; t < TPW; ++t) {
+                const int r0 = 16 * PAIR_WARPS * t, nr = min(16 * PAIR_WARPS, N - r0);
+                __syncthreads();  // the planes, or the rows before, are consumed
+                if (nr <= 0) break;
+                if (t < mine)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+#pragma unroll
+                        for (int j = 0; j < NT; ++j) {
+                            double* x = X + (16 * warp + 8 * i + c8) * LDB + 8 * j + 2 * q;
+                            x[0] = acc[t][i][j][0];
+                            x[1] = acc[t][i][j][1];
+                        }
+                __syncthreads();
+#pragma unroll
+                for (int u = 0; u < YT; ++u) {
+                    const int ty = warp + PAIR_WARPS * u;
+                    if (ty >= NT * NT) continue;
+                    const double* ap = B + (r0 + q) * LDB + 8 * (ty / NT) + c8;
+                    const double* xp = X + q * LDB + 8 * (ty % NT) + c8;
+                    int k = 0;
+#pragma unroll 4
+                    for (; k + 4 < nr; k += 8) {
+                        dm_mma(y[u][0], ap[k * LDB], xp[k * LDB]);
+                        dm_mma(y[u][1], ap[(k + 4) * LDB], xp[(k + 4) * LDB]);
+                    }
+                    if (k < nr) dm_mma(y[u][0], ap[k * LDB], xp[k * LDB]);
+                }
+            }
+            __syncthreads();  // X is consumed
+            double* Y = X;    // [r][8 NT + 1]
+#pragma unroll
+            for (int u = 0; u < YT; ++u) {
+                const int ty = warp + PAIR_WARPS * u;
+                if (ty >= NT * NT) continue;
+                double* yp = Y + (8 * (ty / NT) + c8) * (8 * NT + 1) + 8 * (ty % NT) + 2 * q;
+                yp[0] = y[u][0][0] + y[u][1][0];
+                yp[1] = y[u][0][1] + y[u][1][1];
+            }
+            __syncthreads();
+            double* o = out + (i64)cls * (cols * (cols + 1) / 2);
+            for (int e = tid; e < 64 * NT * NT; e += PAIR_THREADS) {
+                const int r = e / (8 * NT), c = e - r * (8 * NT);
+                if (r < cols && c <= r) o[r * (r + 1) / 2 + c] = Y[r * (8 * NT + 1) + c] + Y[c * (8 * NT + 1) + r];
+            }
+        } else {
+#pragma unroll
+            for (int t = 0; t < TPW; ++t)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int k = 16 * (warp + PAIR_WARPS * t) + 8 * i + c8;
+                    if (k >= N) continue;
+#pragma unroll
+                    for (int j = 0; j < NT; ++j)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const i64 to = cdst[8 * j + 2 * q + h];
+                            if (to >= 0) out[to + (i64)k * cols] = acc[t][i][j][h];
+                        }
+                }
+            __syncthreads();  // the planes are consumed before the next columns' first copy
+        }
+        }
+    }
+}
+
+// the box fits the kernel: rows in the warps' tiles, 16-bit maps, shared memory
+inline bool pair_box_fits(const PairBox& b, int nt) {
+    return b.N <= PAIR_MAX_POINTS && b.F2 < 65535 && pair_axis_keys(b.L) < 32768 &&
+           PairSmem(b, PAIR_MAX_WARPS, nt).bytes <= (size_t)227 * 1024;
+}
+
+template <int W, int NT, int TPW, bool SYM>
+void pair_contract_launch(const PairBox& b, const double* table, const double* bsrc, int cols, int ld, int col0,
+                          double* out, cudaStream_t s) {
+    const size_t smem = PairSmem(b, W, NT).bytes;
+    auto* kernel = k_pair_contract<W, NT, TPW, SYM>;
+    GLI_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 1;
+    GLI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * W, smem));
+    const i64 slots = (i64)context().num_sms * (per_sm > 0 ? per_sm : 1);
+    const unsigned blocks = (unsigned)(b.classes < slots ? b.classes : slots);
+    launch_kernel(kernel, dim3(blocks), dim3(32 * W), smem, s, b, table, bsrc, cols, ld, col0, out);
+}
+
+// A = V[c] B for every class c of the box; nt = column tiles of 8
+template <bool SYM>
+void pair_contract(const PairBox& b, int nt, const double* table, const double* bsrc, int cols, int ld, int col0,
+                   double* out, cudaStream_t s) {
+    auto go = [&](auto n) {
+        constexpr int NT = decltype(n)::value;
+        // two blocks of 8 warps where both fit an SM (228 KB with 1 KB a block)
+        const bool two = b.N <= 256 && 2 * (PairSmem(b, 8, NT).bytes + 1024) <= (size_t)228 * 1024;
+        if (two && b.N <= 128)
+            pair_contract_launch<8, NT, 1, SYM>(b, table, bsrc, cols, ld, col0, out, s);
+        else if (two)
+            pair_contract_launch<8, NT, 2, SYM>(b, table, bsrc, cols, ld, col0, out, s);
+        else if (b.N <= 256)
+            pair_contract_launch<16, NT, 1, SYM>(b, table, bsrc, cols, ld, col0, out, s);
+        else
+            pair_contract_launch<16, NT, 2, SYM>(b, table, bsrc, cols, ld, col0, out, s);
+    };
+    if (nt <= 1)
+        go(std::integral_constant<int, 1>{});
+    else if (nt == 2)
+        go(std::integral_constant<int, 2>{});
+    else if (nt == 3)
+        go(std::integral_constant<int, 3>{});
+    else
+        go(std::integral_constant<int, 4>{});
+}
+
+}  // namespace gli
