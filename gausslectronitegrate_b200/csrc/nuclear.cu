@@ -18,21 +18,32 @@
 // the dense N x N matrix, V_ij = Vk[kx(i,j)][ky(i,j), kz(i,j)] (the sliced
 // tensor-core contractions keep the (kz, ky) order of their batched stage B).
 //
+// Band.  A key's weights are nonzero on the 2 mmax + 1 positions around
+// 3 (i_a + j_a) only (mmax: the outermost factor above tol; 99 of 237 positions
+// on a 24-point axis at tol 1e-8).  Keys are therefore ordered by i_a + j_a, so
+// that the 64 keys of a tile share most of their positions, and a tile's K loop
+// covers just the positions that any of its keys reaches.
+//
 // Batches.  Any number of instances (each its own grid and nuclei, all with
 // the same coefficients and tol) run as one plan: one upload of every
-// instance's descriptor, coordinates and nuclei; one kernel builds every
-// instance's weights, one tabulates every instance's field, one scatters every
-// instance's matrix; each instance's three contractions run on a ring of
-// streams so that small instances overlap.  The plan of a chunk of instances
-// is captured as one CUDA graph and launched once.  Forms: FP64 throughout (the
-// drop-in), or mixed: the three contractions as int8-sliced products on the
-// tensor cores (5 slices), field, weights and scatter in FP64.
+// instance's descriptor, coordinates and nuclei; per pipeline one kernel builds
+// every instance's weights, one tabulates every instance's field, three
+// contract (every instance's tiles in one launch per stage) and one scatters
+// every instance's matrix.  The autotuner chooses how many pipelines (streams)
+// the instances of a chunk are dealt over.  (One launch per instance and stage,
+// captured as a graph on each call, spent more on the capture, on launches under
+// a wave and on their tails than it saved: 200 us of host time per call for one
+// 13 x 16 x 11 instance.)  Forms: FP64 throughout (the drop-in), or mixed: the
+// three contractions as int8-sliced products on the tensor cores (5 slices),
+// field, weights and scatter in FP64, where the autotuner measures that faster.
 #include <math.h>
+#include <string.h>
 
 #include <algorithm>
 #include <string>
 
 #include "autotune.cuh"
+#include "dmma.cuh"
 #include "gli_internal.cuh"
 #include "tc_gemm.cuh"
 
@@ -55,19 +66,32 @@ struct NucInst {
     int n[3];          // axis lengths
     int coord_off[3];  // first coordinate of each axis in the packed coordinate list
     int U[3], u0[3];   // lattice extent and origin (units of 1/6) per axis
+    int P[3];          // U rounded up to even: row pitches (16-byte rows)
     int nk[3];         // axis keys: n (n + 1) / 2
+    int band;          // weights per key (2 mmax + 1); 0: the keys' order is not by position
     int nuc0, nnuc;    // nuclei in the packed nucleus arrays
     i64 N;             // grid points
-    i64 w_off[3];      // weights of each axis in the packed W buffer
-    i64 phi_off;       // field in the packed Phi buffer
-    i64 vk_off;        // key-indexed matrix in the packed Vk buffer
+    i64 w_off[3];      // weights of each axis in the packed W buffer (even)
+    int ks_off[3];     // first position of each key in the packed start list
+    i64 x_off;         // the field; the key-indexed matrix overwrites it (even)
+    i64 h_off;         // the stage-A product H (even)
+    i64 h2_off;        // the stage-B product H2 (even)
     double* out;       // N x N row-major
 };
 
-// W[key][u] of every (instance, axis): key = tri(lo <= hi) over the axis'
-// coordinate list, u a lattice position.  grid (u blocks, key, 3 * instance)
+// Position of key (lo <= hi) of an axis of n points when keys are ordered by
+// lo + hi, then lo: the keys with a smaller sum t < s number floor((s + 1)^2 / 4)
+// up to the middle sum, and mirror beyond it
+__host__ __device__ __forceinline__ int nuc_rank(int n, int lo, int hi) {
+    const int s = lo + hi;
+    const int base = s < n ? (s + 1) * (s + 1) / 4 : n * (n + 1) / 2 - (2 * n - s) * (2 * n - s) / 4;
+    return base + lo - (s >= n ? s - n + 1 : 0);
+}
+
+// W[key][u] of every (instance, axis), u a lattice position (zeros up to the
+// pitch), and the first position of each key.  grid (u blocks, key, 3 * instance)
 __global__ void k_nuc_weights(const NucInst* __restrict__ inst, const double* __restrict__ F, int nf, int nb,
-                              const int* __restrict__ coords, double* __restrict__ W) {
+                              const int* __restrict__ coords, double* __restrict__ W, int* __restrict__ kstart) {
     const NucInst& in = inst[blockIdx.z / 3];
     const int a = blockIdx.z % 3;
     const int key = blockIdx.y;
@@ -75,91 +99,266 @@ __global__ void k_nuc_weights(const NucInst* __restrict__ inst, const double* __
     int hi = (int)((sqrt(8.0 * key + 1.0) - 1.0) * 0.5);
     while (hi * (hi + 1) / 2 > key) --hi;
     while ((hi + 1) * (hi + 2) / 2 <= key) ++hi;
-    const int lo = key - hi * (hi + 1) / 2;
+    const int lo = key - hi * (hi + 1) / 2, rank = nuc_rank(in.n[a], lo, hi);
     const int xa = coords[in.coord_off[a] + lo], xb = coords[in.coord_off[a] + hi];
     const int s = xa > xb ? xa - xb : xb - xa;
-    const int U = in.U[a];
-    double* w = W + in.w_off[a] + (i64)key * U;
-    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < U; u += gridDim.x * blockDim.x) {
+    const int U = in.U[a], P = in.P[a];
+    double* w = W + in.w_off[a] + (i64)rank * P;
+    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < P; u += gridDim.x * blockDim.x) {
         const int m = u + in.u0[a] - 3 * (xa + xb);  // factor logical index
         double v = 0;
-        if (m >= -(nb - 1) && m <= nb - 1) v = F[(i64)s * nf + m + (nb - 1)];
+        if (u < U && m >= -(nb - 1) && m <= nb - 1) v = F[(i64)s * nf + m + (nb - 1)];
         w[u] = v;
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        kstart[in.ks_off[a] + rank] = 3 * (xa + xb) - 6 * coords[in.coord_off[a]];
 }
 
-// the Gaussian-nucleus field at lattice point (u, v, t) of an instance
-__device__ inline double nuc_field_at(const NucInst& in, const double* __restrict__ npos,
-                                      const double* __restrict__ ncharge, int u, int v, int t) {
-    const double px = (u + in.u0[0]) / 6.0, py = (v + in.u0[1]) / 6.0, pz = (t + in.u0[2]) / 6.0;
-    double acc = 0;
-    for (int k = in.nuc0; k < in.nuc0 + in.nnuc; ++k) {
-        const double dx = px - npos[3 * k], dy = py - npos[3 * k + 1], dz = pz - npos[3 * k + 2];
-        const double r2 = dx * dx + dy * dy + dz * dz;
-        // g(r) = erf(r / w) / r with w = 1/3; g(0) = 2 / (sqrt(pi) w).  For
-        // 3 r >= 6, erfc(3 r) <= 2.2e-17 is below a quarter ulp of 1: erf
-        // rounds to 1 and g = 1 / r
-        double g;
-        if (r2 >= 4.0) {
-            g = rsqrt(r2);
-        } else {
-            const double r = sqrt(r2);
-            g = r > 0 ? erf(3.0 * r) / r : 3.3851375012865379;  // 6 / sqrt(pi)
-        }
-        acc += ncharge[k] * g;
-    }
-    return acc;
+// the Gaussian-nucleus field g(r) = erf(r / w) / r with w = 1/3 at squared
+// distance r2; g(0) = 2 / (sqrt(pi) w).  For 3 r >= 6, erfc(3 r) <= 2.2e-17 is
+// below a quarter ulp of 1: erf rounds to 1 and g = 1 / r
+__device__ __forceinline__ double nuc_gaussian(double r2) {
+    if (r2 >= 4.0) return rsqrt(r2);
+    const double r = sqrt(r2);
+    return r > 0 ? erf(3.0 * r) / r : 3.3851375012865379;  // 6 / sqrt(pi)
 }
 
-// Phi[u][v][t] (t fastest) of every instance, position (u + u0x, v + u0y, t + u0z) / 6;
-// grid (row blocks, instance): a block fills whole (u, v) rows
-__global__ void __launch_bounds__(128) k_nuc_field(const NucInst* __restrict__ inst, const double* __restrict__ npos,
-                                                   const double* __restrict__ ncharge, double* __restrict__ Phi) {
+// Phi[u][v][t] (t fastest, pitches P) of every instance, position
+// (u + u0x, v + u0y, t + u0z) / 6; grid (row blocks, instance), a warp fills
+// whole (u, v) rows, four cells per lane and turn: per nucleus the row's part of
+// the squared distance is formed once and each cell costs two FP64
+// multiply-adds and a reciprocal square root.  Bound: the FP64 pipe.  24^3 to
+// 8^3 batch of eight (27 million cells, 6 nuclei): 722 us with a thread per
+// cell, its three coordinates divided by 6 and its whole distance per nucleus.
+constexpr int NUC_FIELD_MAX_T = 2048;  // z positions held in shared memory (axes of 256 points: 1531 + 2 mmax)
+__global__ void __launch_bounds__(256) k_nuc_field(const NucInst* __restrict__ inst, const double* __restrict__ npos,
+                                                   const double* __restrict__ ncharge, double* __restrict__ X) {
+    __shared__ double zs[NUC_FIELD_MAX_T];
     const NucInst& in = inst[blockIdx.y];
-    const int Uy = in.U[1], Uz = in.U[2];
-    const i64 rows = (i64)in.U[0] * Uy;
-    for (i64 row = blockIdx.x; row < rows; row += gridDim.x) {
-        const int u = (int)(row / Uy), v = (int)(row - (i64)u * Uy);
-        double* phi = Phi + in.phi_off + row * Uz;
-        for (int t = threadIdx.x; t < Uz; t += blockDim.x) phi[t] = nuc_field_at(in, npos, ncharge, u, v, t);
+    const int Py = in.P[1], Pz = in.P[2], lane = threadIdx.x & 31;
+    const int rows = in.P[0] * Py, warps = gridDim.x * (blockDim.x >> 5);
+    for (int t = threadIdx.x; t < Pz && t < NUC_FIELD_MAX_T; t += blockDim.x) zs[t] = (t + in.u0[2]) / 6.0;
+    __syncthreads();
+    for (int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += warps) {
+        const int u = row / Py, v = row - u * Py;
+        const double px = (u + in.u0[0]) / 6.0, py = (v + in.u0[1]) / 6.0;
+        double* phi = X + in.x_off + (i64)row * Pz;
+        for (int t0 = 0; t0 < Pz; t0 += 128) {
+            double pz[4], acc[4] = {0.0, 0.0, 0.0, 0.0};
+            const int live = min(4, (Pz - t0 + 31) >> 5);  // (the same in every lane)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int t = t0 + 32 * c + lane;
+                pz[c] = t < NUC_FIELD_MAX_T ? zs[t < Pz ? t : 0] : (t + in.u0[2]) / 6.0;
+            }
+            for (int k = in.nuc0; k < in.nuc0 + in.nnuc; ++k) {
+                const double dx = px - npos[3 * k], dy = py - npos[3 * k + 1], nz = npos[3 * k + 2], q = ncharge[k];
+                const double r2 = dx * dx + dy * dy;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    if (c >= live) break;
+                    const double dz = pz[c] - nz;
+                    acc[c] += q * nuc_gaussian(r2 + dz * dz);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int t = t0 + 32 * c + lane;
+                if (t < Pz) phi[t] = acc[c];
+            }
+        }
     }
 }
 
 // V[i][j] of every instance from its key-indexed block: Vk[kx][ky * nkz + kz]
 // (zfast: the FP64 contractions) or Vk[kx][kz * nky + ky] (the sliced ones).
-// Grid (x pairs, instance): block (ix, jx) writes the (ny nz) x (ny nz)
-// sub-block of rows ix nyz + (iy, iz) and columns jx nyz + (jy, jz), whose
-// entries all lie in the one slice kx = key(ix, jx) (nky nkz entries, read
-// from cache after the first touch; a whole row of V would read every slice,
-// more than L2 holds for a 24^3 instance).  A thread owns columns, decoded
-// once; rows run as (iy, iz) loops, so the inner loop has no division.
-__global__ void __launch_bounds__(256) k_nuc_scatter(const NucInst* __restrict__ inst, const double* __restrict__ Vk,
+//
+// zfast: block (ix, iy, jx) writes the nz x (ny nz) sub-block of rows
+// (ix, iy, .) and columns (jx, ., .).  Its entries lie in the ny lines
+// ky = key(iy, jy) of the slice kx = key(ix, jx): as many lines as fit are
+// copied into shared memory (coalesced), and every row is gathered from
+// there and written as one run of 16-byte stores.  (A thread per column and
+// 8-byte stores, each value gathered from the line in L1, where 32 lanes touch
+// up to 20 cache lines: 868 us for the 2.67 GB of a batch of eight, 3.1 TB/s.)
+// Bound: HBM writes.
+constexpr int NUC_LINE_MAX_Z = 64;                    // z axis of the shared-memory route
+constexpr int NUC_LINES_BYTES = 64 * 1024;            // lines held at a time
+__global__ void __launch_bounds__(256) k_nuc_scatter(const NucInst* __restrict__ inst, const double* __restrict__ X,
                                                      int zfast) {
+    extern __shared__ __align__(16) double lines[];
+    __shared__ uint16_t rank_z[NUC_LINE_MAX_Z * NUC_LINE_MAX_Z];
     const NucInst& in = inst[blockIdx.y];
     const int nx = in.n[0], ny = in.n[1], nz = in.n[2], nky = in.nk[1], nkz = in.nk[2];
     const int nyz = ny * nz;
     const i64 N = in.N;
+    const double* Vk = X + in.x_off;
+    const int items = nx * ny * nx;
+    if (zfast && nz <= NUC_LINE_MAX_Z) {
+        if ((int)blockIdx.x >= items) return;
+        for (int e = threadIdx.x; e < nz * nz; e += blockDim.x) {
+            const int a = e / nz, b = e - a * nz;
+            rank_z[e] = (uint16_t)nuc_rank(nz, min(a, b), max(a, b));
+        }
+        const int group = max(1, min(ny, NUC_LINES_BYTES / (8 * nkz)));
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+        for (int item = blockIdx.x; item < items; item += gridDim.x) {
+            const int jx = item % nx, r = item / nx, iy = r % ny, ix = r / ny;
+            const double* slice = Vk + (i64)nuc_rank(nx, min(ix, jx), max(ix, jx)) * ((i64)nky * nkz);
+            for (int j0 = 0; j0 < ny; j0 += group) {
+                const int cnt = min(group, ny - j0), cols = cnt * nz;
+                __syncthreads();  // the lines before are consumed
+                for (int l = warp; l < cnt; l += warps) {
+                    const int jy = j0 + l;
+                    const double* src = slice + (i64)nuc_rank(ny, min(iy, jy), max(iy, jy)) * nkz;
+                    for (int e = lane; e < nkz; e += 32) lines[l * nkz + e] = __ldg(src + e);
+                }
+                __syncthreads();
+                for (int iz = warp; iz < nz; iz += warps) {
+                    const i64 at = ((i64)(ix * ny + iy) * nz + iz) * N + (i64)jx * nyz + (i64)j0 * nz;
+                    double* out = in.out + at;
+                    const uint16_t* rk = rank_z + iz * nz;
+                    auto value = [&](int l, int jz) { return lines[l * nkz + rk[jz]]; };
+                    // (pairs start on 16-byte boundaries: an odd start leaves its first entry alone)
+                    const int odd = (int)(((uintptr_t)out >> 3) & 1);
+                    if (odd && lane == 0) __stcs(out, value(0, 0));
+                    int c = odd + 2 * lane, l = c / nz, jz = c - l * nz;
+                    for (; c < cols; c += 64) {
+                        const double v0 = value(l, jz);
+                        if (c + 1 < cols) {
+                            const int l1 = jz + 1 < nz ? l : l + 1, z1 = jz + 1 < nz ? jz + 1 : 0;
+                            __stcs(reinterpret_cast<double2*>(out + c), make_double2(v0, value(l1, z1)));
+                        } else {
+                            __stcs(out + c, v0);
+                        }
+                        jz += 64;
+                        while (jz >= nz) {
+                            jz -= nz;
+                            ++l;
+                        }
+                    }
+                }
+            }
+        }
+        return;
+    }
+    // other layouts and long z axes: a thread per column, rows as (iy, iz) loops
     const i64 sy = zfast ? nkz : 1, sz = zfast ? 1 : nky;  // strides of ky and kz in a slice
     for (int pair = blockIdx.x; pair < nx * nx; pair += gridDim.x) {
         const int ix = pair / nx, jx = pair - ix * nx;
-        const int ax = min(ix, jx), bx = max(ix, jx);
-        const double* slice = Vk + in.vk_off + (i64)(bx * (bx + 1) / 2 + ax) * ((i64)nky * nkz);
+        const double* slice = Vk + (i64)nuc_rank(nx, min(ix, jx), max(ix, jx)) * ((i64)nky * nkz);
         double* block = in.out + (i64)ix * nyz * N + (i64)jx * nyz;
         for (int c = threadIdx.x; c < nyz; c += blockDim.x) {
             const int jy = c / nz, jz = c - jy * nz;
             double* col = block + c;
             for (int iy = 0; iy < ny; ++iy) {
-                const int ay = min(iy, jy), by = max(iy, jy);
-                const double* sl = slice + (i64)(by * (by + 1) / 2 + ay) * sy;
+                const double* sl = slice + (i64)nuc_rank(ny, min(iy, jy), max(iy, jy)) * sy;
                 double* out = col + (i64)iy * nz * N;
-                for (int iz = 0; iz < nz; ++iz) {
-                    const int az = min(iz, jz), bz = max(iz, jz);
-                    out[(i64)iz * N] = sl[(i64)(bz * (bz + 1) / 2 + az) * sz];
-                }
+                for (int iz = 0; iz < nz; ++iz)
+                    out[(i64)iz * N] = sl[(i64)nuc_rank(nz, min(iz, jz), max(iz, jz)) * sz];
             }
         }
     }
 }
+
+// One stage of the FP64 contractions over every instance of a pipeline:
+// Y[m][n] = sum_k W[m][k] X[n][k], m a key of the stage's axis, n the rows of
+//   A  X = Phi, n = (u, v) with pitch P1:   Y = H[kz][n]
+//   B  X = H,   n = (kz, u) with pitch P0:  Y = H2[ky][n]
+//   C  X = H2,  n = (ky, kz):               Y = Vk[kx][n]
+// (row pitches make each stage's output the next one's rows as they are; the
+// rows past an axis' extent hold finite values that no later K range reads).
+// Blocks find their instance in `pre`, the tiles before each instance; the key
+// tiles of one n tile are neighbours, so X comes from L2 after the first.  K
+// runs over the positions from the tile's first key's to its last key's last
+// one, both operands K-contiguous 16-byte copies.
+//
+// Bound: the FP64 tensor pipe.  24^3 to 8^3 batch of eight, 6 nuclei: 2.95 ms
+// over full K ranges with 8-byte copies, a launch per instance.
+template <int STAGE>
+struct NucStageOp {
+    static constexpr bool A_KMAJOR = false, B_KMAJOR = false;
+    static constexpr int BN = DM_BN;
+    static constexpr int AXIS = 2 - STAGE;
+    const NucInst* inst;
+    const int* pre;  // ni + 1 tile counts
+    int ni;
+    const double* W;
+    const int* kstart;
+    double* Xb;  // packed buffers
+    double* Hb;
+    double* H2b;
+    struct Block {
+        int mvalid, nvalid, nk;
+        int k0, kend;
+        int pitch;
+        i64 ldy;
+        const double* a;
+        const double* b;
+        double* y;
+    };
+    struct AState {};
+    struct BState {};
+    __device__ bool begin(Block& b) const {
+        // the instance: the last one whose tiles start at or before this block
+        int lo = 0, hi = ni;
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (__ldg(&pre[mid]) <= (int)blockIdx.x) lo = mid;
+            else hi = mid;
+        }
+        const NucInst& in = inst[lo];
+        const int t = (int)blockIdx.x - __ldg(&pre[lo]);
+        const int M = in.nk[AXIS], mt = (M + DM_BM - 1) / DM_BM;
+        const int m0 = t % mt * DM_BM, n0 = t / mt * BN;
+        const int rows = STAGE == 0 ? in.P[0] * in.P[1] : STAGE == 1 ? in.nk[2] * in.P[0] : in.nk[1] * in.nk[2];
+        b.mvalid = min(DM_BM, M - m0);
+        b.nvalid = min(BN, rows - n0);
+        b.pitch = in.P[AXIS];
+        b.kend = in.U[AXIS];
+        b.k0 = 0;
+        if (in.band) {
+            const int* ks = kstart + in.ks_off[AXIS] + m0;
+            b.k0 = ks[0] & ~3;
+            b.kend = min(b.kend, ks[b.mvalid - 1] + in.band);
+        }
+        b.nk = (b.kend - b.k0 + DM_BK - 1) / DM_BK;
+        b.ldy = rows;
+        const double* x = STAGE == 0 ? Xb + in.x_off : STAGE == 1 ? Hb + in.h_off : H2b + in.h2_off;
+        double* y = STAGE == 0 ? Hb + in.h_off : STAGE == 1 ? H2b + in.h2_off : Xb + in.x_off;
+        b.a = W + in.w_off[AXIS] + (i64)m0 * b.pitch + b.k0;
+        b.b = x + (i64)n0 * b.pitch + b.k0;
+        b.y = y + (i64)m0 * b.ldy + n0;
+        return true;
+    }
+    __device__ void a_init(const Block&, AState&) const {}
+    __device__ void b_init(const Block&, BState&) const {}
+    __device__ void a_issue(const Block& b, AState&, int kc, double* tile) const {
+#pragma unroll
+        for (int q = 0; q < DM_BM / 16; ++q) {
+            const int r = dm_pair_row(threadIdx.x, q), k = dm_pair_k(threadIdx.x), kk = kc * DM_BK + k;
+            const int bytes = r < b.mvalid ? dm_pair_bytes(b.k0 + kk, b.kend) : 0;
+            dm_cp16(tile + dm_rowmajor_at(r, k), bytes ? b.a + r * b.pitch + kk : b.a, bytes);
+        }
+    }
+    __device__ void b_issue(const Block& b, BState&, int kc, double* tile) const {
+#pragma unroll
+        for (int q = 0; q < BN / 16; ++q) {
+            const int r = dm_pair_row(threadIdx.x, q), k = dm_pair_k(threadIdx.x), kk = kc * DM_BK + k;
+            const int bytes = r < b.nvalid ? dm_pair_bytes(b.k0 + kk, b.kend) : 0;
+            dm_cp16(tile + dm_rowmajor_at(r, k), bytes ? b.b + r * b.pitch + kk : b.b, bytes);
+        }
+    }
+    __device__ void store(const Block& b, int m, int n, double v0, double v1) const {
+        if (m >= b.mvalid) return;
+        double* y = b.y + m * b.ldy + n;
+        if (n + 1 < b.nvalid && !(b.ldy & 1)) {
+            *reinterpret_cast<double2*>(y) = make_double2(v0, v1);
+        } else {
+            if (n < b.nvalid) y[0] = v0;
+            if (n + 1 < b.nvalid) y[1] = v1;
+        }
+    }
+};
 
 // tiles of a shared-B batched product: batch b, B row block j of nbt
 __global__ void k_shared_b_tiles(int batches, int nbt, int nrows, int bn, int* __restrict__ tb, int* __restrict__ tc,
@@ -189,99 +388,85 @@ struct BatchedRows {
     __device__ bool valid(i64) const { return true; }
 };
 
-// FP64 strided batched GEMM (dense.cu); dgemm_prepare sets its kernel
-// attributes, outside any graph capture
-void dgemm_strided(int M, int N, int K, const double* A, i64 asb, i64 ar, i64 ac, const double* B, i64 bsb, i64 br,
-                   i64 bc, double* C, i64 csb, i64 cr, i64 cc, int batch, bool accumulate, cudaStream_t s);
-void dgemm_prepare();
-
 // host copy of an instance
 struct NucHost {
     NucInst d;
 };
 
-// A: H[kz][(u v)] = sum_t Wz[kz][t] Phi[(u v)][t];  B: H2[ky][kz][u] = sum_v Wy[ky][v] H[kz][u][v];
-// C: Vk[kx][(ky kz)] = sum_u Wx[kx][u] H2[(ky kz)][u]
-static void nuc_contract_fp64(const NucInst& in, const double* W, const double* Phi, double* Vk, cudaStream_t s) {
-    const int* U = in.U;
-    const int* nk = in.nk;
-    const i64 UxUy = (i64)U[0] * U[1], nzy = (i64)nk[2] * nk[1];
-    const double* Wx = W + in.w_off[0];
-    const double* Wy = W + in.w_off[1];
-    const double* Wz = W + in.w_off[2];
-    DevBuf<double> H((i64)nk[2] * UxUy, s), H2(nzy * U[0], s);
-    dgemm_strided(nk[2], (int)UxUy, U[2], Wz, 0, U[2], 1, Phi + in.phi_off, 0, 1, U[2], H.p, 0, UxUy, 1, 1, false,
-                  s);
-    // H2 rows ordered (ky, kz): Vk comes out as [kx][ky][kz], kz innermost (the
-    // scatter's fastest-varying key along a matrix row)
-    dgemm_strided(nk[1], U[0], U[1], Wy, 0, U[1], 1, H.p, UxUy, 1, U[1], H2.p, U[0], (i64)nk[2] * U[0], 1, nk[2],
-                  false, s);
-    dgemm_strided(nk[0], (int)nzy, U[0], Wx, 0, U[0], 1, H2.p, 0, 1, U[0], Vk + in.vk_off, 0, nzy, 1, 1, false, s);
+// doubles of an instance's packed buffers (even): the field and, later, the
+// key-indexed matrix in one; the two intermediate products
+static i64 nuc_even(i64 n) { return (n + 1) & ~(i64)1; }
+static i64 nuc_x_size(const NucInst& in) {
+    return nuc_even(std::max((i64)in.P[0] * in.P[1] * in.P[2], (i64)in.nk[0] * in.nk[1] * in.nk[2]));
 }
+static i64 nuc_h_size(const NucInst& in) { return nuc_even((i64)in.nk[2] * in.P[0] * in.P[1]); }
+static i64 nuc_h2_size(const NucInst& in) { return nuc_even((i64)in.nk[1] * in.nk[2] * in.P[0]); }
 
-static void nuc_contract_mixed(const NucInst& in, const double* W, const double* Phi, double* Vk, int* err,
+static void nuc_contract_mixed(const NucInst& in, const double* W, double* X, double* Hb, double* H2b, int* err,
                                cudaStream_t s) {
     constexpr int S = MIXED_SLICES, BN = tile_n(MIXED_SLICES);
     const int* U = in.U;
+    const int* P = in.P;
+    const double* Phi = X + in.x_off;
+    double *Vk = X + in.x_off, *H = Hb + in.h_off, *H2 = H2b + in.h2_off;
     const int* nk = in.nk;
-    const i64 UxUy = (i64)U[0] * U[1], nzy = (i64)nk[2] * nk[1];
+    const i64 UxUy = (i64)P[0] * P[1], nzy = (i64)nk[2] * nk[1];
     const double* Wx = W + in.w_off[0];
     const double* Wy = W + in.w_off[1];
     const double* Wz = W + in.w_off[2];
-    DevBuf<double> H((i64)nk[2] * UxUy, s), H2(nzy * U[0], s);
     {   // A: rows (u v) of the field against the z keys
         TiledSlices As, Bs;
         const i64 mb = (UxUy + TC_BM - 1) / TC_BM, nbt = (nk[2] + BN - 1) / BN;
         As.alloc(mb, TC_BM, U[2], S, s);
-        slice_tiled(DenseRows{Phi + in.phi_off, U[2]}, UxUy, U[2], As, s);
+        slice_tiled(DenseRows{Phi, P[2]}, UxUy, U[2], As, s);
         Bs.alloc(nbt, BN, U[2], S, s);
-        slice_tiled(DenseRows{Wz, U[2]}, nk[2], U[2], Bs, s);
+        slice_tiled(DenseRows{Wz, P[2]}, nk[2], U[2], Bs, s);
         TileWork w;
         w.a_rows = (int)UxUy;
         w.a_blocks = (int)mb;
         w.n_total = nk[2];
-        w.C = H.p;
+        w.C = H;
         w.rs = 1;
         w.cs = UxUy;
         tc_gemm_tiled(As.view(), Bs.view(), w, (int)nbt, err, s);
     }
     {   // B: batch kz, rows u of H[kz] (K = v) against the y keys (shared by every batch)
         TiledSlices As, Bs;
-        const int mb = (U[0] + TC_BM - 1) / TC_BM, nbt = (nk[1] + BN - 1) / BN;
+        const int mb = (P[0] + TC_BM - 1) / TC_BM, nbt = (nk[1] + BN - 1) / BN;
         As.alloc((i64)nk[2] * mb, TC_BM, U[1], S, s);
-        slice_tiled(BatchedRows{H.p, U[1], U[0], mb}, (i64)nk[2] * U[0], U[1], As, s);
+        slice_tiled(BatchedRows{H, P[1], P[0], mb}, (i64)nk[2] * P[0], U[1], As, s);
         Bs.alloc(nbt, BN, U[1], S, s);
-        slice_tiled(DenseRows{Wy, U[1]}, nk[1], U[1], Bs, s);
+        slice_tiled(DenseRows{Wy, P[1]}, nk[1], U[1], Bs, s);
         const int ntiles = nk[2] * nbt;
         DevBuf<int> tiles(4 * (i64)ntiles, s);
         k_shared_b_tiles<<<(ntiles + 255) / 256, 256, 0, s>>>(nk[2], nbt, nk[1], BN, tiles.p, tiles.p + ntiles,
                                                               tiles.p + 2 * ntiles, tiles.p + 3 * ntiles);
         GLI_CHECK_LAUNCH();
         TileWork w;
-        w.a_rows = U[0];
+        w.a_rows = P[0];
         w.a_blocks = mb;
         w.a_batched = 1;
         w.tile_batch = tiles.p;
         w.tile_col0 = tiles.p + ntiles;
         w.tile_ncols = tiles.p + 2 * ntiles;
         w.tile_bblock = tiles.p + 3 * ntiles;
-        w.C = H2.p;
+        w.C = H2;
         w.rs = 1;
-        w.cs = U[0];
+        w.cs = P[0];
         tc_gemm_tiled(As.view(), Bs.view(), w, ntiles, err, s);
     }
     {   // C: rows (kz ky) of H2 (K = u) against the x keys
         TiledSlices As, Bs;
         const i64 mb = (nzy + TC_BM - 1) / TC_BM, nbt = (nk[0] + BN - 1) / BN;
         As.alloc(mb, TC_BM, U[0], S, s);
-        slice_tiled(DenseRows{H2.p, U[0]}, nzy, U[0], As, s);
+        slice_tiled(DenseRows{H2, P[0]}, nzy, U[0], As, s);
         Bs.alloc(nbt, BN, U[0], S, s);
-        slice_tiled(DenseRows{Wx, U[0]}, nk[0], U[0], Bs, s);
+        slice_tiled(DenseRows{Wx, P[0]}, nk[0], U[0], Bs, s);
         TileWork w;
         w.a_rows = (int)nzy;
         w.a_blocks = (int)mb;
         w.n_total = nk[0];
-        w.C = Vk + in.vk_off;
+        w.C = Vk;
         w.rs = 1;
         w.cs = nzy;
         tc_gemm_tiled(As.view(), Bs.view(), w, (int)nbt, err, s);
@@ -322,87 +507,116 @@ static void ensure_streams(int device, int n) {
     t_ring.ensure(device, n);
 }
 
-// Queues one chunk of instances (descriptors already on the device): weights,
-// field, per-instance contractions on `nstreams` forked streams (int8-sliced
-// tensor-core products when `sliced`, else the FP64 tensor-core GEMM),
-// scatter.  Makes no call that a stream capture forbids.
-static void enqueue_chunk(const std::vector<NucHost>& hosts, const NucInst* d_inst, const double* F, int nf, int nb,
-                          const int* coords, const double* npos, const double* ncharge, bool sliced, int nstreams,
-                          int num_sms, int* err, cudaStream_t s) {
+// kernel attributes: shared memory above the 48 KB default
+static void nuc_prepare() {
+    GLI_CUDA(cudaFuncSetAttribute(k_nuc_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, NUC_LINES_BYTES));
+}
+
+// Queues one chunk of instances, dealt over `pipes` pipelines (largest first,
+// round robin; one pipeline: stream s itself, else forked streams): per
+// pipeline the weights, the field, the three contractions (int8-sliced
+// tensor-core products per instance when `sliced`, else one FP64 tensor-core
+// launch per stage) and the scatter.
+static void run_chunk(const std::vector<NucHost>& hosts, const double* F, int nf, int nb, const int* coords,
+                      const double* npos, const double* ncharge, bool sliced, int pipes, int num_sms, int* err,
+                      cudaStream_t s) {
     const int ni = (int)hosts.size();
-    i64 w_total = 0, phi_total = 0, vk_total = 0;
-    int max_nk = 1, max_u = 1;
-    i64 max_rows = 1;
-    for (const NucHost& h : hosts) {
-        for (int a = 0; a < 3; ++a) {
-            w_total = std::max(w_total, h.d.w_off[a] + (i64)h.d.nk[a] * h.d.U[a]);
-            max_nk = std::max(max_nk, h.d.nk[a]);
-            max_u = std::max(max_u, h.d.U[a]);
-        }
-        const i64 cells = (i64)h.d.U[0] * h.d.U[1] * h.d.U[2];
-        phi_total = std::max(phi_total, h.d.phi_off + cells);
-        vk_total = std::max(vk_total, h.d.vk_off + (i64)h.d.nk[0] * h.d.nk[1] * h.d.nk[2]);
-        max_rows = std::max(max_rows, (i64)h.d.U[0] * h.d.U[1]);
-    }
-    DevBuf<double> W(w_total, s), Phi(phi_total, s), Vk(vk_total, s);
-    k_nuc_weights<<<dim3((unsigned)((max_u + 127) / 128), (unsigned)max_nk, (unsigned)(3 * ni)), 128, 0, s>>>(
-        d_inst, F, nf, nb, coords, W.p);
-    GLI_CHECK_LAUNCH();
-    {
-        const unsigned fb = (unsigned)std::min<i64>(max_rows, std::max<i64>(1, (i64)num_sms * 16));
-        k_nuc_field<<<dim3(fb, (unsigned)ni), 128, 0, s>>>(d_inst, npos, ncharge, Phi.p);
-        GLI_CHECK_LAUNCH();
-    }
-    // per-instance contractions, largest first, round-robin over the streams
+    pipes = std::min(pipes, ni);
     std::vector<int> order(ni);
     for (int k = 0; k < ni; ++k) order[k] = k;
     std::sort(order.begin(), order.end(), [&](int a, int b) { return hosts[a].d.N > hosts[b].d.N; });
-    GLI_CUDA(cudaEventRecord(t_fork, s));
-    for (int k = 0; k < nstreams; ++k) GLI_CUDA(cudaStreamWaitEvent(t_ring.streams[k], t_fork, 0));
-    for (int k = 0; k < ni; ++k) {
-        cudaStream_t st = t_ring.streams[k % nstreams];
-        const NucInst& in = hosts[order[k]].d;
-        if (sliced)
-            nuc_contract_mixed(in, W.p, Phi.p, Vk.p, err, st);
-        else
-            nuc_contract_fp64(in, W.p, Phi.p, Vk.p, st);
+    // descriptors pipeline by pipeline, then the tiles before each instance per stage
+    const size_t dbytes = ni * sizeof(NucInst);
+    std::vector<char> up(dbytes + 3 * (size_t)(ni + pipes) * sizeof(int));
+    NucInst* desc = reinterpret_cast<NucInst*>(up.data());
+    int* pre = reinterpret_cast<int*>(up.data() + dbytes);
+    std::vector<int> first(pipes + 1, 0);
+    i64 w_total = 0, x_total = 0, h_total = 0, h2_total = 0, ks_total = 0;
+    int at = 0;
+    for (int p = 0; p < pipes; ++p) {
+        first[p] = at;
+        for (int k = p; k < ni; k += pipes) desc[at++] = hosts[order[k]].d;
+        const int cnt = at - first[p];
+        for (int st = 0; st < 3; ++st) {
+            int* pr = pre + st * (ni + pipes) + first[p] + p;
+            i64 t = 0;
+            for (int k = 0; k <= cnt; ++k) {
+                if (t >= ((i64)1 << 31)) fail(GLI_ERR_LIMIT, "too many nuclear contraction tiles in one chunk");
+                pr[k] = (int)t;
+                if (k == cnt) break;
+                const NucInst& in = desc[first[p] + k];
+                const i64 rows = st == 0 ? (i64)in.P[0] * in.P[1] : st == 1 ? (i64)in.nk[2] * in.P[0] : (i64)in.nk[1] * in.nk[2];
+                t += (i64)((in.nk[2 - st] + DM_BM - 1) / DM_BM) * ((rows + DM_BN - 1) / DM_BN);
+            }
+        }
     }
-    for (int k = 0; k < nstreams; ++k) {
-        GLI_CUDA(cudaEventRecord(t_ring.events[k], t_ring.streams[k]));
-        GLI_CUDA(cudaStreamWaitEvent(s, t_ring.events[k], 0));
+    first[pipes] = at;
+    for (const NucHost& h : hosts) {
+        for (int a = 0; a < 3; ++a) {
+            w_total = std::max(w_total, h.d.w_off[a] + (i64)h.d.nk[a] * h.d.P[a]);
+            ks_total = std::max<i64>(ks_total, h.d.ks_off[a] + h.d.nk[a]);
+        }
+        x_total = std::max(x_total, h.d.x_off + nuc_x_size(h.d));
+        h_total = std::max(h_total, h.d.h_off + nuc_h_size(h.d));
+        h2_total = std::max(h2_total, h.d.h2_off + nuc_h2_size(h.d));
     }
-    // one block per x pair (ix, jx) of the largest instance
-    i64 max_pairs = 1;
-    for (const NucHost& h : hosts) max_pairs = std::max<i64>(max_pairs, (i64)h.d.n[0] * h.d.n[0]);
-    k_nuc_scatter<<<dim3((unsigned)max_pairs, (unsigned)ni), 256, 0, s>>>(d_inst, Vk.p, sliced ? 0 : 1);
-    GLI_CHECK_LAUNCH();
-}
-
-// Captures the chunk as one CUDA graph and launches it once
-static void run_chunk_graph(const std::vector<NucHost>& hosts, const NucInst* d_inst, const double* F, int nf,
-                            int nb, const int* coords, const double* npos, const double* ncharge, bool sliced,
-                            int nstreams, int num_sms, int* err, cudaStream_t s) {
-    tc_gemm_prepare();
-    dgemm_prepare();
-    GLI_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    cudaGraph_t graph = nullptr;
-    try {
-        enqueue_chunk(hosts, d_inst, F, nf, nb, coords, npos, ncharge, sliced, nstreams, num_sms, err, s);
-    } catch (...) {
-        cudaStreamEndCapture(s, &graph);
-        if (graph) cudaGraphDestroy(graph);
-        cudaGetLastError();
-        throw;
+    DevBuf<char> d_up(up.size(), s);
+    DevBuf<double> W(w_total, s), X(x_total, s), H(h_total, s), H2(h2_total, s);
+    DevBuf<int> ks(ks_total, s);
+    GLI_CUDA(cudaMemcpyAsync(d_up.p, up.data(), up.size(), cudaMemcpyHostToDevice, s));
+    const NucInst* d_inst = reinterpret_cast<const NucInst*>(d_up.p);
+    const int* d_pre = reinterpret_cast<const int*>(d_up.p + dbytes);
+    if (pipes > 1) {
+        GLI_CUDA(cudaEventRecord(t_fork, s));
+        for (int p = 0; p < pipes; ++p) GLI_CUDA(cudaStreamWaitEvent(t_ring.streams[p], t_fork, 0));
     }
-    GLI_CUDA(cudaStreamEndCapture(s, &graph));
-    cudaGraphExec_t exec = nullptr;
-    const cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
-    cudaGraphDestroy(graph);
-    GLI_CUDA(ie);
-    const cudaError_t le = cudaGraphLaunch(exec, s);
-    const cudaError_t se = le == cudaSuccess ? cudaStreamSynchronize(s) : le;
-    cudaGraphExecDestroy(exec);
-    GLI_CUDA(se);
+    for (int p = 0; p < pipes; ++p) {
+        cudaStream_t st = pipes > 1 ? t_ring.streams[p] : s;
+        const int i0 = first[p], cnt = first[p + 1] - i0;
+        const NucInst* di = d_inst + i0;
+        int max_nk = 1, max_p = 1;
+        i64 max_rows = 1, max_items = 1;
+        int lines = 0;
+        for (int k = i0; k < i0 + cnt; ++k) {
+            const NucInst& in = desc[k];
+            for (int a = 0; a < 3; ++a) {
+                max_nk = std::max(max_nk, in.nk[a]);
+                max_p = std::max(max_p, in.P[a]);
+            }
+            max_rows = std::max(max_rows, (i64)in.P[0] * in.P[1]);
+            const bool by_lines = !sliced && in.n[2] <= NUC_LINE_MAX_Z;
+            max_items = std::max(max_items, (i64)in.n[0] * in.n[0] * (by_lines ? in.n[1] : 1));
+            if (by_lines) {
+                const int line = 8 * in.nk[2], held = std::max(1, std::min(in.n[1], NUC_LINES_BYTES / line));
+                lines = std::max(lines, line * held);
+            }
+        }
+        k_nuc_weights<<<dim3((unsigned)((max_p + 127) / 128), (unsigned)max_nk, (unsigned)(3 * cnt)), 128, 0, st>>>(
+            di, F, nf, nb, coords, W.p, ks.p);
+        GLI_CHECK_LAUNCH();
+        const unsigned fb = (unsigned)std::min<i64>((max_rows + 7) / 8, std::max<i64>(1, (i64)num_sms * 16));
+        k_nuc_field<<<dim3(fb, (unsigned)cnt), 256, 0, st>>>(di, npos, ncharge, X.p);
+        GLI_CHECK_LAUNCH();
+        if (sliced) {
+            for (int k = i0; k < i0 + cnt; ++k) nuc_contract_mixed(desc[k], W.p, X.p, H.p, H2.p, err, st);
+        } else {
+            const int* pr[3];
+            for (int q = 0; q < 3; ++q) pr[q] = d_pre + q * (ni + pipes) + i0 + p;
+            const int* h_pr = pre + i0 + p;
+            auto total = [&](int q) { return dim3((unsigned)h_pr[q * (ni + pipes) + cnt]); };
+            dmma_launch(NucStageOp<0>{di, pr[0], cnt, W.p, ks.p, X.p, H.p, H2.p}, total(0), st);
+            dmma_launch(NucStageOp<1>{di, pr[1], cnt, W.p, ks.p, X.p, H.p, H2.p}, total(1), st);
+            dmma_launch(NucStageOp<2>{di, pr[2], cnt, W.p, ks.p, X.p, H.p, H2.p}, total(2), st);
+        }
+        k_nuc_scatter<<<dim3((unsigned)std::min<i64>(max_items, (i64)num_sms * 8), (unsigned)cnt), 256, lines, st>>>(
+            di, X.p, sliced ? 0 : 1);
+        GLI_CHECK_LAUNCH();
+    }
+    if (pipes > 1)
+        for (int p = 0; p < pipes; ++p) {
+            GLI_CUDA(cudaEventRecord(t_ring.events[p], t_ring.streams[p]));
+            GLI_CUDA(cudaStreamWaitEvent(s, t_ring.events[p], 0));
+        }
 }
 
 static thread_local NuclearBatchStats t_nuc_stats;
@@ -454,26 +668,31 @@ void nuclear_batch_device(const double* h_coeffs, i64 nb, const std::vector<Nucl
     std::vector<NucHost> hosts(ni);
     std::vector<int> coords;
     coords.reserve(total_coords);
-    std::vector<double> npos, nq;
-    npos.reserve(3 * total_nuclei);
-    nq.reserve(total_nuclei);
+    std::vector<double> nuc((size_t)(4 * total_nuclei));  // positions, then charges
+    i64 nuc_at = 0;
     for (i64 k = 0; k < ni; ++k) {
         const NuclearJob& j = jobs[k];
         NucInst& in = hosts[k].d;
+        in.band = 2 * h_mmax + 1;
         for (int a = 0; a < 3; ++a) {
             in.n[a] = (int)j.axes[a].size();
             in.coord_off[a] = (int)coords.size();
             coords.insert(coords.end(), j.axes[a].begin(), j.axes[a].end());
             in.u0[a] = 6 * j.axes[a].front() - h_mmax;
             in.U[a] = 6 * (j.axes[a].back() - j.axes[a].front()) + 2 * h_mmax + 1;
+            in.P[a] = (int)nuc_even(in.U[a]);
             in.nk[a] = in.n[a] * (in.n[a] + 1) / 2;
+            // the keys' order (by the sum of their positions in the list) is by
+            // coordinate sum where the list is a run or holds at most two points
+            const int span = j.axes[a].back() - j.axes[a].front();
+            if (in.n[a] > 2 && span != in.n[a] - 1) in.band = 0;
         }
         in.N = (i64)in.n[0] * in.n[1] * in.n[2];
-        in.nuc0 = (int)nq.size();
+        in.nuc0 = (int)nuc_at;
         in.nnuc = j.nn;
-        for (int q = 0; q < j.nn; ++q) {
-            for (int a = 0; a < 3; ++a) npos.push_back(j.nuclei[q].pos[a]);
-            nq.push_back((double)j.nuclei[q].charge);
+        for (int q = 0; q < j.nn; ++q, ++nuc_at) {
+            for (int a = 0; a < 3; ++a) nuc[(size_t)(3 * nuc_at + a)] = j.nuclei[q].pos[a];
+            nuc[(size_t)(3 * total_nuclei + nuc_at)] = (double)j.nuclei[q].charge;
         }
         in.out = j.d_out;
         if ((i64)in.nk[2] * in.nk[1] > ((i64)65535 * TC_BM))
@@ -481,14 +700,14 @@ void nuclear_batch_device(const double* h_coeffs, i64 nb, const std::vector<Nucl
     }
     // chunks: instances whose packed buffers stay under a memory budget (and
     // the weights kernel's grid limit: 3 x instances <= 65535)
-    const i64 budget = (i64)4 << 30;  // bytes of packed W, Phi, Vk per chunk
+    const i64 budget = (i64)6 << 30;  // bytes of packed buffers per chunk
     std::vector<std::pair<i64, i64>> chunks;
     {
         i64 start = 0, bytes = 0;
         for (i64 k = 0; k < ni; ++k) {
             const NucInst& in = hosts[k].d;
-            const i64 sz = 8 * ((i64)in.nk[0] * in.U[0] + (i64)in.nk[1] * in.U[1] + (i64)in.nk[2] * in.U[2] +
-                                (i64)in.U[0] * in.U[1] * in.U[2] + (i64)in.nk[0] * in.nk[1] * in.nk[2]);
+            const i64 sz = 8 * ((i64)in.nk[0] * in.P[0] + (i64)in.nk[1] * in.P[1] + (i64)in.nk[2] * in.P[2] +
+                                nuc_x_size(in) + nuc_h_size(in) + nuc_h2_size(in));
             if (k > start && (bytes + sz > budget || k - start >= 16384)) {
                 chunks.push_back({start, k});
                 start = k;
@@ -498,46 +717,52 @@ void nuclear_batch_device(const double* h_coeffs, i64 nb, const std::vector<Nucl
         }
         chunks.push_back({start, ni});
     }
-    DevBuf<int> d_coords((i64)coords.size(), s);
-    DevBuf<double> d_npos((i64)npos.size(), s), d_nq((i64)nq.size(), s);
-    GLI_CUDA(cudaMemcpyAsync(d_coords.p, coords.data(), coords.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-    GLI_CUDA(cudaMemcpyAsync(d_npos.p, npos.data(), npos.size() * sizeof(double), cudaMemcpyHostToDevice, s));
-    GLI_CUDA(cudaMemcpyAsync(d_nq.p, nq.data(), nq.size() * sizeof(double), cudaMemcpyHostToDevice, s));
-    DevBuf<NucInst> d_inst(ni, s);
-    DevBuf<int> err(1, s);
-    err.zero();
-    // per chunk: offsets within the chunk's packed buffers, then upload the descriptors
+    // one upload: nuclei, then coordinates
+    const size_t nbytes = nuc.size() * sizeof(double);
+    std::vector<char> up(nbytes + coords.size() * sizeof(int));
+    memcpy(up.data(), nuc.data(), nbytes);
+    memcpy(up.data() + nbytes, coords.data(), coords.size() * sizeof(int));
+    DevBuf<char> d_up(up.size(), s);
+    GLI_CUDA(cudaMemcpyAsync(d_up.p, up.data(), up.size(), cudaMemcpyHostToDevice, s));
+    const double* d_npos = reinterpret_cast<const double*>(d_up.p);
+    const double* d_nq = d_npos + 3 * total_nuclei;
+    const int* d_coords = reinterpret_cast<const int*>(d_up.p + nbytes);
+    DevBuf<int> err;
+    if (form == FORM_MIXED) {
+        err.alloc(1, s);
+        err.zero();
+    }
+    // offsets within the chunk's packed buffers
     for (auto& c : chunks) {
-        i64 w = 0, phi = 0, vk = 0;
+        i64 w = 0, x = 0, h = 0, h2 = 0;
+        int ks = 0;
         for (i64 k = c.first; k < c.second; ++k) {
             NucInst& in = hosts[k].d;
             for (int a = 0; a < 3; ++a) {
                 in.w_off[a] = w;
-                w += (i64)in.nk[a] * in.U[a];
+                w += (i64)in.nk[a] * in.P[a];
+                in.ks_off[a] = ks;
+                ks += in.nk[a];
             }
-            in.phi_off = phi;
-            phi += (i64)in.U[0] * in.U[1] * in.U[2];
-            in.vk_off = vk;
-            vk += (i64)in.nk[0] * in.nk[1] * in.nk[2];
+            in.x_off = x;
+            in.h_off = h;
+            in.h2_off = h2;
+            x += nuc_x_size(in);
+            h += nuc_h_size(in);
+            h2 += nuc_h2_size(in);
         }
     }
-    std::vector<NucInst> hd(ni);
-    for (i64 k = 0; k < ni; ++k) hd[k] = hosts[k].d;
-    GLI_CUDA(cudaMemcpyAsync(d_inst.p, hd.data(), ni * sizeof(NucInst), cudaMemcpyHostToDevice, s));
-    // the host staging vectors must outlive the copies
-    GLI_CUDA(cudaStreamSynchronize(s));
 
     const Context& ctx = context();
-    const bool graphs = getenv("GLI_B200_NO_GRAPHS") == nullptr;
     ensure_streams(ctx.device, 8);
+    nuc_prepare();
     for (size_t c = 0; c < chunks.size(); ++c) {
         const std::vector<NucHost> part(hosts.begin() + chunks[c].first, hosts.begin() + chunks[c].second);
-        const NucInst* dptr = d_inst.p + chunks[c].first;
-        // streams for the per-instance contractions and, in the mixed form, the
-        // contraction path: chosen by timing the first chunk of a batch of this
-        // shape (cached per shape key).  Candidate c: c % 16 streams, c >= 16
-        // the int8-sliced tensor-core contractions (mixed form only; they pay
-        // only where the GEMMs are large enough to carry the slicing passes)
+        // pipelines and, in the mixed form, the contraction path: chosen by
+        // timing the first chunk of a batch of this shape (cached per shape
+        // key).  Candidate c: c % 16 pipelines, c >= 16 the int8-sliced
+        // tensor-core contractions (mixed form only; they pay only where the
+        // GEMMs are large enough to carry the slicing passes)
         char key[160];
         snprintf(key, sizeof(key), "nuclear form=%d dev=%d inst=%zu maxN=%lld", form, ctx.device, part.size(),
                  (long long)std::max_element(part.begin(), part.end(), [](const NucHost& a, const NucHost& b) {
@@ -546,12 +771,7 @@ void nuclear_batch_device(const double* h_coeffs, i64 nb, const std::vector<Nucl
         auto run = [&](int cand) {
             const bool sliced = cand >= 16;
             const int nstreams = cand % 16;
-            if (graphs)
-                run_chunk_graph(part, dptr, F.p, nf, (int)nb, d_coords.p, d_npos.p, d_nq.p, sliced, nstreams,
-                                ctx.num_sms, err.p, s);
-            else
-                enqueue_chunk(part, dptr, F.p, nf, (int)nb, d_coords.p, d_npos.p, d_nq.p, sliced, nstreams,
-                              ctx.num_sms, err.p, s);
+            run_chunk(part, F.p, nf, (int)nb, d_coords, d_npos, d_nq, sliced, nstreams, ctx.num_sms, err.p, s);
         };
         std::vector<int> cands = part.size() == 1 ? std::vector<int>{1} : std::vector<int>{1, 2, 4, 8};
         if (form == FORM_MIXED)
@@ -575,7 +795,7 @@ void nuclear_batch_device(const double* h_coeffs, i64 nb, const std::vector<Nucl
         stats.chunks += 1;
     }
     int h_err = 0;
-    GLI_CUDA(cudaMemcpyAsync(&h_err, err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    if (err.p) GLI_CUDA(cudaMemcpyAsync(&h_err, err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     GLI_CUDA(cudaStreamSynchronize(s));
     if (h_err) fail(GLI_ERR_INTERNAL, "tensor-core stage: an mbarrier wait expired (code %d)", h_err);
     stats.instances = ni;

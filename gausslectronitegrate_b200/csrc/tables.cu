@@ -42,22 +42,31 @@ __global__ void k_erida_products(const double* __restrict__ b, int nb, double to
     if (acc != 0) atomicMax(maxabs, s < 0 ? -s : s);
 }
 
-// F[s][m], s = 0..L-1, m = 0..2nb-2 (logical factor index m - (nb-1))
-__global__ void k_factors(const double* __restrict__ b, int nb, int L, double* __restrict__ F) {
-    const int nf = 2 * nb - 1;
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+// F[s][m], s = 0..L-1, m = 0..2nb-2 (logical factor index m - (nb-1)): a warp
+// per entry, its lanes over the pairs i + j = m (a thread per entry summed up
+// to 135 exponentials one after the other: 20 us of latency at the head of
+// every nuclear call)
+__global__ void __launch_bounds__(256) k_factors(const double* __restrict__ b, int nb, int L, double* __restrict__ F) {
+    const int nf = 2 * nb - 1, lane = threadIdx.x & 31;
+    const int m = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int s = blockIdx.y;
     if (m >= nf) return;
     const double prefac = 0.590817950301838675766;  // sqrt(pi) / 3
     double acc = 0;
     const int ilo = m - (nb - 1) > 0 ? m - (nb - 1) : 0;
     const int ihi = m < nb - 1 ? m : nb - 1;
-    for (int i = ilo; i <= ihi; ++i) {
+    for (int i = ilo + lane; i <= ihi; i += 32) {
         const int j = m - i;
         const double e = 0.5 * (double)(3 * s + (i - j));
         acc += prefac * b[i] * b[j] * exp(-e * e);
     }
-    F[(i64)s * nf + m] = acc;
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) F[(i64)s * nf + m] = acc;
+}
+
+static void launch_factors(const double* d_b, int nb, int L, double* d_F, cudaStream_t s) {
+    k_factors<<<dim3((2 * nb - 1 + 7) / 8, L), 256, 0, s>>>(d_b, nb, L, d_F);
+    GLI_CHECK_LAUNCH();
 }
 
 // Pr[pair][x + 2nb-2] for pairs (sa <= sb) in triangular order, masked at tol
@@ -133,9 +142,7 @@ __global__ void k_coulomb_table(int kind, i64 n_entries, double* __restrict__ T)
 }
 
 void factors_device(const double* d_b, int nb, int L, double* d_F, cudaStream_t s) {
-    const int nf = 2 * nb - 1;
-    k_factors<<<dim3((nf + 127) / 128, L), 128, 0, s>>>(d_b, nb, L, d_F);
-    GLI_CHECK_LAUNCH();
+    launch_factors(d_b, nb, L, d_F, s);
 }
 
 // distinct s = u^2 + v^2 (u, v < U): mark, scan, list, and the U x U index
@@ -177,8 +184,7 @@ static void build_lattice_tables(int kind, const double* h_coeffs, i64 nb, i64 L
     } else {
         const i64 nf = 2 * nb - 1, xl = 4 * nb - 3, npairs = L * (L + 1) / 2;
         DevBuf<double> F(L * nf, s);
-        k_factors<<<dim3((unsigned)((nf + 127) / 128), (unsigned)L), 128, 0, s>>>(b.p, (int)nb, (int)L, F.p);
-        GLI_CHECK_LAUNCH();
+        launch_factors(b.p, (int)nb, (int)L, F.p, s);
         prod.alloc(npairs * xl, s);
         k_eri_products<<<dim3((unsigned)((xl + 127) / 128), (unsigned)npairs), 128, 0, s>>>(F.p, (int)nb, tol, prod.p,
                                                                                               maxabs.p);
@@ -302,8 +308,7 @@ double mixed_screen_tol(int kind, const double* h_coeffs, i64 nb, i64 L, double 
         xl = 4 * nb - 3;
         npairs = L * (L + 1) / 2;
         DevBuf<double> F(L * nf, s);
-        k_factors<<<dim3((unsigned)((nf + 127) / 128), (unsigned)L), 128, 0, s>>>(b.p, (int)nb, (int)L, F.p);
-        GLI_CHECK_LAUNCH();
+        launch_factors(b.p, (int)nb, (int)L, F.p, s);
         prod.alloc(npairs * xl, s);
         k_eri_products<<<dim3((unsigned)((xl + 127) / 128), (unsigned)npairs), 128, 0, s>>>(F.p, (int)nb, 0.0, prod.p,
                                                                                               maxabs.p);
