@@ -5,10 +5,11 @@
 // chosen per Op) over K in chunks of 16, three chunks in flight (two for an Op
 // that declares STAGES = 2: the 144-column tiles, so that three blocks still
 // fit on an SM; cp.async groups, the waits are the hardware's own group waits,
-// no flag spins).  Warp w owns the
-// 32 x BN/2 quadrant (w & 1, w >> 1) as 4 x BN/16 m8n8 accumulators; per
-// k-step of 4 it reads 4 A and BN/16 B fragments (one double each) for
-// 4 BN/16 MMAs of 256 FMAs.  BN = 80 serves 65..80 and 129..160 columns in
+// no flag spins).  Warp w owns every other 8-row and 8-column strip (rows
+// 16 i + 8 (w & 1), columns 16 j + 8 (w >> 1)) as 4 x BN/16 m8n8 accumulators,
+// so that a partly filled tile loads the four warps (and their tensor pipes)
+// alike; per k-step of 4 it reads 4 A and BN/16 B fragments (one double each)
+// for 4 BN/16 MMAs of 256 FMAs.  BN = 80 serves 65..80 and 129..160 columns in
 // one and two column tiles (129 keys: 2 tiles instead of 3, measured 20%
 // faster on the stage A shape); BN = 144 holds 129 keys in one tile (another
 // 1.5%: the lattice gathers are made once).
@@ -133,13 +134,56 @@ struct dm_a_landed<Op, std::void_t<decltype(Op::A_LANDED)>> {
     static constexpr bool value = Op::A_LANDED;
 };
 
+// Skipped strips (an Op that declares SKIP): rows (SKIP_M) or columns (SKIP_N)
+// whose operand is zero outside a run of K -- lattice weights, nonzero around
+// their key's position -- take part only in the chunks of their 8-row
+// strip's run.  Op::live_chunks(blk, strip, first, last) gives the chunks
+// [first, last] of a strip (empty: last < first); a mask per chunk, one bit per
+// strip of a warp, is built in shared memory before the main loop.  A skipped
+// MMA would have added products with exact zeros.
+constexpr int SKIP_M = 1, SKIP_N = 2, DM_MAX_CHUNKS = 256;
+template <class Op, class = void>
+struct dm_skip_of {
+    static constexpr int value = 0;
+};
+template <class Op>
+struct dm_skip_of<Op, std::void_t<decltype(Op::SKIP)>> {
+    static constexpr int value = Op::SKIP;
+};
+
+// masks of the two strip groups (even and odd strips) of every chunk
+template <class Op>
+__device__ __forceinline__ void dm_build_masks(const Op& op, const typename Op::Block& blk,
+                                               uint16_t (&live)[2][DM_MAX_CHUNKS]) {
+    constexpr int STRIPS = (dm_skip_of<Op>::value == SKIP_M ? DM_BM : Op::BN) / 8;
+    __shared__ int run[STRIPS];  // first | last << 16 (first > last: empty)
+    for (int t = threadIdx.x; t < STRIPS; t += DM_THREADS) {
+        int first, last;
+        op.live_chunks(blk, t, first, last);
+        run[t] = last < first ? 1 : first | last << 16;
+    }
+    __syncthreads();
+    for (int kc = threadIdx.x; kc < blk.nk; kc += DM_THREADS)
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            unsigned m = 0;
+#pragma unroll
+            for (int t = 0; t < STRIPS / 2; ++t) {
+                const int r = run[2 * t + g];
+                m |= (unsigned)((r & 0xffff) <= kc && kc <= r >> 16) << t;
+            }
+            live[g][kc] = (uint16_t)m;
+        }
+}
+
 // The k loop of one block; FULL: every m8n8 tile of the warp's quadrant holds
 // data, so the MMAs run unpredicated (a runtime predicate per MMA costs about
 // a fifth of the tensor-pipe throughput).
 template <class Op, bool FULL>
 __device__ __forceinline__ void dm_mainloop(const Op& op, const typename Op::Block& blk, typename Op::AState& as,
                                             typename Op::BState& bs, double* smem, int wm, int wn, int mt, int nt,
-                                            double (&acc)[4][Op::BN / 16][2]) {
+                                            const uint16_t* live, double (&acc)[4][Op::BN / 16][2]) {
+    constexpr int SKIP = dm_skip_of<Op>::value;
     constexpr int NJ = Op::BN / 16, STAGE = DM_TILE_A + dm_tile_b(Op::BN), NS = dm_stages_of<Op>::value;
     const int lane = threadIdx.x & 31;
     const int nk = blk.nk;
@@ -156,13 +200,46 @@ __device__ __forceinline__ void dm_mainloop(const Op& op, const typename Op::Blo
         dm_commit();
         const double* a_s = smem + (kc % NS) * STAGE;
         const double* b_s = a_s + DM_TILE_A;
+        if constexpr (SKIP != 0) {
+            const unsigned m = live[kc];
+            if (m == 0) continue;
+            if (!FULL || m != (1u << (SKIP == SKIP_M ? 4 : NJ)) - 1u) {
+#pragma unroll
+                for (int k0 = 0; k0 < DM_BK; k0 += 4) {
+                    if constexpr (SKIP == SKIP_M) {
+                        double bf[NJ];
+#pragma unroll
+                        for (int j = 0; j < NJ; ++j) bf[j] = dm_frag<Op::B_KMAJOR>(b_s, wn + 16 * j, k0, lane);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            if (m >> i & 1u) {
+                                const double af = dm_frag<Op::A_KMAJOR>(a_s, wm + 16 * i, k0, lane);
+#pragma unroll
+                                for (int j = 0; j < NJ; ++j) dm_mma(acc[i][j], af, bf[j]);
+                            }
+                    } else {
+                        double af[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) af[i] = dm_frag<Op::A_KMAJOR>(a_s, wm + 16 * i, k0, lane);
+#pragma unroll
+                        for (int j = 0; j < NJ; ++j)
+                            if (m >> j & 1u) {
+                                const double bf = dm_frag<Op::B_KMAJOR>(b_s, wn + 16 * j, k0, lane);
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) dm_mma(acc[i][j], af[i], bf);
+                            }
+                    }
+                }
+                continue;
+            }
+        }
 #pragma unroll
         for (int k0 = 0; k0 < DM_BK; k0 += 4) {
             double af[4], bf[NJ];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) af[i] = dm_frag<Op::A_KMAJOR>(a_s, wm + 8 * i, k0, lane);
+            for (int i = 0; i < 4; ++i) af[i] = dm_frag<Op::A_KMAJOR>(a_s, wm + 16 * i, k0, lane);
 #pragma unroll
-            for (int j = 0; j < NJ; ++j) bf[j] = dm_frag<Op::B_KMAJOR>(b_s, wn + 8 * j, k0, lane);
+            for (int j = 0; j < NJ; ++j) bf[j] = dm_frag<Op::B_KMAJOR>(b_s, wn + 16 * j, k0, lane);
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -206,7 +283,7 @@ __device__ __forceinline__ void dm_cluster_reduce(const Op& op, const typename O
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
             const bool has = active && i < mt && j < nt;
-            double* d = smem + (wm + 8 * i + (lane >> 2)) * LD + wn + 8 * j + 2 * (lane & 3);
+            double* d = smem + (wm + 16 * i + (lane >> 2)) * LD + wn + 16 * j + 2 * (lane & 3);
             d[0] = has ? acc[i][j][0] : 0.0;
             d[1] = has ? acc[i][j][1] : 0.0;
         }
@@ -292,7 +369,7 @@ __device__ __forceinline__ void dm_split_store(const Op& op, const typename Op::
             if (i < mt && j < nt) {
                 const double o0 = __ldcg(other + ((i * NJ + j) * 2) * DM_THREADS + threadIdx.x);
                 const double o1 = __ldcg(other + ((i * NJ + j) * 2 + 1) * DM_THREADS + threadIdx.x);
-                op.store(blk, wm + 8 * i + (lane >> 2), wn + 8 * j + 2 * (lane & 3), acc[i][j][0] + o0,
+                op.store(blk, wm + 16 * i + (lane >> 2), wn + 16 * j + 2 * (lane & 3), acc[i][j][0] + o0,
                          acc[i][j][1] + o1);
             }
     if (threadIdx.x == 0) op.tickets[slot] = 0u;
@@ -316,11 +393,17 @@ __global__ void __launch_bounds__(DM_THREADS, dm_blocks_of<Op>::value) k_dmma(co
         return;
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wm = (warp & 1) * 32, wn = (warp >> 1) * (Op::BN / 2);
+    const int wm = (warp & 1) * 8, wn = (warp >> 1) * 8;
     typename Op::AState as;
     typename Op::BState bs;
     op.a_init(blk, as);
     op.b_init(blk, bs);
+    const uint16_t* live = nullptr;
+    if constexpr (dm_skip_of<Op>::value != 0) {
+        __shared__ uint16_t s_live[2][DM_MAX_CHUNKS];
+        dm_build_masks(op, blk, s_live);
+        live = s_live[dm_skip_of<Op>::value == SKIP_M ? warp & 1 : warp >> 1];
+    }
 #pragma unroll
     for (int st = 0; st < NS - 1; ++st) {
         if (st < blk.nk) {
@@ -330,17 +413,17 @@ __global__ void __launch_bounds__(DM_THREADS, dm_blocks_of<Op>::value) k_dmma(co
         dm_commit();
     }
     // m8 / n8 tiles of this warp's quadrant that hold rows / columns (warp-uniform)
-    const int mt = min(4, max(0, (blk.mvalid - wm + 7) >> 3));
-    const int nt = min(NJ, max(0, (blk.nvalid - wn + 7) >> 3));
+    const int mt = min(4, max(0, (blk.mvalid - wm + 15) >> 4));
+    const int nt = min(NJ, max(0, (blk.nvalid - wn + 15) >> 4));
     double acc[4][NJ][2];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < NJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
     if (mt == 4 && nt == NJ)
-        dm_mainloop<Op, true>(op, blk, as, bs, dm_smem, wm, wn, mt, nt, acc);
+        dm_mainloop<Op, true>(op, blk, as, bs, dm_smem, wm, wn, mt, nt, live, acc);
     else
-        dm_mainloop<Op, false>(op, blk, as, bs, dm_smem, wm, wn, mt, nt, acc);
+        dm_mainloop<Op, false>(op, blk, as, bs, dm_smem, wm, wn, mt, nt, live, acc);
     dm_wait<0>();
     if constexpr (CLUSTER) {
         dm_cluster_reduce<Op, CLUSTER>(op, blk, true, dm_smem, wm, wn, mt, nt, acc);
@@ -358,7 +441,7 @@ __global__ void __launch_bounds__(DM_THREADS, dm_blocks_of<Op>::value) k_dmma(co
 #pragma unroll
         for (int j = 0; j < NJ; ++j)
             if (i < mt && j < nt)
-                op.store(blk, wm + 8 * i + (lane >> 2), wn + 8 * j + 2 * (lane & 3), acc[i][j][0], acc[i][j][1]);
+                op.store(blk, wm + 16 * i + (lane >> 2), wn + 16 * j + 2 * (lane & 3), acc[i][j][0], acc[i][j][1]);
 }
 
 // (three blocks per SM: 3 x 60 or 69 KB of shared memory, at most 170 registers)

@@ -22,7 +22,9 @@
 // 3 (i_a + j_a) only (mmax: the outermost factor above tol; 99 of 237 positions
 // on a 24-point axis at tol 1e-8).  Keys are therefore ordered by i_a + j_a, so
 // that the 64 keys of a tile share most of their positions, and a tile's K loop
-// covers just the positions that any of its keys reaches.
+// covers just the positions that any of its keys reaches.  Keys whose factor is
+// below tol throughout (|i_a - j_a| from 17 at tol 1e-8) are no keys at all:
+// their matrix entries are zero.
 //
 // Batches.  Any number of instances (each its own grid and nuclei, all with
 // the same coefficients and tol) run as one plan: one upload of every
@@ -40,6 +42,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <map>
 #include <string>
 
 #include "autotune.cuh"
@@ -49,7 +52,8 @@
 
 namespace gli {
 
-__global__ void k_mask_factors(double* __restrict__ F, i64 n, int nf, int nb, double tol, int* __restrict__ mmax) {
+// masks F at tol; reach[0] = largest |m|, reach[1] = largest s of an entry above tol
+__global__ void k_mask_factors(double* __restrict__ F, i64 n, int nf, int nb, double tol, int* __restrict__ reach) {
     const i64 e = (i64)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n) return;
     double v = F[e];
@@ -57,7 +61,8 @@ __global__ void k_mask_factors(double* __restrict__ F, i64 n, int nf, int nb, do
     F[e] = v;
     if (v != 0) {
         const int m = (int)(e % nf) - (nb - 1);
-        atomicMax(mmax, m < 0 ? -m : m);
+        atomicMax(&reach[0], m < 0 ? -m : m);
+        atomicMax(&reach[1], (int)(e / nf));
     }
 }
 
@@ -67,7 +72,9 @@ struct NucInst {
     int coord_off[3];  // first coordinate of each axis in the packed coordinate list
     int U[3], u0[3];   // lattice extent and origin (units of 1/6) per axis
     int P[3];          // U rounded up to even: row pitches (16-byte rows)
-    int nk[3];         // axis keys: n (n + 1) / 2
+    int nk[3];         // axis keys: pairs lo <= hi whose factor is not zero throughout
+    int rk_off[3];     // n x n table: key of (i, j), NUC_DEAD where the factor is zero
+    int key_off[3];    // lo | hi << 8 of each key
     int band;          // weights per key (2 mmax + 1); 0: the keys' order is not by position
     int nuc0, nnuc;    // nuclei in the packed nucleus arrays
     i64 N;             // grid points
@@ -79,31 +86,22 @@ struct NucInst {
     double* out;       // N x N row-major
 };
 
-// Position of key (lo <= hi) of an axis of n points when keys are ordered by
-// lo + hi, then lo: the keys with a smaller sum t < s number floor((s + 1)^2 / 4)
-// up to the middle sum, and mirror beyond it
-__host__ __device__ __forceinline__ int nuc_rank(int n, int lo, int hi) {
-    const int s = lo + hi;
-    const int base = s < n ? (s + 1) * (s + 1) / 4 : n * (n + 1) / 2 - (2 * n - s) * (2 * n - s) / 4;
-    return base + lo - (s >= n ? s - n + 1 : 0);
-}
+constexpr uint16_t NUC_DEAD = 0xffff;
 
 // W[key][u] of every (instance, axis), u a lattice position (zeros up to the
 // pitch), and the first position of each key.  grid (u blocks, key, 3 * instance)
 __global__ void k_nuc_weights(const NucInst* __restrict__ inst, const double* __restrict__ F, int nf, int nb,
-                              const int* __restrict__ coords, double* __restrict__ W, int* __restrict__ kstart) {
+                              const int* __restrict__ coords, const uint16_t* __restrict__ tables,
+                              double* __restrict__ W, int* __restrict__ kstart) {
     const NucInst& in = inst[blockIdx.z / 3];
     const int a = blockIdx.z % 3;
     const int key = blockIdx.y;
     if (key >= in.nk[a]) return;
-    int hi = (int)((sqrt(8.0 * key + 1.0) - 1.0) * 0.5);
-    while (hi * (hi + 1) / 2 > key) --hi;
-    while ((hi + 1) * (hi + 2) / 2 <= key) ++hi;
-    const int lo = key - hi * (hi + 1) / 2, rank = nuc_rank(in.n[a], lo, hi);
+    const int lohi = tables[in.key_off[a] + key], lo = lohi & 0xff, hi = lohi >> 8;
     const int xa = coords[in.coord_off[a] + lo], xb = coords[in.coord_off[a] + hi];
     const int s = xa > xb ? xa - xb : xb - xa;
     const int U = in.U[a], P = in.P[a];
-    double* w = W + in.w_off[a] + (i64)rank * P;
+    double* w = W + in.w_off[a] + (i64)key * P;
     for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < P; u += gridDim.x * blockDim.x) {
         const int m = u + in.u0[a] - 3 * (xa + xb);  // factor logical index
         double v = 0;
@@ -111,7 +109,7 @@ __global__ void k_nuc_weights(const NucInst* __restrict__ inst, const double* __
         w[u] = v;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0)
-        kstart[in.ks_off[a] + rank] = 3 * (xa + xb) - 6 * coords[in.coord_off[a]];
+        kstart[in.ks_off[a] + key] = 3 * (xa + xb) - 6 * coords[in.coord_off[a]];
 }
 
 // the Gaussian-nucleus field g(r) = erf(r / w) / r with w = 1/3 at squared
@@ -123,15 +121,29 @@ __device__ __forceinline__ double nuc_gaussian(double r2) {
     return r > 0 ? erf(3.0 * r) / r : 3.3851375012865379;  // 6 / sqrt(pi)
 }
 
+// 1 / sqrt(x) for 4 <= x < 1e201: the hardware's approximation (PTX
+// rsqrt.approx.ftz.f64, 20 bits) and two Newton steps y += y (1 - x y^2) / 2.
+// The field's cells away from a nucleus need no more than this range, and the
+// general function's handling of the others was most of the field's
+// instructions.
+__device__ __forceinline__ double nuc_rsqrt(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    y = fma(0.5 * y, fma(-x, y * y, 1.0), y);
+    return fma(0.5 * y, fma(-x, y * y, 1.0), y);
+}
+
 // Phi[u][v][t] (t fastest, pitches P) of every instance, position
 // (u + u0x, v + u0y, t + u0z) / 6; grid (row blocks, instance), a warp fills
-// whole (u, v) rows, four cells per lane and turn: per nucleus the row's part of
+// whole (u, v) rows, up to eight cells per lane and turn: per nucleus the row's part of
 // the squared distance is formed once and each cell costs two FP64
-// multiply-adds and a reciprocal square root.  Bound: the FP64 pipe.  24^3 to
-// 8^3 batch of eight (27 million cells, 6 nuclei): 722 us with a thread per
-// cell, its three coordinates divided by 6 and its whole distance per nucleus.
+// multiply-adds and a reciprocal square root.  Bound: the FP64 pipe, 67% busy.
+// 24^3 to 8^3 batch of eight (54 million cells, 6 nuclei): 367 us; 722 us with a
+// thread per cell, its three coordinates divided by 6 and its whole distance per
+// nucleus.
 constexpr int NUC_FIELD_MAX_T = 2048;  // z positions held in shared memory (axes of 256 points: 1531 + 2 mmax)
-__global__ void __launch_bounds__(256) k_nuc_field(const NucInst* __restrict__ inst, const double* __restrict__ npos,
+constexpr int NUC_FIELD_BLOCKS = 3;     // per SM
+__global__ void __launch_bounds__(256, NUC_FIELD_BLOCKS) k_nuc_field(const NucInst* __restrict__ inst, const double* __restrict__ npos,
                                                    const double* __restrict__ ncharge, double* __restrict__ X) {
     __shared__ double zs[NUC_FIELD_MAX_T];
     const NucInst& in = inst[blockIdx.y];
@@ -143,28 +155,52 @@ __global__ void __launch_bounds__(256) k_nuc_field(const NucInst* __restrict__ i
         const int u = row / Py, v = row - u * Py;
         const double px = (u + in.u0[0]) / 6.0, py = (v + in.u0[1]) / 6.0;
         double* phi = X + in.x_off + (i64)row * Pz;
-        for (int t0 = 0; t0 < Pz; t0 += 128) {
-            double pz[4], acc[4] = {0.0, 0.0, 0.0, 0.0};
-            const int live = min(4, (Pz - t0 + 31) >> 5);  // (the same in every lane)
+        auto zs_at = [&](int t) { return t < NUC_FIELD_MAX_T ? zs[t < Pz ? t : 0] : (t + in.u0[2]) / 6.0; };
+        auto cells = [&](auto count, int t0) {
+            constexpr int C = decltype(count)::value;
+            double pz[C], acc[C];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
+            for (int c = 0; c < C; ++c) {
                 const int t = t0 + 32 * c + lane;
-                pz[c] = t < NUC_FIELD_MAX_T ? zs[t < Pz ? t : 0] : (t + in.u0[2]) / 6.0;
+                pz[c] = zs_at(t);
+                acc[c] = 0.0;
             }
             for (int k = in.nuc0; k < in.nuc0 + in.nnuc; ++k) {
                 const double dx = px - npos[3 * k], dy = py - npos[3 * k + 1], nz = npos[3 * k + 2], q = ncharge[k];
                 const double r2 = dx * dx + dy * dy;
+                // (a whole row that has no cell near the nucleus, at distances in range)
+                if (r2 >= 4.0 && r2 < 1e200 && fabs(nz) < 1e99) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    if (c >= live) break;
-                    const double dz = pz[c] - nz;
-                    acc[c] += q * nuc_gaussian(r2 + dz * dz);
+                    for (int c = 0; c < C; ++c) {
+                        const double dz = pz[c] - nz;
+                        acc[c] += q * nuc_rsqrt(r2 + dz * dz);
+                    }
+                } else {
+#pragma unroll 1
+                    for (int c = 0; c < C; ++c) {
+                        const double dz = zs_at(t0 + 32 * c + lane) - nz, g = q * nuc_gaussian(r2 + dz * dz);
+#pragma unroll
+                        for (int e = 0; e < C; ++e)
+                            if (e == c) acc[e] += g;
+                    }
                 }
             }
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
+            for (int c = 0; c < C; ++c) {
                 const int t = t0 + 32 * c + lane;
                 if (t < Pz) phi[t] = acc[c];
+            }
+        };
+        // the row's 32-cell pieces in turns of equal width, at most eight
+        const int pieces = (Pz + 31) >> 5, turns = (pieces + 7) >> 3, width = (pieces + turns - 1) / turns;
+        for (int t0 = 0; t0 < Pz; t0 += 32 * width) {
+            switch (width) {
+                case 8: cells(std::integral_constant<int, 8>{}, t0); break;
+                case 7: cells(std::integral_constant<int, 7>{}, t0); break;
+                case 6: cells(std::integral_constant<int, 6>{}, t0); break;
+                case 5: cells(std::integral_constant<int, 5>{}, t0); break;
+                case 4: cells(std::integral_constant<int, 4>{}, t0); break;
+                default: cells(std::integral_constant<int, 3>{}, t0);
             }
         }
     }
@@ -175,67 +211,91 @@ __global__ void __launch_bounds__(256) k_nuc_field(const NucInst* __restrict__ i
 //
 // zfast: block (ix, iy, jx) writes the nz x (ny nz) sub-block of rows
 // (ix, iy, .) and columns (jx, ., .).  Its entries lie in the ny lines
-// ky = key(iy, jy) of the slice kx = key(ix, jx): as many lines as fit are
-// copied into shared memory (coalesced), and every row is gathered from
-// there and written as one run of 16-byte stores.  (A thread per column and
-// 8-byte stores, each value gathered from the line in L1, where 32 lanes touch
-// up to 20 cache lines: 868 us for the 2.67 GB of a batch of eight, 3.1 TB/s.)
-// Bound: HBM writes.
-constexpr int NUC_LINE_MAX_Z = 64;                    // z axis of the shared-memory route
-constexpr int NUC_LINES_BYTES = 64 * 1024;            // lines held at a time
+// ky = key(iy, jy) of the slice kx = key(ix, jx).  A few lines at a time are read
+// (coalesced) and laid out in shared memory as the output's rows, each value
+// at (lo, hi) and (hi, lo), then copied out row by row in 16-byte stores.
+// Bound: HBM writes.  Batch of eight, 24^3 to 8^3 (2.67 GB): 868 us with a
+// thread per column, 8-byte stores and every value gathered from its line in
+// L1; 778 us gathering it from the line in shared memory; 934 us with two
+// buffers filled by 8-byte cp.async (two copies per value).
+constexpr int NUC_LINE_MAX_Z = 64;         // z axis of the shared-memory route
+constexpr int NUC_ROWS_BYTES = 44 * 1024;  // output rows held at a time: five blocks on an SM
+
+// lines (jy) held at a time, and the row pitch in doubles (6 mod 16: the values
+// of neighbouring keys, on falling diagonals of the square, fall in different banks)
+__host__ __device__ __forceinline__ int nuc_row_pitch(int group, int nz) { return (group * nz + 9) / 16 * 16 + 6; }
+__host__ __device__ __forceinline__ int nuc_line_group(int ny, int nz) {
+    int cap = NUC_ROWS_BYTES / (8 * nz * nz);
+    while (cap > 1 && 8 * nz * nuc_row_pitch(cap, nz) > NUC_ROWS_BYTES) --cap;
+    if (cap < 1) cap = 1;
+    const int turns = (ny + cap - 1) / cap;
+    return (ny + turns - 1) / turns;
+}
+
 __global__ void __launch_bounds__(256) k_nuc_scatter(const NucInst* __restrict__ inst, const double* __restrict__ X,
-                                                     int zfast) {
-    extern __shared__ __align__(16) double lines[];
-    __shared__ uint16_t rank_z[NUC_LINE_MAX_Z * NUC_LINE_MAX_Z];
+                                                     const uint16_t* __restrict__ tables, int zfast) {
+    extern __shared__ __align__(16) double rows[];
     const NucInst& in = inst[blockIdx.y];
     const int nx = in.n[0], ny = in.n[1], nz = in.n[2], nky = in.nk[1], nkz = in.nk[2];
     const int nyz = ny * nz;
     const i64 N = in.N;
     const double* Vk = X + in.x_off;
-    const int items = nx * ny * nx;
+    const uint16_t *rx = tables + in.rk_off[0], *ry = tables + in.rk_off[1], *rz = tables + in.rk_off[2];
     if (zfast && nz <= NUC_LINE_MAX_Z) {
+        const int items = nx * ny * nx;
         if ((int)blockIdx.x >= items) return;
-        for (int e = threadIdx.x; e < nz * nz; e += blockDim.x) {
-            const int a = e / nz, b = e - a * nz;
-            rank_z[e] = (uint16_t)nuc_rank(nz, min(a, b), max(a, b));
-        }
-        const int group = max(1, min(ny, NUC_LINES_BYTES / (8 * nkz)));
+        const int group = nuc_line_group(ny, nz), pitch = nuc_row_pitch(group, nz);
+        const uint16_t* keys = tables + in.key_off[2];
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+        // (the entries of zero factors are never written below)
+        for (int e = threadIdx.x; e < nz * pitch; e += blockDim.x) rows[e] = 0.0;
         for (int item = blockIdx.x; item < items; item += gridDim.x) {
             const int jx = item % nx, r = item / nx, iy = r % ny, ix = r / ny;
-            const double* slice = Vk + (i64)nuc_rank(nx, min(ix, jx), max(ix, jx)) * ((i64)nky * nkz);
+            const int kx = rx[ix * nx + jx];
+            const double* slice = Vk + (i64)kx * ((i64)nky * nkz);
             for (int j0 = 0; j0 < ny; j0 += group) {
                 const int cnt = min(group, ny - j0), cols = cnt * nz;
-                __syncthreads();  // the lines before are consumed
+                __syncthreads();  // the rows before are copied out
                 for (int l = warp; l < cnt; l += warps) {
-                    const int jy = j0 + l;
-                    const double* src = slice + (i64)nuc_rank(ny, min(iy, jy), max(iy, jy)) * nkz;
-                    for (int e = lane; e < nkz; e += 32) lines[l * nkz + e] = __ldg(src + e);
+                    const int ky = kx == NUC_DEAD ? NUC_DEAD : ry[iy * ny + j0 + l];
+                    const bool live = ky != NUC_DEAD;
+                    const double* src = slice + (live ? (i64)ky * nkz : 0);
+                    double* dst = rows + l * nz;
+                    constexpr int V = 5;
+                    for (int e0 = lane; e0 < nkz; e0 += 32 * V) {
+                        double v[V];
+                        int k[V];
+#pragma unroll
+                        for (int u = 0; u < V; ++u) {
+                            const int e = e0 + 32 * u;
+                            v[u] = live && e < nkz ? __ldg(src + e) : 0.0;
+                            k[u] = e < nkz ? __ldg(keys + e) : 0;
+                        }
+#pragma unroll
+                        for (int u = 0; u < V; ++u)
+                            if (e0 + 32 * u < nkz) {
+                                const int lo = k[u] & 0xff, hi = k[u] >> 8;
+                                dst[lo * pitch + hi] = v[u];
+                                dst[hi * pitch + lo] = v[u];
+                            }
+                    }
                 }
                 __syncthreads();
+                double* out0 = in.out + (i64)(ix * ny + iy) * nz * N + (i64)jx * nyz + (i64)j0 * nz;
                 for (int iz = warp; iz < nz; iz += warps) {
-                    const i64 at = ((i64)(ix * ny + iy) * nz + iz) * N + (i64)jx * nyz + (i64)j0 * nz;
-                    double* out = in.out + at;
-                    const uint16_t* rk = rank_z + iz * nz;
-                    auto value = [&](int l, int jz) { return lines[l * nkz + rk[jz]]; };
+                    double* out = out0 + (i64)iz * N;
+                    const double* row = rows + iz * pitch;
                     // (pairs start on 16-byte boundaries: an odd start leaves its first entry alone)
                     const int odd = (int)(((uintptr_t)out >> 3) & 1);
-                    if (odd && lane == 0) __stcs(out, value(0, 0));
-                    int c = odd + 2 * lane, l = c / nz, jz = c - l * nz;
-                    for (; c < cols; c += 64) {
-                        const double v0 = value(l, jz);
-                        if (c + 1 < cols) {
-                            const int l1 = jz + 1 < nz ? l : l + 1, z1 = jz + 1 < nz ? jz + 1 : 0;
-                            __stcs(reinterpret_cast<double2*>(out + c), make_double2(v0, value(l1, z1)));
-                        } else {
-                            __stcs(out + c, v0);
-                        }
-                        jz += 64;
-                        while (jz >= nz) {
-                            jz -= nz;
-                            ++l;
-                        }
+                    if (odd) {
+                        if (lane == 0) __stcs(out, row[0]);
+                        for (int c = 1 + 2 * lane; c + 1 < cols; c += 64)
+                            __stcs(reinterpret_cast<double2*>(out + c), make_double2(row[c], row[c + 1]));
+                    } else {
+                        for (int c = 2 * lane; c + 1 < cols; c += 64)
+                            __stcs(reinterpret_cast<double2*>(out + c), *reinterpret_cast<const double2*>(row + c));
                     }
+                    if (((cols - odd) & 1) && lane == 0 && cols > odd) __stcs(out + cols - 1, row[cols - 1]);
                 }
             }
         }
@@ -244,17 +304,19 @@ __global__ void __launch_bounds__(256) k_nuc_scatter(const NucInst* __restrict__
     // other layouts and long z axes: a thread per column, rows as (iy, iz) loops
     const i64 sy = zfast ? nkz : 1, sz = zfast ? 1 : nky;  // strides of ky and kz in a slice
     for (int pair = blockIdx.x; pair < nx * nx; pair += gridDim.x) {
-        const int ix = pair / nx, jx = pair - ix * nx;
-        const double* slice = Vk + (i64)nuc_rank(nx, min(ix, jx), max(ix, jx)) * ((i64)nky * nkz);
+        const int ix = pair / nx, jx = pair - ix * nx, kx = rx[ix * nx + jx];
+        const double* slice = Vk + (i64)kx * ((i64)nky * nkz);
         double* block = in.out + (i64)ix * nyz * N + (i64)jx * nyz;
         for (int c = threadIdx.x; c < nyz; c += blockDim.x) {
             const int jy = c / nz, jz = c - jy * nz;
             double* col = block + c;
             for (int iy = 0; iy < ny; ++iy) {
-                const double* sl = slice + (i64)nuc_rank(ny, min(iy, jy), max(iy, jy)) * sy;
+                const int ky = kx == NUC_DEAD ? NUC_DEAD : ry[iy * ny + jy];
                 double* out = col + (i64)iy * nz * N;
-                for (int iz = 0; iz < nz; ++iz)
-                    out[(i64)iz * N] = sl[(i64)nuc_rank(nz, min(iz, jz), max(iz, jz)) * sz];
+                for (int iz = 0; iz < nz; ++iz) {
+                    const int kz = ky == NUC_DEAD ? NUC_DEAD : rz[iz * nz + jz];
+                    out[(i64)iz * N] = kz == NUC_DEAD ? 0.0 : slice[ky * sy + kz * sz];
+                }
             }
         }
     }
@@ -270,14 +332,21 @@ __global__ void __launch_bounds__(256) k_nuc_scatter(const NucInst* __restrict__
 // Blocks find their instance in `pre`, the tiles before each instance; the key
 // tiles of one n tile are neighbours, so X comes from L2 after the first.  K
 // runs over the positions from the tile's first key's to its last key's last
-// one, both operands K-contiguous 16-byte copies.
+// one, both operands K-contiguous 16-byte copies, and an 8-key strip takes part
+// only in the chunks it reaches.
 //
-// Bound: the FP64 tensor pipe.  24^3 to 8^3 batch of eight, 6 nuclei: 2.95 ms
-// over full K ranges with 8-byte copies, a launch per instance.
+// Bound: the FP64 tensor pipe, 85% busy on the batch of eight, 24^3 to 8^3,
+// whose three stages take 461 + 410 + 400 us; 2.95 ms over full K ranges with
+// 8-byte copies, a launch per instance.
 template <int STAGE>
 struct NucStageOp {
     static constexpr bool A_KMAJOR = false, B_KMAJOR = false;
     static constexpr int BN = DM_BN;
+    // (short K ranges: a fourth block per SM covers the blocks' starts and ends
+    // better than a third pipeline stage, 5% on each stage; 32-column tiles at
+    // six blocks 4% slower)
+    static constexpr int STAGES = 2, MIN_BLOCKS = 4;
+    static constexpr int SKIP = SKIP_M;
     static constexpr int AXIS = 2 - STAGE;
     const NucInst* inst;
     const int* pre;  // ni + 1 tile counts
@@ -291,6 +360,7 @@ struct NucStageOp {
         int mvalid, nvalid, nk;
         int k0, kend;
         int pitch;
+        int first, last;  // positions that strip (lane & 7) reaches
         i64 ldy;
         const double* a;
         const double* b;
@@ -315,12 +385,18 @@ struct NucStageOp {
         b.nvalid = min(BN, rows - n0);
         b.pitch = in.P[AXIS];
         b.kend = in.U[AXIS];
-        b.k0 = 0;
-        if (in.band) {
+        // the positions that each 8-key strip reaches (its first key's first to
+        // its last key's last), a strip per lane; empty strips reach none
+        const int strip = threadIdx.x & 7, r0 = 8 * strip;
+        b.first = 0;
+        b.last = r0 < b.mvalid ? b.kend - 1 : -1;
+        if (in.band && r0 < b.mvalid) {
             const int* ks = kstart + in.ks_off[AXIS] + m0;
-            b.k0 = ks[0] & ~3;
-            b.kend = min(b.kend, ks[b.mvalid - 1] + in.band);
+            b.first = __ldg(&ks[r0]);
+            b.last = min(b.kend, __ldg(&ks[min(r0 + 7, b.mvalid - 1)]) + in.band) - 1;
         }
+        b.k0 = __shfl_sync(0xffffffffu, b.first, 0) & ~3;
+        b.kend = __reduce_max_sync(0xffffffffu, b.last) + 1;
         b.nk = (b.kend - b.k0 + DM_BK - 1) / DM_BK;
         b.ldy = rows;
         const double* x = STAGE == 0 ? Xb + in.x_off : STAGE == 1 ? Hb + in.h_off : H2b + in.h2_off;
@@ -329,6 +405,10 @@ struct NucStageOp {
         b.b = x + (i64)n0 * b.pitch + b.k0;
         b.y = y + (i64)m0 * b.ldy + n0;
         return true;
+    }
+    __device__ void live_chunks(const Block& b, int, int& first, int& last) const {
+        first = (b.first - b.k0) / DM_BK;  // (thread t asks for strip t)
+        last = b.last < b.first ? -1 : (b.last - b.k0) / DM_BK;
     }
     __device__ void a_init(const Block&, AState&) const {}
     __device__ void b_init(const Block&, BState&) const {}
@@ -507,9 +587,11 @@ static void ensure_streams(int device, int n) {
     t_ring.ensure(device, n);
 }
 
+static_assert(8 * NUC_LINE_MAX_Z * ((NUC_LINE_MAX_Z + 9) / 16 * 16 + 6) <= NUC_ROWS_BYTES, "a line of the longest z axis fits");
+
 // kernel attributes: shared memory above the 48 KB default
 static void nuc_prepare() {
-    GLI_CUDA(cudaFuncSetAttribute(k_nuc_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, NUC_LINES_BYTES));
+    GLI_CUDA(cudaFuncSetAttribute(k_nuc_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, NUC_ROWS_BYTES));
 }
 
 // Queues one chunk of instances, dealt over `pipes` pipelines (largest first,
@@ -518,8 +600,8 @@ static void nuc_prepare() {
 // tensor-core products per instance when `sliced`, else one FP64 tensor-core
 // launch per stage) and the scatter.
 static void run_chunk(const std::vector<NucHost>& hosts, const double* F, int nf, int nb, const int* coords,
-                      const double* npos, const double* ncharge, bool sliced, int pipes, int num_sms, int* err,
-                      cudaStream_t s) {
+                      const double* npos, const double* ncharge, const uint16_t* tables, bool sliced, int pipes, int num_sms,
+                      int* err, cudaStream_t s) {
     const int ni = (int)hosts.size();
     pipes = std::min(pipes, ni);
     std::vector<int> order(ni);
@@ -587,14 +669,13 @@ static void run_chunk(const std::vector<NucHost>& hosts, const double* F, int nf
             const bool by_lines = !sliced && in.n[2] <= NUC_LINE_MAX_Z;
             max_items = std::max(max_items, (i64)in.n[0] * in.n[0] * (by_lines ? in.n[1] : 1));
             if (by_lines) {
-                const int line = 8 * in.nk[2], held = std::max(1, std::min(in.n[1], NUC_LINES_BYTES / line));
-                lines = std::max(lines, line * held);
+                lines = std::max(lines, 8 * in.n[2] * nuc_row_pitch(nuc_line_group(in.n[1], in.n[2]), in.n[2]));
             }
         }
         k_nuc_weights<<<dim3((unsigned)((max_p + 127) / 128), (unsigned)max_nk, (unsigned)(3 * cnt)), 128, 0, st>>>(
-            di, F, nf, nb, coords, W.p, ks.p);
+            di, F, nf, nb, coords, tables, W.p, ks.p);
         GLI_CHECK_LAUNCH();
-        const unsigned fb = (unsigned)std::min<i64>((max_rows + 7) / 8, std::max<i64>(1, (i64)num_sms * 16));
+        const unsigned fb = (unsigned)std::min<i64>((max_rows + 7) / 8, std::max<i64>(1, (i64)num_sms * NUC_FIELD_BLOCKS));
         k_nuc_field<<<dim3(fb, (unsigned)cnt), 256, 0, st>>>(di, npos, ncharge, X.p);
         GLI_CHECK_LAUNCH();
         if (sliced) {
@@ -609,7 +690,7 @@ static void run_chunk(const std::vector<NucHost>& hosts, const double* F, int nf
             dmma_launch(NucStageOp<2>{di, pr[2], cnt, W.p, ks.p, X.p, H.p, H2.p}, total(2), st);
         }
         k_nuc_scatter<<<dim3((unsigned)std::min<i64>(max_items, (i64)num_sms * 8), (unsigned)cnt), 256, lines, st>>>(
-            di, X.p, sliced ? 0 : 1);
+            di, X.p, tables, sliced ? 0 : 1);
         GLI_CHECK_LAUNCH();
     }
     if (pipes > 1)
@@ -648,13 +729,14 @@ void nuclear_batch_device(const double* h_coeffs, i64 nb, const std::vector<Nucl
     DevBuf<double> b(nb, s), F((i64)L * nf, s);
     GLI_CUDA(cudaMemcpyAsync(b.p, h_coeffs, nb * sizeof(double), cudaMemcpyHostToDevice, s));
     factors_device(b.p, (int)nb, L, F.p, s);
-    DevBuf<int> mmax(1, s);
-    GLI_CUDA(cudaMemsetAsync(mmax.p, 0xff, sizeof(int), s));
-    k_mask_factors<<<(unsigned)(((i64)L * nf + 255) / 256), 256, 0, s>>>(F.p, (i64)L * nf, nf, (int)nb, tol, mmax.p);
+    DevBuf<int> reach(2, s);
+    GLI_CUDA(cudaMemsetAsync(reach.p, 0xff, 2 * sizeof(int), s));
+    k_mask_factors<<<(unsigned)(((i64)L * nf + 255) / 256), 256, 0, s>>>(F.p, (i64)L * nf, nf, (int)nb, tol, reach.p);
     GLI_CHECK_LAUNCH();
-    int h_mmax = -1;
-    GLI_CUDA(cudaMemcpyAsync(&h_mmax, mmax.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    int h_reach[2] = {-1, -1};
+    GLI_CUDA(cudaMemcpyAsync(h_reach, reach.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
     GLI_CUDA(cudaStreamSynchronize(s));
+    const int h_mmax = h_reach[0], h_smax = h_reach[1];
     if (h_mmax < 0) {  // every factor below tol
         for (const NuclearJob& j : jobs) {
             const i64 N = (i64)j.axes[0].size() * j.axes[1].size() * j.axes[2].size();
@@ -670,6 +752,34 @@ void nuclear_batch_device(const double* h_coeffs, i64 nb, const std::vector<Nucl
     coords.reserve(total_coords);
     std::vector<double> nuc((size_t)(4 * total_nuclei));  // positions, then charges
     i64 nuc_at = 0;
+    // key tables, one per axis length (and gap of a two-point list)
+    std::vector<uint16_t> tables;
+    struct AxisTable {
+        int rk_off, key_off, nk;
+    };
+    std::map<std::pair<int, int>, AxisTable> axis_tables;
+    auto axis_table = [&](const std::vector<int>& list) {
+        const int n = (int)list.size();
+        const bool run = list.back() - list.front() == n - 1;
+        const std::pair<int, int> id{n, run ? 1 : n == 2 ? list[1] - list[0] : -(int)axis_tables.size() - 1};
+        auto it = axis_tables.find(id);
+        if (it != axis_tables.end()) return it->second;
+        AxisTable t{(int)tables.size(), 0, 0};
+        tables.resize(tables.size() + (size_t)n * n, NUC_DEAD);
+        std::vector<uint16_t> keys;
+        for (int sum = 0; sum <= 2 * (n - 1); ++sum)
+            for (int lo = std::max(0, sum - (n - 1)); 2 * lo <= sum; ++lo) {
+                const int hi = sum - lo;
+                if (list[hi] - list[lo] > h_smax) continue;
+                tables[t.rk_off + lo * n + hi] = tables[t.rk_off + hi * n + lo] = (uint16_t)keys.size();
+                keys.push_back((uint16_t)(lo | hi << 8));
+            }
+        t.key_off = (int)tables.size();
+        t.nk = (int)keys.size();
+        tables.insert(tables.end(), keys.begin(), keys.end());
+        axis_tables[id] = t;
+        return t;
+    };
     for (i64 k = 0; k < ni; ++k) {
         const NuclearJob& j = jobs[k];
         NucInst& in = hosts[k].d;
@@ -681,7 +791,10 @@ void nuclear_batch_device(const double* h_coeffs, i64 nb, const std::vector<Nucl
             in.u0[a] = 6 * j.axes[a].front() - h_mmax;
             in.U[a] = 6 * (j.axes[a].back() - j.axes[a].front()) + 2 * h_mmax + 1;
             in.P[a] = (int)nuc_even(in.U[a]);
-            in.nk[a] = in.n[a] * (in.n[a] + 1) / 2;
+            const AxisTable t = axis_table(j.axes[a]);
+            in.nk[a] = t.nk;
+            in.rk_off[a] = t.rk_off;
+            in.key_off[a] = t.key_off;
             // the keys' order (by the sum of their positions in the list) is by
             // coordinate sum where the list is a run or holds at most two points
             const int span = j.axes[a].back() - j.axes[a].front();
@@ -717,16 +830,18 @@ void nuclear_batch_device(const double* h_coeffs, i64 nb, const std::vector<Nucl
         }
         chunks.push_back({start, ni});
     }
-    // one upload: nuclei, then coordinates
-    const size_t nbytes = nuc.size() * sizeof(double);
-    std::vector<char> up(nbytes + coords.size() * sizeof(int));
+    // one upload: nuclei, coordinates, key tables
+    const size_t nbytes = nuc.size() * sizeof(double), cbytes = coords.size() * sizeof(int);
+    std::vector<char> up(nbytes + cbytes + tables.size() * sizeof(uint16_t));
     memcpy(up.data(), nuc.data(), nbytes);
-    memcpy(up.data() + nbytes, coords.data(), coords.size() * sizeof(int));
+    memcpy(up.data() + nbytes, coords.data(), cbytes);
+    memcpy(up.data() + nbytes + cbytes, tables.data(), tables.size() * sizeof(uint16_t));
     DevBuf<char> d_up(up.size(), s);
     GLI_CUDA(cudaMemcpyAsync(d_up.p, up.data(), up.size(), cudaMemcpyHostToDevice, s));
     const double* d_npos = reinterpret_cast<const double*>(d_up.p);
     const double* d_nq = d_npos + 3 * total_nuclei;
     const int* d_coords = reinterpret_cast<const int*>(d_up.p + nbytes);
+    const uint16_t* d_tables = reinterpret_cast<const uint16_t*>(d_up.p + nbytes + cbytes);
     DevBuf<int> err;
     if (form == FORM_MIXED) {
         err.alloc(1, s);
@@ -771,7 +886,7 @@ void nuclear_batch_device(const double* h_coeffs, i64 nb, const std::vector<Nucl
         auto run = [&](int cand) {
             const bool sliced = cand >= 16;
             const int nstreams = cand % 16;
-            run_chunk(part, F.p, nf, (int)nb, d_coords, d_npos, d_nq, sliced, nstreams, ctx.num_sms, err.p, s);
+            run_chunk(part, F.p, nf, (int)nb, d_coords, d_npos, d_nq, d_tables, sliced, nstreams, ctx.num_sms, err.p, s);
         };
         std::vector<int> cands = part.size() == 1 ? std::vector<int>{1} : std::vector<int>{1, 2, 4, 8};
         if (form == FORM_MIXED)
