@@ -18,8 +18,8 @@
 // Stage A runs over the distinct s = u^2 + v^2 (H depends on u, v only through
 // s); stage C is a per-class warp dot product, or -- when the (pair, key)
 // combinations are few against the classes -- one small GEMM plus a gather.
+#include <limits.h>
 #include <math.h>
-
 #include <stdlib.h>
 #include <string.h>
 
@@ -604,65 +604,92 @@ __global__ void k_pair_lists(i64 words, int nk, const uint32_t* __restrict__ bit
 }
 
 // ---------------------------------------------------------------------------
+// Weight rows are banded: key k's are nonzero on the positions reach[k] only
+// (ERIDA 129^3: 161 of 465), and a class reads only part of the stages' tables:
+//   - its C key is the largest, so a pair of A key a is read at the positions
+//     that any key from a on reaches (from[a]);
+//   - its B key is the smallest, so H[a] is read at v that any key up to a
+//     reaches (upto[a]), and u in from[a]: at s = u^2 + v^2 between the squares
+//     of their ends.
+// So a tile's K loop covers the union of its keys' reaches, an 8-key strip
+// takes part only in the chunks it reaches (SKIP_N), and tiles that no class
+// reads are not computed.  Entries that are not computed are never read: the
+// later stages take their operands as zero outside the ranges above.
+// (ERIDA 129^3, tol 1e-16: stages A, B and the product take 148 + 101 + 21 us;
+// 394 + 198 + 36 us over all positions, with the pairs as 64-row tiles.)
+
+// The K chunks of a block whose strips reach the positions [first, last] (one
+// strip per lane; last < first: none), for part z of P: t0, t1 and nk
+struct KRange {
+    int t0, t1, nk;
+};
+__device__ __forceinline__ KRange k_range(int first, int last, int z, int P) {
+    const int lo = __reduce_min_sync(0xffffffffu, last < first ? INT_MAX : first);
+    const int hi = __reduce_max_sync(0xffffffffu, last < first ? -1 : last);
+    KRange r{0, 0, 0};
+    if (hi < lo) return r;
+    const int base = lo / DM_BK * DM_BK, chunks = (hi + 1 - base + DM_BK - 1) / DM_BK;
+    const int c0 = chunks * z / P, c1 = chunks * (z + 1) / P;
+    r.t0 = base + c0 * DM_BK;
+    r.t1 = min(hi + 1, base + c1 * DM_BK);
+    r.nk = c1 - c0;
+    return r;
+}
+__device__ __forceinline__ void reach_chunks(int reach_first, int reach_last, const KRange& k, int& first, int& last) {
+    first = reach_first <= k.t0 ? 0 : (reach_first - k.t0) / DM_BK;
+    last = reach_last < k.t0 || reach_last < reach_first ? -1 : (reach_last - k.t0) / DM_BK;
+}
+
 // stage A: H[a][j] = sum_t W[aKey[a]][t] T[S[j] + t^2]
 // H depends on (u, v) only through s = u^2 + v^2, so it is evaluated once per
 // distinct s (S, ascending; 10,823 values instead of 31,329 (u, v) at U = 177).
 // As a GEMM: C[j][a] = sum_t G[j][t] W[aKey[a]][t] with G[j][t] = T[S[j] + t^2]
 // gathered tile by tile into shared memory (consecutive j read neighbouring
 // table entries, so a warp's 32 gathers touch a few cache lines), and the
-// FP64 tensor-core tiles of dmma.cuh.  blockIdx.z selects a chunk of t: the
-// split blocks of small problems sum their partial tiles in a cluster; the
-// 144-column tiles split only the m tiles of a partial last wave, in two
-// halves of t (dm_split_store).
-template <int BN_>
+// FP64 tensor-core tiles of dmma.cuh.  blockIdx.z selects a part of the K
+// chunks: the split blocks of small problems sum their partial tiles in a
+// cluster.  `prune` (stage B in FP64): tiles outside the s that any class of
+// their keys reads are left out.
+// DEEP = false: two pipeline stages and four blocks per SM, for grids of
+// several waves.
+template <int BN_, bool DEEP>
 struct StageAOp {
     static constexpr bool A_KMAJOR = true, B_KMAJOR = false;
     static constexpr int BN = BN_;
-    static constexpr int STAGES = BN_ > 80 ? 2 : DM_STAGES;  // 144 columns: three blocks per SM
+    static constexpr int SKIP = SKIP_N;
+    static constexpr int STAGES = DEEP ? 3 : 2, MIN_BLOCKS = DEEP ? 3 : 4;
     static constexpr int NB = BN / 16;  // B element pairs per thread (rows of W are contiguous in t)
-    // W row offsets: 32-bit for the 144-column tiles, whose registers are
-    // scarce (aKey * Up < 2^31 with at most 8,192 keys)
-    using Off = std::conditional_t<(BN_ > 80), int, i64>;
     const double* W;
     const double* T;
     const int* S;
     const int* aKey;
     const PlanCounts* cnt;
-    int nS, U, Up, t_chunk;
-    i64 part_stride;
+    const int2 *reach, *from, *upto;  // null: every position, every tile
+    int nS, U, Up, prune;
     double* H;
-    // tail split (k_dmma's dm_split_store; ws null: none): blocks from nfull on
-    // are the two K halves of the m tiles nfull, nfull + 1, ...
-    int nfull = 0;
-    double* ws = nullptr;
-    unsigned* tickets = nullptr;
-    static constexpr bool TAIL_SPLIT = true;
-    // trusted replays (restore_valid non-null; 64- and 80-column tiles): the
-    // first block restores the kept plan's counts into cnt for the later
-    // kernels (k_restore_plan's work, one launch fewer), and every block reads
-    // the kept counts
+    // trusted replays (restore_valid non-null): the first block restores the
+    // kept plan's counts into cnt for the later kernels (k_restore_plan's work,
+    // one launch fewer), and every block reads the kept counts
     const int* restore_valid = nullptr;
     const PlanCounts* restore_from = nullptr;
     EvalStatus* restore_to = nullptr;
-    __device__ int split_half() const {
-        return ws && (int)blockIdx.x >= nfull ? (int)((blockIdx.x - nfull) & 1) : -1;
-    }
-    __device__ int split_slot() const { return (int)(blockIdx.x - nfull) >> 1; }
     struct Block {
         int mvalid, nvalid, nk;
-        int m0, n0, t0, t1;
-        double* H;
+        int m0, n0;
+        int first, last;  // positions that strip `lane` reaches
+        KRange k;
     };
     struct AState {
         const double* base;  // T + S[j] of this thread's row j
         bool ok;
     };
     struct BState {
-        Off off[NB];  // aKey * Up of this thread's rows, -1 past nA
+        const uint16_t* live;
+        int off[NB];  // aKey * Up of this thread's rows (below 2^31 with at most 8,192 keys), -1 past nA
     };
     __device__ bool begin(Block& b) const {
         const PlanCounts* c = cnt;
-        if (BN_ <= 80 && restore_valid) {
+        if (restore_valid) {
             const bool valid = *restore_valid != 0;
             if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0)
                 restore_status(valid, restore_from, restore_to);
@@ -672,21 +699,37 @@ struct StageAOp {
         const int nA = (int)c->nA;
         b.n0 = blockIdx.y * BN;
         if (b.n0 >= nA) return false;  // grids are sized by a bound on nA
-        const int half = split_half();
-        b.m0 = (half < 0 ? (int)blockIdx.x : nfull + split_slot()) * DM_BM;
+        b.m0 = blockIdx.x * DM_BM;
         b.mvalid = min(DM_BM, nS - b.m0);
         b.nvalid = min(BN, nA - b.n0);
-        if (half < 0) {
-            b.t0 = blockIdx.z * t_chunk;
-            b.t1 = min(U, b.t0 + t_chunk);
-        } else {  // (the host splits only K ranges of at least two chunks)
-            const int hc = ((U + DM_BK - 1) / DM_BK + 1) / 2 * DM_BK;
-            b.t0 = half ? hc : 0;
-            b.t1 = half ? U : min(U, hc);
+        const int lane = threadIdx.x & 31;
+        b.first = INT_MAX;
+        b.last = -1;
+        bool read = !reach;  // some class reads this tile
+        if (!reach && 8 * lane < b.nvalid) {
+            b.first = 0;
+            b.last = U - 1;
         }
-        b.nk = (b.t1 - b.t0 + DM_BK - 1) / DM_BK;
-        b.H = H + (i64)blockIdx.z * part_stride;
-        return b.nk > 0;
+        const int s0 = prune ? S[b.m0] : 0, s1 = prune ? S[b.m0 + b.mvalid - 1] : 0;
+        if (reach && lane < BN / 8)
+            for (int e = 8 * lane; e < min(8 * lane + 8, b.nvalid); ++e) {
+                const int key = __ldg(&aKey[b.n0 + e]);
+                const int2 r = __ldg(&reach[key]);
+                if (prune) {
+                    const int2 u = __ldg(&from[key]), v = __ldg(&upto[key]);
+                    if (u.y < u.x || v.y < v.x || s1 < u.x * u.x + v.x * v.x || s0 > u.y * u.y + v.y * v.y) continue;
+                }
+                read = true;
+                b.first = min(b.first, r.x);
+                b.last = max(b.last, r.y);
+            }
+        if (!__any_sync(0xffffffffu, read)) return false;
+        b.k = k_range(b.first, b.last, blockIdx.z, gridDim.z);
+        b.nk = b.k.nk;
+        return true;
+    }
+    __device__ void live_chunks(const Block& b, int, int& first, int& last) const {
+        reach_chunks(b.first, b.last, b.k, first, last);  // (thread t asks for strip t)
     }
     __device__ void a_init(const Block& b, AState& st) const {
         const int r = dm_kmajor_row(threadIdx.x);
@@ -697,8 +740,8 @@ struct StageAOp {
         const int r = dm_kmajor_row(threadIdx.x);
 #pragma unroll
         for (int q = 0; q < DM_ELEMS; ++q) {
-            const int k = dm_kmajor_k(threadIdx.x, q), t = b.t0 + kc * DM_BK + k;
-            const bool v = st.ok && t < b.t1;
+            const int k = dm_kmajor_k(threadIdx.x, q), t = b.k.t0 + kc * DM_BK + k;
+            const bool v = st.ok && t < b.k.t1;
             dm_cp8(tile + dm_kmajor_at(r, k), v ? st.base + t * t : T, v);
         }
     }
@@ -706,124 +749,152 @@ struct StageAOp {
 #pragma unroll
         for (int q = 0; q < NB; ++q) {
             const int r = dm_pair_row(threadIdx.x, q);
-            st.off[q] = r < b.nvalid ? (Off)aKey[b.n0 + r] * (Off)Up : (Off)-1;
+            st.off[q] = r < b.nvalid ? aKey[b.n0 + r] * Up : -1;
         }
     }
     // pairs (t, t + 1), t even: W rows start at multiples of Up (a multiple of
     // 4) and chunks at multiples of 16, so every pair is 16-byte aligned
     __device__ void b_issue(const Block& b, BState& st, int kc, double* tile) const {
-        const int k = dm_pair_k(threadIdx.x), t = b.t0 + kc * DM_BK + k;
-        const int bytes = dm_pair_bytes(t, b.t1);
+        const int k = dm_pair_k(threadIdx.x), t = b.k.t0 + kc * DM_BK + k;
+        const int bytes = dm_pair_bytes(t, b.k.t1);
+        const unsigned live = st.live[kc];
 #pragma unroll
         for (int q = 0; q < NB; ++q) {
+            if (!dm_live(live, q)) continue;
             const int n = st.off[q] >= 0 ? bytes : 0;
             dm_cp16(tile + dm_rowmajor_at(dm_pair_row(threadIdx.x, q), k), n ? W + st.off[q] + t : W, n);
         }
     }
     __device__ void store(const Block& b, int m, int n, double v0, double v1) const {
         if (m >= b.mvalid) return;
-        double* h = b.H + (i64)(b.n0 + n) * nS + b.m0 + m;
+        double* h = H + (i64)(b.n0 + n) * nS + b.m0 + m;
         if (n < b.nvalid) h[0] = v0;
         if (n + 1 < b.nvalid) h[nS] = v1;
     }
 };
 
 // ---------------------------------------------------------------------------
-// stage B: H2[p][u] = sum_v W[pairB[p]][v] Hf[a(p)][v][u],  Hf[a][v][u] = H[a][sidx[v U + u]]
-// Pairs are ordered by their A key and cut into tiles of 64 pairs of one A key
-// (k_pair_tiles); block (pair tile, 64 u, chunk of v) is one GEMM tile with the
-// pair weights as A (rows read along v) and the expanded H of the tile's A key
-// as B, gathered through sidx straight from H (no expanded copy in memory).
-// The sidx values of the next chunk are loaded one chunk ahead, so the
-// dependent gathers do not wait on them.
-// DEEP = false: two pipeline stages and four blocks per SM (at most 128
-// registers), for grids of several waves (ERIDA 129^3: 199 against 213 us);
-// small grids keep three stages (ERIDA 33^3: 20.5 against 22.5 us)
-template <bool DEEP>
+// stage B: H2[p][u] = sum_v W[pairB[p]][v] H[a(p)][sidx[v U + u]]
+// Pairs are ordered by their A key (their host), then their B key.  A block
+// takes 64 u of one host's pairs, a column tile of them: the host's expanded H
+// is the A operand, gathered through sidx straight from H (once per column
+// tile of pairs; with the pairs as 64-row tiles it was gathered for every tile,
+// and the hosts had to be chosen to fill the tiles), the pair weights the B
+// operand.  u runs over from[a], v over what the pairs' B keys reach.  The sidx
+// values of the next chunk are loaded one chunk ahead, so the dependent gathers
+// do not wait on them.
+template <int BN_, bool DEEP>
 struct StageBOp {
-    static constexpr bool A_KMAJOR = false, B_KMAJOR = true;
-    static constexpr int BN = DM_BN;
+    static constexpr bool A_KMAJOR = true, B_KMAJOR = false;
+    static constexpr int BN = BN_;
+    static constexpr int SKIP = SKIP_N;
     static constexpr int STAGES = DEEP ? 3 : 2, MIN_BLOCKS = DEEP ? 3 : 4;
+    static constexpr int NB = BN / 16;
     const double* W;
     const double* H;
     const int* sidx;
-    const int* rowKey;   // weight key of each tile row
-    const int* rowPair;  // H2 row (pair id) of each tile row
-    const int* tile_batch;
+    const int* aKey;
+    const int* pairB;
+    const int* tile_batch;  // host, first pair and pair count of each column tile
     const int* tile_col0;
     const int* tile_ncols;
-    int nS, U, Up, v_chunk;
-    i64 part_stride;
+    const int2 *reach, *from, *upto;  // null: every position
+    int nS, U, Up;
     double* H2;
     struct Block {
         int mvalid, nvalid, nk;
-        int p0, u0, v0, v1;
-        const double* h;  // H row of the tile's A key
-        double* H2;
+        int p0, u0;
+        int2 u, v;        // positions at which the host's H is computed and read
+        int first, last;  // positions that strip `lane` reaches
+        KRange k;
+        const double* h;  // H row of the host
     };
     struct AState {
-        i64 off[DM_BM / 16];  // weight key * Up of this thread's rows, -1 past the tile
-    };
-    struct BState {
         int sv[DM_ELEMS];  // sidx of the next chunk's elements (-1: zero fill)
     };
+    struct BState {
+        const uint16_t* live;
+        int off[NB];
+    };
     __device__ bool begin(Block& b) const {
-        const int tile = blockIdx.x;
-        b.mvalid = tile_ncols[tile];
-        if (b.mvalid <= 0) return false;  // tiles past the last one
-        b.p0 = tile_col0[tile];
-        b.h = H + (i64)tile_batch[tile] * nS;
-        b.u0 = blockIdx.y * DM_BN;
-        b.nvalid = min(DM_BN, U - b.u0);
-        b.v0 = blockIdx.z * v_chunk;
-        b.v1 = min(U, b.v0 + v_chunk);
-        b.nk = (b.v1 - b.v0 + DM_BK - 1) / DM_BK;
-        b.H2 = H2 + (i64)blockIdx.z * part_stride;
-        return b.nk > 0;
+        b.nvalid = tile_ncols[blockIdx.x];
+        if (b.nvalid <= 0) return false;  // tiles past the last one
+        b.p0 = tile_col0[blockIdx.x];
+        const int host = tile_batch[blockIdx.x];
+        const int lane = threadIdx.x & 31;
+        b.u = b.v = make_int2(0, U - 1);
+        if (reach) {
+            const int key = aKey[host];
+            b.u = __ldg(&from[key]);
+            b.v = __ldg(&upto[key]);
+        }
+        b.u0 = (b.u.x & ~7) + blockIdx.y * DM_BM;
+        b.mvalid = min(DM_BM, b.u.y + 1 - b.u0);
+        if (b.mvalid <= 0) return false;
+        b.h = H + (i64)host * nS;
+        b.first = INT_MAX;
+        b.last = -1;
+        if (!reach && 8 * lane < b.nvalid) {
+            b.first = 0;
+            b.last = U - 1;
+        }
+        if (reach && lane < BN / 8)
+            for (int e = 8 * lane; e < min(8 * lane + 8, b.nvalid); ++e) {
+                const int2 r = __ldg(&reach[pairB[b.p0 + e]]);
+                b.first = min(b.first, r.x);
+                b.last = max(b.last, r.y);
+            }
+        b.k = k_range(b.first, b.last, blockIdx.z, gridDim.z);
+        b.nk = b.k.nk;
+        return true;
     }
-    __device__ void a_init(const Block& b, AState& st) const {
+    __device__ void live_chunks(const Block& b, int, int& first, int& last) const {
+        reach_chunks(b.first, b.last, b.k, first, last);
+    }
+    __device__ void a_load(const Block& b, AState& st, int kc) const {
+        const int r = dm_kmajor_row(threadIdx.x), u = b.u0 + r;
+        const bool row = r < b.mvalid && u >= b.u.x;
 #pragma unroll
-        for (int q = 0; q < DM_BM / 16; ++q) {
+        for (int q = 0; q < DM_ELEMS; ++q) {
+            const int v = b.k.t0 + kc * DM_BK + dm_kmajor_k(threadIdx.x, q);
+            st.sv[q] = (row && v >= b.v.x && v <= b.v.y && v < b.k.t1) ? __ldg(&sidx[v * U + u]) : -1;
+            if (!dcheck(st.sv[q] < nS, 2, st.sv[q])) st.sv[q] = -1;
+        }
+    }
+    __device__ void a_init(const Block& b, AState& st) const { a_load(b, st, 0); }
+    __device__ void a_issue(const Block& b, AState& st, int kc, double* tile) const {
+        const int r = dm_kmajor_row(threadIdx.x);
+#pragma unroll
+        for (int q = 0; q < DM_ELEMS; ++q) {
+            const int sv = st.sv[q];
+            dm_cp8(tile + dm_kmajor_at(r, dm_kmajor_k(threadIdx.x, q)), sv >= 0 ? b.h + sv : b.h, sv >= 0);
+        }
+        if (kc + 1 < b.nk) a_load(b, st, kc + 1);
+    }
+    __device__ void b_init(const Block& b, BState& st) const {
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
             const int r = dm_pair_row(threadIdx.x, q);
-            st.off[q] = r < b.mvalid ? (i64)rowKey[b.p0 + r] * Up : -1;
+            st.off[q] = r < b.nvalid ? pairB[b.p0 + r] * Up : -1;
         }
     }
     // pairs (v, v + 1), v even: 16-byte aligned in the W rows
-    __device__ void a_issue(const Block& b, AState& st, int kc, double* tile) const {
-        const int k = dm_pair_k(threadIdx.x), v = b.v0 + kc * DM_BK + k;
-        const int bytes = dm_pair_bytes(v, b.v1);
+    __device__ void b_issue(const Block& b, BState& st, int kc, double* tile) const {
+        const int k = dm_pair_k(threadIdx.x), v = b.k.t0 + kc * DM_BK + k;
+        const int bytes = dm_pair_bytes(v, b.k.t1);
+        const unsigned live = st.live[kc];
 #pragma unroll
-        for (int q = 0; q < DM_BM / 16; ++q) {
+        for (int q = 0; q < NB; ++q) {
+            if (!dm_live(live, q)) continue;
             const int n = st.off[q] >= 0 ? bytes : 0;
             dm_cp16(tile + dm_rowmajor_at(dm_pair_row(threadIdx.x, q), k), n ? W + st.off[q] + v : W, n);
         }
     }
-    __device__ void b_load(const Block& b, BState& st, int kc) const {
-        const int n = dm_kmajor_row(threadIdx.x), u = b.u0 + n;
-#pragma unroll
-        for (int q = 0; q < DM_ELEMS; ++q) {
-            const int v = b.v0 + kc * DM_BK + dm_kmajor_k(threadIdx.x, q);
-            st.sv[q] = (n < b.nvalid && v < b.v1) ? __ldg(&sidx[v * U + u]) : -1;
-            if (!dcheck(st.sv[q] < nS, 2, st.sv[q])) st.sv[q] = -1;
-        }
-    }
-    __device__ void b_init(const Block& b, BState& st) const { b_load(b, st, 0); }
-    __device__ void b_issue(const Block& b, BState& st, int kc, double* tile) const {
-        const int n = dm_kmajor_row(threadIdx.x);
-#pragma unroll
-        for (int q = 0; q < DM_ELEMS; ++q) {
-            const int sv = st.sv[q];
-            dm_cp8(tile + dm_kmajor_at(n, dm_kmajor_k(threadIdx.x, q)), sv >= 0 ? b.h + sv : b.h, sv >= 0);
-        }
-        if (kc + 1 < b.nk) b_load(b, st, kc + 1);
-    }
     __device__ void store(const Block& b, int m, int n, double v0, double v1) const {
         if (m >= b.mvalid) return;
-        double* h2 = b.H2 + (i64)__ldg(&rowPair[b.p0 + m]) * Up + b.u0 + n;
-        if (n + 1 < b.nvalid)
-            *reinterpret_cast<double2*>(h2) = make_double2(v0, v1);  // Up, u0 and n are even
-        else if (n < b.nvalid)
-            h2[0] = v0;
+        double* h2 = H2 + (i64)(b.p0 + n) * Up + b.u0 + m;
+        if (n < b.nvalid) h2[0] = v0;
+        if (n + 1 < b.nvalid) h2[Up] = v1;
     }
 };
 
@@ -889,7 +960,7 @@ __device__ inline bool choice_runs(int choice, const PlanCounts* c, i64 m) {
 // per class: one warp per class (its pair and C key found from the packed
 // keys), lanes stride over u, shuffle reduction
 __global__ void __launch_bounds__(256) k_stage_c(const double* __restrict__ W, const double* __restrict__ H2,
-                                                  const uint64_t* __restrict__ keys, ClassDecode dec,
+                                                  const int2* __restrict__ reach, const uint64_t* __restrict__ keys, ClassDecode dec,
                                                   const int64_t* __restrict__ idx, int nk,
                                                   const uint32_t* __restrict__ pairBits,
                                                   const uint64_t* __restrict__ pairPre, i64 m, int U, int Up,
@@ -907,8 +978,11 @@ __global__ void __launch_bounds__(256) k_stage_c(const double* __restrict__ W, c
             const i64 pid = pair_id(pairBits, pairPre, (i64)k[1] * nk + k[0]);
             const double* w = W + (i64)k[2] * Up;
             const double* h = H2 + pid * Up;
-            if (dcheck(pid < (i64)cnt->nP && k[2] < nk, 4, pid))
-                for (int u = lane; u < U; u += 32) acc = fma(w[u], h[u], acc);
+            if (dcheck(pid < (i64)cnt->nP && k[2] < nk, 4, pid)) {
+                const int2 r = reach ? __ldg(&reach[k[2]]) : make_int2(0, U - 1);  // (H2 is computed where the C key's weights are nonzero)
+                for (int u = (r.x & ~31) + lane; u <= r.y; u += 32)
+                    if (u >= r.x) acc = fma(w[u], h[u], acc);
+            }
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -927,6 +1001,7 @@ template <int BN_>
 struct ProductOp {
     static constexpr bool A_KMAJOR = false, B_KMAJOR = false;
     static constexpr int BN = BN_;
+    static constexpr int SKIP = SKIP_N;
     static constexpr int STAGES = 2, MIN_BLOCKS = 4;  // four blocks per SM: a grid under a wave splits u in three
     static constexpr int NB = BN / 16;  // B element pairs per thread
     const double* H2;
@@ -936,73 +1011,97 @@ struct ProductOp {
     const int* aKey;
     const uint64_t* kid;  // dense id of each used key
     const PlanCounts* cnt;
+    const int2 *reach, *from;
     i64 m;
-    int choice, U, Up, ldq, u_chunk;
+    int choice, U, Up, ldq;
     double* Q;
     unsigned long long* products;  // count of the products computed (one add per tile)
     struct Block {
         int mvalid, nvalid, nk;
-        int m0, n0, u0, u1;
-        double* Q;
+        int m0, n0;
+        int first, last;  // positions that strip `lane` reaches
+        KRange k;
     };
     struct AState {
-        i64 off[DM_BM / 16];
+        i64 off[DM_BM / 16];  // row * Up, -1 past the tile
+        int lo[DM_BM / 16], hi[DM_BM / 16];  // positions of the row that are computed (lo even)
     };
     struct BState {
-        i64 off[NB];
+        const uint16_t* live;
+        int off[NB];
     };
     __device__ bool begin(Block& b) const {
         if (!choice_runs(choice, cnt, m)) return false;
         b.m0 = blockIdx.x * DM_BM;
         b.mvalid = min(DM_BM, (int)cnt->nP - b.m0);
         if (b.mvalid <= 0) return false;
-        b.n0 = (int)kid[aKey[pairA[b.m0]]] + blockIdx.y * BN;
+        const int key0 = aKey[pairA[b.m0]], lane = threadIdx.x & 31;
+        b.n0 = (int)kid[key0] + blockIdx.y * BN;
         b.nvalid = min(BN, (int)cnt->nku - b.n0);
         if (b.nvalid <= 0) return false;
-        b.u0 = blockIdx.z * u_chunk;
-        b.u1 = min(U, b.u0 + u_chunk);
-        b.nk = (b.u1 - b.u0 + DM_BK - 1) / DM_BK;
-        b.Q = Q;
+        b.first = INT_MAX;
+        b.last = -1;
+        if (!reach && 8 * lane < b.nvalid) {
+            b.first = 0;
+            b.last = U - 1;
+        }
+        if (reach && lane < BN / 8)
+            for (int e = 8 * lane; e < min(8 * lane + 8, b.nvalid); ++e) {
+                const int2 r = __ldg(&reach[keyOf[b.n0 + e]]);
+                b.first = min(b.first, r.x);
+                b.last = max(b.last, r.y);
+            }
+        b.k = k_range(b.first, b.last, blockIdx.z, gridDim.z);
+        b.nk = b.k.nk;
         if (threadIdx.x == 0 && blockIdx.z == 0) atomicAdd(products, (unsigned long long)b.mvalid * b.nvalid);
-        return b.nk > 0;
+        return true;
+    }
+    __device__ void live_chunks(const Block& b, int, int& first, int& last) const {
+        reach_chunks(b.first, b.last, b.k, first, last);
     }
     __device__ void a_init(const Block& b, AState& st) const {
 #pragma unroll
         for (int q = 0; q < DM_BM / 16; ++q) {
             const int r = dm_pair_row(threadIdx.x, q);
             st.off[q] = r < b.mvalid ? (i64)(b.m0 + r) * Up : -1;
+            const int2 u = r >= b.mvalid ? make_int2(0, -1)
+                           : reach       ? __ldg(&from[aKey[pairA[b.m0 + r]]])
+                                         : make_int2(0, U - 1);
+            st.lo[q] = u.x;
+            st.hi[q] = u.y;
         }
     }
     __device__ void b_init(const Block& b, BState& st) const {
 #pragma unroll
         for (int q = 0; q < NB; ++q) {
             const int r = dm_pair_row(threadIdx.x, q);
-            st.off[q] = r < b.nvalid ? (i64)keyOf[b.n0 + r] * Up : -1;
+            st.off[q] = r < b.nvalid ? keyOf[b.n0 + r] * Up : -1;
         }
     }
     // pairs (u, u + 1), u even: H2 and W rows start at multiples of Up (a
     // multiple of 4), so every pair is 16-byte aligned
     __device__ void a_issue(const Block& b, AState& st, int kc, double* tile) const {
-        const int k = dm_pair_k(threadIdx.x), u = b.u0 + kc * DM_BK + k;
-        const int bytes = dm_pair_bytes(u, b.u1);
+        const int k = dm_pair_k(threadIdx.x), u = b.k.t0 + kc * DM_BK + k;
 #pragma unroll
         for (int q = 0; q < DM_BM / 16; ++q) {
-            const int n = st.off[q] >= 0 ? bytes : 0;
+            const int n = u >= st.lo[q] ? dm_pair_bytes(u, min(b.k.t1, st.hi[q] + 1)) : 0;
             dm_cp16(tile + dm_rowmajor_at(dm_pair_row(threadIdx.x, q), k), n ? H2 + st.off[q] + u : H2, n);
         }
     }
     __device__ void b_issue(const Block& b, BState& st, int kc, double* tile) const {
-        const int k = dm_pair_k(threadIdx.x), u = b.u0 + kc * DM_BK + k;
-        const int bytes = dm_pair_bytes(u, b.u1);
+        const int k = dm_pair_k(threadIdx.x), u = b.k.t0 + kc * DM_BK + k;
+        const int bytes = dm_pair_bytes(u, b.k.t1);
+        const unsigned live = st.live[kc];
 #pragma unroll
         for (int q = 0; q < NB; ++q) {
+            if (!dm_live(live, q)) continue;
             const int n = st.off[q] >= 0 ? bytes : 0;
             dm_cp16(tile + dm_rowmajor_at(dm_pair_row(threadIdx.x, q), k), n ? W + st.off[q] + u : W, n);
         }
     }
     __device__ void store(const Block& b, int mm, int n, double v0, double v1) const {
         if (mm >= b.mvalid) return;
-        double* q = b.Q + (i64)(b.m0 + mm) * ldq + b.n0 + n;
+        double* q = Q + (i64)(b.m0 + mm) * ldq + b.n0 + n;
         if (n < b.nvalid) q[0] = v0;
         if (n + 1 < b.nvalid) q[1] = v1;
     }
@@ -1263,87 +1362,31 @@ struct PairRows {  // pair p: row W[pairB[p]], placed in the tiles of its A key
     __device__ bool valid(i64 p) const { return p < (i64)cnt->nP; }
 };
 
-// Balanced hosts of a full pair triangle.  A pair's stage-B row is symmetric
-// in its two keys (sum_v sum_t W_b[v] W_a[t] T[u^2 + v^2 + t^2]), so either
-// key's H row can host it.  Hosting by the larger key gives key a a + 1 rows
-// (ragged tiles: 67% full at 129 keys); when every pair {a, b} of n A keys is
-// present the hosts are chosen instead so that most keys fill whole tiles:
-// keys below y = min(n, 2 bn - 1) form a regular tournament (key i hosts its
-// own pair and i + j mod y for j < reg_count(i, y): at most bn rows), and the
-// keys from y up host every pair with a key below y plus a regular tournament
-// among themselves (129 keys: 132 tiles of 64 instead of 195).
-__host__ __device__ __forceinline__ int reg_count(int i, int y) { return (y & 1) ? (y + 1) / 2 : y / 2 + (i < y / 2); }
-__host__ __device__ __forceinline__ int reg_prefix(int i, int y) {  // rows of the members below i
-    if (y & 1) return i * ((y + 1) / 2);
-    const int h = y / 2;
-    return i <= h ? i * (h + 1) : h * (h + 1) + (i - h) * h;
-}
-__host__ __device__ __forceinline__ int bal_count(int h, int n, int y) {
-    return h < y ? reg_count(h, y) : y + reg_count(h - y, n - y);
-}
-__device__ __forceinline__ int bal_offset(int h, int n, int y) {
-    return h < y ? reg_prefix(h, y) : y * (y + 1) / 2 + (h - y) * y + reg_prefix(h - y, n - y);
-}
-// the partner key of host h's j-th row
-__device__ __forceinline__ int bal_partner(int h, int j, int n, int y) {
-    if (h < y) return (h + j) % y;
-    return j < y ? j : y + (h - y + j - y) % (n - y);
-}
-
-// One block: first pair, pair count and first tile of every A key (pairs are
-// ordered by A key), and the tile list of stage B (tiles of bn rows, each in
-// one host A key); tiles past the last one get no columns.  With row lists
-// (rowPair, rowKey: the H2 row and the weight key of each tile row) a full
-// pair triangle of more than bn keys gets balanced hosts; otherwise the rows
-// are the pairs in order, each hosted by its A key.
+// One block: first pair of every A key (pairs are ordered by A key) and the tile
+// list of stage B (tiles of bn pairs, each in one A key); tiles past the last
+// one get no columns.
 // (pairA, pairB and aKey may have been written earlier in the same kernel:
 // plain coherent loads, no __restrict__)
-__device__ void pair_tiles_block(bool first_ready, const int* pairA, const int* pairB, const int* aKey, int nP, int nA, int nku, int bn, int max_tiles,
+__device__ void pair_tiles_block(bool first_ready, const int* pairA, int nP, int nA, int bn, int max_tiles,
                                  int* __restrict__ first, int* __restrict__ tile0, int* __restrict__ tile_batch,
-                                 int* __restrict__ tile_col0, int* __restrict__ tile_ncols, int* __restrict__ rowPair,
-                                 int* __restrict__ rowKey) {
+                                 int* __restrict__ tile_col0, int* __restrict__ tile_ncols) {
     __shared__ int warp_sums[32];
     __shared__ int carry;
     if (threadIdx.x == 0) carry = 0;
-    for (int t = threadIdx.x; t < max_tiles; t += blockDim.x) tile_ncols[t] = 0;
     // every A key has at least one pair, and pairs are sorted by A key: the
     // first pair of each key is where the key changes (unless the caller
     // filled first[] already)
     if (!first_ready)
         for (int p = threadIdx.x; p < nP; p += blockDim.x)
             if (p == 0 || pairA[p] != pairA[p - 1]) first[pairA[p]] = p;
-    const bool balanced = rowPair && nA > bn && nku == nA && (i64)nP == (i64)nA * (nA + 1) / 2;
-    const int y = min(nA, 2 * bn - 1);
-    if (rowPair) {
-        if (balanced) {
-            // host h's rows in stripes of 8 threads
-            for (int item = threadIdx.x; item < nA * 8; item += blockDim.x) {
-                const int h = item >> 3, d = bal_count(h, nA, y), o = bal_offset(h, nA, y);
-                for (int j = item & 7; j < d; j += 8) {
-                    const int g = bal_partner(h, j, nA, y), hi = max(h, g), lo = min(h, g);
-                    rowPair[o + j] = hi * (hi + 1) / 2 + lo;  // the pair id of (hi, lo) in a full triangle
-                    rowKey[o + j] = aKey[g];
-                }
-            }
-        } else {
-            for (int p = threadIdx.x; p < nP; p += blockDim.x) {
-                rowPair[p] = p;
-                rowKey[p] = pairB[p];
-            }
-        }
-    }
+    for (int t = threadIdx.x; t < max_tiles; t += blockDim.x) tile_ncols[t] = 0;
     __syncthreads();
     for (int base = 0; base < nA; base += blockDim.x) {
         const int a = base + threadIdx.x;
         int lo = 0, npairs = 0;
         if (a < nA) {
-            if (balanced) {
-                lo = bal_offset(a, nA, y);
-                npairs = bal_count(a, nA, y);
-            } else {
-                lo = first[a];
-                npairs = (a + 1 < nA ? first[a + 1] : nP) - lo;
-            }
+            lo = first[a];
+            npairs = (a + 1 < nA ? first[a + 1] : nP) - lo;
         }
         const int nt = (npairs + bn - 1) / bn;
         // block exclusive scan of nt
@@ -1380,44 +1423,37 @@ __device__ void pair_tiles_block(bool first_ready, const int* pairA, const int* 
     }
 }
 
-__global__ void __launch_bounds__(1024) k_pair_tiles(const int* __restrict__ pairA, const int* __restrict__ pairB,
-                                                      const int* __restrict__ aKey, const PlanCounts* __restrict__ cnt,
-                                                      int bn, int max_tiles, int* __restrict__ first,
-                                                      int* __restrict__ tile0, int* __restrict__ tile_batch,
-                                                      int* __restrict__ tile_col0, int* __restrict__ tile_ncols,
-                                                      int* __restrict__ rowPair, int* __restrict__ rowKey) {
-    pair_tiles_block(false, pairA, pairB, aKey, (int)cnt->nP, (int)cnt->nA, (int)cnt->nku, bn, max_tiles, first,
-                     tile0, tile_batch, tile_col0, tile_ncols, rowPair, rowKey);
+__global__ void __launch_bounds__(1024) k_pair_tiles(const int* __restrict__ pairA,
+                                                      const PlanCounts* __restrict__ cnt, int bn, int max_tiles,
+                                                      int* __restrict__ first, int* __restrict__ tile0,
+                                                      int* __restrict__ tile_batch, int* __restrict__ tile_col0,
+                                                      int* __restrict__ tile_ncols) {
+    pair_tiles_block(false, pairA, (int)cnt->nP, (int)cnt->nA, bn, max_tiles, first, tile0, tile_batch, tile_col0,
+                     tile_ncols);
 }
 
 // the tile arrays of one stage B launch: first pair and first tile of every A
-// key, then batch (host A key), first row and row count of every tile, and
-// (FP64 stage B: `rows`) the H2 row and weight key of every tile row
+// key, then batch (A key), first pair and pair count of every tile
 struct PairTiles {
     DevBuf<int> buf;
     int bn = 0;
     i64 max_tiles = 0;
     int *first = nullptr, *tile0 = nullptr, *batch = nullptr, *col0 = nullptr, *ncols = nullptr;
-    int *rowPair = nullptr, *rowKey = nullptr;
     bool built = false;
-    static i64 ints(i64 nA, i64 nP, int tile_pairs, bool rows) {
-        return 2 * nA + 3 * (nP / tile_pairs + nA + 1) + (rows ? 2 * nP : 0);
-    }
+    static i64 ints(i64 nA, i64 nP, int tile_pairs) { return 2 * nA + 3 * (nP / tile_pairs + nA + 1); }
     // mem: nullptr to allocate on the stream, or ints(...) ints lent by an owner
-    void alloc(i64 nA, i64 nP, int tile_pairs, bool rows, cudaStream_t s, int* mem = nullptr) {
+    void alloc(i64 nA, i64 nP, int tile_pairs, cudaStream_t s, int* mem = nullptr) {
         bn = tile_pairs;
         max_tiles = nP / bn + nA + 1;
         if (mem)
-            buf.borrow(mem, ints(nA, nP, tile_pairs, rows), s);
+            buf.borrow(mem, ints(nA, nP, bn), s);
         else
-            buf.alloc(ints(nA, nP, tile_pairs, rows), s);
+            buf.alloc(ints(nA, nP, bn), s);
         first = buf.p;
         tile0 = buf.p + nA;
         batch = buf.p + 2 * nA;
         col0 = batch + max_tiles;
         ncols = col0 + max_tiles;
-        rowPair = rows ? ncols + max_tiles : nullptr;
-        rowKey = rows ? rowPair + nP : nullptr;
     }
 };
 
@@ -1509,8 +1545,7 @@ __global__ void __launch_bounds__(1024) k_plan_small(i64 nk, i64 capA, i64 capP,
                                                      int* __restrict__ pairA, int* __restrict__ pairB, int bn,
                                                      int max_tiles, int* __restrict__ first, int* __restrict__ tile0,
                                                      int* __restrict__ tile_batch, int* __restrict__ tile_col0,
-                                                     int* __restrict__ tile_ncols, int* __restrict__ rowPair,
-                                                     int* __restrict__ rowKey, PlanCounts* __restrict__ cnt,
+                                                     int* __restrict__ tile_ncols, PlanCounts* __restrict__ cnt,
                                                      PlanReuse reuse) {
     __shared__ uint32_t ws[32], total, nku_s;
     __shared__ uint32_t s_bits[PLAN_SMALL_WORDS], s_pre[PLAN_SMALL_WORDS];
@@ -1598,8 +1633,7 @@ __global__ void __launch_bounds__(1024) k_plan_small(i64 nk, i64 capA, i64 capP,
         }
     __syncthreads();
     if (first)
-        pair_tiles_block(true, pairA, pairB, aKey, nP, nA, (int)nku, bn, max_tiles, first, tile0, tile_batch,
-                         tile_col0, tile_ncols, rowPair, rowKey);
+        pair_tiles_block(true, pairA, nP, nA, bn, max_tiles, first, tile0, tile_batch, tile_col0, tile_ncols);
     if (reuse.valid) {
         // save what this plan was made from, for the next replay's check
         for (i64 i = threadIdx.x; i < 2 * nk; i += blockDim.x) reuse.saved_used[i] = used[i];
@@ -1806,38 +1840,20 @@ static void launch_gather(const GatherLaunch& gl, const int64_t* idx, i64 m, dou
 // blocks of a cluster, which sum their partial tiles in distributed shared
 // memory, so Q holds one product per (pair, key).  (Summing slices of Q in the
 // gather instead made ERI 7^3's 3.57 million classes read several values
-// each.)  Returns the blocks per tile; *u_chunk their length of u.
-static int product_split(i64 nP, i64 nku, int U, int num_sms, int* u_chunk) {
+// each.)  Returns the blocks per tile.
+static int product_split(i64 nP, i64 nku, int U, int num_sms) {
     const i64 mt = (nP + DM_BM - 1) / DM_BM, nt = (nku + DM_BN - 1) / DM_BN;
-    *u_chunk = U;
-    const int P = std::min(4, split_count(mt * ((nt + 1) / 2), U, DM_BK, 4 * (i64)num_sms, u_chunk));
-    *u_chunk = ((U + P - 1) / P + DM_BK - 1) / DM_BK * DM_BK;
-    return (U + *u_chunk - 1) / *u_chunk;
-}
-
-// Stage A with 129..144 A keys holds them in one 144-column tile and does not
-// split the whole K range (the partial 144-column tiles would not fit the
-// operand ring for the cluster sum, and summing them through HBM measured
-// slower, ERIDA 129^3 0.439 against 0.410 ms).  Only a last wave under half
-// full is split in K, two blocks per m tile (ERIDA 129^3: 1,072 m tiles on 444
-// block slots, 2.41 waves).  Returns the m tiles split so (0: none).
-static i64 stage_a_tail(i64 nA, int nS, int U, int num_sms) {
-    if (!(nA > 128 && nA <= 144)) return 0;
-    const i64 mb = (nS + DM_BM - 1) / DM_BM;
-    const i64 slots = (i64)dmma_blocks_per_sm<StageAOp<144>>() * num_sms;
-    const i64 tail = mb % slots;
-    return tail > 0 && 2 * tail <= slots && (U + DM_BK - 1) / DM_BK >= 2 ? tail : 0;
+    int u_chunk = U;
+    const int P = std::min(4, split_count(mt * ((nt + 1) / 2), U, DM_BK, 4 * (i64)num_sms, &u_chunk));
+    u_chunk = ((U + P - 1) / P + DM_BK - 1) / DM_BK * DM_BK;
+    return (U + u_chunk - 1) / u_chunk;
 }
 
 // Buffers of the three stages, sized by the plan's counts
 struct StageBufs {
     DevBuf<double> H, H2, Q;
-    DevBuf<double> split_ws;  // stage A's tail split: two partial tiles per split m tile
-    DevBuf<unsigned> tickets;
-    int q_parts = 0, u_chunk = 0;
-    i64 tail = 0;
-    void alloc(const EvalArgs& a, const EvalSizes& sz, bool tc_a, bool product, cudaStream_t s,
-               const PlanStore* keep = nullptr) {
+    int q_parts = 0;
+    void alloc(const EvalArgs& a, const EvalSizes& sz, bool product, cudaStream_t s, const PlanStore* keep = nullptr) {
         const LatticeTables& t = *a.t;
         const int U = (int)t.U, Up = (int)t.Up, nS = (int)t.nS;
         if (sz.nA * (i64)U * U > ((i64)1 << 31))
@@ -1845,18 +1861,12 @@ struct StageBufs {
         H.alloc(sz.nA * (i64)nS, s);
         H2.alloc(sz.nP * (i64)Up, s);
         if (product) {
-            q_parts = product_split(sz.nP, sz.nku, U, a.num_sms, &u_chunk);
+            q_parts = product_split(sz.nP, sz.nku, U, a.num_sms);
             const i64 q = sz.nP * sz.nku;
             if (keep && keep->Q.p && keep->Q.n >= (size_t)q)
                 Q.borrow(keep->Q.p, q, s);  // a graph's own products, kept between its replays
             else
                 Q.alloc(q, s);
-        }
-        tail = tc_a ? 0 : stage_a_tail(sz.nA, nS, U, a.num_sms);
-        if (tail) {
-            split_ws.alloc(tail * 2 * DM_BM * 144, s);
-            tickets.alloc(tail, s);
-            tickets.zero();
         }
     }
 };
@@ -1965,16 +1975,15 @@ static void enqueue_eval(const EvalArgs& a, PlanMode mode, EvalStatus* st, Stage
     // path: ERI 7^3 0.206 against 0.200 ms)
     const bool plan_small = small_pairs && nk <= PLAN_SMALL_KEYS;
     if (plan_small) {
-        const bool sliced = stage_b_sliced(a.mixed, sz.nA, sz.nP, U);
-        const int tbn = sliced ? tile_n(MIXED_SLICES) : DM_BM;
+        const int tbn = stage_b_sliced(a.mixed, sz.nA, sz.nP, U) ? tile_n(MIXED_SLICES) : col_tile(sz.nku);
         if (pstore) {
             pairA.borrow(pstore->pairA.p, sz.nP, s);
             pairB.borrow(pstore->pairB.p, sz.nP, s);
-            tiles.alloc(sz.nA, sz.nP, tbn, !sliced, s, pstore->tiles.p);
+            tiles.alloc(sz.nA, sz.nP, tbn, s, pstore->tiles.p);
         } else {
             pairA.alloc(sz.nP, s);
             pairB.alloc(sz.nP, s);
-            tiles.alloc(sz.nA, sz.nP, tbn, !sliced, s);
+            tiles.alloc(sz.nA, sz.nP, tbn, s);
         }
     }
     // the mixed form runs a stage on the tensor cores when it is large enough
@@ -1982,9 +1991,8 @@ static void enqueue_eval(const EvalArgs& a, PlanMode mode, EvalStatus* st, Stage
     // (decided on the sizes: bounds for bounded plans, counts otherwise)
     StageBufs sb;
     auto stage_bufs = [&]() {
-        const bool tc = a.mixed && sz.nA * (i64)nS >= tc_a_outputs();
         const bool prod = product_pays((double)sz.nP, (double)sz.nku, m) || (bounded && m >= 65536);
-        sb.alloc(a, sz, tc, prod, s, pstore);
+        sb.alloc(a, sz, prod, s, pstore);
     };
     if (known) stage_bufs();
 
@@ -2005,11 +2013,9 @@ static void enqueue_eval(const EvalArgs& a, PlanMode mode, EvalStatus* st, Stage
                           lb ? 1 : 0, fused ? (const int*)pstore->valid.p : (const int*)nullptr);
         }
     }
-    // (a trusted replay whose stage A runs on the FP64 tensor-core GEMM in 64-
-    // or 80-column tiles restores the kept counts in that kernel; the
-    // 144-column tiles have no registers to spare for it)
-    const bool restore_in_a = plan_small && trusted && !(a.mixed && sz.nA * (i64)nS >= tc_a_outputs()) &&
-                              !(sz.nA > 128 && sz.nA <= 144);
+    // (a trusted replay whose stage A runs on the FP64 tensor-core GEMM restores
+    // the kept counts in that kernel)
+    const bool restore_in_a = plan_small && trusted && !(a.mixed && sz.nA * (i64)nS >= tc_a_outputs());
     if (restores != (plan_small && trusted)) fail(GLI_ERR_INTERNAL, "trusted replay without its restoring kernel");
     if (plan_small && trusted) {
         if (!restore_in_a) launch_kernel(k_restore_plan, dim3(1), dim3(32), 0, s, pstore->reuse(true), st);
@@ -2017,7 +2023,7 @@ static void enqueue_eval(const EvalArgs& a, PlanMode mode, EvalStatus* st, Stage
     } else if (plan_small) {
         launch_kernel(k_plan_small, dim3(1), dim3(1024), 0, s, nk, sz.nA, sz.nP, used.p, ids.p, keyOf.p, aId.p, aKey.p, words,
                    pairBits.p, pairPre.p, pairA.p, pairB.p, tiles.bn, (int)tiles.max_tiles, tiles.first, tiles.tile0,
-                   tiles.batch, tiles.col0, tiles.ncols, tiles.rowPair, tiles.rowKey, cnt,
+                   tiles.batch, tiles.col0, tiles.ncols, cnt,
                    pstore ? pstore->reuse(fused) : PlanReuse{});
         tiles.built = true;
     } else {
@@ -2059,10 +2065,13 @@ static void enqueue_eval(const EvalArgs& a, PlanMode mode, EvalStatus* st, Stage
     // the mixed form runs a stage on the tensor cores when it is large enough for
     // them to pay off; smaller stages (latency-bound either way) stay FP64
     const bool tc_a = a.mixed && nA * (i64)nS >= tc_a_outputs();
-    if (restore_in_a && (tc_a || (nA > 128 && nA <= 144)))
+    if (restore_in_a && tc_a)
         fail(GLI_ERR_INTERNAL, "trusted replay: stage A changed path after the plan");
     const bool tc_b = stage_b_sliced(a.mixed, nA, nP, U);
     DevBuf<double>& H2 = sb.H2;
+    const int2* rch = t.banded ? t.key_reach() : nullptr;
+    const int2* rfrom = t.banded ? t.reach_from() : nullptr;
+    const int2* rupto = t.banded ? t.reach_upto() : nullptr;
     t_enq_paths = (tc_a ? 1 : 0) | (tc_b ? 2 : 0);
     timer.mark();
     // ---- stage A
@@ -2085,45 +2094,40 @@ static void enqueue_eval(const EvalArgs& a, PlanMode mode, EvalStatus* st, Stage
         // small problems split the t loop so that enough blocks exist (the
         // partial tiles summed in a cluster)
         const unsigned mb = (unsigned)((nS + DM_BM - 1) / DM_BM);
-        const int bn = (nA > 128 && nA <= 144) ? 144 : col_tile(nA);
+        const int bn = col_tile(nA);
         const unsigned nb = (unsigned)((nA + bn - 1) / bn);
         int t_chunk = U;
-        const int P = bn == 144 ? 1 : split_count((i64)mb * nb, U, DM_BK, DM_SPLIT_TARGET * a.num_sms, &t_chunk);
+        const int P = split_count((i64)mb * nb, U, DM_BK, DM_SPLIT_TARGET * a.num_sms, &t_chunk);
         const dim3 grid(mb, nb, (unsigned)P);
         if (restore_in_a && (mb == 0 || nb == 0))  // (no stage-A block would restore the counts)
             launch_kernel(k_restore_plan, dim3(1), dim3(32), 0, s, pstore->reuse(true), st);
-        auto restoring = [&](auto op) {
+        auto go = [&](auto op) {
             if (restore_in_a && mb > 0 && nb > 0) {
                 op.restore_valid = pstore->valid.p;
                 op.restore_from = pstore->saved_cnt.p;
                 op.restore_to = st;
             }
-            return op;
-        };
-        if (bn == 144) {
-            // one 144-column tile; a last wave under half full split in K
-            // (stage_a_tail)
-            StageAOp<144> op{t.W.p, t.T.p, t.S.p, aKey.p, cnt, nS, U, Up, U, 0, H.p};
-            dim3 g = grid;
-            if (sb.tail) {
-                op.nfull = (int)(mb - sb.tail);
-                op.ws = sb.split_ws.p;
-                op.tickets = sb.tickets.p;
-                g.x = (unsigned)(mb + sb.tail);
-            }
-            dmma_launch(op, g, s);
-        } else if (bn == 80) {
             // a split sums its parts inside a cluster of the P blocks of a tile
-            dmma_launch_cluster(restoring(StageAOp<80>{t.W.p, t.T.p, t.S.p, aKey.p, cnt, nS, U, Up, t_chunk, 0, H.p}),
-                                grid, s);
-        } else {
-            dmma_launch_cluster(restoring(StageAOp<64>{t.W.p, t.T.p, t.S.p, aKey.p, cnt, nS, U, Up, t_chunk, 0, H.p}),
-                                grid, s);
-        }
+            dmma_launch_cluster(op, grid, s);
+        };
+        // (the sliced stage B reads whole rows of H: nothing is left out then)
+        const int prune = t.banded && !tc_b ? 1 : 0;
+        const bool deep = (i64)mb * nb * P <= (i64)DM_SPLIT_TARGET * a.num_sms;
+        auto sized = [&](auto width) {
+            constexpr int BN = decltype(width)::value;
+            if (deep)
+                go(StageAOp<BN, true>{t.W.p, t.T.p, t.S.p, aKey.p, cnt, rch, rfrom, rupto, nS, U, Up, prune, H.p});
+            else
+                go(StageAOp<BN, false>{t.W.p, t.T.p, t.S.p, aKey.p, cnt, rch, rfrom, rupto, nS, U, Up, prune, H.p});
+        };
+        if (bn == 80)
+            sized(std::integral_constant<int, 80>{});
+        else
+            sized(std::integral_constant<int, 64>{});
     }
     timer.mark();
     // ---- stage B
-    if (tiles.built && tiles.bn != (tc_b ? tile_n(MIXED_SLICES) : DM_BM)) tiles.built = false;
+    if (tiles.built && tiles.bn != (tc_b ? tile_n(MIXED_SLICES) : col_tile(nku))) tiles.built = false;
     if (tc_b) {
         constexpr int BN = tile_n(MIXED_SLICES);
         const int mb = (U + TC_BM - 1) / TC_BM;
@@ -2131,10 +2135,9 @@ static void enqueue_eval(const EvalArgs& a, PlanMode mode, EvalStatus* st, Stage
         Hs.alloc(nA * mb, TC_BM, U, MIXED_SLICES, s);
         slice_tiled(ExpandedHRows{H.p, t.sidx.p, cnt, nS, U, mb}, nA * U, U, Hs, s);
         if (!tiles.built) {
-            tiles.alloc(nA, nP, BN, false, s);
-            launch_kernel(k_pair_tiles, dim3(1), dim3(1024), 0, s, pairA.p, pairB.p, aKey.p, cnt, BN,
-                       (int)tiles.max_tiles, tiles.first, tiles.tile0, tiles.batch, tiles.col0, tiles.ncols,
-                       (int*)nullptr, (int*)nullptr);
+            tiles.alloc(nA, nP, BN, s);
+            launch_kernel(k_pair_tiles, dim3(1), dim3(1024), 0, s, pairA.p, cnt, BN, (int)tiles.max_tiles, tiles.first,
+                          tiles.tile0, tiles.batch, tiles.col0, tiles.ncols);
         }
         const i64 max_tiles = tiles.max_tiles;
         Wb.alloc(max_tiles, BN, U, MIXED_SLICES, s);
@@ -2152,44 +2155,37 @@ static void enqueue_eval(const EvalArgs& a, PlanMode mode, EvalStatus* st, Stage
         w.cs = Up;
         tc_gemm_tiled(Hs.view(), Wb.view(), w, (int)max_tiles, &st->tc_err, s);
     } else {
-        // tiles of 64 rows of one host A key, then (tile, 64 u, chunk of v) blocks
+        // (host and column tile of its pairs, 64 u, part of v) blocks; the tile
+        // list is built on the device, the grid follows its bound and the split
+        // the tiles that hold pairs (hosts' last tiles half full); following the
+        // reaches, the u range shrinks with the host
+        const int bn = col_tile(nku);
         if (!tiles.built) {
-            tiles.alloc(nA, nP, DM_BM, true, s);
-            launch_kernel(k_pair_tiles, dim3(1), dim3(1024), 0, s, pairA.p, pairB.p, aKey.p, cnt, DM_BM,
-                       (int)tiles.max_tiles, tiles.first, tiles.tile0, tiles.batch, tiles.col0, tiles.ncols,
-                       tiles.rowPair, tiles.rowKey);
+            tiles.alloc(nA, nP, bn, s);
+            launch_kernel(k_pair_tiles, dim3(1), dim3(1024), 0, s, pairA.p, cnt, bn, (int)tiles.max_tiles, tiles.first,
+                          tiles.tile0, tiles.batch, tiles.col0, tiles.ncols);
         }
-        const i64 max_tiles = tiles.max_tiles;
-        // the tile list is built on the device; the grid follows its bound and
-        // the split follows the tiles that hold pairs: with exact counts (exact
-        // and sized plans) those are known -- a full pair triangle with
-        // balanced hosts fills sum_h ceil(rows_h / 64) tiles, other pair sets
-        // about nP / 64 + nA / 2 -- with bounded plans the bound stands in
-        // (64 u per tile: 80-row K-major gathers measured slower, ERIDA 129^3
-        // stage B 0.32 against 0.21 ms)
-        i64 active = max_tiles;
-        if (!bounded) {
-            if (nku == nA && nP == nA * (nA + 1) / 2 && nA > DM_BM) {
-                const int y = (int)std::min<i64>(nA, 2 * DM_BM - 1);
-                active = 0;
-                for (int h = 0; h < (int)nA; ++h) active += (bal_count(h, (int)nA, y) + DM_BM - 1) / DM_BM;
-            } else {
-                active = std::min<i64>(max_tiles, (nP + DM_BM - 1) / DM_BM + nA / 2);
-            }
-        }
-        const unsigned ub = (unsigned)((U + DM_BN - 1) / DM_BN);
+        const i64 ub = (U + DM_BM - 1) / DM_BM, held = std::min<i64>(tiles.max_tiles, (nP + bn - 1) / bn + nA / 2);
+        const i64 active = t.banded ? (held * ub + 1) / 2 : held * ub;
         int v_chunk = U;
-        const int P = split_count(active * ub, U, DM_BK, DM_SPLIT_TARGET * a.num_sms, &v_chunk);
-        // a split sums its parts inside a cluster of the P blocks of a tile
-        const dim3 grid((unsigned)max_tiles, ub, (unsigned)P);
-        if (active * ub * P >= 4 * (i64)DM_SPLIT_TARGET * a.num_sms)
-            dmma_launch_cluster(StageBOp<false>{t.W.p, H.p, t.sidx.p, tiles.rowKey, tiles.rowPair, tiles.batch,
-                                                tiles.col0, tiles.ncols, nS, U, Up, v_chunk, 0, H2.p},
-                                grid, s);
+        const int P = split_count(active, U, DM_BK, DM_SPLIT_TARGET * a.num_sms, &v_chunk);
+        const dim3 grid((unsigned)tiles.max_tiles, (unsigned)ub, (unsigned)P);
+        const bool deep = active * P <= (i64)DM_SPLIT_TARGET * a.num_sms;
+        auto sized = [&](auto width) {
+            constexpr int BN = decltype(width)::value;
+            if (deep)
+                dmma_launch_cluster(StageBOp<BN, true>{t.W.p, H.p, t.sidx.p, aKey.p, pairB.p, tiles.batch, tiles.col0,
+                                                       tiles.ncols, rch, rfrom, rupto, nS, U, Up, H2.p},
+                                    grid, s);
+            else
+                dmma_launch_cluster(StageBOp<BN, false>{t.W.p, H.p, t.sidx.p, aKey.p, pairB.p, tiles.batch, tiles.col0,
+                                                        tiles.ncols, rch, rfrom, rupto, nS, U, Up, H2.p},
+                                    grid, s);
+        };
+        if (bn == 80)
+            sized(std::integral_constant<int, 80>{});
         else
-            dmma_launch_cluster(StageBOp<true>{t.W.p, H.p, t.sidx.p, tiles.rowKey, tiles.rowPair, tiles.batch,
-                                               tiles.col0, tiles.ncols, nS, U, Up, v_chunk, 0, H2.p},
-                                grid, s);
+            sized(std::integral_constant<int, 64>{});
     }
     timer.mark();
     // ---- stage C: the product form computes every (pair, key) dot product --
@@ -2204,13 +2200,12 @@ static void enqueue_eval(const EvalArgs& a, PlanMode mode, EvalStatus* st, Stage
     if (undecided || product_host) {
         // (Q and its u split sized with the stage buffers: product_split)
         const i64 mt = (nP + DM_BM - 1) / DM_BM, nt = (nku + DM_BN - 1) / DM_BN;
-        const int P = sb.q_parts, u_chunk = sb.u_chunk;
+        const int P = sb.q_parts;
         const i64 ps = nP * nku;
         const DevBuf<double>& Q = sb.Q;
         if (P < 1 || !Q.p) fail(GLI_ERR_INTERNAL, "stage C product without its buffer");
         // (a split sums its parts inside a cluster of the P blocks of a tile)
-        dmma_launch_cluster(ProductOp<64>{H2.p, t.W.p, keyOf.p, pairA.p, aKey.p, ids.p, cnt, m, c_prod, U, Up,
-                                          (int)nku, u_chunk, Q.p, &st->products},
+        dmma_launch_cluster(ProductOp<64>{H2.p, t.W.p, keyOf.p, pairA.p, aKey.p, ids.p, cnt, rch, rfrom, m, c_prod, U, Up, (int)nku, Q.p, &st->products},
                             dim3((unsigned)mt, (unsigned)nt, (unsigned)P), s);
         timer.mark();  // (the class-level kernels of stage C start here)
         t_enq_paths |= (fused ? 2 : 1) << 2;  // the class gather that ran
@@ -2240,7 +2235,7 @@ static void enqueue_eval(const EvalArgs& a, PlanMode mode, EvalStatus* st, Stage
         if (!undecided) timer.mark();  // (no product GEMM: the class-level kernel starts stage C)
         const i64 want = (m + 7) / 8;
         const unsigned gc = (unsigned)(want < (i64)a.num_sms * 16 ? want : (i64)a.num_sms * 16);
-        launch_kernel(k_stage_c, dim3(gc), dim3(256), 0, s, t.W.p, H2.p, keys.p, dec, a.idx, (int)nk, pairBits.p, pairPre.p, m, U, Up,
+        launch_kernel(k_stage_c, dim3(gc), dim3(256), 0, s, t.W.p, H2.p, rch, keys.p, dec, a.idx, (int)nk, pairBits.p, pairPre.p, m, U, Up,
                    cnt, c_class, a.out);
     }
     timer.mark();
@@ -2359,18 +2354,21 @@ static GraphEntry* capture_graph(const EvalArgs& a, const std::shared_ptr<const 
     // function attributes are set outside the capture
     tc_gemm_prepare();
     dgemm_prepare();
-    dmma_prepare<StageAOp<64>>();
-    dmma_prepare<StageAOp<80>>();
-    dmma_prepare<StageAOp<144>>();
-    dmma_blocks_per_sm<StageAOp<144>>();
-    dmma_prepare<StageBOp<true>>();
-    dmma_prepare<StageBOp<false>>();
+    auto prepare = [](auto width) {
+        constexpr int BN = decltype(width)::value;
+        dmma_prepare<StageAOp<BN, true>>();
+        dmma_prepare<StageAOp<BN, false>>();
+        dmma_prepare<StageBOp<BN, true>>();
+        dmma_prepare<StageBOp<BN, false>>();
+        dmma_prepare<StageAOp<BN, true>, true>();
+        dmma_prepare<StageAOp<BN, false>, true>();
+        dmma_prepare<StageBOp<BN, true>, true>();
+        dmma_prepare<StageBOp<BN, false>, true>();
+    };
+    prepare(std::integral_constant<int, 64>{});
+    prepare(std::integral_constant<int, 80>{});
     dmma_prepare<ProductOp<64>>();
     dmma_prepare<ProductOp<64>, true>();
-    dmma_prepare<StageAOp<64>, true>();
-    dmma_prepare<StageAOp<80>, true>();
-    dmma_prepare<StageBOp<true>, true>();
-    dmma_prepare<StageBOp<false>, true>();
     // the sizes of the plan: the sized counts, or the bounds of a bounded plan
     const i64 nk = a.t->nkeys;
     EvalSizes szb = sized;
@@ -2385,12 +2383,9 @@ static GraphEntry* capture_graph(const EvalArgs& a, const std::shared_ptr<const 
     {
         const i64 words = (nk * nk + 31) / 32;
         i64 q_entries = 0;
-        if (product) {
-            int u_chunk = 0;
-            q_entries = szb.nP * szb.nku;
-        }
+        if (product) q_entries = szb.nP * szb.nku;
         e->plan = std::make_unique<PlanStore>();
-        e->plan->alloc(nk, words, szb.nA, szb.nP, PairTiles::ints(szb.nA, szb.nP, 64, true),
+        e->plan->alloc(nk, words, szb.nA, szb.nP, PairTiles::ints(szb.nA, szb.nP, 64),
                        pair_desc_applies(a.d) ? (i64)a.d.N2 : 0, q_entries);
     }
     auto capture = [&](bool trusted, StageTimer* tm, cudaGraphExec_t* exec, long long* launches,

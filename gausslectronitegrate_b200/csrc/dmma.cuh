@@ -1,11 +1,10 @@
 // FP64 tensor-core tiles: mma.sync.m8n8k4.f64 over operand tiles that the
 // caller gathers into shared memory with 8-byte cp.async copies.
 //
-// A block (4 warps) computes a 64 x BN tile of C = A B (BN = 32, 64, 80 or 144,
+// A block (4 warps) computes a 64 x BN tile of C = A B (BN = 32, 64 or 80,
 // chosen per Op) over K in chunks of 16, three chunks in flight (two for an Op
-// that declares STAGES = 2: the 144-column tiles, so that three blocks still
-// fit on an SM; cp.async groups, the waits are the hardware's own group waits,
-// no flag spins).  Warp w owns every other 8-row and 8-column strip (rows
+// that declares STAGES = 2, so that four blocks fit on an SM; cp.async groups,
+// the waits are the hardware's own group waits, no flag spins).  Warp w owns every other 8-row and 8-column strip (rows
 // 16 i + 8 (w & 1), columns 16 j + 8 (w >> 1)) as 4 x BN/16 m8n8 accumulators,
 // so that a partly filled tile loads the four warps (and their tensor pipes)
 // alike; per k-step of 4 it reads 4 A and BN/16 B fragments (one double each)
@@ -111,8 +110,8 @@ __device__ __forceinline__ double dm_frag(const double* s, int row0, int k0, int
 }
 
 // Op interface (all device, const):
-//   static constexpr bool A_KMAJOR, B_KMAJOR;  static constexpr int BN (32, 64,
-//   80 or 144; K-major B tiles have 64 rows); optionally STAGES (2 or 3)
+//   static constexpr bool A_KMAJOR, B_KMAJOR;  static constexpr int BN (32, 64
+//   or 80; K-major B tiles have 64 rows); optionally STAGES (2 or 3)
 //   struct Block { int mvalid, nvalid, nk; ... };       the block's work item
 //   struct AState; struct BState;                       per-thread cached row data
 //   bool begin(Block&)                                  false: nothing to do (uniform)
@@ -138,9 +137,16 @@ struct dm_a_landed<Op, std::void_t<decltype(Op::A_LANDED)>> {
 // whose operand is zero outside a run of K -- lattice weights, nonzero around
 // their key's position -- take part only in the chunks of their 8-row
 // strip's run.  Op::live_chunks(blk, strip, first, last) gives the chunks
-// [first, last] of a strip (empty: last < first); a mask per chunk, one bit per
-// strip of a warp, is built in shared memory before the main loop.  A skipped
-// MMA would have added products with exact zeros.
+// [first, last] of a strip (empty: last < first).  Per chunk and strip parity
+// (a warp's strips are the even or the odd ones) the live strips [lo, hi) are
+// found in shared memory before the main loop (lo | hi << 8; dead strips between
+// live ones count as live).  The main loop branches to code made for that run:
+// a predicate per strip is turned into predicated MMAs, which take the tensor
+// pipe's time whether they execute or not (ERIDA 129^3 stage A: 206 us
+// predicated).  The operand's state gets the runs of the strips that the thread
+// copies (`live`, row-major tiles copied in pairs: its row dm_pair_row(tid, q)
+// lies in strip q of its parity), so that skipped strips are not copied either.
+// A skipped MMA would have added products with exact zeros.
 constexpr int SKIP_M = 1, SKIP_N = 2, DM_MAX_CHUNKS = 256;
 template <class Op, class = void>
 struct dm_skip_of {
@@ -151,7 +157,6 @@ struct dm_skip_of<Op, std::void_t<decltype(Op::SKIP)>> {
     static constexpr int value = Op::SKIP;
 };
 
-// masks of the two strip groups (even and odd strips) of every chunk
 template <class Op>
 __device__ __forceinline__ void dm_build_masks(const Op& op, const typename Op::Block& blk,
                                                uint16_t (&live)[2][DM_MAX_CHUNKS]) {
@@ -166,14 +171,46 @@ __device__ __forceinline__ void dm_build_masks(const Op& op, const typename Op::
     for (int kc = threadIdx.x; kc < blk.nk; kc += DM_THREADS)
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
-            unsigned m = 0;
+            int lo = STRIPS / 2, hi = 0;
 #pragma unroll
             for (int t = 0; t < STRIPS / 2; ++t) {
                 const int r = run[2 * t + g];
-                m |= (unsigned)((r & 0xffff) <= kc && kc <= r >> 16) << t;
+                if ((r & 0xffff) <= kc && kc <= r >> 16) {
+                    lo = min(lo, t);
+                    hi = t + 1;
+                }
             }
-            live[g][kc] = (uint16_t)m;
+            live[g][kc] = (uint16_t)(hi > lo ? lo | hi << 8 : 0);
         }
+    __syncthreads();
+}
+__device__ __forceinline__ bool dm_live(unsigned run, int strip) {
+    return strip >= (int)(run & 0xffu) && strip < (int)(run >> 8);
+}
+
+// f(LO, HI) for the run [lo, hi) of N strips
+template <int LO, int N, class F>
+__device__ __forceinline__ void dm_run_from(int hi, F&& f) {
+    using std::integral_constant;
+    static_assert(N <= 5, "five strips per warp");
+    switch (hi - LO) {
+        case 1: f(integral_constant<int, LO>{}, integral_constant<int, LO + 1>{}); break;
+        case 2: if constexpr (LO + 2 <= N) f(integral_constant<int, LO>{}, integral_constant<int, LO + 2>{}); break;
+        case 3: if constexpr (LO + 3 <= N) f(integral_constant<int, LO>{}, integral_constant<int, LO + 3>{}); break;
+        case 4: if constexpr (LO + 4 <= N) f(integral_constant<int, LO>{}, integral_constant<int, LO + 4>{}); break;
+        case 5: if constexpr (LO + 5 <= N) f(integral_constant<int, LO>{}, integral_constant<int, LO + 5>{}); break;
+    }
+}
+template <int N, class F>
+__device__ __forceinline__ void dm_run(unsigned run, F&& f) {
+    const int hi = run >> 8;
+    switch (run & 0xffu) {
+        case 0: dm_run_from<0, N>(hi, f); break;
+        case 1: if constexpr (N > 1) dm_run_from<1, N>(hi, f); break;
+        case 2: if constexpr (N > 2) dm_run_from<2, N>(hi, f); break;
+        case 3: if constexpr (N > 3) dm_run_from<3, N>(hi, f); break;
+        case 4: if constexpr (N > 4) dm_run_from<4, N>(hi, f); break;
+    }
 }
 
 // The k loop of one block; FULL: every m8n8 tile of the warp's quadrant holds
@@ -201,37 +238,26 @@ __device__ __forceinline__ void dm_mainloop(const Op& op, const typename Op::Blo
         const double* a_s = smem + (kc % NS) * STAGE;
         const double* b_s = a_s + DM_TILE_A;
         if constexpr (SKIP != 0) {
-            const unsigned m = live[kc];
-            if (m == 0) continue;
-            if (!FULL || m != (1u << (SKIP == SKIP_M ? 4 : NJ)) - 1u) {
+            // (strips past the tile's rows or columns hold zeros: no run covers
+            // them alone, and their results are not stored)
+            dm_run<SKIP == SKIP_M ? 4 : NJ>(live[kc], [&](auto lo, auto hi) {
+                constexpr int LO = decltype(lo)::value, HI = decltype(hi)::value;
+                constexpr int I0 = SKIP == SKIP_M ? LO : 0, I1 = SKIP == SKIP_M ? HI : 4;
+                constexpr int J0 = SKIP == SKIP_M ? 0 : LO, J1 = SKIP == SKIP_M ? NJ : HI;
 #pragma unroll
                 for (int k0 = 0; k0 < DM_BK; k0 += 4) {
-                    if constexpr (SKIP == SKIP_M) {
-                        double bf[NJ];
+                    double af[4], bf[NJ];
 #pragma unroll
-                        for (int j = 0; j < NJ; ++j) bf[j] = dm_frag<Op::B_KMAJOR>(b_s, wn + 16 * j, k0, lane);
+                    for (int i = I0; i < I1; ++i) af[i] = dm_frag<Op::A_KMAJOR>(a_s, wm + 16 * i, k0, lane);
 #pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            if (m >> i & 1u) {
-                                const double af = dm_frag<Op::A_KMAJOR>(a_s, wm + 16 * i, k0, lane);
+                    for (int j = J0; j < J1; ++j) bf[j] = dm_frag<Op::B_KMAJOR>(b_s, wn + 16 * j, k0, lane);
 #pragma unroll
-                                for (int j = 0; j < NJ; ++j) dm_mma(acc[i][j], af, bf[j]);
-                            }
-                    } else {
-                        double af[4];
+                    for (int i = I0; i < I1; ++i)
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) af[i] = dm_frag<Op::A_KMAJOR>(a_s, wm + 16 * i, k0, lane);
-#pragma unroll
-                        for (int j = 0; j < NJ; ++j)
-                            if (m >> j & 1u) {
-                                const double bf = dm_frag<Op::B_KMAJOR>(b_s, wn + 16 * j, k0, lane);
-#pragma unroll
-                                for (int i = 0; i < 4; ++i) dm_mma(acc[i][j], af[i], bf);
-                            }
-                    }
+                        for (int j = J0; j < J1; ++j) dm_mma(acc[i][j], af[i], bf[j]);
                 }
-                continue;
-            }
+            });
+            continue;
         }
 #pragma unroll
         for (int k0 = 0; k0 < DM_BK; k0 += 4) {
@@ -264,13 +290,13 @@ struct dm_blocks_of<Op, std::void_t<decltype(Op::MIN_BLOCKS)>> {
 // block leaves its partial tile in its own shared memory, and after a cluster
 // barrier every block sums its share of the tile's rows over the cluster's
 // blocks through distributed shared memory, in the order of their ranks (the
-// same order on every run), and stores it.  The Op then writes every part to
-// the same destination (part stride 0).  Every block of a cluster reaches both
-// cluster barriers: a block without work contributes zeros.
+// same order on every run), and stores it.  Op::begin gives the same answer to
+// every block of a cluster (its parts differ in their K range only, which may
+// be empty), so that all of them or none reach the cluster barriers.
 constexpr int DM_RED_LD = 2;  // doubles of padding per reduction-tile row
 
 template <class Op, bool CLUSTER>
-__device__ __forceinline__ void dm_cluster_reduce(const Op& op, const typename Op::Block& blk, bool active,
+__device__ __forceinline__ void dm_cluster_reduce(const Op& op, const typename Op::Block& blk,
                                                   double* smem, int wm, int wn, int mt, int nt,
                                                   const double (&acc)[4][Op::BN / 16][2]) {
     constexpr int NJ = Op::BN / 16, LD = Op::BN + DM_RED_LD;
@@ -282,7 +308,7 @@ __device__ __forceinline__ void dm_cluster_reduce(const Op& op, const typename O
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
-            const bool has = active && i < mt && j < nt;
+            const bool has = i < mt && j < nt;
             double* d = smem + (wm + 16 * i + (lane >> 2)) * LD + wn + 16 * j + 2 * (lane & 3);
             d[0] = has ? acc[i][j][0] : 0.0;
             d[1] = has ? acc[i][j][1] : 0.0;
@@ -290,7 +316,7 @@ __device__ __forceinline__ void dm_cluster_reduce(const Op& op, const typename O
     cg::cluster_group cl = cg::this_cluster();
     cl.sync();
     const int P = (int)cl.num_blocks(), r = (int)cl.block_rank();
-    if (active) {
+    {
         // block r sums rows [r0, r1) of the tile: per column pair, the P
         // partial pairs are loaded first (16-byte distributed shared-memory
         // loads, all in flight together) and then added in rank order
@@ -300,6 +326,9 @@ __device__ __forceinline__ void dm_cluster_reduce(const Op& op, const typename O
 #pragma unroll
         for (int q = 0; q < 8; ++q)
             part[q] = reinterpret_cast<const double2*>(cl.map_shared_rank(smem, q < P ? q : 0));
+        // (neighbouring threads read neighbouring pairs of a row: taking rows
+        // instead, for Ops whose output is contiguous that way, spreads the remote
+        // reads and measured slower, ERIDA 33^3 stage B 23.5 against 18.6 us)
         for (int e = r0 * PAIRS + threadIdx.x; e < r1 * PAIRS; e += blockDim.x) {
             const int row = e / PAIRS, c = 2 * (e % PAIRS);
             const int off = (row * LD + c) / 2;  // LD and c are even: 16-byte aligned pairs
@@ -320,78 +349,16 @@ __device__ __forceinline__ void dm_cluster_reduce(const Op& op, const typename O
     cl.sync();  // no block leaves while another still reads its tile
 }
 
-// Tail split (an Op that declares TAIL_SPLIT): the last, partial wave of a
-// launch would leave most SMs idle, so its m tiles are each computed by two
-// blocks over the two halves of K, and the blocks of a full wave's worth of
-// tiles run whole before them.  Both halves write their partial tile to
-// global scratch in the threads' own fragment order (coalesced, no shared
-// memory), then take a ticket for the tile; the second to arrive adds the
-// other's partial to its own and stores the sum (a + b = b + a exactly, so
-// the result does not depend on which half came second), and resets the
-// ticket for the next evaluation.  No block waits on another.
-//   Op::split_half()  -1 for a whole tile, else 0 or 1 (uniform in a block)
-//   Op::split_slot()  the tile's scratch slot; Op::ws, Op::tickets
-template <class Op, class = void>
-struct dm_tail_split {
-    static constexpr bool value = false;
-};
-template <class Op>
-struct dm_tail_split<Op, std::void_t<decltype(Op::TAIL_SPLIT)>> {
-    static constexpr bool value = Op::TAIL_SPLIT;
-};
-
-template <class Op>
-__device__ __forceinline__ void dm_split_store(const Op& op, const typename Op::Block& blk, int half, int wm, int wn,
-                                               int mt, int nt, const double (&acc)[4][Op::BN / 16][2]) {
-    constexpr int NJ = Op::BN / 16, TILE = DM_BM * Op::BN;
-    const int lane = threadIdx.x & 31, slot = op.split_slot();
-    __shared__ unsigned s_ticket;
-    double* mine = op.ws + ((i64)slot * 2 + half) * TILE;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < NJ; ++j)
-            if (i < mt && j < nt) {
-                __stcg(mine + ((i * NJ + j) * 2) * DM_THREADS + threadIdx.x, acc[i][j][0]);
-                __stcg(mine + ((i * NJ + j) * 2 + 1) * DM_THREADS + threadIdx.x, acc[i][j][1]);
-            }
-    __threadfence();  // the partial is visible before the ticket is taken
-    __syncthreads();
-    if (threadIdx.x == 0) s_ticket = atomicAdd(op.tickets + slot, 1u);
-    __syncthreads();
-    if (s_ticket == 0) return;  // the other half arrives second and sums
-    __threadfence();
-    const double* other = op.ws + ((i64)slot * 2 + (half ^ 1)) * TILE;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < NJ; ++j)
-            if (i < mt && j < nt) {
-                const double o0 = __ldcg(other + ((i * NJ + j) * 2) * DM_THREADS + threadIdx.x);
-                const double o1 = __ldcg(other + ((i * NJ + j) * 2 + 1) * DM_THREADS + threadIdx.x);
-                op.store(blk, wm + 16 * i + (lane >> 2), wn + 16 * j + 2 * (lane & 3), acc[i][j][0] + o0,
-                         acc[i][j][1] + o1);
-            }
-    if (threadIdx.x == 0) op.tickets[slot] = 0u;
-}
-
 template <class Op, bool CLUSTER = false>
 __global__ void __launch_bounds__(DM_THREADS, dm_blocks_of<Op>::value) k_dmma(const Op op) {
     constexpr int NJ = Op::BN / 16, STAGE = DM_TILE_A + dm_tile_b(Op::BN), NS = dm_stages_of<Op>::value;
-    static_assert(Op::BN == 64 || ((Op::BN == 80 || Op::BN == 32 || Op::BN == 144) && !Op::B_KMAJOR),
-                  "column tiles of 64, or 32, 80 and 144 read row-major");
+    static_assert(Op::BN == 64 || ((Op::BN == 80 || Op::BN == 32) && !Op::B_KMAJOR),
+                  "column tiles of 64, or 32 and 80 read row-major");
     static_assert(NS >= 2 && NS <= 3, "two or three stages");
     static_assert(!CLUSTER || DM_BM * (Op::BN + DM_RED_LD) <= NS * STAGE, "reduction tile exceeds the operand ring");
     extern __shared__ __align__(16) double dm_smem[];
     typename Op::Block blk;
-    const bool active = op.begin(blk);
-    if (!active) {
-        if constexpr (CLUSTER) {
-            double none[4][NJ][2];
-            dm_cluster_reduce<Op, CLUSTER>(op, blk, false, dm_smem, 0, 0, 0, 0, none);
-        }
-        return;
-    }
+    if (!op.begin(blk)) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wm = (warp & 1) * 8, wn = (warp >> 1) * 8;
     typename Op::AState as;
@@ -403,6 +370,9 @@ __global__ void __launch_bounds__(DM_THREADS, dm_blocks_of<Op>::value) k_dmma(co
         __shared__ uint16_t s_live[2][DM_MAX_CHUNKS];
         dm_build_masks(op, blk, s_live);
         live = s_live[dm_skip_of<Op>::value == SKIP_M ? warp & 1 : warp >> 1];
+        // (this thread copies rows (tid >> 3) + 16 q of the skipped operand: strips of one parity)
+        if constexpr (dm_skip_of<Op>::value == SKIP_M) as.live = s_live[threadIdx.x >> 6 & 1];
+        else bs.live = s_live[threadIdx.x >> 6 & 1];
     }
 #pragma unroll
     for (int st = 0; st < NS - 1; ++st) {
@@ -420,21 +390,14 @@ __global__ void __launch_bounds__(DM_THREADS, dm_blocks_of<Op>::value) k_dmma(co
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < NJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-    if (mt == 4 && nt == NJ)
+    if (dm_skip_of<Op>::value != 0 || (mt == 4 && nt == NJ))
         dm_mainloop<Op, true>(op, blk, as, bs, dm_smem, wm, wn, mt, nt, live, acc);
-    else
+    else if constexpr (dm_skip_of<Op>::value == 0)
         dm_mainloop<Op, false>(op, blk, as, bs, dm_smem, wm, wn, mt, nt, live, acc);
     dm_wait<0>();
     if constexpr (CLUSTER) {
-        dm_cluster_reduce<Op, CLUSTER>(op, blk, true, dm_smem, wm, wn, mt, nt, acc);
+        dm_cluster_reduce<Op, CLUSTER>(op, blk, dm_smem, wm, wn, mt, nt, acc);
         return;
-    }
-    if constexpr (dm_tail_split<Op>::value) {
-        const int half = op.split_half();
-        if (half >= 0) {
-            dm_split_store(op, blk, half, wm, wn, mt, nt, acc);
-            return;
-        }
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)

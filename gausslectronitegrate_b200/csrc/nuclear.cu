@@ -366,7 +366,9 @@ struct NucStageOp {
         const double* b;
         double* y;
     };
-    struct AState {};
+    struct AState {
+        const uint16_t* live;
+    };
     struct BState {};
     __device__ bool begin(Block& b) const {
         // the instance: the last one whose tiles start at or before this block
@@ -412,9 +414,11 @@ struct NucStageOp {
     }
     __device__ void a_init(const Block&, AState&) const {}
     __device__ void b_init(const Block&, BState&) const {}
-    __device__ void a_issue(const Block& b, AState&, int kc, double* tile) const {
+    __device__ void a_issue(const Block& b, AState& st, int kc, double* tile) const {
+        const unsigned live = st.live[kc];
 #pragma unroll
         for (int q = 0; q < DM_BM / 16; ++q) {
+            if (!dm_live(live, q)) continue;
             const int r = dm_pair_row(threadIdx.x, q), k = dm_pair_k(threadIdx.x), kk = kc * DM_BK + k;
             const int bytes = r < b.mvalid ? dm_pair_bytes(b.k0 + kk, b.kend) : 0;
             dm_cp16(tile + dm_rowmajor_at(r, k), bytes ? b.a + r * b.pitch + kk : b.a, bytes);

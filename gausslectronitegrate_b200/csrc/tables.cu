@@ -124,6 +124,22 @@ __global__ void k_fold_weights(int kind, const double* __restrict__ P, int nb, i
     W[key * Up + m] = v;
 }
 
+// first and last nonzero weight of every key, a warp per key
+__global__ void __launch_bounds__(256) k_key_reach(const double* __restrict__ W, i64 nkeys, int U, int Up,
+                                                   int2* __restrict__ reach) {
+    const i64 key = (i64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (key >= nkeys) return;
+    int first = U, last = -1;
+    for (int u = threadIdx.x & 31; u < U; u += 32)
+        if (W[key * Up + u] != 0.0) {
+            first = min(first, u);
+            last = max(last, u);
+        }
+    first = __reduce_min_sync(0xffffffffu, first);
+    last = __reduce_max_sync(0xffffffffu, last);
+    if ((threadIdx.x & 31) == 0) reach[key] = make_int2(first, last);
+}
+
 // T[n]: Coulomb interaction of two normalised Gaussians of width w at distance
 // sqrt(n)/den, erf(dist / (sqrt2 w)) / dist, with limit sqrt(2/pi)/w at n = 0.
 //   ERI   (kind 1): w = 1/3,       den = 6  ->  erf(sqrt(n)/(2 sqrt2)) * 6/sqrt(n)
@@ -205,9 +221,35 @@ static void build_lattice_tables(int kind, const double* h_coeffs, i64 nb, i64 L
     k_fold_weights<<<dim3((unsigned)((t.Up + 127) / 128), (unsigned)t.nkeys), 128, 0, s>>>(
         kind, prod.p, (int)nb, (int)L, t.nkeys, (int)t.U, (int)t.Up, t.W.p);
     GLI_CHECK_LAUNCH();
+    t.reach.alloc((size_t)(3 * t.nkeys));
+    k_key_reach<<<(unsigned)((t.nkeys + 7) / 8), 256, 0, s>>>(t.W.p, t.nkeys, (int)t.U, (int)t.Up, t.reach.p);
+    GLI_CHECK_LAUNCH();
+    std::vector<int2> reach((size_t)(3 * t.nkeys));
+    GLI_CUDA(cudaMemcpyAsync(reach.data(), t.reach.p, t.nkeys * sizeof(int2), cudaMemcpyDeviceToHost, s));
     t.T.alloc(t.tlen);
     k_coulomb_table<<<(unsigned)((t.tlen + 255) / 256), 256, 0, s>>>(kind, t.tlen, t.T.p);
     GLI_CHECK_LAUNCH();
+
+    GLI_CUDA(cudaStreamSynchronize(s));
+    {
+        const i64 n = t.nkeys;
+        i64 total = 0, live = 0;
+        for (i64 k = 0; k < n; ++k)
+            if (reach[k].y >= reach[k].x) {
+                total += reach[k].y - reach[k].x + 1;
+                ++live;
+            }
+        t.banded = 4 * total < 3 * live * t.U;
+        int2 from = make_int2((int)t.U, -1), upto = from;
+        for (i64 k = 0; k < n; ++k) {
+            upto = make_int2(std::min(upto.x, reach[k].x), std::max(upto.y, reach[k].y));
+            reach[2 * n + k] = upto;
+            const int2 r = reach[n - 1 - k];
+            from = make_int2(std::min(from.x, r.x), std::max(from.y, r.y));
+            reach[2 * n - 1 - k] = make_int2(from.x & ~1, from.y);
+        }
+        GLI_CUDA(cudaMemcpyAsync(t.reach.p + n, reach.data() + n, 2 * n * sizeof(int2), cudaMemcpyHostToDevice, s));
+    }
 
     const i64 U = t.U, smax = 2 * (U - 1) * (U - 1) + 1;
     DevBuf<uint32_t> mark(smax, s);
