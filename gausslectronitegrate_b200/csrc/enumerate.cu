@@ -20,29 +20,31 @@
 // point p (the unshifted copies are part of every orbit), a canonical tuple has
 // omin[i] = i and omin[q] >= i for each other point q.
 //
-// ERIDA, one pass (k_enum_collect): a thread per slot; each block gathers its
-// survivors in shared memory and sorts them (within a block ascending index is
-// the (slot, partner) order, and blocks cover increasing index ranges), then
-// appends them to a scratch buffer; a scan of the blocks' counts and a copy
-// place the runs in block order.  129^3: 1.4 ms.
+// ERIDA, live slots in closed form: a point that is the smallest of its images
+// is (-a, -b, -c) with a >= b >= c >= 0, so the live slots are numbered by the
+// tetrahedral index of (a, b, c), descending.  A warp takes one slot, a lane each
+// of its 27 partners, and keeps the ballot of the survivors (k_erida_slots); a
+// scan of their counts and a pass over the ballots write the list
+// (k_erida_place).  The orbit test is arithmetic too: the copies' points compare
+// by their sorted absolute coordinates, and where a point's image is the slot's
+// point itself, six axis permutations give the smallest partner (the signs
+// follow, or are free where a coordinate is zero).  33^3: 388 us for a thread per
+// point of the grid over all 48 images, 2 us now; 129^3 1.27 ms, 40 us now.
 //
 // ERI, live slots: at 7^3, 168,092 of the 40 million slots (i, j, k) hold a
 // canonical class, and a thread per slot leaves most lanes of a warp idle
 // beside one busy slot.  The slots that pass the filter are compacted first
-// (k_enum_live); a warp then takes each live slot's partner candidates 32 at
+// (k_enum_live; grids of at most ENUM_DIRECT_SLOTS slots skip it, and its host
+// round trip); a warp then takes each live slot's partner candidates 32 at
 // a time in ascending order, keeps the survivors (placed in order by its
 // ballots) in shared memory and appends them to a scratch buffer, and a scan
-// of the slots' counts and a copy place the runs (k_enum_slots_collect).  7^3:
-// 25 ms against 146 ms for a thread per slot in two passes.  (The same
-// scheme for ERIDA, whose live slots have only 27 cheap candidates each,
-// measured slower at 129^3: 3.6 against 1.4 ms; it serves the ERIDA tests of
-// the live-slot fallback.)
+// of the slots' counts and a copy place the runs (k_enum_slots_collect).
 //
-// Fallbacks, when a block's or a slot's survivors exceed its buffer or the
-// scratch buffer fills: two passes (count, scan, write), over the live slots
-// (k_enum_slots) for ERI and over every slot (k_enum_erida) for ERIDA.  The
-// thread-per-slot two passes of ERI (k_enum_eri) remain for the tests.  The
-// output is sorted by construction on every path.
+// Fallbacks, when a slot's survivors exceed its buffer or the scratch buffer
+// fills: two passes (count, scan, write) over the live slots (k_enum_slots).
+// The thread-per-slot two passes (k_enum_erida, k_enum_eri) and the live-slot
+// passes for ERIDA remain for the tests.  The output is sorted by construction
+// on every path.
 #include <algorithm>
 #include <climits>
 #include <cstdlib>
@@ -137,8 +139,8 @@ __device__ inline void eri_candidates(const SymGrid& G, i64 t, Emit&& emit) {
                     if (G.omin[l] < (int)i) continue;
                     const int bz = min(lo[2], p[3][2]) + max(hi[2], p[3][2]);
                     const int bias[3] = {bx, by, bz};
-                    const i64 idx = base + l;
-                    if (canonical_quad(G, p, bias, idx)) emit(idx);
+                    const int pts[4] = {(int)i, (int)j, (int)k, (int)l};
+                    if (canonical_quad(G, pts, bias)) emit(base + l);
                 }
             }
         }
@@ -153,19 +155,125 @@ __device__ inline void slot_candidates(const SymGrid& G, i64 t, Emit&& emit) {
         eri_candidates(G, t, emit);
 }
 
-// smallest linear index among the 48 O_h images of each grid point
-__global__ void k_orbit_min(SymGrid G, int* __restrict__ omin) {
+// smallest linear index among the 48 O_h images of each grid point, and (images
+// non-null: ERI) the images themselves, 16 bits each
+__global__ void k_orbit_min(SymGrid G, int* __restrict__ omin, uint4* __restrict__ images) {
     const i64 p = (i64)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= G.N) return;
     int q[3];
     point_of(G, p, q);
     i64 best = p;
+    uint32_t w[4] = {0, 0, 0, 0};
     for (int g = 0; g < 48; ++g) {
         int r[3];
         oh_apply(g, q, r);
-        best = min(best, lin3(G, r));
+        const i64 l = lin3(G, r);
+        best = min(best, l);
+        if (!images) continue;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k == (g >> 1 & 3)) w[k] = g & 1 ? w[k] | (uint32_t)l << 16 : (uint32_t)l;
+        if ((g & 7) == 7) images[p * 6 + (g >> 3)] = make_uint4(w[0], w[1], w[2], w[3]);
     }
     omin[p] = (int)best;
+}
+
+// ---------------------------------------------------------------------------
+// ERIDA: live slots in closed form
+
+// live slot s (ascending linear index) of extent e -> (a, b, c): the tetrahedral
+// index from the other end
+__device__ __forceinline__ void erida_slot_point(i64 t, int& a, int& b, int& c) {
+    a = (int)cbrt(6.0 * (double)t);
+    while ((i64)(a + 1) * (a + 2) * (a + 3) / 6 <= t) ++a;
+    while ((i64)a * (a + 1) * (a + 2) / 6 > t) --a;
+    const i64 r = t - (i64)a * (a + 1) * (a + 2) / 6;
+    b = (int)((sqrt(8.0 * (double)r + 1.0) - 1.0) * 0.5);
+    while ((i64)(b + 1) * (b + 2) / 2 <= r) ++b;
+    while ((i64)b * (b + 1) / 2 > r) --b;
+    c = (int)(r - (i64)b * (b + 1) / 2);
+}
+
+// sorted absolute coordinates, largest first, 10 bits each: a larger key is a
+// smaller smallest image
+__device__ __forceinline__ uint32_t orbit_key(int x, int y, int z) {
+    const int a = absi(x), b = absi(y), c = absi(z);
+    const int hi = max(a, max(b, c)), lo = min(a, min(b, c));
+    return (uint32_t)hi << 20 | (uint32_t)(a + b + c - hi - lo) << 10 | (uint32_t)lo;
+}
+
+// does some O_h element that takes q to (-a, -b, -c) take r below j?
+__device__ __forceinline__ bool partner_below(const int q[3], const int r[3], int a, int b, int c, const int j[3]) {
+    bool below = false;
+#pragma unroll
+    for (int perm = 0; perm < 6; ++perm) {
+        const int a0 = perm < 2 ? 0 : perm < 4 ? 1 : 2;
+        const int a1 = perm == 0 ? 1 : perm == 1 ? 2 : perm == 2 ? 0 : perm == 3 ? 2 : perm == 4 ? 0 : 1;
+        const int a2 = 3 - a0 - a1;
+        const bool maps = absi(q[a0]) == a && absi(q[a1]) == b && absi(q[a2]) == c;
+        const int x = q[a0] == 0 ? -absi(r[a0]) : q[a0] > 0 ? -r[a0] : r[a0];
+        const int y = q[a1] == 0 ? -absi(r[a1]) : q[a1] > 0 ? -r[a1] : r[a1];
+        const int z = q[a2] == 0 ? -absi(r[a2]) : q[a2] > 0 ? -r[a2] : r[a2];
+        below = below || (maps && (x < j[0] || (x == j[0] && (y < j[1] || (y == j[1] && z < j[2])))));
+    }
+    return below;
+}
+
+// a warp per live slot: masks[s] = ballot of its surviving partners (lane
+// 9 tx + 3 ty + tz, ascending j), counts[s] their number
+__global__ void __launch_bounds__(256) k_erida_slots(SymGrid G, i64 nlive, uint32_t* __restrict__ masks,
+                                                     uint32_t* __restrict__ counts) {
+    const i64 s = (i64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (s >= nlive) return;
+    const int lane = threadIdx.x & 31;
+    int a, b, c;
+    erida_slot_point(nlive - 1 - s, a, b, c);
+    const uint32_t key = (uint32_t)a << 20 | (uint32_t)b << 10 | (uint32_t)c;
+    const int tx = lane / 9, ty = lane / 3 % 3, tz = lane % 3;
+    const int p[3] = {-a, -b, -c}, j[3] = {a - 1 + tx, b - 1 + ty, c - 1 + tz};
+    bool keep = lane < 27 && j[0] >= p[0];
+    for (int x = 0; x < 3; ++x) keep = keep && absi(j[x]) <= G.e;
+    if (keep) {
+        const int bias[3] = {tx - 1, ty - 1, tz - 1};
+        for (int m = 0; m < 8 && keep; ++m) {
+            if ((m & 1 && !bias[0]) || (m & 2 && !bias[1]) || (m & 4 && !bias[2])) continue;
+            int q0[3], q1[3];
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                const int sft = m >> x & 1 ? bias[x] : 0;
+                q0[x] = p[x] - sft;
+                q1[x] = j[x] - sft;
+            }
+            const uint32_t k0 = orbit_key(q0[0], q0[1], q0[2]), k1 = orbit_key(q1[0], q1[1], q1[2]);
+            keep = k0 <= key && k1 <= key;
+            if (keep && k0 == key) keep = !partner_below(q0, q1, a, b, c, j);
+            if (keep && k1 == key) keep = !partner_below(q1, q0, a, b, c, j);
+        }
+    }
+    const unsigned ballot = __ballot_sync(0xffffffffu, keep);
+    if (lane == 0) {
+        masks[s] = ballot;
+        counts[s] = __popc(ballot);
+    }
+}
+
+// the classes of slot s, a thread per slot, at dest[s]
+__global__ void __launch_bounds__(256) k_erida_place(SymGrid G, i64 nlive, const uint32_t* __restrict__ masks,
+                                                     const uint64_t* __restrict__ dest, int64_t* __restrict__ out) {
+    const i64 s = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= nlive) return;
+    uint32_t m = masks[s];
+    if (!m) return;
+    int a, b, c;
+    erida_slot_point(nlive - 1 - s, a, b, c);
+    const int p[3] = {-a, -b, -c};
+    const i64 base = lin3(G, p) * G.N;
+    int64_t* o = out + dest[s];
+    for (; m; m &= m - 1) {
+        const int l = __ffs(m) - 1;
+        const int j[3] = {a - 1 + l / 9, b - 1 + l / 3 % 3, c - 1 + l % 3};
+        *o++ = base + lin3(G, j);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -201,72 +309,13 @@ __global__ void k_enum_eri(SymGrid G, uint32_t* __restrict__ counts, const uint6
 }
 
 // ---------------------------------------------------------------------------
-// one pass (ERIDA: blocks of slots; ERI: live slots)
+// one pass over the live slots
 
 struct EnumStatus {
     unsigned long long used;  // scratch entries reserved
-    int overflow;             // 1: a block's (or slot's) survivors exceeded its buffer; 2: the scratch buffer filled
+    uint64_t total;           // classes in the list (the scan of the runs)
+    int overflow;             // 1: a slot's survivors exceeded its buffer; 2: the scratch buffer filled
 };
-
-// ERIDA in one pass: a thread per slot, survivors sorted per block
-constexpr int ENUM_BLOCK = 128;  // slots per block
-constexpr int ENUM_CAP = 2048;   // survivors a block can hold (16 KB)
-
-template <int KIND>
-__global__ void __launch_bounds__(ENUM_BLOCK) k_enum_collect(SymGrid G, i64 slots, int64_t* __restrict__ scratch,
-                                                             unsigned long long cap, uint32_t* __restrict__ run_n,
-                                                             unsigned long long* __restrict__ run_off,
-                                                             EnumStatus* __restrict__ st) {
-    __shared__ int64_t buf[ENUM_CAP];
-    __shared__ int n;
-    __shared__ unsigned long long off;
-    if (threadIdx.x == 0) n = 0;
-    __syncthreads();
-    const i64 t = (i64)blockIdx.x * ENUM_BLOCK + threadIdx.x;
-    if (t < slots)
-        slot_candidates<KIND>(G, t, [&](i64 idx) {
-            const int k = atomicAdd(&n, 1);
-            if (k < ENUM_CAP) buf[k] = idx;
-        });
-    __syncthreads();
-    const int cnt = n;  // the same for every thread: the returns below are uniform
-    if (cnt == 0 || cnt > ENUM_CAP) {
-        if (threadIdx.x == 0) {
-            run_n[blockIdx.x] = 0;
-            if (cnt > ENUM_CAP) atomicOr(&st->overflow, 1);
-        }
-        return;
-    }
-    // bitonic sort, padded to a power of two with the largest index
-    int np = 1;
-    while (np < cnt) np <<= 1;
-    for (int k = cnt + threadIdx.x; k < np; k += ENUM_BLOCK) buf[k] = LLONG_MAX;
-    __syncthreads();
-    for (int k = 2; k <= np; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < np; i += ENUM_BLOCK) {
-                const int x = i ^ j;
-                if (x > i) {
-                    const int64_t a = buf[i], b = buf[x];
-                    if ((a > b) == ((i & k) == 0)) {
-                        buf[i] = b;
-                        buf[x] = a;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    if (threadIdx.x == 0) {
-        off = atomicAdd(&st->used, (unsigned long long)cnt);
-        const bool fits = off + cnt <= cap;
-        run_n[blockIdx.x] = fits ? (uint32_t)cnt : 0u;
-        run_off[blockIdx.x] = off;
-        if (!fits) atomicOr(&st->overflow, 2);
-    }
-    __syncthreads();
-    if (off + cnt > cap) return;
-    for (int k = threadIdx.x; k < cnt; k += ENUM_BLOCK) scratch[off + k] = buf[k];
-}
 
 // each slot's run from the scratch buffer to its place (dest: exclusive scan
 // of the run lengths in slot order); one warp per run
@@ -284,44 +333,28 @@ __global__ void k_enum_place(const int64_t* __restrict__ scratch, const uint32_t
     }
 }
 
-// scratch entries: ERIDA lists have L (L + 1) (L + 2) / 6 classes; ERI lists
-// about N^4 / 3,900 at L = 7 (and a falling fraction beyond), so N^4 / 1024
-// with a floor; at most 2^26 entries (512 MB); a list that does not fit takes
-// the two passes
-static i64 enum_scratch(int kind, const SymGrid& G) {
-    const double L = G.L, N = (double)G.N;
-    const double want = kind == 0 ? L * (L + 1) * (L + 2) / 6 + 1024 : N * N * N * N / 1024 + (1 << 20);
-    return (i64)std::min(want, (double)((i64)1 << 26));
+// scratch entries of ERI lists, which hold about N^4 / 3,900 classes at L = 7
+// (and a falling fraction beyond): N^4 / 1024 with a floor; at most 2^26 entries
+// (512 MB); a list that does not fit takes the two passes
+static i64 enum_scratch(const SymGrid& G) {
+    const double N = (double)G.N;
+    return (i64)std::min(N * N * N * N / 1024 + (1 << 20), (double)((i64)1 << 26));
 }
 
-// one pass into out (allocated here); false when it did not fit
-template <int KIND>
-static bool enumerate_one_pass(const SymGrid& G, i64 slots, int64_t** d_out, i64* total, int num_sms,
-                               cudaStream_t s) {
-    const i64 runs = (slots + ENUM_BLOCK - 1) / ENUM_BLOCK;
-    const i64 cap = enum_scratch(KIND, G);
-    DevBuf<int64_t> scratch(cap, s);
-    DevBuf<uint32_t> run_n(runs, s);
-    DevBuf<unsigned long long> run_off(runs, s);
-    DevBuf<EnumStatus> st(1, s);
-    st.zero();
-    k_enum_collect<KIND><<<(unsigned)runs, ENUM_BLOCK, 0, s>>>(G, slots, scratch.p, (unsigned long long)cap, run_n.p,
-                                                               run_off.p, st.p);
+// the ERIDA list through the live slots in closed form
+static i64 enumerate_erida(const SymGrid& G, int64_t** d_out, cudaStream_t s) {
+    const i64 e = G.e, nlive = (e + 1) * (e + 2) * (e + 3) / 6;
+    DevBuf<uint32_t> masks(nlive, s), counts(nlive, s);
+    DevBuf<uint64_t> dest(nlive, s);
+    k_erida_slots<<<(unsigned)((nlive + 7) / 8), 256, 0, s>>>(G, nlive, masks.p, counts.p);
     GLI_CHECK_LAUNCH();
-    DevBuf<uint64_t> dest(runs, s);
-    const i64 n = exclusive_scan_u32(run_n.p, dest.p, runs, s);  // synchronises
-    EnumStatus h;
-    GLI_CUDA(cudaMemcpyAsync(&h, st.p, sizeof(h), cudaMemcpyDeviceToHost, s));
-    GLI_CUDA(cudaStreamSynchronize(s));
-    if (h.overflow) return false;
+    const i64 total = exclusive_scan_u32(counts.p, dest.p, nlive, s);
     int64_t* out = nullptr;
-    GLI_CUDA(cudaMallocAsync((void**)&out, (n > 0 ? n : 1) * sizeof(int64_t), s));
-    const unsigned grid = (unsigned)std::max<i64>(1, std::min<i64>((runs + 7) / 8, (i64)num_sms * 16));
-    k_enum_place<<<grid, 256, 0, s>>>(scratch.p, run_n.p, run_off.p, dest.p, runs, out);
+    GLI_CUDA(cudaMallocAsync((void**)&out, (total > 0 ? total : 1) * sizeof(int64_t), s));
+    k_erida_place<<<(unsigned)((nlive + 255) / 256), 256, 0, s>>>(G, nlive, masks.p, dest.p, out);
     GLI_CHECK_LAUNCH();
     *d_out = out;
-    *total = n;
-    return true;
+    return total;
 }
 
 // can slot t hold a canonical class: the omin filter (ERIDA: i canonical;
@@ -435,8 +468,9 @@ __device__ inline uint32_t eri_slot_walk(const SymGrid& G, i64 t, int lane, Emit
                     const int bias[3] = {min(lo[0], p[3][0]) + max(hi[0], p[3][0]),
                                          min(lo[1], p[3][1]) + max(hi[1], p[3][1]),
                                          min(lo[2], p[3][2]) + max(hi[2], p[3][2])};
+                    const int pts[4] = {(int)i, (int)j, (int)k, (int)l};
                     idx = base + l;
-                    keep = canonical_quad(G, p, bias, idx);
+                    keep = canonical_quad(G, pts, bias);
                 }
             }
             const unsigned b = __ballot_sync(0xffffffffu, keep);
@@ -487,7 +521,12 @@ __global__ void __launch_bounds__(256) k_enum_slots_collect(SymGrid G, const int
     const i64 warps = (i64)gridDim.x * (blockDim.x >> 5);
     int64_t* mine = buf[warp];
     for (i64 sl = (i64)blockIdx.x * (blockDim.x >> 5) + warp; sl < nlive; sl += warps) {
-        const uint32_t c = slot_walk<KIND>(G, slot_ids[sl], lane, [&](i64 idx, uint32_t rank) {
+        // (without slot_ids: every slot, the dead ones passed over here)
+        if (!slot_ids && !slot_live<KIND>(G, sl)) {
+            if (lane == 0) run_n[sl] = 0u;
+            continue;
+        }
+        const uint32_t c = slot_walk<KIND>(G, slot_ids ? slot_ids[sl] : sl, lane, [&](i64 idx, uint32_t rank) {
             if (idx >= 0 && rank < ENUM_SLOT_CAP) mine[rank] = idx;
         });
         __syncwarp();
@@ -506,18 +545,53 @@ __global__ void __launch_bounds__(256) k_enum_slots_collect(SymGrid G, const int
     }
 }
 
+// grids of at most this many slots (3^3: 19,683) are walked without compacting
+// the live ones first: a warp passes over a dead slot in less time than the host
+// takes to learn their number
+constexpr i64 ENUM_DIRECT_SLOTS = 1 << 16;
+
 // collect = false: the count and write passes over the live slots (the
 // fallback of a slot with more survivors than a warp's buffer)
 template <int KIND>
 static i64 enumerate_live(const SymGrid& G, bool collect, int64_t** d_out, int num_sms, cudaStream_t s) {
     const i64 slots = KIND == 0 ? G.N : G.N * G.N * G.N;
+    int64_t* out = nullptr;
+    // one pass: survivors kept per warp, appended to scratch, placed in slot
+    // order; false when they do not fit
+    auto one_pass = [&](const int64_t* ids, i64 n, i64* total) {
+        const unsigned grid = (unsigned)std::max<i64>(1, std::min<i64>((n + 7) / 8, (i64)num_sms * 16));
+        const i64 cap = enum_scratch(G);
+        DevBuf<int64_t> scratch(cap, s);
+        DevBuf<uint32_t> run_n(n, s);
+        DevBuf<unsigned long long> run_off(n, s);
+        DevBuf<uint64_t> dest(n, s);
+        DevBuf<EnumStatus> st(1, s);
+        st.zero();
+        k_enum_slots_collect<KIND><<<grid, 256, 0, s>>>(G, ids, n, scratch.p, (unsigned long long)cap, run_n.p,
+                                                        run_off.p, st.p);
+        GLI_CHECK_LAUNCH();
+        exclusive_scan_u32_dev(run_n.p, dest.p, n, &st.p->total, s);
+        EnumStatus h;
+        GLI_CUDA(cudaMemcpyAsync(&h, st.p, sizeof(h), cudaMemcpyDeviceToHost, s));
+        GLI_CUDA(cudaStreamSynchronize(s));
+        if (h.overflow) return false;
+        *total = (i64)h.total;
+        GLI_CUDA(cudaMallocAsync((void**)&out, (h.total > 0 ? h.total : 1) * sizeof(int64_t), s));
+        k_enum_place<<<grid, 256, 0, s>>>(scratch.p, run_n.p, run_off.p, dest.p, n, out);
+        GLI_CHECK_LAUNCH();
+        return true;
+    };
+    i64 total = 0;
+    if (collect && slots <= ENUM_DIRECT_SLOTS && one_pass(nullptr, slots, &total)) {
+        *d_out = out;
+        return total;
+    }
     const i64 nb = (slots + 255) / 256;
     DevBuf<uint32_t> bc(nb, s);
     DevBuf<uint64_t> bo(nb, s);
     k_enum_live<KIND, false><<<(unsigned)nb, 256, 0, s>>>(G, slots, bc.p, nullptr, nullptr);
     GLI_CHECK_LAUNCH();
     const i64 nlive = exclusive_scan_u32(bc.p, bo.p, nb, s);
-    int64_t* out = nullptr;
     if (nlive == 0) {
         GLI_CUDA(cudaMallocAsync((void**)&out, sizeof(int64_t), s));
         *d_out = out;
@@ -526,36 +600,16 @@ static i64 enumerate_live(const SymGrid& G, bool collect, int64_t** d_out, int n
     DevBuf<int64_t> ids(nlive, s);
     k_enum_live<KIND, true><<<(unsigned)nb, 256, 0, s>>>(G, slots, nullptr, bo.p, ids.p);
     GLI_CHECK_LAUNCH();
-    const unsigned grid = (unsigned)std::max<i64>(1, std::min<i64>((nlive + 7) / 8, (i64)num_sms * 16));
-    if (collect) {
-        // one pass: survivors kept per warp, appended to scratch, placed in slot order
-        const i64 cap = enum_scratch(KIND, G);
-        DevBuf<int64_t> scratch(cap, s);
-        DevBuf<uint32_t> run_n(nlive, s);
-        DevBuf<unsigned long long> run_off(nlive, s);
-        DevBuf<EnumStatus> st(1, s);
-        st.zero();
-        k_enum_slots_collect<KIND><<<grid, 256, 0, s>>>(G, ids.p, nlive, scratch.p, (unsigned long long)cap,
-                                                        run_n.p, run_off.p, st.p);
-        GLI_CHECK_LAUNCH();
-        DevBuf<uint64_t> dest(nlive, s);
-        const i64 n = exclusive_scan_u32(run_n.p, dest.p, nlive, s);  // synchronises
-        EnumStatus h;
-        GLI_CUDA(cudaMemcpyAsync(&h, st.p, sizeof(h), cudaMemcpyDeviceToHost, s));
-        GLI_CUDA(cudaStreamSynchronize(s));
-        if (!h.overflow) {
-            GLI_CUDA(cudaMallocAsync((void**)&out, (n > 0 ? n : 1) * sizeof(int64_t), s));
-            k_enum_place<<<grid, 256, 0, s>>>(scratch.p, run_n.p, run_off.p, dest.p, nlive, out);
-            GLI_CHECK_LAUNCH();
-            *d_out = out;
-            return n;
-        }
+    if (collect && one_pass(ids.p, nlive, &total)) {
+        *d_out = out;
+        return total;
     }
+    const unsigned grid = (unsigned)std::max<i64>(1, std::min<i64>((nlive + 7) / 8, (i64)num_sms * 16));
     DevBuf<uint32_t> counts(nlive, s);
     DevBuf<uint64_t> offsets(nlive, s);
     k_enum_slots<KIND, false><<<grid, 256, 0, s>>>(G, ids.p, nlive, counts.p, nullptr, nullptr);
     GLI_CHECK_LAUNCH();
-    const i64 total = exclusive_scan_u32(counts.p, offsets.p, nlive, s);
+    total = exclusive_scan_u32(counts.p, offsets.p, nlive, s);
     GLI_CUDA(cudaMallocAsync((void**)&out, (total > 0 ? total : 1) * sizeof(int64_t), s));
     k_enum_slots<KIND, true><<<grid, 256, 0, s>>>(G, ids.p, nlive, nullptr, offsets.p, out);
     GLI_CHECK_LAUNCH();
@@ -574,21 +628,23 @@ i64 enumerate_device(int kind, const GridDesc& g, int64_t** d_out, cudaStream_t 
     if (kind == 1 && G.L > 17) fail(GLI_ERR_LIMIT, "ERI enumeration supports grids up to 17^3 (got %d^3)", G.L);
     if (kind == 0 && G.L > 1025) fail(GLI_ERR_LIMIT, "ERIDA enumeration supports grids up to 1025^3");
     const i64 slots = kind == 0 ? G.N : G.N * G.N * G.N;
-    DevBuf<int> omin(G.N, s);
-    k_orbit_min<<<(unsigned)((G.N + 255) / 256), 256, 0, s>>>(G, omin.p);
-    GLI_CHECK_LAUNCH();
-    G.omin = omin.p;
-    // live slots in one pass.  For their tests, GLI_B200_ENUM_TWO_PASS selects
-    // the thread-per-slot two passes, and the value "live" the count and write
-    // passes over the live slots.
+    // For their tests, GLI_B200_ENUM_TWO_PASS selects the thread-per-slot two
+    // passes, and the value "live" the count and write passes over the live
+    // slots.
     const char* two = getenv("GLI_B200_ENUM_TWO_PASS");
     const bool live_two = two && strcmp(two, "live") == 0;
+    if (kind == 0 && !two) return enumerate_erida(G, d_out, s);
+    DevBuf<int> omin(G.N, s);
+    DevBuf<uint4> images;
+    if (kind == 1) images.alloc(6 * G.N, s);
+    k_orbit_min<<<(unsigned)((G.N + 255) / 256), 256, 0, s>>>(G, omin.p, images.p);
+    GLI_CHECK_LAUNCH();
+    G.omin = omin.p;
+    G.images = images.p;
     if (!two || live_two) {
         const int sms = context().num_sms;
         if (kind == 1) return enumerate_live<1>(G, !live_two, d_out, sms, s);
-        if (live_two) return enumerate_live<0>(G, false, d_out, sms, s);
-        i64 total = 0;
-        if (enumerate_one_pass<0>(G, slots, d_out, &total, sms, s)) return total;
+        return enumerate_live<0>(G, false, d_out, sms, s);
     }
     DevBuf<uint32_t> counts(slots, s);
     DevBuf<uint64_t> offsets(slots, s);

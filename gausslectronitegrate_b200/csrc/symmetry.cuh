@@ -4,6 +4,8 @@
 // (src/eri_integrals.c:240-291, src/erida_integrals.c:209-234) with the
 // bias-shift loops of the enumerators and fill routines.
 #pragma once
+#include <limits.h>
+
 #include "gli_internal.cuh"
 
 namespace gli {
@@ -13,6 +15,7 @@ struct SymGrid {
     int L;   // 2e + 1
     i64 N;   // L^3
     const int* omin = nullptr;  // enumeration: smallest linear index among each point's 48 O_h images
+    const uint4* images = nullptr;  // ERI enumeration: the 48 images themselves, 16 bits each (N <= 65535), 6 uint4 a point
 };
 
 __device__ inline i64 lin3(const SymGrid& G, const int q[3]) {
@@ -44,27 +47,43 @@ __device__ inline bool canonical_pair(const SymGrid& G, const int p[2][3], const
     return true;
 }
 
-// ERI: is (p0, p1, p2, p3) the smallest index of its orbit?
-__device__ inline bool canonical_quad(const SymGrid& G, const int p[4][3], const int bias[3], i64 idx) {
-    const i64 N2 = G.N * G.N;
+// ERI: is (l0, l1, l2, l3) (linear point indices, l0 the leading one) the
+// smallest index of its orbit?  An image's index leads with its smallest
+// point.  omin rules a shifted copy out at once when no point of it has an image
+// at l0 or below, and decides at once when one lies below; only copies with an
+// image at l0 look at their images, read eight per load from the table.  The
+// index pairs compare in 32 bits (N^2 < 2^32).
+__device__ inline bool canonical_quad(const SymGrid& G, const int l[4], const int bias[3]) {
+    const uint32_t N = (uint32_t)G.N;
+    const uint32_t ij = l[0] * N + l[1], kl = l[2] * N + l[3];
     for (int bx = 0; bx <= absi(bias[0]); ++bx)
         for (int by = 0; by <= absi(bias[1]); ++by)
             for (int bz = 0; bz <= absi(bias[2]); ++bz) {
-                const int sft[3] = {bx * bias[0], by * bias[1], bz * bias[2]};
-                int q[4][3];
-                for (int k = 0; k < 4; ++k)
-                    for (int a = 0; a < 3; ++a) q[k][a] = p[k][a] - sft[a];
-                for (int g = 0; g < 48; ++g) {
-                    i64 l4[4];
-                    for (int k = 0; k < 4; ++k) {
-                        int r[3];
-                        oh_apply(g, q[k], r);
-                        l4[k] = lin3(G, r);
+                const int sft = ((bx * bias[0]) * G.L + by * bias[1]) * G.L + bz * bias[2];
+                int q[4], least = INT_MAX;
+                for (int k = 0; k < 4; ++k) {
+                    q[k] = l[k] - sft;
+                    least = min(least, G.omin[q[k]]);
+                }
+                if (least < l[0]) return false;
+                if (least > l[0]) continue;
+                for (int c = 0; c < 6; ++c) {
+                    uint4 im[4];
+                    for (int k = 0; k < 4; ++k) im[k] = __ldg(G.images + (i64)q[k] * 6 + c);
+#pragma unroll
+                    for (int h = 0; h < 8; ++h) {
+                        uint32_t r[4];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const uint32_t w = h < 2 ? im[k].x : h < 4 ? im[k].y : h < 6 ? im[k].z : im[k].w;
+                            r[k] = h & 1 ? w >> 16 : w & 0xffffu;
+                        }
+                        if (min(min(r[0], r[1]), min(r[2], r[3])) != (uint32_t)l[0]) continue;
+                        const uint32_t ab = min(r[0], r[1]) * N + max(r[0], r[1]);
+                        const uint32_t cd = min(r[2], r[3]) * N + max(r[2], r[3]);
+                        const uint32_t first = min(ab, cd), second = max(ab, cd);
+                        if (first < ij || (first == ij && second < kl)) return false;
                     }
-                    i64 ab = l4[0] <= l4[1] ? l4[0] * G.N + l4[1] : l4[1] * G.N + l4[0];
-                    i64 cd = l4[2] <= l4[3] ? l4[2] * G.N + l4[3] : l4[3] * G.N + l4[2];
-                    if (ab > cd) { i64 t = ab; ab = cd; cd = t; }
-                    if (ab * N2 + cd < idx) return false;
                 }
             }
     return true;
