@@ -29,16 +29,17 @@
 // by their sorted absolute coordinates, and where a point's image is the slot's
 // point itself, six axis permutations give the smallest partner (the signs
 // follow, or are free where a coordinate is zero).  33^3: 388 us for a thread per
-// point of the grid over all 48 images, 2 us now; 129^3 1.27 ms, 40 us now.
+// point of the grid over all 48 images, 5 us now; the 129^3 list 1.4 ms, now 0.16
+// ms with its copy.
 //
 // ERI, live slots: at 7^3, 168,092 of the 40 million slots (i, j, k) hold a
 // canonical class, and a thread per slot leaves most lanes of a warp idle
 // beside one busy slot.  The slots that pass the filter are compacted first
-// (k_enum_live; grids of at most ENUM_DIRECT_SLOTS slots skip it, and its host
-// round trip); a warp then takes each live slot's partner candidates 32 at
+// (k_enum_live; 3^3 skips it, k_enum_small); a warp then takes each live slot's partner candidates 32 at
 // a time in ascending order, keeps the survivors (placed in order by its
 // ballots) in shared memory and appends them to a scratch buffer, and a scan
-// of the slots' counts and a copy place the runs (k_enum_slots_collect).
+// of the slots' counts and a copy place the runs (k_enum_slots_collect).  7^3:
+// 25 ms with arithmetic images of every copy, 3.5 ms reading them from the table.
 //
 // Fallbacks, when a slot's survivors exceed its buffer or the scratch buffer
 // fills: two passes (count, scan, write) over the live slots (k_enum_slots).
@@ -106,15 +107,40 @@ __device__ inline int axis_partners(int lo, int hi, int e, int lmin, signed char
     return n;
 }
 
+// ERI slot t = (i N + j) N + k -> points, and a point's coordinates, in 32-bit
+// arithmetic where the slots fit it (grids up to 11^3): 64-bit divisions took
+// most of a small grid's walk
+__device__ __forceinline__ void eri_slot_points(const SymGrid& G, i64 t, int& i, int& j, int& k) {
+    const uint32_t N = (uint32_t)G.N;
+    if (N <= 1625) {
+        const uint32_t u = (uint32_t)t, ij = u / N;
+        k = (int)(u - ij * N);
+        i = (int)(ij / N);
+        j = (int)(ij - i * N);
+    } else {
+        const uint32_t ij = (uint32_t)(t / N);  // (N^2 < 2^32)
+        k = (int)(t - (i64)ij * N);
+        i = (int)(ij / N);
+        j = (int)(ij - i * N);
+    }
+}
+__device__ __forceinline__ void point32(const SymGrid& G, int lin, int p[3]) {
+    const int r = lin / G.L, x = r / G.L;
+    p[2] = lin - r * G.L - G.e;
+    p[1] = r - x * G.L - G.e;
+    p[0] = x - G.e;
+}
+
 // ERI: slot t = (i, j, k)
 template <class Emit>
 __device__ inline void eri_candidates(const SymGrid& G, i64 t, Emit&& emit) {
-    const i64 i = t / (G.N * G.N), j = (t / G.N) % G.N, k = t % G.N;
-    if (G.omin[i] != (int)i || G.omin[j] < (int)i || G.omin[k] < (int)i) return;
+    int i, j, k;
+    eri_slot_points(G, t, i, j, k);
+    if (G.omin[i] != i || G.omin[j] < i || G.omin[k] < i) return;
     int p[4][3];
-    point_of(G, i, p[0]);
-    point_of(G, j, p[1]);
-    point_of(G, k, p[2]);
+    point32(G, i, p[0]);
+    point32(G, j, p[1]);
+    point32(G, k, p[2]);
     // reference x-ordering: i <= j, i <= k (and k <= l below) on the x coordinate
     if (p[0][0] <= p[1][0] && p[0][0] <= p[2][0]) {
         signed char sx[MAX_AXIS], sy[MAX_AXIS], sz[MAX_AXIS];
@@ -126,7 +152,7 @@ __device__ inline void eri_candidates(const SymGrid& G, i64 t, Emit&& emit) {
         const int nx = axis_partners(lo[0], hi[0], G.e, p[2][0], sx);
         const int ny = axis_partners(lo[1], hi[1], G.e, -G.e, sy);
         const int nz = axis_partners(lo[2], hi[2], G.e, -G.e, sz);
-        const i64 base = ((i * G.N + j) * G.N + k) * G.N;
+        const i64 base = t * G.N;
         for (int ax = 0; ax < nx; ++ax) {
             p[3][0] = sx[ax];
             const int bx = min(lo[0], p[3][0]) + max(hi[0], p[3][0]);
@@ -139,7 +165,7 @@ __device__ inline void eri_candidates(const SymGrid& G, i64 t, Emit&& emit) {
                     if (G.omin[l] < (int)i) continue;
                     const int bz = min(lo[2], p[3][2]) + max(hi[2], p[3][2]);
                     const int bias[3] = {bx, by, bz};
-                    const int pts[4] = {(int)i, (int)j, (int)k, (int)l};
+                    const int pts[4] = {i, j, k, (int)l};
                     if (canonical_quad(G, pts, bias)) emit(base + l);
                 }
             }
@@ -156,26 +182,29 @@ __device__ inline void slot_candidates(const SymGrid& G, i64 t, Emit&& emit) {
 }
 
 // smallest linear index among the 48 O_h images of each grid point, and (images
-// non-null: ERI) the images themselves, 16 bits each
-__global__ void k_orbit_min(SymGrid G, int* __restrict__ omin, uint4* __restrict__ images) {
-    const i64 p = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= G.N) return;
-    int q[3];
-    point_of(G, p, q);
-    i64 best = p;
-    uint32_t w[4] = {0, 0, 0, 0};
-    for (int g = 0; g < 48; ++g) {
-        int r[3];
-        oh_apply(g, q, r);
-        const i64 l = lin3(G, r);
-        best = min(best, l);
-        if (!images) continue;
+// non-null: ERI) the images themselves, 16 bits each; eight lanes a point, six of
+// them with eight images each
+__global__ void __launch_bounds__(256) k_orbit_min(SymGrid G, int* __restrict__ omin, uint4* __restrict__ images) {
+    const i64 p = (i64)blockIdx.x * (blockDim.x >> 3) + (threadIdx.x >> 3);
+    const int c = threadIdx.x & 7;
+    int best = INT_MAX;
+    if (p < G.N && c < 6) {
+        int q[3];
+        point32(G, (int)p, q);
+        uint32_t w[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (k == (g >> 1 & 3)) w[k] = g & 1 ? w[k] | (uint32_t)l << 16 : (uint32_t)l;
-        if ((g & 7) == 7) images[p * 6 + (g >> 3)] = make_uint4(w[0], w[1], w[2], w[3]);
+        for (int h = 0; h < 8; ++h) {
+            int r[3];
+            oh_apply(8 * c + h, q, r);
+            const int l = ((r[0] + G.e) * G.L + r[1] + G.e) * G.L + r[2] + G.e;
+            best = min(best, l);
+            w[h >> 1] = h & 1 ? w[h >> 1] | (uint32_t)l << 16 : (uint32_t)l;
+        }
+        if (images) images[p * 6 + c] = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    omin[p] = (int)best;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
+    if (p < G.N && c == 0) omin[p] = best;
 }
 
 // ---------------------------------------------------------------------------
@@ -363,13 +392,12 @@ static i64 enumerate_erida(const SymGrid& G, int64_t** d_out, cudaStream_t s) {
 template <int KIND>
 __device__ inline bool slot_live(const SymGrid& G, i64 t) {
     if (KIND == 0) return G.omin[t] == (int)t;
-    const i64 N = G.N;
-    const i64 i = t / (N * N), j = (t / N) % N, k = t % N;
-    if (G.omin[i] != (int)i || G.omin[j] < (int)i || G.omin[k] < (int)i) return false;
+    int i, j, k;
+    eri_slot_points(G, t, i, j, k);
+    if (G.omin[i] != i || G.omin[j] < i || G.omin[k] < i) return false;
     // x coordinate: the leading digit of the x-major linear index
-    const i64 LL = (i64)G.L * G.L;
-    const i64 xi = i / LL;
-    return xi <= j / LL && xi <= k / LL;
+    const int x0 = i / (G.L * G.L) * (G.L * G.L);
+    return x0 <= j && x0 <= k;
 }
 
 // WRITE = false: live slots per block of 256; WRITE = true: their ids at the
@@ -437,11 +465,12 @@ template <class Emit>
 __device__ inline uint32_t eri_slot_walk(const SymGrid& G, i64 t, int lane, Emit&& emit) {
     const i64 N = G.N;
     {
-        const i64 i = t / (N * N), j = (t / N) % N, k = t % N;
+        int i, j, k;
+        eri_slot_points(G, t, i, j, k);
         int p[4][3];
-        point_of(G, i, p[0]);
-        point_of(G, j, p[1]);
-        point_of(G, k, p[2]);
+        point32(G, i, p[0]);
+        point32(G, j, p[1]);
+        point32(G, k, p[2]);
         signed char sx[MAX_AXIS], sy[MAX_AXIS], sz[MAX_AXIS];
         int lo[3], hi[3];
         for (int a = 0; a < 3; ++a) {
@@ -463,12 +492,12 @@ __device__ inline uint32_t eri_slot_walk(const SymGrid& G, i64 t, int lane, Emit
                 p[3][0] = sx[ax];
                 p[3][1] = sy[ay];
                 p[3][2] = sz[az];
-                const i64 l = lin3(G, p[3]);
-                if (G.omin[l] >= (int)i) {
+                const int l = ((p[3][0] + G.e) * G.L + p[3][1] + G.e) * G.L + p[3][2] + G.e;
+                if (G.omin[l] >= i) {
                     const int bias[3] = {min(lo[0], p[3][0]) + max(hi[0], p[3][0]),
                                          min(lo[1], p[3][1]) + max(hi[1], p[3][1]),
                                          min(lo[2], p[3][2]) + max(hi[2], p[3][2])};
-                    const int pts[4] = {(int)i, (int)j, (int)k, (int)l};
+                    const int pts[4] = {i, j, k, l};
                     idx = base + l;
                     keep = canonical_quad(G, pts, bias);
                 }
@@ -521,12 +550,7 @@ __global__ void __launch_bounds__(256) k_enum_slots_collect(SymGrid G, const int
     const i64 warps = (i64)gridDim.x * (blockDim.x >> 5);
     int64_t* mine = buf[warp];
     for (i64 sl = (i64)blockIdx.x * (blockDim.x >> 5) + warp; sl < nlive; sl += warps) {
-        // (without slot_ids: every slot, the dead ones passed over here)
-        if (!slot_ids && !slot_live<KIND>(G, sl)) {
-            if (lane == 0) run_n[sl] = 0u;
-            continue;
-        }
-        const uint32_t c = slot_walk<KIND>(G, slot_ids ? slot_ids[sl] : sl, lane, [&](i64 idx, uint32_t rank) {
+        const uint32_t c = slot_walk<KIND>(G, slot_ids[sl], lane, [&](i64 idx, uint32_t rank) {
             if (idx >= 0 && rank < ENUM_SLOT_CAP) mine[rank] = idx;
         });
         __syncwarp();
@@ -545,10 +569,77 @@ __global__ void __launch_bounds__(256) k_enum_slots_collect(SymGrid G, const int
     }
 }
 
-// grids of at most this many slots (3^3: 19,683) are walked without compacting
-// the live ones first: a warp passes over a dead slot in less time than the host
-// takes to learn their number
-constexpr i64 ENUM_DIRECT_SLOTS = 1 << 16;
+// ERI grids up to 3^3 (at most 27 partners a slot): a block per slot of the live
+// leading points (those in closed form as for ERIDA: 4 of 27), without compacting
+// the live slots and the host round trip for their number.  The few slots do not
+// fill the GPU, so each is spread out: a warp takes four partners, eight lanes
+// each, a lane per shifted copy.  (3^3: 53 us with a warp per slot and a lane per
+// partner, one chain of up to eight copies' images.)
+constexpr int ENUM_SMALL_L = 3;
+
+__global__ void __launch_bounds__(256) k_enum_small(SymGrid G, i64 npoints, int64_t* __restrict__ scratch,
+                                                    unsigned long long cap, uint32_t* __restrict__ run_n,
+                                                    unsigned long long* __restrict__ run_off,
+                                                    EnumStatus* __restrict__ st) {
+    __shared__ unsigned kept;
+    const int N = (int)G.N, N2 = N * N, sl = blockIdx.x, lane = threadIdx.x & 31;
+    int a, b, c;
+    erida_slot_point(npoints - 1 - sl / N2, a, b, c);
+    const int p0[3] = {-a, -b, -c};
+    const i64 t = lin3(G, p0) * N2 + sl % N2;
+    if (!slot_live<1>(G, t)) {
+        if (threadIdx.x == 0) run_n[sl] = 0u;
+        return;
+    }
+    if (threadIdx.x == 0) kept = 0u;
+    __syncthreads();
+    int i, j, k, p[4][3], lo[3], hi[3];
+    eri_slot_points(G, t, i, j, k);
+    point32(G, i, p[0]);
+    point32(G, j, p[1]);
+    point32(G, k, p[2]);
+    signed char sx[MAX_AXIS], sy[MAX_AXIS], sz[MAX_AXIS];
+    for (int x = 0; x < 3; ++x) {
+        lo[x] = min(min(p[0][x], p[1][x]), p[2][x]);
+        hi[x] = max(max(p[0][x], p[1][x]), p[2][x]);
+    }
+    const int nx = axis_partners(lo[0], hi[0], G.e, p[2][0], sx);
+    const int ny = axis_partners(lo[1], hi[1], G.e, -G.e, sy);
+    const int nz = axis_partners(lo[2], hi[2], G.e, -G.e, sz);
+    const int total = nx * ny * nz;  // (at most 27)
+    auto partner = [&](int cand, int q[3]) {
+        q[0] = sx[cand / (nz * ny)];
+        q[1] = sy[cand / nz % ny];
+        q[2] = sz[cand % nz];
+        return ((q[0] + G.e) * G.L + q[1] + G.e) * G.L + q[2] + G.e;
+    };
+    const int cand = threadIdx.x >> 3, m = lane & 7;
+    bool keep = false;
+    if (cand < total) {
+        const int l = partner(cand, p[3]);
+        if (G.omin[l] >= i) {
+            int bias[3];
+            for (int x = 0; x < 3; ++x) bias[x] = min(lo[x], p[3][x]) + max(hi[x], p[3][x]);
+            const int pts[4] = {i, j, k, l};
+            keep = !copy_exists(bias, m) || canonical_copy(G, pts, copy_shift(G, bias, m));
+        }
+    }
+    const unsigned vote = __ballot_sync(0xffffffffu, keep) >> (lane & 24) & 0xffu;
+    if (m == 0 && vote == 0xffu) atomicOr(&kept, 1u << cand);  // a partner survives in all its copies
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    const unsigned list = kept, n = __popc(list);
+    unsigned long long off = 0;
+    if (n && lane == 0) off = atomicAdd(&st->used, (unsigned long long)n);
+    off = __shfl_sync(0xffffffffu, off, 0);
+    const bool fits = off + n <= cap;
+    if (lane == 0) {
+        run_n[sl] = fits ? n : 0u;
+        run_off[sl] = off;
+        if (!fits) atomicOr(&st->overflow, 2);
+    }
+    if (fits && list >> lane & 1u) scratch[off + __popc(list & ((1u << lane) - 1u))] = t * N + partner(lane, p[3]);
+}
 
 // collect = false: the count and write passes over the live slots (the
 // fallback of a slot with more survivors than a warp's buffer)
@@ -567,8 +658,12 @@ static i64 enumerate_live(const SymGrid& G, bool collect, int64_t** d_out, int n
         DevBuf<uint64_t> dest(n, s);
         DevBuf<EnumStatus> st(1, s);
         st.zero();
-        k_enum_slots_collect<KIND><<<grid, 256, 0, s>>>(G, ids, n, scratch.p, (unsigned long long)cap, run_n.p,
-                                                        run_off.p, st.p);
+        if (ids)
+            k_enum_slots_collect<KIND><<<grid, 256, 0, s>>>(G, ids, n, scratch.p, (unsigned long long)cap, run_n.p,
+                                                            run_off.p, st.p);
+        else
+            k_enum_small<<<(unsigned)n, 256, 0, s>>>(G, n / (G.N * G.N), scratch.p, (unsigned long long)cap, run_n.p,
+                                                     run_off.p, st.p);
         GLI_CHECK_LAUNCH();
         exclusive_scan_u32_dev(run_n.p, dest.p, n, &st.p->total, s);
         EnumStatus h;
@@ -582,7 +677,8 @@ static i64 enumerate_live(const SymGrid& G, bool collect, int64_t** d_out, int n
         return true;
     };
     i64 total = 0;
-    if (collect && slots <= ENUM_DIRECT_SLOTS && one_pass(nullptr, slots, &total)) {
+    if (KIND == 1 && collect && G.L <= ENUM_SMALL_L &&
+        one_pass(nullptr, (i64)(G.e + 1) * (G.e + 2) * (G.e + 3) / 6 * G.N * G.N, &total)) {
         *d_out = out;
         return total;
     }
@@ -637,7 +733,7 @@ i64 enumerate_device(int kind, const GridDesc& g, int64_t** d_out, cudaStream_t 
     DevBuf<int> omin(G.N, s);
     DevBuf<uint4> images;
     if (kind == 1) images.alloc(6 * G.N, s);
-    k_orbit_min<<<(unsigned)((G.N + 255) / 256), 256, 0, s>>>(G, omin.p, images.p);
+    k_orbit_min<<<(unsigned)((G.N + 31) / 32), 256, 0, s>>>(G, omin.p, images.p);
     GLI_CHECK_LAUNCH();
     G.omin = omin.p;
     G.images = images.p;

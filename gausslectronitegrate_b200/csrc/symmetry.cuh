@@ -53,39 +53,45 @@ __device__ inline bool canonical_pair(const SymGrid& G, const int p[2][3], const
 // at l0 or below, and decides at once when one lies below; only copies with an
 // image at l0 look at their images, read eight per load from the table.  The
 // index pairs compare in 32 bits (N^2 < 2^32).
-__device__ inline bool canonical_quad(const SymGrid& G, const int l[4], const int bias[3]) {
+__device__ inline bool canonical_copy(const SymGrid& G, const int l[4], int sft) {  // (the copy moved by -sft)
     const uint32_t N = (uint32_t)G.N;
     const uint32_t ij = l[0] * N + l[1], kl = l[2] * N + l[3];
-    for (int bx = 0; bx <= absi(bias[0]); ++bx)
-        for (int by = 0; by <= absi(bias[1]); ++by)
-            for (int bz = 0; bz <= absi(bias[2]); ++bz) {
-                const int sft = ((bx * bias[0]) * G.L + by * bias[1]) * G.L + bz * bias[2];
-                int q[4], least = INT_MAX;
-                for (int k = 0; k < 4; ++k) {
-                    q[k] = l[k] - sft;
-                    least = min(least, G.omin[q[k]]);
-                }
-                if (least < l[0]) return false;
-                if (least > l[0]) continue;
-                for (int c = 0; c < 6; ++c) {
-                    uint4 im[4];
-                    for (int k = 0; k < 4; ++k) im[k] = __ldg(G.images + (i64)q[k] * 6 + c);
+    int q[4], least = INT_MAX;
+    for (int k = 0; k < 4; ++k) {
+        q[k] = l[k] - sft;
+        least = min(least, G.omin[q[k]]);
+    }
+    if (least != l[0]) return least > l[0];
+    for (int c = 0; c < 6; ++c) {
+        uint4 im[4];
+        for (int k = 0; k < 4; ++k) im[k] = __ldg(G.images + (i64)q[k] * 6 + c);
 #pragma unroll
-                    for (int h = 0; h < 8; ++h) {
-                        uint32_t r[4];
+        for (int h = 0; h < 8; ++h) {
+            uint32_t r[4];
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const uint32_t w = h < 2 ? im[k].x : h < 4 ? im[k].y : h < 6 ? im[k].z : im[k].w;
-                            r[k] = h & 1 ? w >> 16 : w & 0xffffu;
-                        }
-                        if (min(min(r[0], r[1]), min(r[2], r[3])) != (uint32_t)l[0]) continue;
-                        const uint32_t ab = min(r[0], r[1]) * N + max(r[0], r[1]);
-                        const uint32_t cd = min(r[2], r[3]) * N + max(r[2], r[3]);
-                        const uint32_t first = min(ab, cd), second = max(ab, cd);
-                        if (first < ij || (first == ij && second < kl)) return false;
-                    }
-                }
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t w = h < 2 ? im[k].x : h < 4 ? im[k].y : h < 6 ? im[k].z : im[k].w;
+                r[k] = h & 1 ? w >> 16 : w & 0xffffu;
             }
+            if (min(min(r[0], r[1]), min(r[2], r[3])) != (uint32_t)l[0]) continue;
+            const uint32_t ab = min(r[0], r[1]) * N + max(r[0], r[1]);
+            const uint32_t cd = min(r[2], r[3]) * N + max(r[2], r[3]);
+            const uint32_t first = min(ab, cd), second = max(ab, cd);
+            if (first < ij || (first == ij && second < kl)) return false;
+        }
+    }
+    return true;
+}
+// the shift of copy m (bit a: moved by the bias of axis a) as a linear index
+__device__ __forceinline__ int copy_shift(const SymGrid& G, const int bias[3], int m) {
+    return ((m & 1 ? bias[0] : 0) * G.L + (m & 2 ? bias[1] : 0)) * G.L + (m & 4 ? bias[2] : 0);
+}
+__device__ __forceinline__ bool copy_exists(const int bias[3], int m) {
+    return !((m & 1 && !bias[0]) || (m & 2 && !bias[1]) || (m & 4 && !bias[2]));
+}
+__device__ inline bool canonical_quad(const SymGrid& G, const int l[4], const int bias[3]) {
+    for (int m = 0; m < 8; ++m)
+        if (copy_exists(bias, m) && !canonical_copy(G, l, copy_shift(G, bias, m))) return false;
     return true;
 }
 
