@@ -5,9 +5,12 @@
 // HBM write (8 bytes per entry, almost all zero).  Row i = (ax, ay, az) has
 // its nonzeros on three lines through i: the x line (columns bx P + c, P =
 // ny nz, c = ay nz + az), the y line and the z line inside the x block bx = ax.
-// A block writes whole rows with 16-byte stores; each thread walks its columns
+// A block writes one row with 16-byte stores; each thread walks its columns
 // with the x block and the in-block offset updated incrementally (no division
-// per entry), and only the x block of the row itself decodes (y, z).
+// per entry), and only the x block of the row itself decodes (y, z).  24^3 (1.53
+// GB): 215 us, 7.1 TB/s, where filling the same buffer takes 204 us; 262 us with
+// eight blocks per SM walking the rows, whose last rows left SMs idle, and every
+// entry compared with the lines.
 #include <math.h>
 #include <stdlib.h>
 
@@ -68,37 +71,30 @@ __global__ void __launch_bounds__(256) k_kinetic_matrix(const double* __restrict
     __syncthreads();
     const int P = ny * nz, N = nx * P;
     const int step = 2 * blockDim.x;
-    for (int row = blockIdx.x; row < N; row += gridDim.x) {
-        const int ax = row / P, c = row - ax * P, ay = c / nz, az = c - ay * nz;
-        double* r = out + (i64)row * N;
-        // a row starting on an odd double writes its first entry alone, so
-        // that the pairs stored as double2 sit on 16-byte boundaries
-        const int j0 = (int)(((i64)row * N) & 1);
-        if (j0 && threadIdx.x == 0) r[0] = kinetic_entry(k1, ax, ay, az, c, nz, 0, 0);
-        int j = j0 + 2 * threadIdx.x;
-        int bx = j / P, q = j - bx * P;
-        for (; j + 1 < N; j += step) {
-            const double v0 = kinetic_entry(k1, ax, ay, az, c, nz, bx, q);
-            const int q1 = q + 1 < P ? q + 1 : 0, bx1 = q + 1 < P ? bx : bx + 1;
-            const double v1 = kinetic_entry(k1, ax, ay, az, c, nz, bx1, q1);
-            *reinterpret_cast<double2*>(r + j) = make_double2(v0, v1);
-            q += step;
-            while (q >= P) {
-                q -= P;
-                ++bx;
-            }
+    const int row = blockIdx.x;
+    const int ax = row / P, c = row - ax * P, ay = c / nz, az = c - ay * nz;
+    double* r = out + (i64)row * N;
+    // a row starting on an odd double writes its first entry alone, so
+    // that the pairs stored as double2 sit on 16-byte boundaries
+    const int j0 = (int)(((i64)row * N) & 1);
+    if (j0 && threadIdx.x == 0) r[0] = kinetic_entry(k1, ax, ay, az, c, nz, 0, 0);
+    int j = j0 + 2 * threadIdx.x;
+    int bx = j / P, q = j - bx * P;
+    for (; j + 1 < N; j += step) {
+        const int q1 = q + 1 < P ? q + 1 : 0, bx1 = q + 1 < P ? bx : bx + 1;
+        double2 v = make_double2(0.0, 0.0);
+        if (q == c || q1 == c || bx == ax || bx1 == ax) {  // (few pairs: the row's own x block and the x line)
+            v.x = kinetic_entry(k1, ax, ay, az, c, nz, bx, q);
+            v.y = kinetic_entry(k1, ax, ay, az, c, nz, bx1, q1);
         }
-        if (j < N) r[j] = kinetic_entry(k1, ax, ay, az, c, nz, bx, q);  // an unpaired last entry
+        *reinterpret_cast<double2*>(r + j) = v;
+        q += step;
+        while (q >= P) {
+            q -= P;
+            ++bx;
+        }
     }
-}
-
-// blocks of the matrix kernel: rows spread over a few waves of the current
-// device's SMs (an attribute query: no context state of the library is made)
-static unsigned kinetic_blocks(i64 N) {
-    int dev = 0, sms = 148;
-    GLI_CUDA(cudaGetDevice(&dev));
-    GLI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    return (unsigned)std::min<i64>(N, (i64)sms * 8);
+    if (j < N) r[j] = kinetic_entry(k1, ax, ay, az, c, nz, bx, q);  // an unpaired last entry
 }
 
 void kinetic_table_device(const double* h_coeffs, i64 nb, i64 L, double* d_k1, cudaStream_t s) {
@@ -115,7 +111,7 @@ void kinetic_matrix_device(const double* h_coeffs, i64 nb, const GridDesc& g, do
     kinetic_table_device(h_coeffs, nb, L, k1.p, s);
     const i64 N = g.points();
     if (N >= ((i64)1 << 31)) fail(GLI_ERR_LIMIT, "kinetic matrix of %lld points exceeds the row index range", (long long)N);
-    k_kinetic_matrix<<<kinetic_blocks(N), 256, 0, s>>>(k1.p, (int)L, (int)g.num[0], (int)g.num[1], (int)g.num[2],
+    k_kinetic_matrix<<<(unsigned)N, 256, 0, s>>>(k1.p, (int)L, (int)g.num[0], (int)g.num[1], (int)g.num[2],
                                                        d_out);
     GLI_CHECK_LAUNCH();
 }
@@ -233,7 +229,7 @@ static void kinetic_matrix_noalloc(const double* d_coeffs, i64 nb, const GridDes
     k_kinetic_1d<<<(unsigned)L, 256, 0, s>>>(d_coeffs, (int)nb, table);
     GLI_CHECK_LAUNCH();
     const i64 N = g.points();
-    k_kinetic_matrix<<<kinetic_blocks(N), 256, 0, s>>>(table, (int)L, (int)g.num[0], (int)g.num[1], (int)g.num[2],
+    k_kinetic_matrix<<<(unsigned)N, 256, 0, s>>>(table, (int)L, (int)g.num[0], (int)g.num[1], (int)g.num[2],
                                                        d_out);
     GLI_CHECK_LAUNCH();
 }
