@@ -209,8 +209,9 @@ __global__ void __launch_bounds__(256, NUC_FIELD_BLOCKS) k_nuc_field(const NucIn
 // V[i][j] of every instance from its key-indexed block: Vk[kx][ky * nkz + kz]
 // (zfast: the FP64 contractions) or Vk[kx][kz * nky + ky] (the sliced ones).
 //
-// zfast: block (ix, iy, jx) writes the nz x (ny nz) sub-block of rows
-// (ix, iy, .) and columns (jx, ., .).  Its entries lie in the ny lines
+// zfast: item (iy, ix <= jx) writes the nz x (ny nz) sub-blocks of rows
+// (ix, iy, .) and columns (jx, ., .) and of rows (jx, iy, .) and columns
+// (ix, ., .), which hold the same values.  They lie in the ny lines
 // ky = key(iy, jy) of the slice kx = key(ix, jx).  A few lines at a time are read
 // (coalesced) and laid out in shared memory as the output's rows, each value
 // at (lo, hi) and (hi, lo), then copied out row by row in 16-byte stores.
@@ -242,7 +243,7 @@ __global__ void __launch_bounds__(256) k_nuc_scatter(const NucInst* __restrict__
     const double* Vk = X + in.x_off;
     const uint16_t *rx = tables + in.rk_off[0], *ry = tables + in.rk_off[1], *rz = tables + in.rk_off[2];
     if (zfast && nz <= NUC_LINE_MAX_Z) {
-        const int items = nx * ny * nx;
+        const int items = nx * (nx + 1) / 2 * ny;
         if ((int)blockIdx.x >= items) return;
         const int group = nuc_line_group(ny, nz), pitch = nuc_row_pitch(group, nz);
         const uint16_t* keys = tables + in.key_off[2];
@@ -250,7 +251,12 @@ __global__ void __launch_bounds__(256) k_nuc_scatter(const NucInst* __restrict__
         // (the entries of zero factors are never written below)
         for (int e = threadIdx.x; e < nz * pitch; e += blockDim.x) rows[e] = 0.0;
         for (int item = blockIdx.x; item < items; item += gridDim.x) {
-            const int jx = item % nx, r = item / nx, iy = r % ny, ix = r / ny;
+            // (iy, ix <= jx): the sub-blocks (ix, iy, jx) and (jx, iy, ix) hold the same values
+            const int iy = item % ny, xp = item / ny;
+            int jx = (int)((sqrtf(8.0f * xp + 1.0f) - 1.0f) * 0.5f);
+            while ((jx + 1) * (jx + 2) / 2 <= xp) ++jx;
+            while (jx * (jx + 1) / 2 > xp) --jx;
+            const int ix = xp - jx * (jx + 1) / 2;
             const int kx = rx[ix * nx + jx];
             const double* slice = Vk + (i64)kx * ((i64)nky * nkz);
             for (int j0 = 0; j0 < ny; j0 += group) {
@@ -281,9 +287,12 @@ __global__ void __launch_bounds__(256) k_nuc_scatter(const NucInst* __restrict__
                     }
                 }
                 __syncthreads();
-                double* out0 = in.out + (i64)(ix * ny + iy) * nz * N + (i64)jx * nyz + (i64)j0 * nz;
-                for (int iz = warp; iz < nz; iz += warps) {
-                    double* out = out0 + (i64)iz * N;
+                double* const block0 = in.out + (i64)(ix * ny + iy) * nz * N + (i64)jx * nyz + (i64)j0 * nz;
+                double* const block1 = in.out + (i64)(jx * ny + iy) * nz * N + (i64)ix * nyz + (i64)j0 * nz;
+                const int nrows = ix == jx ? nz : 2 * nz;
+                for (int r = warp; r < nrows; r += warps) {
+                    const int iz = r < nz ? r : r - nz;
+                    double* out = (r < nz ? block0 : block1) + (i64)iz * N;
                     const double* row = rows + iz * pitch;
                     // (pairs start on 16-byte boundaries: an odd start leaves its first entry alone)
                     const int odd = (int)(((uintptr_t)out >> 3) & 1);
@@ -671,7 +680,7 @@ static void run_chunk(const std::vector<NucHost>& hosts, const double* F, int nf
             }
             max_rows = std::max(max_rows, (i64)in.P[0] * in.P[1]);
             const bool by_lines = !sliced && in.n[2] <= NUC_LINE_MAX_Z;
-            max_items = std::max(max_items, (i64)in.n[0] * in.n[0] * (by_lines ? in.n[1] : 1));
+            max_items = std::max(max_items, by_lines ? (i64)in.n[0] * (in.n[0] + 1) / 2 * in.n[1] : (i64)in.n[0] * in.n[0]);
             if (by_lines) {
                 lines = std::max(lines, 8 * in.n[2] * nuc_row_pitch(nuc_line_group(in.n[1], in.n[2]), in.n[2]));
             }
