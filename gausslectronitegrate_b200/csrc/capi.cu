@@ -5,11 +5,16 @@
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
+#ifdef __SSE2__
+#include <emmintrin.h>
+#endif
 
 #include <algorithm>
+#include <atomic>
+#include <new>
+#include <system_error>
 #include <thread>
 #include <vector>
-#include <new>
 
 #include "gli_internal.cuh"
 
@@ -45,70 +50,66 @@ T* host_alloc(i64 count) {
 }
 
 
-// Large device -> host copies into pageable memory (dense kinetic and nuclear
-// matrices, dense tensors: up to GBs) go through two page-locked staging
-// buffers: the DMA of one chunk overlaps the host copy of the previous one,
-// which is split over a few threads (one core's memcpy into freshly mapped
-// pages runs far below the link's rate).  Synchronous; smaller copies are one
-// asynchronous cudaMemcpyAsync on the stream.
-struct StagedD2H {
-    static constexpr size_t kChunk = (size_t)32 << 20;
-    void* pin[2] = {nullptr, nullptr};
-    cudaEvent_t ev[2] = {nullptr, nullptr};
+// Copies of several MB between the device and pageable host memory (class lists
+// and values, dense matrices and tensors) go through a ring of page-locked
+// pieces, 64 of 1 MB per thread, so that up to eight host threads copy pieces
+// between the ring and the caller's memory while the DMA engine moves others:
+// one core's memcpy, and its page faults in fresh result memory, run at a fifth
+// of the link's rate.  The calling thread queues the DMAs in order and is the
+// only one that calls CUDA.  Pieces on their way in are written past the caches
+// (stage_piece): a DMA of lines that another core has just written waits for
+// their write-back, 29 GB/s against 55 GB/s.  (57 MB of class list and values in:
+// 3.6 ms through two 16 MB buffers filled by threads started for each of them,
+// 2.5 ms through the ring with memcpy, 1.5 ms with streaming stores and four
+// threads; the link alone takes 1.06 ms.)
+struct StagingRing {
+    static constexpr size_t kPiece = (size_t)1 << 20;
+    static constexpr int kSlots = 64;
+    char* pin = nullptr;
+    cudaEvent_t ev[kSlots] = {};
+    int device = -1;  // of the events
     void ensure() {
-        for (int k = 0; k < 2; ++k) {
-            if (!pin[k]) GLI_CUDA(cudaHostAlloc(&pin[k], kChunk, cudaHostAllocDefault));
-            if (!ev[k]) GLI_CUDA(cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming));
-        }
+        int dev = 0;
+        GLI_CUDA(cudaGetDevice(&dev));
+        if (!pin) GLI_CUDA(cudaHostAlloc((void**)&pin, kPiece * kSlots, cudaHostAllocPortable));
+        if (dev != device)
+            for (auto& e : ev) {
+                if (e) {
+                    GLI_CUDA(cudaEventSynchronize(e));
+                    GLI_CUDA(cudaEventDestroy(e));
+                }
+                e = nullptr;
+                GLI_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            }
+        device = dev;
     }
-    ~StagedD2H() {
-        for (int k = 0; k < 2; ++k) {
-            if (pin[k]) cudaFreeHost(pin[k]);
-            if (ev[k]) cudaEventDestroy(ev[k]);
-        }
+    char* slot(size_t p) { return pin + p % kSlots * kPiece; }
+    cudaEvent_t event(size_t p) { return ev[p % kSlots]; }
+    ~StagingRing() {
+        if (pin) cudaFreeHost(pin);
+        for (auto& e : ev)
+            if (e) cudaEventDestroy(e);
     }
 };
-static thread_local StagedD2H t_staged;
+static thread_local StagingRing t_ring;
 
-static void parallel_memcpy(void* dst, const void* src, size_t bytes) {
-    const unsigned hw = std::thread::hardware_concurrency();
-    const int nt = (int)std::min<size_t>(std::min<size_t>(8, hw > 1 ? hw / 2 : 1), std::max<size_t>(1, bytes >> 22));
-    if (nt <= 1) {
-        memcpy(dst, src, bytes);
-        return;
-    }
-    const size_t part = (bytes / nt + 63) / 64 * 64;
-    std::vector<std::thread> th;
-    for (int k = 1; k < nt; ++k) {
-        const size_t b0 = std::min(bytes, k * part), b1 = std::min(bytes, (k + 1) * part);
-        if (b1 > b0) th.emplace_back([=] { memcpy((char*)dst + b0, (const char*)src + b0, b1 - b0); });
-    }
-    memcpy(dst, src, std::min(bytes, part));
-    for (auto& t : th) t.join();
+// copy into a slot with streaming stores (slots are 16-byte aligned)
+static void stage_piece(char* dst, const char* src, size_t len) {
+#ifdef __SSE2__
+    size_t o = 0;
+    for (; o + 64 <= len; o += 64)
+        for (int q = 0; q < 64; q += 16)
+            _mm_stream_si128((__m128i*)(dst + o + q), _mm_loadu_si128((const __m128i*)(src + o + q)));
+    memcpy(dst + o, src + o, len - o);
+    _mm_sfence();
+#else
+    memcpy(dst, src, len);
+#endif
 }
 
-template <class T>
-void to_host(T* h, const T* d, i64 n, cudaStream_t s) {
-    const size_t bytes = (size_t)n * sizeof(T);
-    if (bytes < 2 * StagedD2H::kChunk) {
-        if (n) GLI_CUDA(cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, s));
-        return;
-    }
-    t_staged.ensure();
-    const size_t chunks = (bytes + StagedD2H::kChunk - 1) / StagedD2H::kChunk;
-    for (size_t c = 0; c <= chunks; ++c) {
-        if (c < chunks) {
-            const size_t off = c * StagedD2H::kChunk, len = std::min(StagedD2H::kChunk, bytes - off);
-            GLI_CUDA(cudaMemcpyAsync(t_staged.pin[c & 1], (const char*)d + off, len, cudaMemcpyDeviceToHost, s));
-            GLI_CUDA(cudaEventRecord(t_staged.ev[c & 1], s));
-        }
-        if (c > 0) {  // the previous chunk: wait for its DMA, copy it out of the staging buffer
-            const size_t p = c - 1, off = p * StagedD2H::kChunk, len = std::min(StagedD2H::kChunk, bytes - off);
-            GLI_CUDA(cudaEventSynchronize(t_staged.ev[p & 1]));
-            parallel_memcpy((char*)h + off, t_staged.pin[p & 1], len);
-        }
-    }
-}
+// below this size the driver's own staging of a pageable copy is as fast as
+// starting the threads (about 80 us)
+static constexpr size_t kStagedBytes = (size_t)2 << 20;
 
 static bool host_pinned(const void* p) {
     cudaPointerAttributes a = {};
@@ -119,32 +120,126 @@ static bool host_pinned(const void* p) {
     return a.type == cudaMemoryTypeHost;
 }
 
-// Host -> device copies of long arrays in pageable memory (class lists and
-// values of the reference-facing calls: tens of MB) go through the same two
-// page-locked staging buffers: the host copy of one chunk, split over a few
-// threads, overlaps the DMA of the previous one.  Returns with the last DMAs
-// queued on s (the buffers are not rewritten before their events complete).
+// The host threads of one staged copy: each takes the next piece, waits until
+// `go` has passed it, copies it and marks it done.  Joined on every path.
+struct PieceWorkers {
+    std::vector<std::thread> threads;
+    std::vector<std::atomic<char>> done;
+    std::atomic<size_t> next{0}, go{0};
+    std::atomic<bool> stop{false};
+    explicit PieceWorkers(size_t pieces) : done(pieces) {}
+    template <class Copy>
+    bool start(unsigned most, Copy copy) {  // false: no thread could be started
+        const unsigned hw = std::thread::hardware_concurrency();
+        const size_t n = std::min<size_t>({(size_t)most, hw > 1 ? hw / 2 : 1, done.size()});
+        for (size_t k = 0; k < n; ++k) {
+            try {
+                threads.emplace_back([this, copy] {
+                    for (size_t p; (p = next.fetch_add(1)) < done.size();) {
+                        while (go.load(std::memory_order_acquire) <= p) {
+                            if (stop.load()) return;
+                            std::this_thread::yield();
+                        }
+                        copy(p);
+                        done[p].store(1, std::memory_order_release);
+                    }
+                });
+            } catch (const std::system_error&) {
+                break;
+            }
+        }
+        return !threads.empty();
+    }
+    void wait(size_t p) {
+        while (!done[p].load(std::memory_order_acquire)) std::this_thread::yield();
+    }
+    ~PieceWorkers() {
+        stop = true;
+        for (auto& t : threads) t.join();
+    }
+};
+
+// device -> host; synchronous for staged copies, else queued on s
 template <class T>
-void to_device(DevBuf<T>& d, const T* h, i64 n, cudaStream_t s) {
-    d.alloc(n, s);
-    const size_t bytes = (size_t)n * sizeof(T);
-    constexpr size_t kChunk = (size_t)16 << 20;
-    if (bytes < kChunk || host_pinned(h)) {
-        if (n) GLI_CUDA(cudaMemcpyAsync(d.p, h, bytes, cudaMemcpyHostToDevice, s));
-        return;
+void to_host(T* h, const T* d, i64 n, cudaStream_t s) {
+    const size_t bytes = (size_t)n * sizeof(T), pieces = (bytes + StagingRing::kPiece - 1) / StagingRing::kPiece;
+    auto plain = [&] {
+        if (n) GLI_CUDA(cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, s));
+    };
+    if (bytes < kStagedBytes || host_pinned(h)) return plain();
+    t_ring.ensure();
+    StagingRing& ring = t_ring;
+    auto len = [&](size_t p) { return std::min(StagingRing::kPiece, bytes - p * StagingRing::kPiece); };
+    PieceWorkers w(pieces);
+    if (!w.start(8, [&ring, h, len](size_t p) { memcpy((char*)h + p * StagingRing::kPiece, ring.slot(p), len(p)); }))
+        return plain();
+    auto queue = [&](size_t p) {
+        GLI_CUDA(cudaMemcpyAsync(ring.slot(p), (const char*)d + p * StagingRing::kPiece, len(p),
+                                 cudaMemcpyDeviceToHost, s));
+        GLI_CUDA(cudaEventRecord(ring.event(p), s));
+    };
+    for (size_t p = 0; p < std::min<size_t>(pieces, StagingRing::kSlots); ++p) queue(p);
+    for (size_t p = 0; p < pieces; ++p) {
+        GLI_CUDA(cudaEventSynchronize(ring.event(p)));
+        w.go.store(p + 1, std::memory_order_release);
+        // the slot of a piece copied out half a ring ago takes the next DMA
+        const size_t half = StagingRing::kSlots / 2;
+        if (p >= half && p - half + StagingRing::kSlots < pieces) {
+            w.wait(p - half);
+            queue(p - half + StagingRing::kSlots);
+        }
     }
-    t_staged.ensure();
-    for (int k = 0; k < 2; ++k) GLI_CUDA(cudaEventSynchronize(t_staged.ev[k]));  // earlier uses of the buffers
-    const size_t chunks = (bytes + kChunk - 1) / kChunk;
-    for (size_t c = 0; c < chunks; ++c) {
-        const size_t off = c * kChunk, len = std::min(kChunk, bytes - off);
-        const int k = (int)(c & 1);
-        if (c >= 2) GLI_CUDA(cudaEventSynchronize(t_staged.ev[k]));  // the buffer's previous DMA is done
-        parallel_memcpy(t_staged.pin[k], (const char*)h + off, len);
-        GLI_CUDA(cudaMemcpyAsync((char*)d.p + off, t_staged.pin[k], len, cudaMemcpyHostToDevice, s));
-        GLI_CUDA(cudaEventRecord(t_staged.ev[k], s));
-    }
+    for (size_t p = 0; p < pieces; ++p) w.wait(p);
 }
+
+// Host -> device copies of several arrays as one staged copy; returns with the
+// last DMAs queued on s (the ring is not rewritten before they complete).
+struct Upload {
+    struct Piece {
+        char* dst;
+        const char* src;
+        size_t len;
+    };
+    cudaStream_t s;
+    std::vector<Piece> pieces;
+    explicit Upload(cudaStream_t stream) : s(stream) {}
+    template <class T>
+    void add(DevBuf<T>& d, const T* h, i64 n) {
+        d.alloc(n, s);
+        const size_t bytes = (size_t)n * sizeof(T);
+        if (bytes < kStagedBytes || host_pinned(h)) {
+            if (n) GLI_CUDA(cudaMemcpyAsync(d.p, h, bytes, cudaMemcpyHostToDevice, s));
+            return;
+        }
+        for (size_t o = 0; o < bytes; o += StagingRing::kPiece)
+            pieces.push_back({(char*)d.p + o, (const char*)h + o, std::min(StagingRing::kPiece, bytes - o)});
+    }
+    void run() {
+        if (pieces.empty()) return;
+        t_ring.ensure();
+        StagingRing& ring = t_ring;
+        const size_t n = pieces.size();
+        for (auto& e : ring.ev) GLI_CUDA(cudaEventSynchronize(e));  // earlier uses of the slots
+        PieceWorkers w(n);
+        const Piece* pc = pieces.data();
+        w.go = std::min<size_t>(n, StagingRing::kSlots);
+        if (!w.start(4, [&ring, pc](size_t p) { stage_piece(ring.slot(p), pc[p].src, pc[p].len); })) {
+            for (const Piece& p : pieces) GLI_CUDA(cudaMemcpyAsync(p.dst, p.src, p.len, cudaMemcpyHostToDevice, s));
+            return;
+        }
+        for (size_t p = 0; p < n; ++p) {
+            w.wait(p);
+            GLI_CUDA(cudaMemcpyAsync(pc[p].dst, ring.slot(p), pc[p].len, cudaMemcpyHostToDevice, s));
+            GLI_CUDA(cudaEventRecord(ring.event(p), s));
+            // the slot of a piece sent half a ring ago takes the next copy
+            const size_t half = StagingRing::kSlots / 2;
+            if (p >= half && p - half + StagingRing::kSlots < n) {
+                GLI_CUDA(cudaEventSynchronize(ring.event(p - half)));
+                w.go.store(p - half + StagingRing::kSlots + 1, std::memory_order_release);
+            }
+        }
+    }
+};
 
 void check_gdata(const struct gausslet_data* g) {
     if (!g || !g->coefficients || g->indices.num <= 0 || g->indices.num % 2 != 1)
@@ -560,8 +655,10 @@ void fill_dense_erida_matrix(const struct sparse_erida_gausslet_integrals* erida
         cudaStream_t s = ctx.stream;
         DevBuf<int64_t> di;
         DevBuf<double> dv, out(N * N, s);
-        to_device(di, (const int64_t*)erida->two_indices, erida->num_entries, s);
-        to_device(dv, (const double*)erida->integral_values, erida->num_entries, s);
+        Upload up(s);
+        up.add(di, (const int64_t*)erida->two_indices, erida->num_entries);
+        up.add(dv, (const double*)erida->integral_values, erida->num_entries);
+        up.run();
         gli::fill_dense_device(0, gs, di.p, dv.p, erida->num_entries, gd, out.p, s);
         to_host(erida_matrix, out.p, N * N, s);
         GLI_CUDA(cudaStreamSynchronize(s));
@@ -578,9 +675,11 @@ void project_sparse_erida_gausslet_integrals(const struct sparse_erida_gausslet_
         cudaStream_t s = ctx.stream;
         DevBuf<int64_t> di;
         DevBuf<double> dv, db, out(M * M * M * M, s);
-        to_device(di, (const int64_t*)erida->two_indices, erida->num_entries, s);
-        to_device(dv, (const double*)erida->integral_values, erida->num_entries, s);
-        to_device(db, basis, N * M, s);
+        Upload up(s);
+        up.add(di, (const int64_t*)erida->two_indices, erida->num_entries);
+        up.add(dv, (const double*)erida->integral_values, erida->num_entries);
+        up.add(db, basis, N * M);
+        up.run();
         gli::project_device(0, g, di.p, dv.p, erida->num_entries, db.p, M, out.p, s);
         to_host(eri_proj, out.p, M * M * M * M, s);
         GLI_CUDA(cudaStreamSynchronize(s));
@@ -651,8 +750,10 @@ void fill_dense_eri_tensor(const struct sparse_eri_gausslet_integrals* eri, cons
         cudaStream_t s = ctx.stream;
         DevBuf<int64_t> di;
         DevBuf<double> dv, out(N * N * N * N, s);
-        to_device(di, (const int64_t*)eri->four_indices, eri->num_entries, s);
-        to_device(dv, (const double*)eri->integral_values, eri->num_entries, s);
+        Upload up(s);
+        up.add(di, (const int64_t*)eri->four_indices, eri->num_entries);
+        up.add(dv, (const double*)eri->integral_values, eri->num_entries);
+        up.run();
         gli::fill_dense_device(1, gs, di.p, dv.p, eri->num_entries, gd, out.p, s);
         to_host(eri_tensor, out.p, N * N * N * N, s);
         GLI_CUDA(cudaStreamSynchronize(s));
@@ -669,9 +770,11 @@ void apply_sparse_eri_tensor(const struct sparse_eri_gausslet_integrals* eri, co
         cudaStream_t s = ctx.stream;
         DevBuf<int64_t> di;
         DevBuf<double> dv, dst, out(N * N * ns, s);
-        to_device(di, (const int64_t*)eri->four_indices, eri->num_entries, s);
-        to_device(dv, (const double*)eri->integral_values, eri->num_entries, s);
-        to_device(dst, states, N * N * ns, s);
+        Upload up(s);
+        up.add(di, (const int64_t*)eri->four_indices, eri->num_entries);
+        up.add(dv, (const double*)eri->integral_values, eri->num_entries);
+        up.add(dst, states, N * N * ns);
+        up.run();
         gli::apply_eri_device(g, di.p, dv.p, eri->num_entries, dst.p, ns, out.p, s);
         to_host(ret, out.p, N * N * ns, s);
         GLI_CUDA(cudaStreamSynchronize(s));
@@ -688,9 +791,11 @@ void project_sparse_eri_gausslet_integrals(const struct sparse_eri_gausslet_inte
         cudaStream_t s = ctx.stream;
         DevBuf<int64_t> di;
         DevBuf<double> dv, db, out(M * M * M * M, s);
-        to_device(di, (const int64_t*)eri->four_indices, eri->num_entries, s);
-        to_device(dv, (const double*)eri->integral_values, eri->num_entries, s);
-        to_device(db, basis, N * M, s);
+        Upload up(s);
+        up.add(di, (const int64_t*)eri->four_indices, eri->num_entries);
+        up.add(dv, (const double*)eri->integral_values, eri->num_entries);
+        up.add(db, basis, N * M);
+        up.run();
         gli::project_device(1, g, di.p, dv.p, eri->num_entries, db.p, M, out.p, s);
         to_host(eri_proj, out.p, M * M * M * M, s);
         GLI_CUDA(cudaStreamSynchronize(s));
