@@ -139,20 +139,15 @@ __device__ __forceinline__ uint32_t pd_field(int dax, int sax) {
     return (uint32_t)abs(dax) | ((uint32_t)sax << 8);
 }
 
-// descriptor of every point pair h = p N + q (N^2 entries); skip (sized
-// replays): when *skip is set the table kept with the replay's saved plan is
-// current (a function of the grid alone, made by the replay that made the plan)
-__global__ void k_pair_desc(ClassDecode d, uint2* __restrict__ pd, const int* __restrict__ skip) {
-    if (skip && *skip) return;
-    const uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
-    if ((uint64_t)h >= d.N2) return;
+// descriptor of the point pair h = p N + q (one of N^2)
+__device__ __forceinline__ uint2 pair_desc(const ClassDecode& d, uint32_t h) {
     const uint32_t p = h / d.n32, q = h - p * d.n32;
     int a[3], b[3];
     decode_pt(d, p, a);
     decode_pt(d, q, b);
     uint32_t f[3];
     for (int x = 0; x < 3; ++x) f[x] = pd_field(a[x] - b[x], a[x] + b[x] - 2 * d.is[x]);
-    pd[h] = make_uint2(f[0] | (f[1] << 16), f[2]);
+    return make_uint2(f[0] | (f[1] << 16), f[2]);
 }
 
 // key of one axis from the two pair fields (|d01| | s01 << 8, |d23| | s23 << 8):
@@ -271,6 +266,34 @@ __device__ __forceinline__ void restore_status(bool valid, const PlanCounts* __r
     st->bad = 0;
     st->tc_err = 0;
     st->products = 0ull;
+}
+
+// The first kernel of an evaluation that marks its classes: the status block
+// and the `nmark` words of key flags and pair bits cleared, and the pair
+// descriptors of the grid made (pd non-null; skip, sized replays: when *skip
+// is set the table kept with the replay's saved plan is current, a function of
+// the grid alone).  Bound: one launch's latency, 1.5 us.  The three memset
+// nodes and the descriptor kernel it takes the place of took 14 us of a graph.
+__global__ void __launch_bounds__(256) k_begin(EvalStatus* __restrict__ st, uint32_t* __restrict__ marks, i64 nmark,
+                                               ClassDecode d, uint2* __restrict__ pd, const int* __restrict__ skip) {
+    const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x, step = (i64)gridDim.x * blockDim.x;
+    if (t < (i64)(sizeof(EvalStatus) / sizeof(uint32_t))) reinterpret_cast<uint32_t*>(st)[t] = 0u;
+    for (i64 i = t; i < nmark; i += step) marks[i] = 0u;
+    if (!pd || (skip && *skip)) return;
+    for (i64 h = t; h < (i64)d.N2; h += step) pd[h] = pair_desc(d, (uint32_t)h);
+}
+
+// The status block, written to page-locked host memory by the last kernel of
+// an evaluation (visible to the host once it has synchronised): 5 us with its
+// launch, against 8 to 13 us for a copy engine's transfer.  Both together: ERI
+// 3^3 values 49 to 41 us, ERIDA 33^3 73 to 67 us, ERI 7^3 102 to 98 us.
+__global__ void k_report(const EvalStatus* __restrict__ st, EvalStatus* __restrict__ host) {
+    static_assert(sizeof(EvalStatus) % sizeof(uint64_t) == 0 && sizeof(EvalStatus) <= 32 * sizeof(uint64_t), "");
+    if (threadIdx.x < sizeof(EvalStatus) / sizeof(uint64_t))
+        reinterpret_cast<uint64_t*>(host)[threadIdx.x] = reinterpret_cast<const uint64_t*>(st)[threadIdx.x];
+}
+static void report_status(const EvalStatus* st, EvalStatus* h_status, cudaStream_t s) {
+    launch_kernel(k_report, dim3(1), dim3(32), 0, s, st, h_status);
 }
 
 // Decodes every class once (its packed keys are kept for the later passes)
@@ -1890,7 +1913,6 @@ static void enqueue_eval(const EvalArgs& a, PlanMode mode, EvalStatus* st, Stage
     // stage A's first block): no memset node ahead of it
     const bool restores = trusted && (bounded || mode == PLAN_SIZED) && (nk * nk + 31) / 32 <= 8 * 1024 &&
                           nk <= PLAN_SMALL_KEYS;
-    if (!restores) GLI_CUDA(cudaMemsetAsync(st, 0, sizeof(EvalStatus), s));
     PlanCounts* cnt = &st->cnt;
     if (bounded) {
         sz.nku = nk;
@@ -1899,19 +1921,18 @@ static void enqueue_eval(const EvalArgs& a, PlanMode mode, EvalStatus* st, Stage
         sz.nP = std::min(nk * (nk + 1) / 2, m);
     }
     // Bounded and sized evaluations know every size here: all their buffers
-    // are allocated and zeroed before the first kernel, so that a captured
-    // graph has its allocation and memset nodes at the root and its kernels
-    // follow one another directly
+    // are allocated before the first kernel, so that a captured graph has its
+    // allocation nodes at the root and its kernels follow one another directly
     const bool known = mode != PLAN_EXACT;
     // usedKey and usedA side by side so that one scan serves both; pair flags
     // over all key pairs (slot k2 * nk + k1)
     const i64 words = (nk * nk + 31) / 32;
-    DevBuf<uint32_t> used, pairBits;
+    DevBuf<uint32_t> marks, used, pairBits;
+    const i64 used_words = (2 * nk + 63) / 64 * 64, mark_words = used_words + words;
     if (!trusted) {
-        used.alloc(2 * nk, s);
-        pairBits.alloc(words, s);
-        used.zero();
-        pairBits.zero();
+        marks.alloc(mark_words, s);
+        used.borrow(marks.p, 2 * nk, s);
+        pairBits.borrow(marks.p + used_words, words, s);
     }
     const unsigned cb = (unsigned)((m + 255) / 256);
     const unsigned kb = (unsigned)((nk + 255) / 256);
@@ -1996,9 +2017,14 @@ static void enqueue_eval(const EvalArgs& a, PlanMode mode, EvalStatus* st, Stage
     };
     if (known) stage_bufs();
 
-    if (dec.pd && !trusted)
-        launch_kernel(k_pair_desc, dim3((unsigned)((dec.N2 + 255) / 256)), dim3(256), 0, s, dec, pdesc.p, pd_skip);
-    else if (!dec.pd && dec.kind == 1)
+    if (!restores) {
+        // (a trusted replay of a large plan has its tables: only the status is cleared)
+        const i64 nm = trusted ? 0 : mark_words, npd = dec.pd && !trusted ? (i64)dec.N2 : 0;
+        const i64 gb = std::min<i64>((std::max<i64>(nm, npd) + 255) / 256, (i64)a.num_sms * 8);
+        launch_kernel(k_begin, dim3((unsigned)std::max<i64>(gb, 1)), dim3(256), 0, s, st, marks.p, nm, dec,
+                      npd ? pdesc.p : (uint2*)nullptr, pd_skip);
+    }
+    if (!dec.pd && dec.kind == 1)
         launch_kernel(k_point_table, dim3((unsigned)((dec.N + 255) / 256)), dim3(256), 0, s, dec, pts.p);
     if (!trusted) {
         const size_t lb = mark_local_bytes(nk);
@@ -2514,7 +2540,7 @@ static void sparse_values_enqueue(int kind, const double* h_coeffs, i64 nb, cons
         GLI_CUDA(cudaGraphLaunch(trust ? e->exec_trust : e->exec, s));
         add_launches(trust ? e->launches_trust : e->launches);
         t_paths = e->paths;
-        GLI_CUDA(cudaMemcpyAsync(h_status, e->status.p, sizeof(EvalStatus), cudaMemcpyDeviceToHost, s));
+        report_status(e->status.p, h_status, s);
         *sized = e;
         return;
     }
@@ -2522,7 +2548,7 @@ static void sparse_values_enqueue(int kind, const double* h_coeffs, i64 nb, cons
     EvalSizes sz;
     enqueue_eval(a, bounded ? PLAN_BOUNDED : PLAN_EXACT, st.p, timer, sz, s);
     t_paths = t_enq_paths;
-    GLI_CUDA(cudaMemcpyAsync(h_status, st.p, sizeof(EvalStatus), cudaMemcpyDeviceToHost, s));
+    report_status(st.p, h_status, s);
     // the exact counts of this list size the graph that its next evaluations replay
     if (graphs && !bounded && sized_plan_fits(t.nkeys)) capture_graph(a, tp, ctx.device, s, PLAN_SIZED, sz, t_timing);
 }
@@ -2868,7 +2894,7 @@ static void sparse_values_pinned(int kind, const double* h_coeffs, i64 nb, const
                 GLI_CUDA(cudaMemcpyAsync(h_out + b, d_val + b, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost,
                                          s_out));
         }
-        GLI_CUDA(cudaMemcpyAsync(hs, e->status.p, sizeof(EvalStatus), cudaMemcpyDeviceToHost, s));
+        report_status(e->status.p, hs, s);
         GLI_CUDA(cudaStreamSynchronize(s_out));
         GLI_CUDA(cudaStreamSynchronize(s));
         t_paths = e->paths;
