@@ -99,22 +99,33 @@ __device__ __forceinline__ int pair_class(const PairBox& b, int i, int j) {
     return (f[0] * b.F[1] + f[1]) * b.F[2] + f[2];
 }
 
+// 8-byte asynchronous copy without the compiler's ordering of other memory
+// accesses (the kernel's barriers and waits order it): between two k steps it
+// must not hold back the next step's loads
+__device__ __forceinline__ void pair_cp8(double* dst, const double* src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src));
+}
+
 // Shared memory of k_pair_contract (the launch and the kernel agree on it)
 struct PairSmem {
     int ldb;      // doubles per row of B: 4 or 12 mod 16, so that fragment reads have no bank conflicts
     int planes;   // doubles: two buffers of n0 planes (the epilogue's tiles reuse them)
     int brows;    // rows of B
     int map_ld;   // uint16 per row of the (y z) x (y z) maps
+    int sum, part, rows;  // (SYM epilogue) Y, the warps' parts of it and the 8-row strips of Y they hold at a time
     size_t bytes;
     __host__ __device__ PairSmem(const PairBox& b, int warps, int nt) {
         ldb = 8 * nt + 4;
-        const int rows = b.N < 16 * warps ? (b.N + 15) / 16 * 16 : 16 * warps;
         planes = 2 * b.n[0] * b.PS;
-        if (planes < rows * ldb) planes = rows * ldb;
-        if (planes < 8 * nt * (8 * nt + 1)) planes = 8 * nt * (8 * nt + 1);
+        sum = b.PS;  // (past the next class's first plane)
+        part = sum + 8 * nt * (8 * nt + 1);
+        const int strip = warps * 64 * nt;
+        if (planes < part + strip) planes = part + strip;
+        rows = (planes - part) / strip < nt ? (planes - part) / strip : nt;
         brows = b.N + 4;
         map_ld = 4 * b.S;
-        bytes = 8 * ((size_t)planes + (size_t)brows * ldb + 2 * 8 * (size_t)nt) + 4 * ((size_t)b.F2 + b.F[0] + b.F[1] + b.F[2]) +
+        bytes = 8 * ((size_t)planes + (size_t)brows * ldb + 2 * 8 * (size_t)nt) + 6 * ((size_t)b.F2 + b.F[0] + b.F[1] + b.F[2]) +
                 2 * ((size_t)2 * b.nyz + 1) * map_ld;
     }
 };
@@ -133,21 +144,30 @@ struct PairSmem {
 // The k loop runs over the x planes of l.  V[c] restricted to l's plane needs
 // one plane of values per x coordinate of k (F1 F2 each): they are copied from
 // the key table with 8-byte cp.async into one of two buffers while the previous
-// plane is contracted.  A fragments are read from there through a map
-// (yz of k, yz of l) -> value, 16 bits each, the same for every plane; rows
-// and columns outside the triangle (or the box) point at the plane's zero.
-// Bound: the FP64 tensor pipe, 47% busy (343 points, 20 orbitals); the rest is
-// the planes' copies, the barriers between planes and the blocks' start and
-// end.  Measured on a B200, first two contractions: 216 points and 32 orbitals
-// 1.09 ms (a contraction per point pair, its slab staged from the key table:
-// 5.25 ms), 343 points and 20 orbitals 5.2 ms (23.7 ms); the whole projection
-// calls 9.9 to 5.4 ms and 28.0 to 9.2 ms, the apply at 5^3 points and 4 states
-// 12.8 to 0.57 ms (0.24 ms of kernels).
+// plane is contracted, one value per thread between two k steps (all copies
+// ahead of the plane's first MMA left the tensor pipe idle behind them: 5.19
+// against 4.88 ms at 343 points and 20 orbitals).  V fragments are read from
+// there through a map (yz of k, yz of l) -> value, 16 bits each, the same for
+// every plane; rows and columns outside the triangle (or the box) point at the
+// plane's zero.  V is the right operand: an accumulator tile holds A^T, eight
+// columns by eight rows k, and is as it stands the left operand of Y^T = A^T B
+// (the values of one lane have k of equal parity), so the second contraction
+// needs no trip of A through shared memory, and every warp takes part in it.
+// The next class's keys are made under the last plane, its first plane's copies
+// under that contraction.
+// Bound: the FP64 tensor pipe, 55% busy (343 points, 20 orbitals), with the
+// shared-memory pipe 59% busy (V fragments, and copies whose 32 values lie in
+// about as many lines).  Measured on a B200, first two contractions: 216 points
+// and 32 orbitals 1.04 ms (a contraction per point pair, its slab staged from
+// the key table: 5.25 ms), 343 points and 20 orbitals 4.44 ms (23.7 ms; A through
+// shared memory 4.88 ms); the whole projection calls 9.9 to 3.8 ms and 28.0 to
+// 6.5 ms, the apply at 5^3 points and 4 states 12.7 to 0.50 ms (0.16 ms of this
+// kernel; 0.21 ms with four column tiles multiplied whatever the class's pairs).
 //
 // A warp owns up to two 16-row tiles (rows 16 (w + W t)) and keeps their
 // accumulators over all planes, so each B fragment serves all its tiles.  The
 // FP64 MMAs of four warps per scheduler hide each other's issue gaps and the
-// map and value loads (two warps with three tiles each kept the FP64 tensor
+// map and value loads (loads issued a step ahead gained nothing, 4.54 ms) (two warps with three tiles each kept the FP64 tensor
 // pipe 39% busy): two blocks of 8 warps on an SM, or one of 16 where the
 // planes and B of one box take more than half of the shared memory.
 template <int W, int NT, int TPW, bool SYM>
@@ -168,10 +188,20 @@ __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : 1)
     int* kx = reinterpret_cast<int*>(yz + F2);
     int* ky = kx + box.F[0];
     int* kz = ky + box.F[1];
-    uint16_t* map = reinterpret_cast<uint16_t*>(kz + box.F[2]);  // nyz rows: every l
+    uint16_t* fields = reinterpret_cast<uint16_t*>(kz + box.F[2]);  // coordinate positions lo | hi << 8 of x, y, z fields
+    uint16_t* fyz = fields + box.F[0] + box.F[1] + box.F[2];        // y field | z field << 8 of a plane's values
+    uint16_t* map = fyz + F2;                                       // nyz rows: every l
     uint16_t* tmap = map + nyz * map_ld;                          // nyz rows: l >= k only
     uint16_t* zrow = tmap + nyz * map_ld;                         // a row of zeros
-    // the maps, and B where every class has the same
+    // the maps, the fields, and B where every class has the same
+    const int nfields = box.F[0] + box.F[1] + box.F[2];
+    for (int g = tid; g < nfields; g += PAIR_THREADS) {
+        const int a = g < box.F[0] ? 0 : g < box.F[0] + box.F[1] ? 1 : 2;
+        int lo, hi;
+        pair_field(g - (a > 0 ? box.F[0] : 0) - (a > 1 ? box.F[1] : 0), lo, hi);
+        fields[g] = (uint16_t)(lo | hi << 8);
+    }
+    for (int e = tid; e < F2; e += PAIR_THREADS) fyz[e] = (uint16_t)(e / box.F[2] | e % box.F[2] << 8);
     for (int e = tid; e < nyz * map_ld; e += PAIR_THREADS) {
         const int k = e / map_ld, l = e - k * map_ld;
         int v = F2;
@@ -200,34 +230,86 @@ __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : 1)
             row_m[t][i] = (r - row_k[t][i] * nyz) * map_ld + q;
         }
 
-    for (int cls = blockIdx.x; cls < box.classes; cls += gridDim.x) {
-        int f[3], lo[3], hi[3], d[3], s[3];
-        f[2] = cls % box.F[2];
-        f[1] = cls / box.F[2] % box.F[1];
-        f[0] = cls / F2;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            pair_field(f[a], lo[a], hi[a]);
-            d[a] = box.c[a][hi[a]] - box.c[a][lo[a]];
-            s[a] = box.c[a][hi[a]] + box.c[a][lo[a]];
+    __syncthreads();  // the fields
+
+    // the axis keys of class cls with every field: bit 15 marks the y and z
+    // fields of one coordinate
+    auto keys = [&](int cls) {
+        for (int g = tid; g < nfields; g += PAIR_THREADS) {
+            const int a = g < box.F[0] ? 0 : g < box.F[0] + box.F[1] ? 1 : 2;
+            const int f = a == 0 ? cls / F2 : a == 1 ? box.F[0] + cls / box.F[2] % box.F[1]
+                                                     : box.F[0] + box.F[1] + cls % box.F[2];
+            const int p1 = fields[f], p2 = fields[g], h1 = p1 >> 8, l1 = p1 & 255, h2 = p2 >> 8, l2 = p2 & 255;
+            const int xl = box.c[a][l1], xh = box.c[a][h1], yl = box.c[a][l2], yh = box.c[a][h2];
+            kx[g] = pair_axis_key(xh - xl, yh - yl, xh + xl - yh - yl, box.L) | (a && l2 == h2 ? 1 << 15 : 0);
         }
-        __syncthreads();  // the previous class is done with the tables, the planes and (apply) B
-        for (int a = 0, o = 0; a < 3; o += box.F[a], ++a)
-            for (int g = tid; g < box.F[a]; g += PAIR_THREADS) {
-                int l2, h2;
-                pair_field(g, l2, h2);
-                const int d2 = box.c[a][h2] - box.c[a][l2], s2 = box.c[a][h2] + box.c[a][l2];
-                kx[o + g] = pair_axis_key(d[a], d2, s[a] - s2, box.L);
-            }
-        for (int e = tid; e < 2 * box.n[0]; e += PAIR_THREADS) planes[e * PS + F2] = 0.0;
-        __syncthreads();
+    };
+    auto key_pairs = [&]() {
         for (int e = tid; e < F2; e += PAIR_THREADS) {
-            const int fy = e / box.F[2], fz = e - fy * box.F[2];
-            int l2, h2, l3, h3;
-            pair_field(fy, l2, h2);
-            pair_field(fz, l3, h3);
-            const uint32_t a = min(ky[fy], kz[fz]), b = max(ky[fy], kz[fz]);
-            yz[e] = a | b << 15 | (l2 == h2 && l3 == h3 ? 1u << 31 : 0u);
+            const uint32_t f = fyz[e], y = ky[f & 255], z = kz[f >> 8];
+            const uint32_t a = min(y & 0x7fffu, z & 0x7fffu), b = max(y & 0x7fffu, z & 0x7fffu);
+            yz[e] = a | b << 15 | (y & z) >> 15 << 31;
+        }
+    };
+    auto zeros = [&]() {
+        for (int e = tid; e < 2 * box.n[0]; e += PAIR_THREADS) planes[e * PS + F2] = 0.0;
+    };
+    // copies the values of l's plane glx into its buffer, one value per
+    // thread and call: value ge of the plane for k's x coordinate gk
+    int glx = 0, gend = 0, gk = 0, ge = 0;
+    uint32_t gx = 0;
+    auto gen_wrap = [&]() {
+        while (ge >= F2 && gk < gend) {
+            ge -= F2;
+            ++gk;
+        }
+        const int h = max(gk, glx);
+        if (gk < gend) gx = kx[h * (h + 1) / 2 + min(gk, glx)];
+    };
+    auto gen_plane = [&](int lx) {
+        glx = lx;
+        gend = lx >= box.n[0] ? 0 : SYM ? lx + 1 : box.n[0];
+        gk = 0;
+        ge = tid;
+        gen_wrap();
+    };
+    auto gen_one = [&]() {
+        if (gk >= gend) return;
+        const uint32_t v = yz[ge], a = v & 0x7fffu, b = v >> 15 & 0x7fffu;
+        pair_cp8(planes + ((glx & 1) * box.n[0] + gk) * PS + ge,
+                 table + tetra_index32(min(a, gx), max(a, min(b, gx)), max(b, gx)));
+        ge += PAIR_THREADS;
+        if (ge >= F2) gen_wrap();
+    };
+    auto gen_first = [&]() {
+        gen_plane(0);
+        while (gk < gend) gen_one();
+        dm_commit();
+    };
+    if (SYM) {
+        keys(blockIdx.x);
+        zeros();
+        __syncthreads();
+        key_pairs();
+        __syncthreads();
+        gen_first();
+    }
+
+    for (int cls = blockIdx.x; cls < box.classes; cls += gridDim.x) {
+        int lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
+        if (!SYM) {
+            const int f[3] = {cls / F2, box.F[0] + cls / box.F[2] % box.F[1], box.F[0] + box.F[1] + cls % box.F[2]};
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const int p = fields[f[a]];
+                lo[a] = p & 255;
+                hi[a] = p >> 8;
+            }
+            __syncthreads();  // the previous class is done with the tables, the planes and B
+            keys(cls);
+            zeros();
+            __syncthreads();
+            key_pairs();
         }
         int axes = 0;  // (apply) axes on which the class's two coordinates differ
         if (!SYM) {
@@ -270,21 +352,6 @@ __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : 1)
                 dm_cp8(B + r * LDB + c, from >= 0 ? bsrc + from + (i64)r * ld : bsrc, from >= 0);
             }
         }
-        __syncthreads();
-        // copies the values of l's plane lx into a buffer
-        auto stage = [&](int lx, double* buf) {
-            const int cnt = SYM ? lx + 1 : box.n[0];
-            for (int kxi = 0; kxi < cnt; ++kxi) {
-                const int h = max(kxi, lx);
-                const uint32_t x = kx[h * (h + 1) / 2 + min(kxi, lx)];
-                double* dst = buf + kxi * PS;
-                for (int e = tid; e < F2; e += PAIR_THREADS) {
-                    const uint32_t v = yz[e], a = v & 0x7fffu, b = v >> 15 & 0x7fffu;
-                    dm_cp8(dst + e, table + tetra_index32(min(a, x), max(a, min(b, x)), max(b, x)), true);
-                }
-            }
-            dm_commit();
-        };
         double acc[TPW][2][NT][2];
 #pragma unroll
         for (int t = 0; t < TPW; ++t)
@@ -292,15 +359,18 @@ __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : 1)
             for (int i = 0; i < 2; ++i)
 #pragma unroll
                 for (int j = 0; j < NT; ++j) acc[t][i][j][0] = acc[t][i][j][1] = 0.0;
-        stage(0, planes);
+        if (!SYM) gen_first();
+        const int next = cls + gridDim.x;
+        const int live = SYM ? NT : min(NT, (bcols - ct + 7) / 8);  // column tiles in use
         for (int lx = 0; lx < box.n[0]; ++lx) {
             double* buf = planes + (lx & 1) * box.n[0] * PS;
             dm_wait<0>();
             if (SYM)  // the diagonal k = l, halved by the thread that copied it
-                for (int e = tid; e < F2; e += PAIR_THREADS)
+                for (int e = (unsigned)(tid + PAIR_THREADS * F2 - lx * F2) % PAIR_THREADS; e < F2; e += PAIR_THREADS)
                     if (yz[e] >> 31) buf[lx * PS + e] *= 0.5;
             __syncthreads();  // the plane has landed everywhere; the other buffer is consumed
-            if (lx + 1 < box.n[0]) stage(lx + 1, planes + ((lx + 1) & 1) * box.n[0] * PS);
+            gen_plane(lx + 1);
+            if (SYM && lx + 1 == box.n[0] && next < box.classes) keys(next);  // (every copy of this class is queued)
             // rows that meet this plane (offsets into the maps and the values)
             const int rows = SYM ? (lx + 1) * nyz : N, xmax = SYM ? lx + 1 : box.n[0];
             int mo[TPW][2], po[TPW][2];
@@ -317,103 +387,113 @@ __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : 1)
                 }
             }
             const int bo = lay.planes + (lx * nyz + q) * LDB + c8;
-            auto steps = [&](auto active) {
-                constexpr int A = decltype(active)::value;
+            auto steps = [&](auto active, auto columns) {
+                constexpr int A = decltype(active)::value, J = decltype(columns)::value;
                 auto step = [&](int st, bool last) {
                     // (past the plane's last point B is taken as zero, not only
                     // A: a state or orbital may hold infinities in the next plane)
                     const bool in = !last || 4 * st + q < nyz;
-                    double bf[NT];
+                    double bf[J];
 #pragma unroll
-                    for (int j = 0; j < NT; ++j) bf[j] = in ? sm[bo + st * 4 * LDB + 8 * j] : 0.0;
+                    for (int j = 0; j < J; ++j) bf[j] = in ? sm[bo + st * 4 * LDB + 8 * j] : 0.0;
 #pragma unroll
                     for (int t = 0; t < A; ++t) {
                         const double a0 = sm[po[t][0] + map[mo[t][0] + 4 * st]], a1 = sm[po[t][1] + map[mo[t][1] + 4 * st]];
 #pragma unroll
-                        for (int j = 0; j < NT; ++j) dm_mma(acc[t][0][j], a0, bf[j]);
+                        for (int j = 0; j < J; ++j) dm_mma(acc[t][0][j], bf[j], a0);
 #pragma unroll
-                        for (int j = 0; j < NT; ++j) dm_mma(acc[t][1][j], a1, bf[j]);
+                        for (int j = 0; j < J; ++j) dm_mma(acc[t][1][j], bf[j], a1);
                     }
                 };
 #pragma unroll 2
-                for (int st = 0; st < box.S - 1; ++st) step(st, false);
+                for (int st = 0; st < box.S - 1; ++st) {
+                    step(st, false);
+                    gen_one();
+                }
                 step(box.S - 1, true);
             };
+            auto planes_of = [&](auto active) {
+                if constexpr (!SYM && NT > 1) {
+                    if (live == 1) return steps(active, std::integral_constant<int, 1>{});
+                    if constexpr (NT > 2)
+                        if (live == 2) return steps(active, std::integral_constant<int, 2>{});
+                }
+                steps(active, std::integral_constant<int, NT>{});
+            };
             if constexpr (TPW >= 2)
-                if (nact == 2) steps(std::integral_constant<int, 2>{});
-            if (nact == 1) steps(std::integral_constant<int, 1>{});
+                if (nact == 2) planes_of(std::integral_constant<int, 2>{});
+            if (nact == 1) planes_of(std::integral_constant<int, 1>{});
+            while (gk < gend) gen_one();
+            dm_commit();
         }
         if constexpr (SYM) {
-            // Y[r][s] = sum_k B[k][r] A[k][s]: the rows of A through shared memory,
-            // 128 at a time; NT^2 tiles of Y over the warps
-            constexpr int YT = (NT * NT + PAIR_WARPS - 1) / PAIR_WARPS;
-            // (two chains of MMAs per tile of Y: one chain over 343 rows waits
-            // on its own latency)
-            double y[YT][2][2];
+            // Y^T[s][r] = sum_k A[k][s] B[k][r]: an accumulator tile (s, k) is
+            // itself the left operand of two MMAs over its k of equal parity; each
+            // warp's rows give a part of Y^T, summed in shared memory
+            __syncthreads();  // the planes are consumed, the next class's keys made
+            if (next < box.classes) key_pairs();
+            double* Y = sm + lay.sum;  // [s][8 NT + 1]
+            double* part = sm + lay.part;
+            for (int i0 = 0; i0 < NT; i0 += lay.rows) {
 #pragma unroll
-            for (int t = 0; t < YT; ++t) y[t][0][0] = y[t][0][1] = y[t][1][0] = y[t][1][1] = 0.0;
-            double* X = planes;
+                for (int is = 0; is < NT; ++is) {
+                    if (is < i0 || is >= i0 + lay.rows) continue;
+                    double y[NT][2];
 #pragma unroll
-            for (int t = 0; t < TPW; ++t) {
-                const int r0 = 16 * PAIR_WARPS * t, nr = min(16 * PAIR_WARPS, N - r0);
-                __syncthreads();  // the planes, or the rows before, are consumed
-                if (nr <= 0) break;
-                if (t < mine)
+                    for (int j = 0; j < NT; ++j) y[j][0] = y[j][1] = 0.0;
 #pragma unroll
-                    for (int i = 0; i < 2; ++i)
+                    for (int t = 0; t < TPW; ++t)
+                        if (t < mine) {
 #pragma unroll
-                        for (int j = 0; j < NT; ++j) {
-                            double* x = X + (16 * warp + 8 * i + c8) * LDB + 8 * j + 2 * q;
-                            x[0] = acc[t][i][j][0];
-                            x[1] = acc[t][i][j][1];
+                            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                                for (int h = 0; h < 2; ++h) {
+                                    const int k = 16 * (warp + PAIR_WARPS * t) + 8 * i + 2 * q + h;
+#pragma unroll
+                                    for (int j = 0; j < NT; ++j)
+                                        dm_mma(y[j], acc[t][i][is][h], k < N ? B[k * LDB + 8 * j + c8] : 0.0);
+                                }
                         }
-                __syncthreads();
+                    double* p = part + (((is - i0) * PAIR_WARPS + warp) * 8 + c8) * 8 * NT + 2 * q;
 #pragma unroll
-                for (int u = 0; u < YT; ++u) {
-                    const int ty = warp + PAIR_WARPS * u;
-                    if (ty >= NT * NT) continue;
-                    const double* ap = B + (r0 + q) * LDB + 8 * (ty / NT) + c8;
-                    const double* xp = X + q * LDB + 8 * (ty % NT) + c8;
-                    int k = 0;
-#pragma unroll 4
-                    for (; k + 4 < nr; k += 8) {
-                        dm_mma(y[u][0], ap[k * LDB], xp[k * LDB]);
-                        dm_mma(y[u][1], ap[(k + 4) * LDB], xp[(k + 4) * LDB]);
-                    }
-                    if (k < nr) dm_mma(y[u][0], ap[k * LDB], xp[k * LDB]);
+                    for (int j = 0; j < NT; ++j) p[8 * j] = y[j][0], p[8 * j + 1] = y[j][1];
                 }
-            }
-            __syncthreads();  // X is consumed
-            double* Y = X;    // [r][8 NT + 1]
+                __syncthreads();
+                // the next class's first plane: its copies land meanwhile
+                if (i0 == 0 && next < box.classes) gen_first();
+                const int n = min(lay.rows, NT - i0) * 64 * NT;
+                for (int e = tid; e < n; e += PAIR_THREADS) {
+                    const double* p = part + e / (64 * NT) * (PAIR_WARPS * 64 * NT) + e % (64 * NT);
+                    double v = 0.0;
 #pragma unroll
-            for (int u = 0; u < YT; ++u) {
-                const int ty = warp + PAIR_WARPS * u;
-                if (ty >= NT * NT) continue;
-                double* yp = Y + (8 * (ty / NT) + c8) * (8 * NT + 1) + 8 * (ty % NT) + 2 * q;
-                yp[0] = y[u][0][0] + y[u][1][0];
-                yp[1] = y[u][0][1] + y[u][1][1];
+                    for (int w = 0; w < PAIR_WARPS; ++w) v += p[w * 64 * NT];
+                    Y[(8 * i0 + e / (8 * NT)) * (8 * NT + 1) + e % (8 * NT)] = v;
+                }
+                __syncthreads();
             }
-            __syncthreads();
             double* o = out + (i64)cls * (cols * (cols + 1) / 2);
             for (int e = tid; e < 64 * NT * NT; e += PAIR_THREADS) {
                 const int r = e / (8 * NT), c = e - r * (8 * NT);
                 if (r < cols && c <= r) o[r * (r + 1) / 2 + c] = Y[r * (8 * NT + 1) + c] + Y[c * (8 * NT + 1) + r];
             }
+            __syncthreads();  // Y is consumed
+            zeros();
         } else {
 #pragma unroll
-            for (int t = 0; t < TPW; ++t)
+            for (int j = 0; j < NT; ++j) {
+                if (j >= live) break;
+                const i64 to = cdst[8 * j + c8];
+                if (to < 0) continue;
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const int k = 16 * (warp + PAIR_WARPS * t) + 8 * i + c8;
-                    if (k >= N) continue;
+                for (int t = 0; t < TPW; ++t)
 #pragma unroll
-                    for (int j = 0; j < NT; ++j)
+                    for (int i = 0; i < 2; ++i)
 #pragma unroll
                         for (int h = 0; h < 2; ++h) {
-                            const i64 to = cdst[8 * j + 2 * q + h];
-                            if (to >= 0) out[to + (i64)k * cols] = acc[t][i][j][h];
+                            const int k = 16 * (warp + PAIR_WARPS * t) + 8 * i + 2 * q + h;
+                            if (k < N) out[to + (i64)k * cols] = acc[t][i][j][h];
                         }
-                }
+            }
             __syncthreads();  // the planes are consumed before the next columns' first copy
         }
         }
