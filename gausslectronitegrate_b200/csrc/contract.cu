@@ -1223,89 +1223,63 @@ __global__ void __launch_bounds__(256, PD ? 8 : 6) k_gather_q_plan(const double*
                                                         const uint2* __restrict__ bitpre, int ldq,
                                                         PlanCounts* __restrict__ cnt, double* __restrict__ out) {
     if (cnt->overflow) return;
-    const bool vec = ((uintptr_t)idx & 15) == 0 && ((uintptr_t)out & 15) == 0;
-    const i64 groups = (m + 3) / 4, stride = (i64)gridDim.x * blockDim.x;
-    // one group of four classes per thread and step, at most 32 registers:
-    // eight blocks per SM hide the dependent loads better than two groups
-    // at four blocks (ERI 7^3 stage C 45 against 49 us)
-    constexpr int G = 1;
     bool miss = false;
-    for (i64 g0 = (i64)blockIdx.x * blockDim.x + threadIdx.x; g0 < groups; g0 += G * stride) {
-        int64_t c[G][4];
+    // A warp's lanes take consecutive classes, four rounds of 32: neighbours in
+    // a list read neighbouring descriptors, pairs and products, so a load of the
+    // warp meets few lines (ERI 7^3, 3.57 million classes: 22 us; four
+    // consecutive classes per lane with 16-byte index loads and stores 26 us).
+    // Bound: integer instructions (about 120 per class, the ALU 68% busy); the
+    // list and the values are 57 MB, 8.7 us.
+    const i64 step = (i64)gridDim.x * blockDim.x * 4;
+    for (i64 n0 = ((i64)blockIdx.x * blockDim.x + (threadIdx.x & ~31)) * 4 + (threadIdx.x & 31); n0 < m; n0 += step) {
+        const int left = (int)min((i64)128, m - n0);  // of round v: 32 v < left
+        const int64_t* ip = idx + n0;
+        double* op = out + n0;
+        int64_t c[4];
 #pragma unroll
-        for (int h = 0; h < G; ++h) {
-            const i64 n0 = 4 * (g0 + h * stride);
-            if (vec && n0 + 3 < m) {
-                const longlong2 a = __ldg(reinterpret_cast<const longlong2*>(idx + n0));
-                const longlong2 b = __ldg(reinterpret_cast<const longlong2*>(idx + n0 + 2));
-                c[h][0] = a.x, c[h][1] = a.y, c[h][2] = b.x, c[h][3] = b.y;
-            } else {
+        for (int v = 0; v < 4; ++v) c[v] = 32 * v < left ? __ldg(ip + 32 * v) : 0;
+        int q[4];
+        uint64_t base = PD_NO_BASE;
+        uint2 da = make_uint2(0, 0);
 #pragma unroll
-                for (int v = 0; v < 4; ++v) c[h][v] = n0 + v < m ? __ldg(&idx[n0 + v]) : 0;
-            }
-        }
-        int q[G][4];
-#pragma unroll
-        for (int h = 0; h < G; ++h) {
-            const i64 n0 = 4 * (g0 + h * stride);
-            uint64_t base = PD_NO_BASE;
-            uint2 da = make_uint2(0, 0);
-            int last_slot = -1, last_pid = -1;
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                q[h][v] = -1;
-                if (n0 + v >= m) continue;
-                int s0, s1, s2;
-                if constexpr (PD) {
-                    if (!pd_class_keys(dec, c[h][v], base, da, s0, s1, s2)) {
-                        miss = true;
-                        continue;
-                    }
-                } else {
-                    int k[3];
-                    if (!class_keys(dec, c[h][v], k)) {
-                        miss = true;
-                        continue;
-                    }
-                    s0 = k[0], s1 = k[1], s2 = k[2];
-                }
-                if (!dcheck(s0 >= 0 && s2 < nk, 1, s2)) continue;
-                const int slot = s1 * nk + s0;
-                if (slot != last_slot) {
-                    last_slot = slot;
-                    const uint2 bp = __ldg(&bitpre[slot >> 5]);  // (bits, pairs before the word)
-                    const uint32_t bit = (uint32_t)(slot & 31);
-                    last_pid = (bp.x >> bit) & 1u ? (int)(bp.y + __popc(bp.x & ((1u << bit) - 1u))) : -1;
-                }
-                const uint32_t k0 = __ldg(&kk[s2]);  // key id, bit 31: a key the list uses
-                if (last_pid < 0 || !(k0 >> 31)) {
+        for (int v = 0; v < 4; ++v) {
+            q[v] = -1;
+            if (32 * v >= left) continue;
+            int s0, s1, s2;
+            if constexpr (PD) {
+                if (!pd_class_keys(dec, c[v], base, da, s0, s1, s2)) {
                     miss = true;
                     continue;
                 }
-                q[h][v] = last_pid * ldq + (int)(k0 & 0x7fffffffu);  // (Q has fewer than 2^31 entries)
-            }
-        }
-        double acc[G][4];
-#pragma unroll
-        for (int h = 0; h < G; ++h)
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                acc[h][v] = 0.0;
-                if (q[h][v] >= 0 && dcheck(q[h][v] < nq, 3, q[h][v])) acc[h][v] = Q[q[h][v]];
-            }
-#pragma unroll
-        for (int h = 0; h < G; ++h) {
-            const i64 n0 = 4 * (g0 + h * stride);
-            if (n0 >= m) continue;
-            if (vec && n0 + 3 < m) {
-                reinterpret_cast<double2*>(out + n0)[0] = make_double2(acc[h][0], acc[h][1]);
-                reinterpret_cast<double2*>(out + n0)[1] = make_double2(acc[h][2], acc[h][3]);
             } else {
-#pragma unroll
-                for (int v = 0; v < 4; ++v)
-                    if (n0 + v < m) out[n0 + v] = acc[h][v];
+                int k[3];
+                if (!class_keys(dec, c[v], k)) {
+                    miss = true;
+                    continue;
+                }
+                s0 = k[0], s1 = k[1], s2 = k[2];
             }
+            if (!dcheck(s0 >= 0 && s2 < nk, 1, s2)) continue;
+            const int slot = s1 * nk + s0;
+            const uint2 bp = __ldg(&bitpre[slot >> 5]);  // (bits, pairs before the word)
+            const uint32_t bit = (uint32_t)(slot & 31);
+            const uint32_t k0 = __ldg(&kk[s2]);  // key id, bit 31: a key the list uses
+            if (!((bp.x >> bit) & 1u) || !(k0 >> 31)) {
+                miss = true;
+                continue;
+            }
+            const int pid = (int)(bp.y + __popc(bp.x & ((1u << bit) - 1u)));
+            q[v] = pid * ldq + (int)(k0 & 0x7fffffffu);  // (Q has fewer than 2^31 entries)
         }
+        double acc[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            acc[v] = 0.0;
+            if (q[v] >= 0 && dcheck(q[v] < nq, 3, q[v])) acc[v] = Q[q[v]];
+        }
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+            if (32 * v < left) op[32 * v] = acc[v];
     }
     if (miss) atomicExch(reinterpret_cast<unsigned long long*>(&cnt->overflow), 1ull);
 }
