@@ -122,25 +122,30 @@ __device__ __forceinline__ double nuc_gaussian(double r2) {
 }
 
 // 1 / sqrt(x) for 4 <= x < 1e201: the hardware's approximation (PTX
-// rsqrt.approx.ftz.f64, 20 bits) and two Newton steps y += y (1 - x y^2) / 2.
+// rsqrt.approx.ftz.f64: y, 20 bits) and one step of third order,
+// y (1 + e / 2 + 3 e^2 / 8) with e = 1 - x y^2, whose remainder is 5/16 e^3 <
+// 2^-60.  y^2 of the short y is exact, so e is rounded once and the result is
+// off by little more than its own rounding (two Newton steps, eight operations
+// for five: 0.83 ulp at most, here 0.51).
 // The field's cells away from a nucleus need no more than this range, and the
 // general function's handling of the others was most of the field's
 // instructions.
 __device__ __forceinline__ double nuc_rsqrt(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    y = fma(0.5 * y, fma(-x, y * y, 1.0), y);
-    return fma(0.5 * y, fma(-x, y * y, 1.0), y);
+    const double e = fma(-x, y * y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
 // Phi[u][v][t] (t fastest, pitches P) of every instance, position
 // (u + u0x, v + u0y, t + u0z) / 6; grid (row blocks, instance), a warp fills
 // whole (u, v) rows, up to eight cells per lane and turn: per nucleus the row's part of
-// the squared distance is formed once and each cell costs two FP64
-// multiply-adds and a reciprocal square root.  Bound: the FP64 pipe, 67% busy.
-// 24^3 to 8^3 batch of eight (54 million cells, 6 nuclei): 367 us; 722 us with a
-// thread per cell, its three coordinates divided by 6 and its whole distance per
-// nucleus.
+// the squared distance is formed once and each cell costs eight FP64
+// operations and the hardware's approximation.  Bound: the FP64 pipe (13 x 16 x
+// 11 points, 5 nuclei, 74 million of these: 36 us, the pipe's own time 33;
+// 41 us with two Newton steps).  24^3 to 8^3 batch of eight, with two Newton
+// steps: 367 us; 722 us with a thread per cell, its three coordinates divided
+// by 6 and its whole distance per nucleus.
 constexpr int NUC_FIELD_MAX_T = 2048;  // z positions held in shared memory (axes of 256 points: 1531 + 2 mmax)
 constexpr int NUC_FIELD_BLOCKS = 3;     // per SM
 __global__ void __launch_bounds__(256, NUC_FIELD_BLOCKS) k_nuc_field(const NucInst* __restrict__ inst, const double* __restrict__ npos,
