@@ -39,7 +39,8 @@
 // a time in ascending order, keeps the survivors (placed in order by its
 // ballots) in shared memory and appends them to a scratch buffer, and a scan
 // of the slots' counts and a copy place the runs (k_enum_slots_collect).  7^3:
-// 25 ms with arithmetic images of every copy, 3.5 ms reading them from the table.
+// 25 ms with arithmetic images of every copy, 3.5 ms reading them from the table, 2.9
+// ms testing two images at a time for one that leads with i.
 //
 // Fallbacks, when a slot's survivors exceed its buffer or the scratch buffer
 // fills: two passes (count, scan, write) over the live slots (k_enum_slots).
@@ -181,10 +182,19 @@ __device__ inline void slot_candidates(const SymGrid& G, i64 t, Emit&& emit) {
         eri_candidates(G, t, emit);
 }
 
+// status of the pass over the live slots
+struct EnumStatus {
+    unsigned long long used;  // scratch entries reserved
+    uint64_t total;           // classes in the list (the scan of the runs)
+    int overflow;             // 1: a slot's survivors exceeded its buffer; 2: the scratch buffer filled
+};
+
 // smallest linear index among the 48 O_h images of each grid point, and (images
 // non-null: ERI) the images themselves, 16 bits each; eight lanes a point, six of
-// them with eight images each
-__global__ void __launch_bounds__(256) k_orbit_min(SymGrid G, int* __restrict__ omin, uint4* __restrict__ images) {
+// them with eight images each.  Clears the status of the pass that follows.
+__global__ void __launch_bounds__(256) k_orbit_min(SymGrid G, int* __restrict__ omin, uint4* __restrict__ images,
+                                                   EnumStatus* __restrict__ st) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *st = EnumStatus{0ull, 0ull, 0};
     const i64 p = (i64)blockIdx.x * (blockDim.x >> 3) + (threadIdx.x >> 3);
     const int c = threadIdx.x & 7;
     int best = INT_MAX;
@@ -340,12 +350,6 @@ __global__ void k_enum_eri(SymGrid G, uint32_t* __restrict__ counts, const uint6
 // ---------------------------------------------------------------------------
 // one pass over the live slots
 
-struct EnumStatus {
-    unsigned long long used;  // scratch entries reserved
-    uint64_t total;           // classes in the list (the scan of the runs)
-    int overflow;             // 1: a slot's survivors exceeded its buffer; 2: the scratch buffer filled
-};
-
 // each slot's run from the scratch buffer to its place (dest: exclusive scan
 // of the run lengths in slot order); one warp per run
 __global__ void k_enum_place(const int64_t* __restrict__ scratch, const uint32_t* __restrict__ run_n,
@@ -377,11 +381,29 @@ static i64 enumerate_erida(const SymGrid& G, int64_t** d_out, cudaStream_t s) {
     DevBuf<uint64_t> dest(nlive, s);
     k_erida_slots<<<(unsigned)((nlive + 7) / 8), 256, 0, s>>>(G, nlive, masks.p, counts.p);
     GLI_CHECK_LAUNCH();
-    const i64 total = exclusive_scan_u32(counts.p, dest.p, nlive, s);
     int64_t* out = nullptr;
-    GLI_CUDA(cudaMallocAsync((void**)&out, (total > 0 ? total : 1) * sizeof(int64_t), s));
-    k_erida_place<<<(unsigned)((nlive + 255) / 256), 256, 0, s>>>(G, nlive, masks.p, dest.p, out);
-    GLI_CHECK_LAUNCH();
+    auto place = [&](i64 entries) {
+        GLI_CUDA(cudaMallocAsync((void**)&out, std::max<i64>(entries, 1) * sizeof(int64_t), s));
+        k_erida_place<<<(unsigned)((nlive + 255) / 256), 256, 0, s>>>(G, nlive, masks.p, dest.p, out);
+        GLI_CHECK_LAUNCH();
+    };
+    // A slot has at most 27 partners: lists whose bound takes at most 32 MB
+    // (191 points per axis) are placed before the host reads their length, which
+    // saves a round trip in the middle (20 us of 33^3's 190).
+    const i64 bound = 27 * nlive;
+    i64 total = 0;
+    if (bound <= ((i64)4 << 20)) {
+        DevBuf<uint64_t> len(1, s);
+        exclusive_scan_u32_dev(counts.p, dest.p, nlive, len.p, s);
+        place(bound);
+        uint64_t h = 0;
+        GLI_CUDA(cudaMemcpyAsync(&h, len.p, sizeof(h), cudaMemcpyDeviceToHost, s));
+        GLI_CUDA(cudaStreamSynchronize(s));
+        total = (i64)h;
+    } else {
+        total = exclusive_scan_u32(counts.p, dest.p, nlive, s);
+        place(total);
+    }
     *d_out = out;
     return total;
 }
@@ -573,8 +595,10 @@ __global__ void __launch_bounds__(256) k_enum_slots_collect(SymGrid G, const int
 // leading points (those in closed form as for ERIDA: 4 of 27), without compacting
 // the live slots and the host round trip for their number.  The few slots do not
 // fill the GPU, so each is spread out: a warp takes four partners, eight lanes
-// each, a lane per shifted copy.  (3^3: 53 us with a warp per slot and a lane per
-// partner, one chain of up to eight copies' images.)
+// each, a lane per shifted copy.  Bound: instructions, 69% of the issue slots
+// (3^3: 14 us; 23 us with every warp making the slot's points and partner lists
+// for itself, 53 us with a warp per slot and a lane per partner, one chain of up
+// to eight copies' images).
 constexpr int ENUM_SMALL_L = 3;
 
 __global__ void __launch_bounds__(256) k_enum_small(SymGrid G, i64 npoints, int64_t* __restrict__ scratch,
@@ -582,45 +606,53 @@ __global__ void __launch_bounds__(256) k_enum_small(SymGrid G, i64 npoints, int6
                                                     unsigned long long* __restrict__ run_off,
                                                     EnumStatus* __restrict__ st) {
     __shared__ unsigned kept;
+    __shared__ int s_pts[3], s_lo[3], s_hi[3], s_n[3];  // the slot's points; per axis their box and the partners
+    __shared__ signed char s_part[3][4];
     const int N = (int)G.N, N2 = N * N, sl = blockIdx.x, lane = threadIdx.x & 31;
-    int a, b, c;
-    erida_slot_point(npoints - 1 - sl / N2, a, b, c);
-    const int p0[3] = {-a, -b, -c};
-    const i64 t = lin3(G, p0) * N2 + sl % N2;
-    if (!slot_live<1>(G, t)) {
+    // the slot, made by the first warp, a lane per axis
+    if (threadIdx.x < 32) {
+        const int r = (int)npoints - 1 - sl / N2;  // the leading point's number, as erida_slot_point
+        int a = 0, b = 0;
+        while ((a + 1) * (a + 2) * (a + 3) / 6 <= r) ++a;
+        const int rb = r - a * (a + 1) * (a + 2) / 6;
+        while ((b + 1) * (b + 2) / 2 <= rb) ++b;
+        const int p0[3] = {-a, -b, b * (b + 1) / 2 - rb};
+        const int jk = sl % N2, i = (int)lin3(G, p0), j = jk / N, k = jk - j * N;
+        const bool live = slot_live<1>(G, (i64)i * N2 + jk);
+        if (lane < 3) {
+            const int pw = lane == 0 ? G.L * G.L : lane == 1 ? G.L : 1;
+            const int x = i / pw % G.L - G.e, y = j / pw % G.L - G.e, z = k / pw % G.L - G.e;
+            const int lo = min(min(x, y), z), hi = max(max(x, y), z);
+            s_pts[lane] = lane == 0 ? i : lane == 1 ? j : k;
+            s_lo[lane] = lo;
+            s_hi[lane] = hi;
+            s_n[lane] = live ? axis_partners(lo, hi, G.e, lane ? -G.e : z, s_part[lane]) : 0;
+        }
+        if (lane == 0) kept = 0u;
+    }
+    __syncthreads();
+    const int i = s_pts[0], nx = s_n[0], ny = s_n[1], nz = s_n[2], total = nx * ny * nz;  // (at most 27)
+    if (!total) {
         if (threadIdx.x == 0) run_n[sl] = 0u;
         return;
     }
-    if (threadIdx.x == 0) kept = 0u;
-    __syncthreads();
-    int i, j, k, p[4][3], lo[3], hi[3];
-    eri_slot_points(G, t, i, j, k);
-    point32(G, i, p[0]);
-    point32(G, j, p[1]);
-    point32(G, k, p[2]);
-    signed char sx[MAX_AXIS], sy[MAX_AXIS], sz[MAX_AXIS];
-    for (int x = 0; x < 3; ++x) {
-        lo[x] = min(min(p[0][x], p[1][x]), p[2][x]);
-        hi[x] = max(max(p[0][x], p[1][x]), p[2][x]);
-    }
-    const int nx = axis_partners(lo[0], hi[0], G.e, p[2][0], sx);
-    const int ny = axis_partners(lo[1], hi[1], G.e, -G.e, sy);
-    const int nz = axis_partners(lo[2], hi[2], G.e, -G.e, sz);
-    const int total = nx * ny * nz;  // (at most 27)
+    const i64 t = (i64)i * N2 + sl % N2;
     auto partner = [&](int cand, int q[3]) {
-        q[0] = sx[cand / (nz * ny)];
-        q[1] = sy[cand / nz % ny];
-        q[2] = sz[cand % nz];
+        const int yz = cand / nz, x = yz / ny;
+        q[0] = s_part[0][x];
+        q[1] = s_part[1][yz - x * ny];
+        q[2] = s_part[2][cand - yz * nz];
         return ((q[0] + G.e) * G.L + q[1] + G.e) * G.L + q[2] + G.e;
     };
     const int cand = threadIdx.x >> 3, m = lane & 7;
+    int q[3];
     bool keep = false;
     if (cand < total) {
-        const int l = partner(cand, p[3]);
+        const int l = partner(cand, q);
         if (G.omin[l] >= i) {
             int bias[3];
-            for (int x = 0; x < 3; ++x) bias[x] = min(lo[x], p[3][x]) + max(hi[x], p[3][x]);
-            const int pts[4] = {i, j, k, l};
+            for (int x = 0; x < 3; ++x) bias[x] = min(s_lo[x], q[x]) + max(s_hi[x], q[x]);
+            const int pts[4] = {i, s_pts[1], s_pts[2], l};
             keep = !copy_exists(bias, m) || canonical_copy(G, pts, copy_shift(G, bias, m));
         }
     }
@@ -638,17 +670,20 @@ __global__ void __launch_bounds__(256) k_enum_small(SymGrid G, i64 npoints, int6
         run_off[sl] = off;
         if (!fits) atomicOr(&st->overflow, 2);
     }
-    if (fits && list >> lane & 1u) scratch[off + __popc(list & ((1u << lane) - 1u))] = t * N + partner(lane, p[3]);
+    if (fits && list >> lane & 1u) scratch[off + __popc(list & ((1u << lane) - 1u))] = t * N + partner(lane, q);
 }
 
 // collect = false: the count and write passes over the live slots (the
 // fallback of a slot with more survivors than a warp's buffer)
 template <int KIND>
-static i64 enumerate_live(const SymGrid& G, bool collect, int64_t** d_out, int num_sms, cudaStream_t s) {
+static i64 enumerate_live(const SymGrid& G, bool collect, EnumStatus* st, int64_t** d_out, int num_sms, cudaStream_t s) {
     const i64 slots = KIND == 0 ? G.N : G.N * G.N * G.N;
     int64_t* out = nullptr;
     // one pass: survivors kept per warp, appended to scratch, placed in slot
-    // order; false when they do not fit
+    // order; false when they do not fit.  Without slot ids (k_enum_small) the
+    // list's length is bounded by 27 partners a slot, so it is placed before the
+    // host reads the length (a round trip, 20 us).
+    bool clear = true;  // (the status, by k_orbit_min)
     auto one_pass = [&](const int64_t* ids, i64 n, i64* total) {
         const unsigned grid = (unsigned)std::max<i64>(1, std::min<i64>((n + 7) / 8, (i64)num_sms * 16));
         const i64 cap = enum_scratch(G);
@@ -656,24 +691,32 @@ static i64 enumerate_live(const SymGrid& G, bool collect, int64_t** d_out, int n
         DevBuf<uint32_t> run_n(n, s);
         DevBuf<unsigned long long> run_off(n, s);
         DevBuf<uint64_t> dest(n, s);
-        DevBuf<EnumStatus> st(1, s);
-        st.zero();
+        if (!clear) GLI_CUDA(cudaMemsetAsync(st, 0, sizeof(EnumStatus), s));
+        clear = false;
+        auto place = [&](i64 entries) {
+            GLI_CUDA(cudaMallocAsync((void**)&out, std::max<i64>(entries, 1) * sizeof(int64_t), s));
+            k_enum_place<<<grid, 256, 0, s>>>(scratch.p, run_n.p, run_off.p, dest.p, n, out);
+            GLI_CHECK_LAUNCH();
+        };
         if (ids)
             k_enum_slots_collect<KIND><<<grid, 256, 0, s>>>(G, ids, n, scratch.p, (unsigned long long)cap, run_n.p,
-                                                            run_off.p, st.p);
+                                                            run_off.p, st);
         else
             k_enum_small<<<(unsigned)n, 256, 0, s>>>(G, n / (G.N * G.N), scratch.p, (unsigned long long)cap, run_n.p,
-                                                     run_off.p, st.p);
+                                                     run_off.p, st);
         GLI_CHECK_LAUNCH();
-        exclusive_scan_u32_dev(run_n.p, dest.p, n, &st.p->total, s);
+        exclusive_scan_u32_dev(run_n.p, dest.p, n, &st->total, s);
+        if (!ids) place(27 * n);
         EnumStatus h;
-        GLI_CUDA(cudaMemcpyAsync(&h, st.p, sizeof(h), cudaMemcpyDeviceToHost, s));
+        GLI_CUDA(cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, s));
         GLI_CUDA(cudaStreamSynchronize(s));
-        if (h.overflow) return false;
+        if (h.overflow) {
+            if (out) cudaFreeAsync(out, s);
+            out = nullptr;
+            return false;
+        }
         *total = (i64)h.total;
-        GLI_CUDA(cudaMallocAsync((void**)&out, (h.total > 0 ? h.total : 1) * sizeof(int64_t), s));
-        k_enum_place<<<grid, 256, 0, s>>>(scratch.p, run_n.p, run_off.p, dest.p, n, out);
-        GLI_CHECK_LAUNCH();
+        if (ids) place(*total);
         return true;
     };
     i64 total = 0;
@@ -733,14 +776,15 @@ i64 enumerate_device(int kind, const GridDesc& g, int64_t** d_out, cudaStream_t 
     DevBuf<int> omin(G.N, s);
     DevBuf<uint4> images;
     if (kind == 1) images.alloc(6 * G.N, s);
-    k_orbit_min<<<(unsigned)((G.N + 31) / 32), 256, 0, s>>>(G, omin.p, images.p);
+    DevBuf<EnumStatus> st(1, s);
+    k_orbit_min<<<(unsigned)((G.N + 31) / 32), 256, 0, s>>>(G, omin.p, images.p, st.p);
     GLI_CHECK_LAUNCH();
     G.omin = omin.p;
     G.images = images.p;
     if (!two || live_two) {
         const int sms = context().num_sms;
-        if (kind == 1) return enumerate_live<1>(G, !live_two, d_out, sms, s);
-        return enumerate_live<0>(G, false, d_out, sms, s);
+        if (kind == 1) return enumerate_live<1>(G, !live_two, st.p, d_out, sms, s);
+        return enumerate_live<0>(G, false, st.p, d_out, sms, s);
     }
     DevBuf<uint32_t> counts(slots, s);
     DevBuf<uint64_t> offsets(slots, s);

@@ -62,22 +62,28 @@ __device__ inline bool canonical_copy(const SymGrid& G, const int l[4], int sft)
         least = min(least, G.omin[q[k]]);
     }
     if (least != l[0]) return least > l[0];
+    const uint32_t both = (uint32_t)l[0] * 0x10001u;
     for (int c = 0; c < 6; ++c) {
         uint4 im[4];
         for (int k = 0; k < 4; ++k) im[k] = __ldg(G.images + (i64)q[k] * 6 + c);
 #pragma unroll
-        for (int h = 0; h < 8; ++h) {
-            uint32_t r[4];
+        for (int h = 0; h < 4; ++h) {  // two images of each point in a word
+            uint32_t w[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const uint32_t w = h < 2 ? im[k].x : h < 4 ? im[k].y : h < 6 ? im[k].z : im[k].w;
-                r[k] = h & 1 ? w >> 16 : w & 0xffffu;
+            for (int k = 0; k < 4; ++k) w[k] = h == 0 ? im[k].x : h == 1 ? im[k].y : h == 2 ? im[k].z : im[k].w;
+            const uint32_t off = __vimin3_u16x2(__vimin3_u16x2(w[0], w[1], w[2]), w[3], w[3]) ^ both;
+            if ((off & 0xffffu) && off >> 16) continue;
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                if (u ? off >> 16 : off & 0xffffu) continue;
+                uint32_t r[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) r[k] = u ? w[k] >> 16 : w[k] & 0xffffu;
+                const uint32_t ab = min(r[0], r[1]) * N + max(r[0], r[1]);
+                const uint32_t cd = min(r[2], r[3]) * N + max(r[2], r[3]);
+                const uint32_t first = min(ab, cd), second = max(ab, cd);
+                if (first < ij || (first == ij && second < kl)) return false;
             }
-            if (min(min(r[0], r[1]), min(r[2], r[3])) != (uint32_t)l[0]) continue;
-            const uint32_t ab = min(r[0], r[1]) * N + max(r[0], r[1]);
-            const uint32_t cd = min(r[2], r[3]) * N + max(r[2], r[3]);
-            const uint32_t first = min(ab, cd), second = max(ab, cd);
-            if (first < ij || (first == ij && second < kl)) return false;
         }
     }
     return true;
