@@ -144,13 +144,54 @@ __global__ void k_check_complete(SymGrid G, const int64_t* __restrict__ idx, i64
     if (orbit_min_quad(G, p, bias) != v) atomicOr(bad, 1);
 }
 
-__global__ void k_key_table(SymGrid G, const int64_t* __restrict__ idx, const double* __restrict__ val, i64 m,
-                            double* __restrict__ table) {
-    const i64 n = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= m) return;
-    int p[4][3];
-    eri_points(G, idx[n], p);
-    table[eri_key_slot(p, G.L)] = val[n];
+// The key table of a complete list: each class's value to the slot of its keys.
+// canon non-null: the canonical list, which the class list has to equal; where
+// it does not, *bad is set and nothing is written (so that every slot written is
+// the slot of a class of the grid).  The points' coordinates come from shared
+// memory; one estimated 64-bit quotient (N^4 < 2^53) and 32-bit arithmetic.
+// Bound: HBM reads of the two lists and the values, and the scattered writes.
+// 7^3, 3.57 million classes: 41 us; 78 us as a comparison of the lists, and
+// a pass with four points' 64-bit divisions for each class.
+constexpr int KEY_TABLE_POINTS = 4096;  // (key tables end at 14 points per axis)
+__global__ void __launch_bounds__(256) k_key_table(SymGrid G, const int64_t* __restrict__ canon,
+                                                   const int64_t* __restrict__ idx, const double* __restrict__ val,
+                                                   i64 m, double* __restrict__ table, int* __restrict__ bad) {
+    __shared__ uint32_t pt[KEY_TABLE_POINTS];  // coordinates from the grid's corner, 8 bits each
+    const uint32_t N = (uint32_t)G.N, L = (uint32_t)G.L;
+    for (uint32_t p = threadIdx.x; p < N; p += blockDim.x) {
+        const uint32_t r = p / L, x = r / L;
+        pt[p] = x | (r - x * L) << 8 | (p - r * L) << 16;
+    }
+    __syncthreads();
+    const i64 N2 = (i64)N * N;
+    const double inv = 1.0 / (double)N2;
+    bool differ = false;
+    for (i64 n = (i64)blockIdx.x * blockDim.x + threadIdx.x; n < m; n += (i64)gridDim.x * blockDim.x) {
+        const i64 v = idx[n];
+        if (canon && v != canon[n]) {
+            differ = true;
+            continue;
+        }
+        i64 hi = (i64)((double)v * inv), lo = v - hi * N2;
+        if (lo < 0) {
+            --hi;
+            lo += N2;
+        } else if (lo >= N2) {
+            ++hi;
+            lo -= N2;
+        }
+        const uint32_t ij = (uint32_t)hi, kl = (uint32_t)lo, i = ij / N, k = kl / N;
+        const uint32_t pi = pt[i], pj = pt[ij - i * N], pk = pt[k], pl = pt[kl - k * N];
+        int key[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const int ci = pi >> 8 * a & 255, cj = pj >> 8 * a & 255, ck = pk >> 8 * a & 255, cl = pl >> 8 * a & 255;
+            key[a] = pair_axis_key(ci - cj, ck - cl, ci + cj - ck - cl, (int)L);
+        }
+        const int a = min(key[0], key[1]), b = max(key[0], key[1]);
+        table[tetra_index32(min(a, key[2]), max(a, min(b, key[2])), max(b, key[2]))] = val[n];
+    }
+    if (differ) atomicOr(bad, 1);
 }
 
 // rows [row0, row0 + nrows) of the (ij) x (kl) flattening of the dense grid D,
@@ -168,15 +209,6 @@ __global__ void k_fill_eri_rows_keyed(DenseGrid D, const double* __restrict__ ta
         dense_point(D, kl % D.N, p[3]);
         out[e] = table[eri_key_slot(p, L)];
     }
-}
-
-// points of a dense grid (x-major), for the slab fill
-__global__ void k_dense_points(DenseGrid D, short4* __restrict__ pt) {
-    const i64 n = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= D.N) return;
-    int p[3];
-    dense_point(D, n, p);
-    pt[n] = make_short4((short)p[0], (short)p[1], (short)p[2], 0);
 }
 
 // slab i of the (i j k l) tensor, S[(j N + k) N + l] = V[i j k l], its first
@@ -516,47 +548,66 @@ static CanonicalList canonical_eri_list(const GridDesc& g, i64 e, cudaStream_t s
     return c;
 }
 
-// bad = 1 where the list differs from the canonical list
-__global__ void k_equal_lists(const int64_t* __restrict__ a, const int64_t* __restrict__ b, i64 m,
-                              int* __restrict__ bad) {
-    bool differ = false;
-    for (i64 n = (i64)blockIdx.x * blockDim.x + threadIdx.x; n < m; n += (i64)gridDim.x * blockDim.x)
-        differ = differ || a[n] != b[n];
-    if (differ) atomicOr(bad, 1);
-}
-
 // Key table of a complete ERI class list, or an empty buffer when the list is
 // not the complete canonical list of its grid (then entries are looked up).
+// begin: whether the list can be complete (its grid's table is small enough and
+// its length is the canonical list's).  queue: the table, and whether the list
+// is complete, on the stream.  valid: the answer, after a wait; a table queued
+// for a list that is not complete holds unset values and must not be used for a
+// result.
 struct KeyTable {
     DevBuf<double> t;
-    bool ok = false;
+    DevBuf<int> bad;
+    CanonicalList canon;
+    i64 slots = 0;
+    bool ok = false, asked = false;
+    bool begin(const SymGrid& G, const GridDesc& g, i64 m, cudaStream_t s) {
+        if (m <= 0) return false;
+        const i64 nk = pair_axis_keys((int)G.L);
+        slots = nk * (nk + 1) * (nk + 2) / 6;
+        if (slots > ((i64)1 << 29)) return false;  // above 4 GB: keep the lookups
+        canon = canonical_eri_list(g, G.e, s);
+        return canon.count == m;
+    }
+    void queue(const SymGrid& G, const int64_t* d_idx, const double* d_val, i64 m, cudaStream_t s) {
+        if (G.N > KEY_TABLE_POINTS) fail(GLI_ERR_INTERNAL, "key table of %lld points", (long long)G.N);
+        bad.alloc(1, s);
+        bad.zero();
+        if (!canon.d) {  // (before the table: only canonical indices may be decoded)
+            k_check_complete<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(G, d_idx, m, bad.p);
+            GLI_CHECK_LAUNCH();
+            asked = true;
+            ok = true;
+            if (!valid(s)) return;
+        }
+        t.alloc(slots, s);
+        const Context& c = context();
+        k_key_table<<<(unsigned)std::min<i64>((m + 255) / 256, (i64)c.num_sms * 8), 256, 0, s>>>(
+            G, canon.d, d_idx, d_val, m, t.p, bad.p);
+        GLI_CHECK_LAUNCH();
+        ok = true;
+        asked = canon.d != nullptr;
+    }
+    bool valid(cudaStream_t s) {
+        if (asked) {
+            asked = false;
+            int h = 0;
+            GLI_CUDA(cudaMemcpyAsync(&h, bad.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+            GLI_CUDA(cudaStreamSynchronize(s));
+            if (h) {
+                ok = false;
+                t.release();
+            }
+        }
+        return ok;
+    }
 };
 
 static void build_key_table(const SymGrid& G, const GridDesc& g, const int64_t* d_idx, const double* d_val, i64 m,
                             KeyTable& kt, cudaStream_t s) {
-    kt.ok = false;
-    if (m <= 0) return;
-    const i64 L = G.L;
-    const i64 nk = pair_axis_keys((int)L);
-    const i64 slots = nk * (nk + 1) * (nk + 2) / 6;
-    if (slots > ((i64)1 << 29)) return;  // above 4 GB: keep the lookups
-    const CanonicalList canon = canonical_eri_list(g, G.e, s);
-    if (canon.count != m) return;
-    DevBuf<int> bad(1, s);
-    bad.zero();
-    if (canon.d)
-        k_equal_lists<<<grid_for(m), 256, 0, s>>>(d_idx, canon.d, m, bad.p);
-    else
-        k_check_complete<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(G, d_idx, m, bad.p);
-    GLI_CHECK_LAUNCH();
-    int h = 0;
-    GLI_CUDA(cudaMemcpyAsync(&h, bad.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    GLI_CUDA(cudaStreamSynchronize(s));
-    if (h) return;
-    kt.t.alloc(slots, s);
-    k_key_table<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(G, d_idx, d_val, m, kt.t.p);
-    GLI_CHECK_LAUNCH();
-    kt.ok = true;
+    if (!kt.begin(G, g, m, s)) return;
+    kt.queue(G, d_idx, d_val, m, s);
+    kt.valid(s);
 }
 
 void fill_dense_device(int kind, const GridDesc& sparse, const int64_t* d_idx, const double* d_val, i64 m,
@@ -620,7 +671,7 @@ void apply_eri_device(const GridDesc& g, const int64_t* d_idx, const double* d_v
     const DenseGrid D = dense_of(g);
     const i64 N = D.N, N2 = N * N;
     KeyTable kt;
-    build_key_table(G, g, d_idx, d_val, m, kt, s);
+    if (kt.begin(G, g, m, s)) kt.queue(G, d_idx, d_val, m, s);
     if (kt.ok && G.L <= PAIR_MAX_AXIS) {
         std::vector<int> coords[3];
         for (int a = 0; a < 3; ++a)
@@ -637,9 +688,11 @@ void apply_eri_device(const GridDesc& g, const int64_t* d_idx, const double* d_v
                 k_apply_sum<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(C.p, (int)N, cols, (int)ns, (int)c0, d_ret);
                 GLI_CHECK_LAUNCH();
             }
-            return;
+            // (a list that is not complete is found here, and expanded below)
+            if (kt.valid(s)) return;
         }
     }
+    kt.valid(s);
     // chunk of rows i of V[i][j][k][l]: for one i, the (j, k, l) block is N^3
     const i64 per_i = N2 * N;
     i64 ci = (i64)(256 << 20) / (per_i * 8);
@@ -824,10 +877,35 @@ void project_device(int kind, const GridDesc& g, const int64_t* d_idx, const dou
     // 7^3 onto 32 orbitals: the slab as FP64-level int8 slices on the tcgen05
     // tensor cores took 0.44 s, dominated by writing the slices)
     KeyTable kt;
-    build_key_table(G, g, d_idx, d_val, m, kt, s);
-    const bool slab32 = kt.ok && N2 * N < ((i64)1 << 32);
-    DevBuf<short4> pt;
+    std::vector<double> hb;
+    if (kt.begin(G, g, m, s)) {
+        // (the basis is read before the table is queued, and looked through on
+        // the host while that is made)
+        if (N2 * N < ((i64)1 << 32)) {
+            hb.resize((size_t)(N * M));
+            GLI_CUDA(cudaMemcpyAsync(hb.data(), d_basis, N * M * sizeof(double), cudaMemcpyDeviceToHost, s));
+            GLI_CUDA(cudaStreamSynchronize(s));
+        }
+        kt.queue(G, d_idx, d_val, m, s);
+    }
+    std::vector<i64> act;
+    for (i64 i = 0; i < (hb.empty() ? 0 : N); ++i)
+        for (i64 c = 0; c < M; ++c)
+            if (hb[(size_t)(i * M + c)] != 0.0) {
+                act.push_back(i);
+                break;
+            }
     std::vector<short4> hpt;
+    for (const i64 i : act) {
+        const int yz = D.num[1] * D.num[2], r = (int)(i % yz);
+        hpt.push_back(make_short4((short)(D.istart[0] + i / yz), (short)(D.istart[1] + r / D.num[2]),
+                                  (short)(D.istart[2] + r % D.num[2]), 0));
+    }
+    std::vector<double> hbc;  // the rows that are not zero
+    if ((i64)act.size() < N)
+        for (const i64 i : act) hbc.insert(hbc.end(), hb.begin() + i * M, hb.begin() + (i + 1) * M);
+    const bool slab32 = kt.valid(s) && N2 * N < ((i64)1 << 32);
+    DevBuf<short4> pt;
     // Rows of the basis that are zero contribute nothing: with the key table
     // (entries computed from point coordinates) the contraction runs over the
     // points whose rows are nonzero only -- a basis on a sub-grid of the sparse
@@ -836,38 +914,14 @@ void project_device(int kind, const GridDesc& g, const int64_t* d_idx, const dou
     const double* bx = d_basis;
     DevBuf<double> bcomp;
     if (slab32) {
-        pt.alloc(N, s);
-        k_dense_points<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(D, pt.p);
-        GLI_CHECK_LAUNCH();
-        hpt.resize(N);
-        std::vector<double> hb((size_t)(N * M));
-        GLI_CUDA(cudaMemcpyAsync(hpt.data(), pt.p, N * sizeof(short4), cudaMemcpyDeviceToHost, s));
-        GLI_CUDA(cudaMemcpyAsync(hb.data(), d_basis, N * M * sizeof(double), cudaMemcpyDeviceToHost, s));
-        GLI_CUDA(cudaStreamSynchronize(s));
-        std::vector<i64> act;
-        for (i64 i = 0; i < N; ++i)
-            for (i64 c = 0; c < M; ++c)
-                if (hb[(size_t)(i * M + c)] != 0.0) {
-                    act.push_back(i);
-                    break;
-                }
         if (act.empty()) {
             GLI_CUDA(cudaMemsetAsync(d_out, 0, M * M * M * M * sizeof(double), s));
             return;
         }
         if ((i64)act.size() < N) {
             Nx = (i64)act.size();
-            std::vector<short4> hp((size_t)Nx);
-            std::vector<double> hbc((size_t)(Nx * M));
-            for (i64 a = 0; a < Nx; ++a) {
-                hp[(size_t)a] = hpt[(size_t)act[(size_t)a]];
-                for (i64 c = 0; c < M; ++c) hbc[(size_t)(a * M + c)] = hb[(size_t)(act[(size_t)a] * M + c)];
-            }
-            hpt.swap(hp);
-            GLI_CUDA(cudaMemcpyAsync(pt.p, hpt.data(), Nx * sizeof(short4), cudaMemcpyHostToDevice, s));
             bcomp.alloc(Nx * M, s);
             GLI_CUDA(cudaMemcpyAsync(bcomp.p, hbc.data(), Nx * M * sizeof(double), cudaMemcpyHostToDevice, s));
-            GLI_CUDA(cudaStreamSynchronize(s));  // the host vectors go out of scope
             bx = bcomp.p;
         }
     }
@@ -920,6 +974,11 @@ void project_device(int kind, const GridDesc& g, const int64_t* d_idx, const dou
                 return;
             }
         }
+    }
+    if (slab32) {
+        pt.alloc(Nx, s);
+        GLI_CUDA(cudaMemcpyAsync(pt.p, hpt.data(), Nx * sizeof(short4), cudaMemcpyHostToDevice, s));
+        GLI_CUDA(cudaStreamSynchronize(s));  // the host vectors go out of scope
     }
     // V[i j k l] = V[j i k l]: the two first contractions run over the pairs
     // j <= i only, W[i][j] = B^T V[i j] B (M x M), and W[j][i] = W[i][j] is
