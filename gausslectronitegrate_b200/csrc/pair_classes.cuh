@@ -155,14 +155,17 @@ struct PairSmem {
 // needs no trip of A through shared memory, and every warp takes part in it.
 // The next class's keys are made under the last plane, its first plane's copies
 // under that contraction.
+// A tile's k steps that lie before all its rows in the diagonal plane are zero
+// and left out (343 points: 4.43 to 4.26 ms).
 // Bound: the FP64 tensor pipe, 55% busy (343 points, 20 orbitals), with the
 // shared-memory pipe 59% busy (V fragments, and copies whose 32 values lie in
-// about as many lines).  Measured on a B200, first two contractions: 216 points
-// and 32 orbitals 1.04 ms (a contraction per point pair, its slab staged from
-// the key table: 5.25 ms), 343 points and 20 orbitals 4.44 ms (23.7 ms; A through
-// shared memory 4.88 ms); the whole projection calls 9.9 to 3.8 ms and 28.0 to
-// 6.5 ms, the apply at 5^3 points and 4 states 12.7 to 0.50 ms (0.16 ms of this
-// kernel; 0.21 ms with four column tiles multiplied whatever the class's pairs).
+// about as many lines; contiguous copies in their place measured 4.03 ms).
+// Measured on a B200, first two contractions: 216 points and 32 orbitals 0.98
+// ms (a contraction per point pair, its slab staged from the key table: 5.25
+// ms), 343 points and 20 orbitals 4.26 ms (23.7 ms; A through shared memory 4.88
+// ms); the whole projection calls 9.9 to 3.5 ms and 28.0 to 6.4 ms, the apply at
+// 5^3 points and 4 states 12.7 to 0.48 ms (0.16 ms of this kernel; 0.21 ms with
+// four column tiles multiplied whatever the class's pairs).
 //
 // A warp owns up to two 16-row tiles (rows 16 (w + W t)) and keeps their
 // accumulators over all planes, so each B fragment serves all its tiles.  The
@@ -374,9 +377,14 @@ __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : 1)
             // rows that meet this plane (offsets into the maps and the values)
             const int rows = SYM ? (lx + 1) * nyz : N, xmax = SYM ? lx + 1 : box.n[0];
             int mo[TPW][2], po[TPW][2];
+            // first k step of a tile: below it, in the diagonal plane, l lies
+            // before every row of the tile
+            int from[TPW];
             int nact = 0;
 #pragma unroll
             for (int t = 0; t < TPW; ++t) {
+                const int below = 16 * (warp + PAIR_WARPS * t) - lx * nyz;
+                from[t] = SYM && below > 0 ? below >> 2 : 0;
                 if (16 * (warp + PAIR_WARPS * t) < rows) nact = t + 1;
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
@@ -387,7 +395,7 @@ __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : 1)
                 }
             }
             const int bo = lay.planes + (lx * nyz + q) * LDB + c8;
-            auto steps = [&](auto active, auto columns) {
+            auto steps = [&](auto active, auto columns, int st0, int st1) {
                 constexpr int A = decltype(active)::value, J = decltype(columns)::value;
                 auto step = [&](int st, bool last) {
                     // (past the plane's last point B is taken as zero, not only
@@ -406,23 +414,26 @@ __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : 1)
                     }
                 };
 #pragma unroll 2
-                for (int st = 0; st < box.S - 1; ++st) {
+                for (int st = st0; st < min(st1, box.S - 1); ++st) {
                     step(st, false);
                     gen_one();
                 }
-                step(box.S - 1, true);
+                if (st1 == box.S) step(box.S - 1, true);
             };
-            auto planes_of = [&](auto active) {
+            auto planes_of = [&](auto active, int st0, int st1) {
                 if constexpr (!SYM && NT > 1) {
-                    if (live == 1) return steps(active, std::integral_constant<int, 1>{});
+                    if (live == 1) return steps(active, std::integral_constant<int, 1>{}, st0, st1);
                     if constexpr (NT > 2)
-                        if (live == 2) return steps(active, std::integral_constant<int, 2>{});
+                        if (live == 2) return steps(active, std::integral_constant<int, 2>{}, st0, st1);
                 }
-                steps(active, std::integral_constant<int, NT>{});
+                steps(active, std::integral_constant<int, NT>{}, st0, st1);
             };
             if constexpr (TPW >= 2)
-                if (nact == 2) planes_of(std::integral_constant<int, 2>{});
-            if (nact == 1) planes_of(std::integral_constant<int, 1>{});
+                if (nact == 2) {
+                    if (SYM) planes_of(std::integral_constant<int, 1>{}, from[0], from[1]);
+                    planes_of(std::integral_constant<int, 2>{}, from[1], box.S);
+                }
+            if (nact == 1) planes_of(std::integral_constant<int, 1>{}, from[0], box.S);
             while (gk < gend) gen_one();
             dm_commit();
         }
