@@ -702,14 +702,13 @@ def run_projection(args):
         E = eri.project(basis)
         ms.append(1e3 * (time.perf_counter() - t0))
     clk = clocks.stop()
-    # the FLOPs the contraction executes: the first two contractions run over
-    # the pairs j <= i of the tensor's (i j) symmetry, n (n + 1) / 2 of n^2,
-    # and the first over the l >= k chunks of each slab's rows (64-row tiles
-    # start their K loop at their smallest k: tiles at k0 = 0, 64, 128, 192)
+    # the FLOPs the contraction executes: the first two contractions once per
+    # pair class (21 unordered coordinate pairs per axis), the first over the
+    # planes l >= k by the points' x coordinate (21 of 36 pairs of planes), then
+    # the other pair's indices against the packed class blocks
     n, M = 216, W.ERI6_STATES
-    pairs = n * (n + 1) / 2
-    kept = sum(min(64, n - k0) * (n - k0 // 16 * 16) for k0 in range(0, n, 64)) / (n * n)
-    flops = 2.0 * (pairs * n * n * M * kept + pairs * n * M * M + n ** 2 * M ** 3 + n * M ** 4)
+    classes, P = 21 ** 3, M * (M + 1) / 2
+    flops = 2.0 * (classes * (n * n * 21 / 36 * M + n * M * M) + n * n * P * M + n * P * M * M)
     step = statistics.median(ms)
     peak = C.c_double()
     gli.lib().gli_b200_measure_fp64_peak(C.byref(peak))
@@ -723,8 +722,8 @@ def run_projection(args):
                    "max_abs_E": float(np.abs(E).max())},
         "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",
                      "frac": achieved / peak.value if peak.value else None,
-                     "algorithmic_flops_per_step": flops, "kernel": "k_dmma<KeyedSlabOp> + k_dmma<StridedOp>",
-                     "flops_counted": "executed: first two contractions over the i >= j pairs, the first over the l >= k chunks",
+                     "algorithmic_flops_per_step": flops, "kernel": "k_pair_contract + k_dmma<ClassBlocksOp> + k_dmma<StridedOp>",
+                     "flops_counted": "executed: first two contractions per pair class, the first over the planes l >= k",
                      "peak_source": "measured FP64 peak on this device (gli_b200_measure_fp64_peak)",
                      "note": "host-API step: includes the 8 MB output copy"},
         "clocks": clk}), flush=True)
@@ -734,8 +733,7 @@ def run_projection(args):
 def run_nuclear_batch(args):
     """Config: 256 linear H_n chains (n uniform in 2..8, bonds 1.0-3.0 bohr,
     jitter N(0, 0.1) bohr), each on its own centred grid of 8^3..24^3 points at
-    0.5 bohr; every matrix written to its own device buffer; one call per step
-    (one CUDA graph per chunk of instances).  Metric: instances per second and
+    0.5 bohr; every matrix written to its own device buffer; one call per step.  Metric: instances per second and
     matrix GB/s written; the mixed form's max abs error against FP64 in Ha on
     the first instances."""
     import torch
@@ -937,10 +935,13 @@ def roofline(paths, dom, st, plan, U, m, fp64_peak):
         achieved = flops / (ms * 1e-3) / 1e12 if ms > 0 else None
         return {"bound": "fp64", "stage": dom[0], "kernel": kernel,
                 "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
-                "frac": achieved / fp64_peak if achieved and fp64_peak else None,
+                "frac": achieved / fp64_peak if achieved and fp64_peak and achieved <= fp64_peak else None,
                 "peak_source": "measured FP64 peak on this device (gli_b200_measure_fp64_peak: "
                                "max of FMA and m8n8k4 MMA probes)",
-                "algorithmic_flops_per_launch": flops, "traffic": None}
+                "algorithmic_flops_per_launch": flops,
+                "flops_counted": "over the whole lattice; on wide grids stages A and B leave out the positions where a "
+                                 "key's weights are zero (no fraction where the count exceeds what can be executed)",
+                "traffic": None}
     S, BN = 5, 96
     nsp = (nS + 127) // 128 * 128
     bytes_ = {"A": S * nsp * kp + S * ((nA + BN - 1) // BN * BN) * kp + 8 * nA * nS,

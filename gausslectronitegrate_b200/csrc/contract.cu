@@ -2243,8 +2243,8 @@ static void enqueue_eval(const EvalArgs& a, PlanMode mode, EvalStatus* st, Stage
 
 // ---------------------------------------------------------------------------
 // CUDA graphs of evaluations.  A bounded or sized evaluation issues no host
-// synchronisation, so the whole launch sequence (allocations, memsets and about
-// 15 kernels) is captured once and replayed: every replay recomputes everything
+// synchronisation, so the whole launch sequence (allocations and its kernels)
+// is captured once and replayed: every replay recomputes everything
 // from the class list in device memory; only the launch overhead is saved.
 // A graph is keyed by what fixes its launch sequence and its pointers: the
 // table set (kept alive by the entry), the grid, the class-list pointer and

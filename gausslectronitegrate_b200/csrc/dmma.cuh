@@ -10,8 +10,7 @@
 // alike; per k-step of 4 it reads 4 A and BN/16 B fragments (one double each)
 // for 4 BN/16 MMAs of 256 FMAs.  BN = 80 serves 65..80 and 129..160 columns in
 // one and two column tiles (129 keys: 2 tiles instead of 3, measured 20%
-// faster on the stage A shape); BN = 144 holds 129 keys in one tile (another
-// 1.5%: the lattice gathers are made once).
+// faster on the stage A shape).
 //
 // The operand sources are arbitrary: an Op class says, per tile element, where
 // the double comes from (a strided matrix, a lattice-table gather, a gather

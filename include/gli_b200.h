@@ -301,9 +301,9 @@ int gli_b200_sparse_values(int kind, const struct gausslet_data* gdata,
  * and writes its N_k x N_k row-major matrix to the device buffer d_out[k];
  * all instances share the coefficients and tol.  form GLI_FORM_FP64 is the
  * reference's arithmetic; GLI_FORM_MIXED runs the three lattice contractions
- * as int8-sliced tensor-core products (about 1e-9 relative).  Each chunk of
- * instances is one CUDA graph launch; the number of concurrent instance
- * pipelines is chosen by the autotuner.  Batches the reference's
+ * as int8-sliced tensor-core products (about 1e-9 relative).  A chunk of
+ * instances is one upload and one launch per stage and pipeline; the number of
+ * concurrent instance pipelines is chosen by the autotuner.  Batches the reference's
  * compute_nuclear_gausslet_integrals (include/nuclear_integrals.h:40-43,
  * src/nuclear_integrals.c:133-266). */
 int gli_b200_nuclear_batch_dev(const struct gausslet_data* gdata, glong num_instances,
@@ -317,7 +317,7 @@ int gli_b200_nuclear_batch(const struct gausslet_data* gdata, glong num_instance
 	const struct cartesian_grid_3d* grids, const glong* nuclei_offsets,
 	const struct atomic_nucleus* nuclei, double tol, int form, double* const* h_out);
 
-/* instances, graph chunks and concurrent instance pipelines of the calling
+/* instances, chunks and concurrent instance pipelines of the calling
  * thread's last nuclear batch (no reference counterpart) */
 void gli_b200_last_nuclear_batch(glong out[3]);
 
