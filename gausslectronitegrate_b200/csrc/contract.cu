@@ -2089,6 +2089,15 @@ static void enqueue_eval(const EvalArgs& a, PlanMode mode, EvalStatus* st, Stage
         w.C = H.p;
         w.rs = 1;
         w.cs = nS;
+        if (t.banded) {
+            w.keys = aKey.p;
+            w.reach = rch;
+            if (!tc_b) {  // (the sliced stage B reads whole rows of H)
+                w.from = rfrom;
+                w.upto = rupto;
+                w.S = t.S.p;
+            }
+        }
         tc_gemm_tiled(a.G, Wa.view(), w, nbt, &st->tc_err, s);
     } else {
         // small problems split the t loop so that enough blocks exist (the

@@ -243,6 +243,13 @@ struct TileWork {
     const int64_t* n_dev = nullptr;
     double* C = nullptr;
     i64 rs = 0, cs = 0;
+    // column n's key and the K positions first..last outside which its B row is
+    // zero (null: whole rows); from, upto, S (null: every tile is computed): the
+    // (u, v) positions at which C is read for a key, and u^2 + v^2 of A's rows in
+    // ascending order
+    const int* keys = nullptr;
+    const int2 *reach = nullptr, *from = nullptr, *upto = nullptr;
+    const int* S = nullptr;
 };
 
 // sets the kernels' shared-memory attribute on the current device (once per
