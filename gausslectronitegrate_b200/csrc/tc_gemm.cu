@@ -180,10 +180,12 @@ __global__ void __launch_bounds__(256, 1) k_tc_gemm(TiledOperand A, TiledOperand
     const int rows_valid = min(TC_BM, w.a_rows - mt * TC_BM);
     if (ncols <= 0 || rows_valid <= 0) return;  // uniform across the CTA
     const i64 a_rb = w.a_batched ? (i64)batch * w.a_blocks + mt : mt;
+    const int n16 = (ncols + 15) & ~15;  // columns in use, whole MMA widths (at most TC_BN)
     const int nkc = A.nkc;
     // The chunks in which some column of the tile has a nonzero weight (zero
     // digits add nothing), and whether the tile is read at all: the same in every
-    // warp.  (Stage A at ERIDA 129^3: 108 us; 129 us over the whole lattice.
+    // warp.  (Stage A at ERIDA 129^3, 96 + 33 columns: 129 us over the whole lattice,
+    // 108 us by reaches, 101 us with MMAs and stores of the columns in use only.
     // One tile an SM: its loads, MMAs and stores follow one another.)
     int kc0 = 0, kc1 = nkc;
     if (w.reach) {
@@ -247,7 +249,7 @@ __global__ void __launch_bounds__(256, 1) k_tc_gemm(TiledOperand A, TiledOperand
         }
     } else if (warp == 1 && lane == 0) {
         // MMA issuer
-        constexpr uint32_t idesc = idesc_s8(TC_BM, TC_BN);
+        const uint32_t idesc = idesc_s8(TC_BM, n16);
         constexpr uint32_t SBO = (TC_BK / 16) * 128;
         for (int kc = kc0; kc < kc1; ++kc) {
             const int s = (kc - kc0) % NST, round = (kc - kc0) / NST;
@@ -289,17 +291,15 @@ __global__ void __launch_bounds__(256, 1) k_tc_gemm(TiledOperand A, TiledOperand
     __syncthreads();
 
     if (!abort_flag) {
-        // eight warps: warp w reads TMEM lanes 32 (w % 4) .. (its rows) and half
-        // of the columns
+        // eight warps: warp w reads TMEM lanes 32 (w % 4) .. (its rows) and every
+        // other group of 16 columns in use
         const int quarter = warp & 3, half = warp >> 2;
         const int row = quarter * 32 + lane;
         const bool live = row < rows_valid;
         const int ea = live ? A.e[a_rb * TC_BM + row] : 0;
         double* crow = w.C + (i64)(mt * TC_BM + row) * w.rs;
         const int* eb = B.e + b_rb * TC_BN;
-        constexpr int HALF = TC_BN / 2;
-        static_assert(HALF % 16 == 0, "column halves of whole 16-column loads");
-        for (int c0 = half * HALF; c0 < (half + 1) * HALF; c0 += 16) {
+        for (int c0 = 16 * half; c0 < ncols; c0 += 32) {
             uint32_t v[R][16];
 #pragma unroll
             for (int r = 0; r < R; ++r)
