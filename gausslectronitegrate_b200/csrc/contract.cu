@@ -780,7 +780,7 @@ struct StageAOp {
     __device__ void b_issue(const Block& b, BState& st, int kc, double* tile) const {
         const int k = dm_pair_k(threadIdx.x), t = b.k.t0 + kc * DM_BK + k;
         const int bytes = dm_pair_bytes(t, b.k.t1);
-        const unsigned live = st.live[kc];
+        const unsigned live = st.live[dm_run_entry(kc)];
 #pragma unroll
         for (int q = 0; q < NB; ++q) {
             if (!dm_live(live, q)) continue;
@@ -905,7 +905,7 @@ struct StageBOp {
     __device__ void b_issue(const Block& b, BState& st, int kc, double* tile) const {
         const int k = dm_pair_k(threadIdx.x), v = b.k.t0 + kc * DM_BK + k;
         const int bytes = dm_pair_bytes(v, b.k.t1);
-        const unsigned live = st.live[kc];
+        const unsigned live = st.live[dm_run_entry(kc)];
 #pragma unroll
         for (int q = 0; q < NB; ++q) {
             if (!dm_live(live, q)) continue;
@@ -1114,7 +1114,7 @@ struct ProductOp {
     __device__ void b_issue(const Block& b, BState& st, int kc, double* tile) const {
         const int k = dm_pair_k(threadIdx.x), u = b.k.t0 + kc * DM_BK + k;
         const int bytes = dm_pair_bytes(u, b.k.t1);
-        const unsigned live = st.live[kc];
+        const unsigned live = st.live[dm_run_entry(kc)];
 #pragma unroll
         for (int q = 0; q < NB; ++q) {
             if (!dm_live(live, q)) continue;

@@ -156,31 +156,44 @@ struct dm_skip_of<Op, std::void_t<decltype(Op::SKIP)>> {
     static constexpr int value = Op::SKIP;
 };
 
+// The runs of at most DM_MAX_CHUNKS chunks are held (4,096 positions, the
+// lattice limit of the class lists).  A longer K range (nuclear matrices: the two
+// points of an axis may lie any distance apart) shares the last entry among the
+// chunks from it on: a strip is live there if it is live in any of them.
+__host__ __device__ __forceinline__ int dm_run_entry(int kc) { return kc < DM_MAX_CHUNKS ? kc : DM_MAX_CHUNKS - 1; }
+// a strip's chunks [first, last] as entries, first | last << 16 (first > last: empty)
+__host__ __device__ __forceinline__ int dm_strip_run(int first, int last) {
+    return last < first ? 1 : dm_run_entry(first) | dm_run_entry(last) << 16;
+}
+// the live strips of parity g at an entry
+template <int STRIPS>
+__host__ __device__ __forceinline__ uint16_t dm_live_run(const int* run, int g, int entry) {
+    int lo = STRIPS / 2, hi = 0;
+#pragma unroll
+    for (int t = 0; t < STRIPS / 2; ++t) {
+        const int r = run[2 * t + g];
+        if ((r & 0xffff) <= entry && entry <= r >> 16) {
+            if (lo > t) lo = t;
+            hi = t + 1;
+        }
+    }
+    return (uint16_t)(hi > lo ? lo | hi << 8 : 0);
+}
+
 template <class Op>
 __device__ __forceinline__ void dm_build_masks(const Op& op, const typename Op::Block& blk,
                                                uint16_t (&live)[2][DM_MAX_CHUNKS]) {
     constexpr int STRIPS = (dm_skip_of<Op>::value == SKIP_M ? DM_BM : Op::BN) / 8;
-    __shared__ int run[STRIPS];  // first | last << 16 (first > last: empty)
+    __shared__ int run[STRIPS];
     for (int t = threadIdx.x; t < STRIPS; t += DM_THREADS) {
         int first, last;
         op.live_chunks(blk, t, first, last);
-        run[t] = last < first ? 1 : first | last << 16;
+        run[t] = dm_strip_run(first, last);
     }
     __syncthreads();
-    for (int kc = threadIdx.x; kc < blk.nk; kc += DM_THREADS)
+    for (int e = threadIdx.x; e < min(blk.nk, DM_MAX_CHUNKS); e += DM_THREADS)
 #pragma unroll
-        for (int g = 0; g < 2; ++g) {
-            int lo = STRIPS / 2, hi = 0;
-#pragma unroll
-            for (int t = 0; t < STRIPS / 2; ++t) {
-                const int r = run[2 * t + g];
-                if ((r & 0xffff) <= kc && kc <= r >> 16) {
-                    lo = min(lo, t);
-                    hi = t + 1;
-                }
-            }
-            live[g][kc] = (uint16_t)(hi > lo ? lo | hi << 8 : 0);
-        }
+        for (int g = 0; g < 2; ++g) live[g][e] = dm_live_run<STRIPS>(run, g, e);
     __syncthreads();
 }
 __device__ __forceinline__ bool dm_live(unsigned run, int strip) {
@@ -239,7 +252,7 @@ __device__ __forceinline__ void dm_mainloop(const Op& op, const typename Op::Blo
         if constexpr (SKIP != 0) {
             // (strips past the tile's rows or columns hold zeros: no run covers
             // them alone, and their results are not stored)
-            dm_run<SKIP == SKIP_M ? 4 : NJ>(live[kc], [&](auto lo, auto hi) {
+            dm_run<SKIP == SKIP_M ? 4 : NJ>(live[dm_run_entry(kc)], [&](auto lo, auto hi) {
                 constexpr int LO = decltype(lo)::value, HI = decltype(hi)::value;
                 constexpr int I0 = SKIP == SKIP_M ? LO : 0, I1 = SKIP == SKIP_M ? HI : 4;
                 constexpr int J0 = SKIP == SKIP_M ? 0 : LO, J1 = SKIP == SKIP_M ? NJ : HI;

@@ -429,7 +429,7 @@ struct NucStageOp {
     __device__ void a_init(const Block&, AState&) const {}
     __device__ void b_init(const Block&, BState&) const {}
     __device__ void a_issue(const Block& b, AState& st, int kc, double* tile) const {
-        const unsigned live = st.live[kc];
+        const unsigned live = st.live[dm_run_entry(kc)];
 #pragma unroll
         for (int q = 0; q < DM_BM / 16; ++q) {
             if (!dm_live(live, q)) continue;
