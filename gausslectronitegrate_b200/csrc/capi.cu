@@ -593,7 +593,8 @@ double compute_nuclear_gausslet_integral(const struct gausslet_data* gdata,
         gli::Context& ctx = gli::context();
         cudaStream_t s = ctx.stream;
         DevBuf<double> d(N * N, s);
-        gli::nuclear_matrix_device(gdata->coefficients, gdata->indices.num, axes, nuclei, num_nuclei, tol, d.p, s);
+        gli::nuclear_matrix_device(gdata->coefficients, gdata->indices.num, axes, nuclei, num_nuclei, tol, d.p, s,
+                                   true);
         std::vector<double> h(N * N);
         to_host(h.data(), d.p, N * N, s);
         GLI_CUDA(cudaStreamSynchronize(s));

@@ -201,9 +201,13 @@ void kinetic_table_device(const double* h_coeffs, i64 nb, i64 L, double* d_k1, c
 // tables.cu: per-shift Gaussian-pair factors F[s][m], s = 0..L-1, m = 0..2nb-2
 void factors_device(const double* d_b, int nb, int L, double* d_F, cudaStream_t s);
 
-// nuclear.cu: dense nuclear matrix over the product of three axis coordinate lists
+// nuclear.cu: dense nuclear matrix over the product of three axis coordinate
+// lists.  far_only: the caller reads only entries between the lists' ends on
+// every axis (a single entry); zeros when the ends of an axis lie too far apart
+// for any factor
 void nuclear_matrix_device(const double* h_coeffs, i64 nb, const std::vector<int> axes[3],
-                           const struct atomic_nucleus* nuclei, int nn, double tol, double* d_out, cudaStream_t s);
+                           const struct atomic_nucleus* nuclei, int nn, double tol, double* d_out, cudaStream_t s,
+                           bool far_only = false);
 
 // one instance of a nuclear batch: ascending coordinate lists per axis, its
 // nuclei (host memory) and its N x N output (device memory)
@@ -212,6 +216,7 @@ struct NuclearJob {
     const struct atomic_nucleus* nuclei = nullptr;
     int nn = 0;
     double* d_out = nullptr;
+    bool far_only = false;  // only entries between the lists' ends on every axis are read
 };
 struct NuclearBatchStats {
     i64 instances = 0, chunks = 0;

@@ -729,7 +729,7 @@ void nuclear_batch_device(const double* h_coeffs, i64 nb, const std::vector<Nucl
     if (jobs.empty()) return;
     NuclearBatchStats stats;
     // factor shifts needed: 0 .. max |i_a - j_a| over every instance
-    int L = 1;
+    i64 L = 1;
     i64 total_nuclei = 0, total_coords = 0;
     for (const NuclearJob& j : jobs) {
         if (j.nn <= 0 || !j.nuclei) fail(GLI_ERR_ARGUMENT, "every instance needs at least one nucleus");
@@ -738,24 +738,36 @@ void nuclear_batch_device(const double* h_coeffs, i64 nb, const std::vector<Nucl
         for (int a = 0; a < 3; ++a) {
             if (j.axes[a].empty() || j.axes[a].size() > 256)
                 fail(GLI_ERR_LIMIT, "axis %d has %zu points (1..256)", a, j.axes[a].size());
-            L = std::max(L, j.axes[a].back() - j.axes[a].front() + 1);
+            L = std::max(L, (i64)j.axes[a].back() - j.axes[a].front() + 1);
             total_coords += (i64)j.axes[a].size();
         }
         total_nuclei += j.nn;
     }
     const int nf = (int)(2 * nb - 1);
-    DevBuf<double> b(nb, s), F((i64)L * nf, s);
+    // (a factor of shift s holds exp(-(3 s + i - j)^2 / 4), |i - j| < nb: zero in
+    // FP64 from 3 s - nb = 55 on, so larger shifts need no rows)
+    L = std::min<i64>(L, (nb + 55) / 3 + 2);
+    DevBuf<double> b(nb, s), F(L * nf, s);
     GLI_CUDA(cudaMemcpyAsync(b.p, h_coeffs, nb * sizeof(double), cudaMemcpyHostToDevice, s));
-    factors_device(b.p, (int)nb, L, F.p, s);
+    factors_device(b.p, (int)nb, (int)L, F.p, s);
     DevBuf<int> reach(2, s);
     GLI_CUDA(cudaMemsetAsync(reach.p, 0xff, 2 * sizeof(int), s));
-    k_mask_factors<<<(unsigned)(((i64)L * nf + 255) / 256), 256, 0, s>>>(F.p, (i64)L * nf, nf, (int)nb, tol, reach.p);
+    k_mask_factors<<<(unsigned)((L * nf + 255) / 256), 256, 0, s>>>(F.p, L * nf, nf, (int)nb, tol, reach.p);
     GLI_CHECK_LAUNCH();
     int h_reach[2] = {-1, -1};
     GLI_CUDA(cudaMemcpyAsync(h_reach, reach.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
     GLI_CUDA(cudaStreamSynchronize(s));
     const int h_mmax = h_reach[0], h_smax = h_reach[1];
-    if (h_mmax < 0) {  // every factor below tol
+    // an entry between two points further apart on an axis than any factor
+    // reaches is zero: nothing to tabulate (the lattice box of the points grows
+    // with the cube of their distance)
+    bool dead = jobs.size() == 1 && jobs[0].far_only;
+    if (dead) {
+        i64 gap = 0;
+        for (const auto& list : jobs[0].axes) gap = std::max(gap, (i64)list.back() - list.front());
+        dead = gap > h_smax;
+    }
+    if (h_mmax < 0 || dead) {  // every factor below tol
         for (const NuclearJob& j : jobs) {
             const i64 N = (i64)j.axes[0].size() * j.axes[1].size() * j.axes[2].size();
             GLI_CUDA(cudaMemsetAsync(j.d_out, 0, N * N * sizeof(double), s));
@@ -936,13 +948,15 @@ void nuclear_batch_device(const double* h_coeffs, i64 nb, const std::vector<Nucl
 }
 
 void nuclear_matrix_device(const double* h_coeffs, i64 nb, const std::vector<int> axes[3],
-                           const struct atomic_nucleus* nuclei, int nn, double tol, double* d_out, cudaStream_t s) {
+                           const struct atomic_nucleus* nuclei, int nn, double tol, double* d_out, cudaStream_t s,
+                           bool far_only) {
     if (nn <= 0) fail(GLI_ERR_ARGUMENT, "at least one nucleus is required");
     std::vector<NuclearJob> jobs(1);
     for (int a = 0; a < 3; ++a) jobs[0].axes[a] = axes[a];
     jobs[0].nuclei = nuclei;
     jobs[0].nn = nn;
     jobs[0].d_out = d_out;
+    jobs[0].far_only = far_only;
     nuclear_batch_device(h_coeffs, nb, jobs, tol, FORM_FP64, s);
 }
 

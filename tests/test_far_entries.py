@@ -106,3 +106,13 @@ def test_far_entries_in_the_bounds_checked_build():
     env = dict(os.environ, GLI_B200_LIBRARY=DEBUG_LIB)
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, env=env, timeout=900)
     assert r.returncode == 0 and "gaps ok" in r.stdout, r.stdout + r.stderr
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("gap", [(700, 700, 700), (1, 100_000, 0), (1_000_000, -1_000_000, 1_000_000)])
+def test_entries_far_apart_are_zero(gap):
+    # the lattice box between such points takes terabytes: no factor reaches, nothing is tabulated
+    import gausslectronitegrate_b200 as gli
+    got = gli.compute_nuclear_gausslet_integral(g10(), [(0, 0, 0), gap], POS, Q, 1e-8)
+    assert not np.any(Oracle().factors(g10(), max(map(abs, gap)), 0.0)[0])
+    assert got == 0.0
