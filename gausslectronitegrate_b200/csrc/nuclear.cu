@@ -121,31 +121,13 @@ __device__ __forceinline__ double nuc_gaussian(double r2) {
     return r > 0 ? erf(3.0 * r) / r : 3.3851375012865379;  // 6 / sqrt(pi)
 }
 
-// 1 / sqrt(x) for 4 <= x < 1e201: the hardware's approximation (PTX
-// rsqrt.approx.ftz.f64: y, 20 bits) and one step of third order,
-// y (1 + e / 2 + 3 e^2 / 8) with e = 1 - x y^2, whose remainder is 5/16 e^3 <
-// 2^-60.  y^2 of the short y is exact, so e is rounded once and the result is
-// off by little more than its own rounding (two Newton steps, eight operations
-// for five: 0.83 ulp at most, here 0.51).
-// The field's cells away from a nucleus need no more than this range, and the
-// general function's handling of the others was most of the field's
-// instructions.
-__device__ __forceinline__ double nuc_rsqrt(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y * y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
 // Phi[u][v][t] (t fastest, pitches P) of every instance, position
 // (u + u0x, v + u0y, t + u0z) / 6; grid (row blocks, instance), a warp fills
 // whole (u, v) rows, up to eight cells per lane and turn: per nucleus the row's part of
-// the squared distance is formed once and each cell costs eight FP64
-// operations and the hardware's approximation.  Bound: the FP64 pipe (13 x 16 x
-// 11 points, 5 nuclei, 74 million of these: 36 us, the pipe's own time 33;
-// 41 us with two Newton steps).  24^3 to 8^3 batch of eight, with two Newton
-// steps: 367 us; 722 us with a thread per cell, its three coordinates divided
-// by 6 and its whole distance per nucleus.
+// the squared distance is formed once and each cell costs two FP64
+// multiply-adds and a reciprocal square root.  Bound: the issue slots (64% busy,
+// the FP64 pipe 41%).  13 x 16 x 11 points and 5 nuclei, 171 x 189 x 159 cells:
+// 45 us.
 constexpr int NUC_FIELD_MAX_T = 2048;  // z positions held in shared memory (axes of 256 points: 1531 + 2 mmax)
 constexpr int NUC_FIELD_BLOCKS = 3;     // per SM
 __global__ void __launch_bounds__(256, NUC_FIELD_BLOCKS) k_nuc_field(const NucInst* __restrict__ inst, const double* __restrict__ npos,
@@ -173,12 +155,12 @@ __global__ void __launch_bounds__(256, NUC_FIELD_BLOCKS) k_nuc_field(const NucIn
             for (int k = in.nuc0; k < in.nuc0 + in.nnuc; ++k) {
                 const double dx = px - npos[3 * k], dy = py - npos[3 * k + 1], nz = npos[3 * k + 2], q = ncharge[k];
                 const double r2 = dx * dx + dy * dy;
-                // (a whole row that has no cell near the nucleus, at distances in range)
-                if (r2 >= 4.0 && r2 < 1e200 && fabs(nz) < 1e99) {
+                // (a whole row that has no cell near the nucleus: g = 1 / r throughout)
+                if (r2 >= 4.0 && !isnan(nz)) {
 #pragma unroll
                     for (int c = 0; c < C; ++c) {
                         const double dz = pz[c] - nz;
-                        acc[c] += q * nuc_rsqrt(r2 + dz * dz);
+                        acc[c] += q * rsqrt(r2 + dz * dz);
                     }
                 } else {
 #pragma unroll 1
