@@ -1680,8 +1680,6 @@ static TiledOperand lattice_g_slices(const LatticeTables& t, cudaStream_t s) {
     return t.g_sliced->view;
 }
 
-void dgemm_prepare();  // dense.cu: attributes of the strided FP64 GEMM
-
 static thread_local bool t_timing = false;
 static thread_local ContractStats t_last;
 static thread_local int t_paths = 0;  // tensor-core stages of the evaluation being completed
@@ -2360,9 +2358,10 @@ static GraphEntry* capture_graph(const EvalArgs& a, const std::shared_ptr<const 
         e->num[k] = a.d.num[k];
     }
     e->status.alloc(1);
-    // function attributes are set outside the capture
-    tc_gemm_prepare();
-    dgemm_prepare();
+    // function attributes are set outside the capture.  (The first one of a
+    // translation unit loads its kernels, several milliseconds in a process' first
+    // evaluation: no unit is touched that this evaluation does not launch from.)
+    if (a.mixed) tc_gemm_prepare();
     auto prepare = [](auto width) {
         constexpr int BN = decltype(width)::value;
         dmma_prepare<StageAOp<BN, true>>();

@@ -454,15 +454,6 @@ static void dgemm(int M, int N, int K, MatView A, MatView B, double* C, i64 csb,
         dmma_launch(StridedOp<false, false>{M, N, K, A, B, C, csb, cr, cc, acc}, grid, s);
 }
 
-void dgemm_prepare() {
-    dmma_prepare<StridedOp<true, true>>();
-    dmma_prepare<StridedOp<true, false>>();
-    dmma_prepare<StridedOp<false, true>>();
-    dmma_prepare<StridedOp<false, false>>();
-    dmma_prepare<StridedOp<true, false, 32>>();
-    dmma_prepare<StridedOp<false, false, 32>>();
-}
-
 void dgemm_strided(int M, int N, int K, const double* A, i64 asb, i64 ar, i64 ac, const double* B, i64 bsb, i64 br,
                    i64 bc, double* C, i64 csb, i64 cr, i64 cc, int batch, bool accumulate, cudaStream_t s) {
     dgemm(M, N, K, MatView{A, asb, ar, ac}, MatView{B, bsb, br, bc}, C, csb, cr, cc, batch, accumulate, s);
