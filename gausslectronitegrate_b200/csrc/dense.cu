@@ -32,6 +32,7 @@
 // GEMM as it stages the operand tiles (KeyedSlabOp, at most 32 orbitals), or
 // fills the slab first (k_fill_slab_keyed) and contracts it.
 #include <algorithm>
+#include <cmath>
 #include <map>
 #include <mutex>
 
@@ -880,12 +881,16 @@ void project_device(int kind, const GridDesc& g, const int64_t* d_idx, const dou
         kt.queue(G, d_idx, d_val, m, s);
     }
     std::vector<i64> act;
-    for (i64 i = 0; i < (hb.empty() ? 0 : N); ++i)
-        for (i64 c = 0; c < M; ++c)
-            if (hb[(size_t)(i * M + c)] != 0.0) {
-                act.push_back(i);
-                break;
-            }
+    bool finite = true;
+    for (i64 i = 0; i < (hb.empty() ? 0 : N); ++i) {
+        bool any = false;
+        for (i64 c = 0; c < M; ++c) {
+            const double v = hb[(size_t)(i * M + c)];
+            any = any || v != 0.0;
+            finite = finite && std::isfinite(v);
+        }
+        if (any) act.push_back(i);
+    }
     std::vector<short4> hpt;
     for (const i64 i : act) {
         const int yz = D.num[1] * D.num[2], r = (int)(i % yz);
@@ -916,8 +921,9 @@ void project_device(int kind, const GridDesc& g, const int64_t* d_idx, const dou
             bx = bcomp.p;
         }
     }
-    if (slab32 && M <= 32) {
-        // The active points in their box (the product of their coordinates per
+    if (slab32 && M <= 32 && finite) {
+        // (infinite coefficients go the general way: the pair classes' zero
+        // triangles and padding rows would make them undefined.)  The active points in their box (the product of their coordinates per
         // axis; a sub-grid is its own box): the first two contractions once per
         // pair class.  A box of over twice the active points (orbitals on
         // scattered points) would contract mostly zero rows, and one beyond the
