@@ -3,6 +3,7 @@
 // runs its device work on the thread's stream and, on failure, prints one line
 // to stderr, records the status and returns empty results.
 #include <math.h>
+#include <sched.h>
 #include <stdlib.h>
 #include <string.h>
 #ifdef __SSE2__
@@ -120,6 +121,13 @@ static bool host_pinned(const void* p) {
     return a.type == cudaMemoryTypeHost;
 }
 
+// CPUs that the process may run on (hardware_concurrency() counts the machine's)
+static unsigned usable_cpus() {
+    cpu_set_t set;
+    if (sched_getaffinity(0, sizeof(set), &set) == 0 && CPU_COUNT(&set) > 0) return (unsigned)CPU_COUNT(&set);
+    return std::max(1u, std::thread::hardware_concurrency());
+}
+
 // The host threads of one staged copy: each takes the next piece, waits until
 // `go` has passed it, copies it and marks it done.  Joined on every path.
 struct PieceWorkers {
@@ -129,9 +137,8 @@ struct PieceWorkers {
     std::atomic<bool> stop{false};
     explicit PieceWorkers(size_t pieces) : done(pieces) {}
     template <class Copy>
-    bool start(unsigned most, Copy copy) {  // false: no thread could be started
-        const unsigned hw = std::thread::hardware_concurrency();
-        const size_t n = std::min<size_t>({(size_t)most, hw > 1 ? hw / 2 : 1, done.size()});
+    bool start(unsigned most, Copy copy) {  // false: no thread could be started, or no CPU for one
+        const size_t n = std::min<size_t>({(size_t)most, usable_cpus() / 2, done.size()});
         for (size_t k = 0; k < n; ++k) {
             try {
                 threads.emplace_back([this, copy] {
