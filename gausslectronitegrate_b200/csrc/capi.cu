@@ -51,6 +51,13 @@ T* host_alloc(i64 count) {
 }
 
 
+// CPUs that the process may run on (hardware_concurrency() counts the machine's)
+static unsigned usable_cpus() {
+    cpu_set_t set;
+    if (sched_getaffinity(0, sizeof(set), &set) == 0 && CPU_COUNT(&set) > 0) return (unsigned)CPU_COUNT(&set);
+    return std::max(1u, std::thread::hardware_concurrency());
+}
+
 // Copies of several MB between the device and pageable host memory (class lists
 // and values, dense matrices and tensors) go through a ring of page-locked
 // pieces, 64 of 1 MB per thread, so that up to eight host threads copy pieces
@@ -69,10 +76,15 @@ struct StagingRing {
     char* pin = nullptr;
     cudaEvent_t ev[kSlots] = {};
     int device = -1;  // of the events
-    void ensure() {
+    bool ensure() {  // false: no CPU for a thread, or the page-locked memory is not to be had
+        if (usable_cpus() < 2) return false;
         int dev = 0;
         GLI_CUDA(cudaGetDevice(&dev));
-        if (!pin) GLI_CUDA(cudaHostAlloc((void**)&pin, kPiece * kSlots, cudaHostAllocPortable));
+        if (!pin && cudaHostAlloc((void**)&pin, kPiece * kSlots, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            pin = nullptr;
+            return false;
+        }
         if (dev != device)
             for (auto& e : ev) {
                 if (e) {
@@ -83,6 +95,7 @@ struct StagingRing {
                 GLI_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
             }
         device = dev;
+        return true;
     }
     char* slot(size_t p) { return pin + p % kSlots * kPiece; }
     cudaEvent_t event(size_t p) { return ev[p % kSlots]; }
@@ -119,13 +132,6 @@ static bool host_pinned(const void* p) {
         return false;
     }
     return a.type == cudaMemoryTypeHost;
-}
-
-// CPUs that the process may run on (hardware_concurrency() counts the machine's)
-static unsigned usable_cpus() {
-    cpu_set_t set;
-    if (sched_getaffinity(0, sizeof(set), &set) == 0 && CPU_COUNT(&set) > 0) return (unsigned)CPU_COUNT(&set);
-    return std::max(1u, std::thread::hardware_concurrency());
 }
 
 // The host threads of one staged copy: each takes the next piece, waits until
@@ -174,7 +180,7 @@ void to_host(T* h, const T* d, i64 n, cudaStream_t s) {
         if (n) GLI_CUDA(cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, s));
     };
     if (bytes < kStagedBytes || host_pinned(h)) return plain();
-    t_ring.ensure();
+    if (!t_ring.ensure()) return plain();
     StagingRing& ring = t_ring;
     auto len = [&](size_t p) { return std::min(StagingRing::kPiece, bytes - p * StagingRing::kPiece); };
     PieceWorkers w(pieces);
@@ -223,17 +229,17 @@ struct Upload {
     }
     void run() {
         if (pieces.empty()) return;
-        t_ring.ensure();
+        auto plain = [&] {
+            for (const Piece& p : pieces) GLI_CUDA(cudaMemcpyAsync(p.dst, p.src, p.len, cudaMemcpyHostToDevice, s));
+        };
+        if (!t_ring.ensure()) return plain();
         StagingRing& ring = t_ring;
         const size_t n = pieces.size();
         for (auto& e : ring.ev) GLI_CUDA(cudaEventSynchronize(e));  // earlier uses of the slots
         PieceWorkers w(n);
         const Piece* pc = pieces.data();
         w.go = std::min<size_t>(n, StagingRing::kSlots);
-        if (!w.start(4, [&ring, pc](size_t p) { stage_piece(ring.slot(p), pc[p].src, pc[p].len); })) {
-            for (const Piece& p : pieces) GLI_CUDA(cudaMemcpyAsync(p.dst, p.src, p.len, cudaMemcpyHostToDevice, s));
-            return;
-        }
+        if (!w.start(4, [&ring, pc](size_t p) { stage_piece(ring.slot(p), pc[p].src, pc[p].len); })) return plain();
         for (size_t p = 0; p < n; ++p) {
             w.wait(p);
             GLI_CUDA(cudaMemcpyAsync(pc[p].dst, ring.slot(p), pc[p].len, cudaMemcpyHostToDevice, s));
