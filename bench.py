@@ -499,7 +499,8 @@ def run_ours(args):
     # the dominant kernel: stage A, stage B, or one of stage C's two kernels
     # (its product GEMM, and the class gather or per-class dots after it)
     dom = max(("A", "B", "C_product", "C_class"), key=lambda k: st[k])
-    roof = roofline(paths[chosen], dom, st, st["plan"], U, m, peak.value)
+    roof = roofline(paths[chosen], dom, st, st["plan"], U, m, peak.value,
+                    mean_key_reach(KIND, b, spec[0][1], screening[chosen]["product_threshold"]))
     # (measured DRAM bytes per launch are keyed by stage; "C" is the class gather)
     tkey = {"C_class": "C"}.get(dom, dom) + (":tc" if roof["bound"] == "hbm" and dom in ("A", "B") else "")
     roof["traffic"] = measured_traffic(f"{args.workload}:{tkey}")
@@ -898,7 +899,44 @@ def lattice_nS(U):
     return int(np.unique((u[:, None] ** 2 + u[None, :] ** 2).ravel()).size)
 
 
-def roofline(paths, dom, st, plan, U, m, fp64_peak):
+def mean_key_reach(kind, b, L, tol):
+    """Share of the lattice positions on which an axis key's weights are
+    nonzero, averaged over the keys of a grid of L points per axis.  A key's
+    weights are its product vector (entries above tol) laid around three times
+    its coordinate difference and folded at zero."""
+    b = np.asarray(b, dtype=np.float64)
+    i = np.arange(b.size)
+    if kind == "erida":
+        products, shifts = [2 * np.pi / 9 * np.convolve(b, b[::-1])], range(L)
+    else:
+        F = []
+        for s in range(L):
+            g = np.sqrt(np.pi) / 3 * np.outer(b, b) * np.exp(-(0.5 * (3 * s + i[:, None] - i[None, :])) ** 2)
+            F.append(np.bincount((i[:, None] + i[None, :]).ravel(), g.ravel()))
+        products = [np.convolve(F[lo], F[hi][::-1]) for hi in range(L) for lo in range(hi + 1)]
+        shifts = range(2 * L - 1)
+    spans = []  # (first, last) offset of each product vector's entries above tol
+    for p in products:
+        at = np.flatnonzero(np.abs(p) > tol) - (p.size - 1) // 2
+        if at.size:
+            spans.append((int(at[0]), int(at[-1])))
+    if not spans:
+        return 0.0
+    U = 3 * (len(shifts) - 1) + max(max(-f, l) for f, l in spans) + 1
+    reach = []
+    for c in shifts:
+        for f, l in spans:
+            lo, hi = 3 * c + f, 3 * c + l
+            first = lo if lo > 0 else -hi if hi < 0 else 0  # (folded: positions |lo|..|hi|)
+            reach.append(max(abs(lo), abs(hi)) - first + 1)
+    return float(np.mean(reach)) / U
+
+
+# below this mean reach the library's stages leave out positions without weights
+BANDED_REACH = 0.75
+
+
+def roofline(paths, dom, st, plan, U, m, fp64_peak, reach=1.0):
     """Roofline entry of the dominant kernel (from the library's stage events:
     stage A, stage B, or one of stage C's two kernels, C_product and C_class).
     FP64 kernels (the FP64 tensor-core GEMM k_dmma, or the per-class dots of
@@ -911,7 +949,9 @@ def roofline(paths, dom, st, plan, U, m, fp64_peak):
     (pair, key) products the product GEMM computed, 0 when stage C ran per
     class (one length-U dot product per class).  The class gather after the
     product GEMM moves 16 bytes per class (the class index in, its value out)
-    against the measured HBM bandwidth."""
+    against the measured HBM bandwidth.  reach = mean_key_reach of the form's
+    tables: where it is below BANDED_REACH the stages execute less than the
+    whole lattice's FLOPs, so the rate is an effective one and has no fraction."""
     nA, nP, nku, product = plan
     ms = st[dom]
     nS = lattice_nS(U)
@@ -933,14 +973,16 @@ def roofline(paths, dom, st, plan, U, m, fp64_peak):
         kernel = {"A": "k_dmma<StageAOp>", "B": "k_dmma<StageBOp>", "C_product": "k_dmma<ProductOp>",
                   "C_class": "k_stage_c"}[dom]
         achieved = flops / (ms * 1e-3) / 1e12 if ms > 0 else None
+        banded = reach < BANDED_REACH
         return {"bound": "fp64", "stage": dom[0], "kernel": kernel,
                 "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
-                "frac": achieved / fp64_peak if achieved and fp64_peak and achieved <= fp64_peak else None,
+                "frac": achieved / fp64_peak if achieved and fp64_peak and not banded else None,
                 "peak_source": "measured FP64 peak on this device (gli_b200_measure_fp64_peak: "
                                "max of FMA and m8n8k4 MMA probes)",
                 "algorithmic_flops_per_launch": flops,
-                "flops_counted": "over the whole lattice; on wide grids stages A and B leave out the positions where a "
-                                 "key's weights are zero (no fraction where the count exceeds what can be executed)",
+                "flops_counted": ("an effective rate: over the whole lattice, of which a key's weights reach "
+                                  f"{reach:.0%} on average; the stages and the product leave the rest out"
+                                  if banded else "over the whole lattice"),
                 "traffic": None}
     S, BN = 5, 96
     nsp = (nS + 127) // 128 * 128
