@@ -1018,8 +1018,8 @@ __global__ void __launch_bounds__(256) k_stage_c(const double* __restrict__ W, c
 // Q at its pair (A key a, B key) and its largest key c >= a, and pairs are
 // ordered by A key, so the column tiles of a row tile start at the key of its
 // first A key: keys below it are never read (129 ERIDA keys: 166 blocks
-// instead of 396).  blockIdx.z selects a chunk of u; the chunks' partial
-// products go to separate slices of Q, summed by k_gather_q.
+// instead of 396).  blockIdx.z selects a part of the K chunks; the parts'
+// partial products are summed in a cluster.
 template <int BN_>
 struct ProductOp {
     static constexpr bool A_KMAJOR = false, B_KMAJOR = false;
@@ -2498,8 +2498,8 @@ static EvalArgs eval_args(int kind, const double* h_coeffs, i64 nb, const GridDe
     return a;
 }
 
-// Queues one evaluation on stream s and an asynchronous copy of its status
-// block into h_status (pinned); the caller synchronises and checks it.
+// Queues one evaluation on stream s and the kernel that writes its status
+// block into h_status (page-locked); the caller synchronises and checks it.
 // *sized receives the graph that was replayed (null otherwise): when its
 // status reports an overflow (a sized plan outgrown, or a class outside a
 // reused plan), the caller drops it and calls again, which plans anew.

@@ -435,20 +435,6 @@ void dmma_prepare() {
     done.fetch_or(bit);
 }
 
-// blocks of k_dmma<Op> resident on one SM (registers and shared memory)
-template <class Op>
-int dmma_blocks_per_sm() {
-    static std::atomic<int> cached{0};
-    int v = cached.load();
-    if (v > 0) return v;
-    dmma_prepare<Op>();
-    GLI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_dmma<Op>, DM_THREADS,
-                                                           dm_smem(Op::BN, dm_stages_of<Op>::value)));
-    v = v > 0 ? v : 1;
-    cached.store(v);
-    return v;
-}
-
 // one launch of k_dmma<Op> on grid `grid`
 template <class Op>
 void dmma_launch(const Op& op, dim3 grid, cudaStream_t s) {
@@ -458,7 +444,7 @@ void dmma_launch(const Op& op, dim3 grid, cudaStream_t s) {
 }
 
 // the same with K split over grid.z (2..8) blocks that sum their partial tiles
-// in a cluster (the Op's part stride must be 0)
+// in a cluster
 template <class Op>
 void dmma_launch_cluster(const Op& op, dim3 grid, cudaStream_t s) {
     if (grid.x == 0 || grid.y == 0 || grid.z == 0) return;

@@ -157,7 +157,7 @@ struct PairSmem {
 // under that contraction.
 // A tile's k steps that lie before all its rows in the diagonal plane are zero
 // and left out (343 points: 4.43 to 4.26 ms).
-// Bound: the FP64 tensor pipe, 55% busy (343 points, 20 orbitals), with the
+// Bound: the FP64 tensor pipe, 50% busy (343 points, 20 orbitals), with the
 // shared-memory pipe 59% busy (V fragments, and copies whose 32 values lie in
 // about as many lines; contiguous copies in their place measured 4.03 ms).
 // Measured on a B200, first two contractions: 216 points and 32 orbitals 0.98
@@ -170,9 +170,10 @@ struct PairSmem {
 // A warp owns up to two 16-row tiles (rows 16 (w + W t)) and keeps their
 // accumulators over all planes, so each B fragment serves all its tiles.  The
 // FP64 MMAs of four warps per scheduler hide each other's issue gaps and the
-// map and value loads (loads issued a step ahead gained nothing, 4.54 ms) (two warps with three tiles each kept the FP64 tensor
-// pipe 39% busy): two blocks of 8 warps on an SM, or one of 16 where the
-// planes and B of one box take more than half of the shared memory.
+// map and value loads: two blocks of 8 warps on an SM, or one of 16 where the
+// planes and B of one box take more than half of the shared memory.  (Two warps
+// per scheduler with three tiles each kept the FP64 tensor pipe 39% busy; loads
+// issued a step ahead gained nothing, 4.54 ms.)
 template <int W, int NT, int TPW, bool SYM>
 __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : 1)
     k_pair_contract(const PairBox box, const double* __restrict__ table, const double* __restrict__ bsrc, int cols,

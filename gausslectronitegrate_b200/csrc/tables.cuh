@@ -85,16 +85,7 @@ std::shared_ptr<const LatticeTables> lattice_tables(int kind, const double* h_co
 constexpr double MIXED_SCREEN_BOUND = 1e-9;
 double mixed_screen_tol(int kind, const double* h_coeffs, i64 nb, i64 L, double tol, double* bound, cudaStream_t s);
 
-// dense ERI key of one axis: shift pair (|s01|, |s23|) unordered and |c|/3
-__host__ __device__ inline i64 eri_axis_key(i64 s01, i64 s23, i64 cc, i64 L) {
-    i64 a = s01 < 0 ? -s01 : s01;
-    i64 b = s23 < 0 ? -s23 : s23;
-    if (a > b) { i64 t = a; a = b; b = t; }
-    const i64 c = cc < 0 ? -cc : cc;
-    return (b * (b + 1) / 2 + a) * (2 * L - 1) + c;
-}
-
-// the same key in 32-bit arithmetic (keys < 2^21)
+// dense ERI key of one axis: shift pair (|s01|, |s23|) unordered and |c|/3 (keys < 2^21)
 __host__ __device__ inline int eri_axis_key32(int s01, int s23, int cc, int L) {
     int a = s01 < 0 ? -s01 : s01;
     int b = s23 < 0 ? -s23 : s23;
