@@ -97,8 +97,12 @@ struct StagingRing {
         device = dev;
         return true;
     }
-    char* slot(size_t p) { return pin + p % kSlots * kPiece; }
-    cudaEvent_t event(size_t p) { return ev[p % kSlots]; }
+    // Each copy begins at the slot after the last one's: a DMA into lines that a
+    // core's cache still holds from the copy before runs at 10 GB/s, not 55.
+    size_t base = 0;
+    void advance(size_t pieces) { base = (base + pieces) % kSlots; }
+    char* slot(size_t p) { return pin + (base + p) % kSlots * kPiece; }
+    cudaEvent_t event(size_t p) { return ev[(base + p) % kSlots]; }
     ~StagingRing() {
         if (pin) cudaFreeHost(pin);
         for (auto& e : ev)
@@ -121,9 +125,15 @@ static void stage_piece(char* dst, const char* src, size_t len) {
 #endif
 }
 
-// below this size the driver's own staging of a pageable copy is as fast as
-// starting the threads (about 80 us)
-static constexpr size_t kStagedBytes = (size_t)2 << 20;
+// Below these sizes the driver's own staging of a pageable copy is as fast as
+// starting the threads (about 80 us).  Out, into memory that was written before:
+// 2 MB 498 us of a call plain and 664 staged, 5.5 MB 843 and 921, 8 MB 1,084 and
+// 1,076, 16 MB 1,790 and 1,540 (fresh memory 3,900 and 1,140 at 8 MB).  In: 2 x
+// 2 MB 457 and 446, 2 x 3 MB 598 and 520.
+static constexpr size_t kStagedIn = (size_t)2 << 20, kStagedOut = (size_t)8 << 20;
+// Results from this size on go out in pieces of 4 MB, whole huge pages of the
+// caller's memory per thread (128 MB: 8.2 to 6.5 ms; 12 MB 0.78 to 0.9).
+static constexpr size_t kLargeOut = (size_t)64 << 20;
 
 static bool host_pinned(const void* p) {
     cudaPointerAttributes a = {};
@@ -175,34 +185,36 @@ struct PieceWorkers {
 // device -> host; synchronous for staged copies, else queued on s
 template <class T>
 void to_host(T* h, const T* d, i64 n, cudaStream_t s) {
-    const size_t bytes = (size_t)n * sizeof(T), pieces = (bytes + StagingRing::kPiece - 1) / StagingRing::kPiece;
+    const size_t bytes = (size_t)n * sizeof(T);
     auto plain = [&] {
         if (n) GLI_CUDA(cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, s));
     };
-    if (bytes < kStagedBytes || host_pinned(h)) return plain();
+    if (bytes < kStagedOut || host_pinned(h)) return plain();
     if (!t_ring.ensure()) return plain();
     StagingRing& ring = t_ring;
-    auto len = [&](size_t p) { return std::min(StagingRing::kPiece, bytes - p * StagingRing::kPiece); };
+    const size_t unit = bytes >= kLargeOut ? 4 : 1, piece = unit * StagingRing::kPiece;  // (unit: ring slots a piece)
+    const size_t slots = StagingRing::kSlots / unit, pieces = (bytes + piece - 1) / piece;
+    if (unit > 1) ring.base = 0;
+    auto len = [=](size_t p) { return std::min(piece, bytes - p * piece); };
     PieceWorkers w(pieces);
-    if (!w.start(8, [&ring, h, len](size_t p) { memcpy((char*)h + p * StagingRing::kPiece, ring.slot(p), len(p)); }))
+    if (!w.start(8, [&ring, h, len, unit, piece](size_t p) { memcpy((char*)h + p * piece, ring.slot(p * unit), len(p)); }))
         return plain();
     auto queue = [&](size_t p) {
-        GLI_CUDA(cudaMemcpyAsync(ring.slot(p), (const char*)d + p * StagingRing::kPiece, len(p),
-                                 cudaMemcpyDeviceToHost, s));
-        GLI_CUDA(cudaEventRecord(ring.event(p), s));
+        GLI_CUDA(cudaMemcpyAsync(ring.slot(p * unit), (const char*)d + p * piece, len(p), cudaMemcpyDeviceToHost, s));
+        GLI_CUDA(cudaEventRecord(ring.event(p * unit), s));
     };
-    for (size_t p = 0; p < std::min<size_t>(pieces, StagingRing::kSlots); ++p) queue(p);
+    for (size_t p = 0; p < std::min(pieces, slots); ++p) queue(p);
     for (size_t p = 0; p < pieces; ++p) {
-        GLI_CUDA(cudaEventSynchronize(ring.event(p)));
+        GLI_CUDA(cudaEventSynchronize(ring.event(p * unit)));
         w.go.store(p + 1, std::memory_order_release);
         // the slot of a piece copied out half a ring ago takes the next DMA
-        const size_t half = StagingRing::kSlots / 2;
-        if (p >= half && p - half + StagingRing::kSlots < pieces) {
-            w.wait(p - half);
-            queue(p - half + StagingRing::kSlots);
+        if (p >= slots / 2 && p - slots / 2 + slots < pieces) {
+            w.wait(p - slots / 2);
+            queue(p - slots / 2 + slots);
         }
     }
     for (size_t p = 0; p < pieces; ++p) w.wait(p);
+    ring.advance(pieces * unit);
 }
 
 // Host -> device copies of several arrays as one staged copy; returns with the
@@ -220,7 +232,7 @@ struct Upload {
     void add(DevBuf<T>& d, const T* h, i64 n) {
         d.alloc(n, s);
         const size_t bytes = (size_t)n * sizeof(T);
-        if (bytes < kStagedBytes || host_pinned(h)) {
+        if (bytes < kStagedIn || host_pinned(h)) {
             if (n) GLI_CUDA(cudaMemcpyAsync(d.p, h, bytes, cudaMemcpyHostToDevice, s));
             return;
         }
@@ -251,6 +263,7 @@ struct Upload {
                 w.go.store(p - half + StagingRing::kSlots + 1, std::memory_order_release);
             }
         }
+        ring.advance(n);
     }
 };
 
