@@ -923,10 +923,14 @@ void project_device(int kind, const GridDesc& g, const int64_t* d_idx, const dou
     }
     if (slab32 && M <= 32 && finite) {
         // (infinite coefficients go the general way: the pair classes' zero
-        // triangles and padding rows would make them undefined.)  The active points in their box (the product of their coordinates per
-        // axis; a sub-grid is its own box): the first two contractions once per
-        // pair class.  A box of over twice the active points (orbitals on
-        // scattered points) would contract mostly zero rows, and one beyond the
+        // triangles and padding rows would make them undefined.)  The active
+        // points in their box (the product of their coordinates per axis; a
+        // sub-grid is its own box): the first two contractions once per pair
+        // class.  A box of over one and a half times the active points (orbitals
+        // on scattered points) would contract mostly zero rows, which the general
+        // contraction leaves out: whole calls through the box and without it, ms,
+        // 6^3 and 32 orbitals at 1.2, 1.5, 2 times 3.3, 3.3, 3.3 and 5.2, 3.6, 2.8,
+        // 7^3 and 20 orbitals 6.2, 6.2, 6.2 and 13.8, 7.4, 3.9.  A box beyond the
         // kernel's rows or shared memory does not fit it.
         std::vector<int> coords[3];
         for (i64 a = 0; a < Nx; ++a) {
@@ -944,7 +948,7 @@ void project_device(int kind, const GridDesc& g, const int64_t* d_idx, const dou
             fits = fits && c.size() <= PAIR_MAX_AXIS;
             points *= (i64)c.size();
         }
-        if (fits && points <= 2 * Nx) {
+        if (fits && 2 * points <= 3 * Nx) {
             const PairBox box = make_pair_box((int)G.L, coords);
             if (pair_box_fits(box, nt)) {
                 const double* bb = bx;
