@@ -932,8 +932,9 @@ def mean_key_reach(kind, b, L, tol):
     return float(np.mean(reach)) / U
 
 
-# below this mean reach the library's stages leave out positions without weights
-BANDED_REACH = 0.75
+# from this many positions left out by a key on average, the library's stages
+# follow the keys' reaches
+BANDED_LEFT_OUT = 64
 
 
 def roofline(paths, dom, st, plan, U, m, fp64_peak, reach=1.0):
@@ -950,8 +951,8 @@ def roofline(paths, dom, st, plan, U, m, fp64_peak, reach=1.0):
     class (one length-U dot product per class).  The class gather after the
     product GEMM moves 16 bytes per class (the class index in, its value out)
     against the measured HBM bandwidth.  reach = mean_key_reach of the form's
-    tables: where it is below BANDED_REACH the stages execute less than the
-    whole lattice's FLOPs, so the rate is an effective one and has no fraction."""
+    tables: where it leaves out BANDED_LEFT_OUT positions the stages execute less than
+    the whole lattice's FLOPs, so the rate is an effective one and has no fraction."""
     nA, nP, nku, product = plan
     ms = st[dom]
     nS = lattice_nS(U)
@@ -973,7 +974,7 @@ def roofline(paths, dom, st, plan, U, m, fp64_peak, reach=1.0):
         kernel = {"A": "k_dmma<StageAOp>", "B": "k_dmma<StageBOp>", "C_product": "k_dmma<ProductOp>",
                   "C_class": "k_stage_c"}[dom]
         achieved = flops / (ms * 1e-3) / 1e12 if ms > 0 else None
-        banded = reach < BANDED_REACH
+        banded = (1 - reach) * U >= BANDED_LEFT_OUT
         return {"bound": "fp64", "stage": dom[0], "kernel": kernel,
                 "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
                 "frac": achieved / fp64_peak if achieved and fp64_peak and not banded else None,

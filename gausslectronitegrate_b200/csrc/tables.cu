@@ -239,7 +239,7 @@ static void build_lattice_tables(int kind, const double* h_coeffs, i64 nb, i64 L
                 total += reach[k].y - reach[k].x + 1;
                 ++live;
             }
-        t.banded = 4 * total < 3 * live * t.U;
+        t.banded = live > 0 && live * t.U - total >= BANDED_LEFT_OUT * live;
         int2 from = make_int2((int)t.U, -1), upto = from;
         for (i64 k = 0; k < n; ++k) {
             upto = make_int2(std::min(upto.x, reach[k].x), std::max(upto.y, reach[k].y));

@@ -36,6 +36,17 @@ struct TiledTable {
     TiledOperand view;
 };
 
+// Positions that a key leaves out on average from which the stages follow the
+// keys' reaches: four chunks of the K loops.  Fewer chunks save less than the
+// dependent loads at a block's start cost.  Whole evaluations without and with
+// the reaches, us: ERI 7^3 91 and 106 (22 positions left out at tol 1e-16), 71
+// and 88 (23 at 1e-8), 64 and 74 (26 at 1e-5); ERIDA 33^3 56 and 63 (50), 57 and
+// 57 (55), 54 and 47 (68 at 1e-5); 41^3 75 and 72 (67; an eighth of the list 63
+// and 67), 49^3 83 and 82 (87), 57^3 121 and 94 (107), 65^3 153 and 119 (129),
+// 129^3 656 and 291 (313).  (A limit on the share of the lattice, three
+// quarters, put ERI 7^3 at 1e-8 and ERIDA 33^3 on the wrong side.)
+constexpr i64 BANDED_LEFT_OUT = 64;
+
 struct LatticeTables {
     int kind = 0;            // 0 = ERIDA, 1 = ERI
     int device = 0;
@@ -53,10 +64,8 @@ struct LatticeTables {
     // for keys in ascending order, those of any key from k on (x rounded down to
     // even) and of any key up to k: nkeys each, one after the other
     DevMem<int2> reach;
-    // the keys reach less than 3/4 of the positions on average: the stages then
-    // follow the reaches (fewer positions, but more dependent loads at a
-    // block's start: stage A of the mixed ERI 7^3, whose keys reach nearly all of
-    // 113 positions, takes 20.3 us without them and 23.0 us with them)
+    // the keys leave out at least BANDED_LEFT_OUT positions on average: the stages
+    // then follow the reaches
     bool banded = false;
     const int2* key_reach() const { return reach.p; }
     const int2* reach_from() const { return reach.p + nkeys; }

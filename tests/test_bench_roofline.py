@@ -15,7 +15,7 @@ STAGES = {"A": 0.15, "B": 0.1, "C_product": 0.02, "C_class": 0.01}
 
 
 @pytest.mark.parametrize("dom", ["A", "B", "C_product", "C_class"])
-@pytest.mark.parametrize("kind,L,U,banded", [("erida", 129, 465, True), ("erida", 33, 177, True), ("eri", 7, 141, False)])
+@pytest.mark.parametrize("kind,L,U,banded", [("erida", 129, 465, True), ("erida", 33, 177, False), ("eri", 7, 141, False)])
 def test_fraction_only_where_the_whole_lattice_is_executed(dom, kind, L, U, banded):
     reach = bench.mean_key_reach(kind, g10(), L, 1e-16)
     product = 0 if dom == "C_class" else 370_177
