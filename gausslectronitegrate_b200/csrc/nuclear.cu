@@ -127,7 +127,8 @@ __device__ __forceinline__ double nuc_gaussian(double r2) {
 // the squared distance is formed once and each cell costs two FP64
 // multiply-adds and a reciprocal square root.  Bound: the issue slots (64% busy,
 // the FP64 pipe 41%).  13 x 16 x 11 points and 5 nuclei, 171 x 189 x 159 cells:
-// 45 us.
+// 45 us; the batch of eight, 24^3 to 8^3, 376 us (71%, 49%), 722 us with a thread
+// per cell, its coordinates divided by 6 and its whole distance per nucleus.
 constexpr int NUC_FIELD_MAX_T = 2048;  // z positions held in shared memory (axes of 256 points: 1531 + 2 mmax)
 constexpr int NUC_FIELD_BLOCKS = 3;     // per SM
 __global__ void __launch_bounds__(256, NUC_FIELD_BLOCKS) k_nuc_field(const NucInst* __restrict__ inst, const double* __restrict__ npos,
@@ -331,8 +332,8 @@ __global__ void __launch_bounds__(256) k_nuc_scatter(const NucInst* __restrict__
 // one, both operands K-contiguous 16-byte copies, and an 8-key strip takes part
 // only in the chunks it reaches.
 //
-// Bound: the FP64 tensor pipe, 85% busy on the batch of eight, 24^3 to 8^3,
-// whose three stages take 461 + 410 + 400 us; 2.95 ms over full K ranges with
+// Bound: the FP64 tensor pipe, 75% busy on the batch of eight, 24^3 to 8^3,
+// whose three stages take 381 + 348 + 345 us; 2.95 ms over full K ranges with
 // 8-byte copies, a launch per instance.
 template <int STAGE>
 struct NucStageOp {
